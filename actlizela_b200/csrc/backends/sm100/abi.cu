@@ -6,7 +6,6 @@
 #include "gdn_common.cuh"
 
 #include <climits>
-#include <vector>
 
 namespace gdn_sm100 {
 namespace {
@@ -45,15 +44,19 @@ bool geometry_ok(int b, int t, int hk, int hv) {
 constexpr int kStageMask = 0x30, kPrepareOnly = 0x10, kWalkOnly = 0x20, kSegmentShift = 8, kMaxSegments = 16;
 constexpr int kWalkFlagMask = 0xc0, kHomogeneousBit = 0x40, kUntilDecayedBit = 0x80;
 constexpr int kParallelShift = 16, kMaxParallel = 8, kOffsetTailBit = 0x100000, kPairBit = 0x200000;
+// kernel family 4: the single-launch tensor-core forward (gdn_fused.cu): one segment, no stage restriction
+constexpr int kFused = 4;
+bool is_fused(int config) { return (config & 0xf) == kFused; }
 bool config_ok(int config) {
   const int segments = (config >> kSegmentShift) & 0xff, parallel = (config >> kParallelShift) & 0xf;
-  if (config < 0 || (config & 0xf) > 3 ||
+  if (config < 0 || (config & 0xf) > kFused ||
       (config & ~(kStageMask | kWalkFlagMask | 0xf | (0xff << kSegmentShift) | (0xf << kParallelShift) | kOffsetTailBit | kPairBit)) != 0)
     return false;
   if ((config & kOffsetTailBit) && (config & ~kOffsetTailBit) != (1 | kWalkOnly)) return false;
   if ((config & kPairBit) && (config & ~kPairBit) != (1 | kWalkOnly)) return false;
   if ((config & kWalkFlagMask) && ((config & 0xf) != 1 || (config & kStageMask) != kWalkOnly)) return false;
-  if (parallel > kMaxParallel || (parallel > 1 && ((config & 0xf) != 1 || (config & kWalkFlagMask)))) return false;
+  if (parallel > kMaxParallel || (parallel > 1 && (((config & 0xf) != 1 && !is_fused(config)) || (config & kWalkFlagMask)))) return false;
+  if (is_fused(config) && ((config & kStageMask) || segments > 1)) return false;
   return (config & kStageMask) != kStageMask && segments <= kMaxSegments;
 }
 // parallel sub-segments for a launch that walks `chunks` chunks per (batch, value head)
@@ -66,6 +69,13 @@ int segments_of(int config, const Geometry& geo) {
   if ((config & 0xf) != 1 || (config & kStageMask) || segments < 2) return 1;
   const int chunks = geo.chunks();
   return segments > chunks ? chunks : segments;
+}
+
+// workspace a call needs: the factors of every block, or (single-launch form) the flag words of the sub-segments
+long long scratch_bytes(const Geometry& geo, int config, int segments) {
+  if (!is_fused(config)) return workspace_bytes(geo, segments);
+  const long long flags = fused_workspace_bytes(geo, parallel_of(config, geo.chunks()));
+  return flags > 256 ? flags : 256;
 }
 
 // Second stream and events of the segmented forward, created by configure() for the current device.
@@ -111,23 +121,6 @@ int launch_prepare_tc(int, const Inputs& in, const Geometry& geo, const Workspac
 }
 int launch_walk_tc(int, const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream) {
   return launch_walk_umma(in, geo, ws, stream);
-}
-
-// Offsets table of the packed mode from DEVICE offsets: cu_seqlens[0..n] (forced into 0 <= ... <= total and
-// non-decreasing, so that no later index can leave the tensors) followed by the chunk prefix.
-__global__ void varlen_table_kernel(const int* __restrict__ cu_seqlens, int n_seqs, int total, int* __restrict__ table) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int chunks = 0, previous = 0;
-  table[0] = 0;
-  table[n_seqs + 1] = 0;
-  for (int i = 1; i <= n_seqs; ++i) {
-    int at = cu_seqlens[i];
-    at = at < previous ? previous : (at > total ? total : at);
-    chunks += (at - previous + kChunk - 1) / kChunk;
-    table[i] = at;
-    table[n_seqs + 1 + i] = chunks;
-    previous = at;
-  }
 }
 
 // One affine step of a 128x128 state block, out = M @ S + b, by the 256 threads of a CTA (each 64 outputs).
@@ -254,6 +247,7 @@ int map_status_page() {
   if ((e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&on_device), g_status_pages[device], 0)) != cudaSuccess)
     return int(e);
   if (int rc = set_status_mirror_umma(on_device)) return rc;
+  if (int rc = set_status_mirror_fused(on_device)) return rc;
   if (int rc = set_status_mirror_gemm(on_device)) return rc;
   g_status_mapped[device] = true;
   return 0;
@@ -270,6 +264,7 @@ volatile int* status_page_of_current_device() {
 extern "C" int actlize_la_sm100_configure(void) {
   if (int rc = configure_simt()) return rc;
   if (int rc = configure_umma()) return rc;
+  if (int rc = configure_fused()) return rc;
   if (int rc = configure_out_proj()) return rc;
   if (int rc = map_status_page()) return rc;
   return create_segment_streams();
@@ -296,18 +291,20 @@ extern "C" int actlize_la_sm100_select(int b, int t, int hk, int hv, int gate_fp
     while ((long long)(root + 1) * (root + 1) <= chunks / 8) ++root;
     segments = root < 1 ? 1 : (root > 8 ? 8 : root);
   }
-  return kPolicyDefault | (kPolicyDefault == 1 ? (segments << kSegmentShift) | (int(parallel) << kParallelShift) : 0);
+  if (kPolicyDefault == kFused) segments = 1;
+  return kPolicyDefault | (segments << kSegmentShift) | (int(parallel) << kParallelShift);
 }
 
 extern "C" long long actlize_la_sm100_workspace_bytes(int b, int t, int hk, int hv, int config) {
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config)) return -1;
   const Geometry geo{b, t, hk, hv};
-  return workspace_bytes(geo, segments_of(config, geo));
+  return scratch_bytes(geo, config, segments_of(config, geo));
 }
 
 extern "C" int actlize_la_sm100_launches_per_forward(int config) {
   if (!config_ok(config)) return -1;
   if (config & kStageMask) return 1;
+  if (is_fused(config)) return ((config >> kParallelShift) & 0xf) > 1 ? 2 : 1;
   const int segments = (config >> kSegmentShift) & 0xff;
   return ((config & 0xf) == 1 && segments > 1) ? 2 * segments : 2;
 }
@@ -326,6 +323,7 @@ extern "C" int actlize_la_sm100_device_status(int* status4, int reset) {
   if (reset) {
     for (int i = 0; i < 4; ++i) page[i] = 0;
     if (int rc = clear_device_status_umma()) return rc;
+    if (int rc = clear_device_status_fused()) return rc;
     if (int rc = clear_device_status_gemm()) return rc;
   }
   return 0;
@@ -354,11 +352,17 @@ extern "C" int actlize_la_sm100_selftest_walk_stall(
 
 extern "C" int actlize_la_sm100_walk_plan_counts(int* counts2, int reset) {
   if (!counts2) return int(cudaErrorInvalidValue);
-  return read_walk_plan_counts(counts2, reset);
+  int single[2];
+  if (int rc = read_walk_plan_counts(counts2, reset)) return rc;
+  if (int rc = read_fused_plan_counts(single, reset)) return rc;
+  counts2[0] += single[0];
+  counts2[1] += single[1];
+  return 0;
 }
 
 namespace {
 int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config, int segments, cudaStream_t stream);
+int run_fused(const Inputs& in, Geometry geo, int config, void* workspace, cudaStream_t stream);
 }
 
 extern "C" int actlize_la_sm100_forward_prepared(
@@ -370,7 +374,7 @@ extern "C" int actlize_la_sm100_forward_prepared(
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config)) return int(cudaErrorInvalidValue);
   Geometry geo{b, t, hk, hv};
   const int segments = segments_of(config, geo);
-  if (workspace_bytes_given < workspace_bytes(geo, segments)) return int(cudaErrorInvalidValue);
+  if (workspace_bytes_given < scratch_bytes(geo, config, segments)) return int(cudaErrorInvalidValue);
   if ((reinterpret_cast<uintptr_t>(workspace) & 255) || (reinterpret_cast<uintptr_t>(q) & 15) ||
       (reinterpret_cast<uintptr_t>(k) & 15) || (reinterpret_cast<uintptr_t>(v) & 15) ||
       (reinterpret_cast<uintptr_t>(output) & 15))
@@ -384,11 +388,16 @@ extern "C" int actlize_la_sm100_forward_prepared(
                   initial, static_cast<__nv_bfloat16*>(output), final_state, gate_fp32 ? 1 : 0,
                   ((config & kHomogeneousBit) ? kWalkHomogeneous : 0) | ((config & kUntilDecayedBit) ? kWalkUntilDecayed : 0) |
                       ((config & kOffsetTailBit) ? kWalkTail : 0) | ((config & kPairBit) ? kWalkPair : 0)};
+  if (is_fused(config)) return run_fused(in, geo, config, workspace, static_cast<cudaStream_t>(opaque_stream));
   const Workspace ws = carve_workspace(workspace, geo);
   return run_forward(in, geo, ws, config, segments, static_cast<cudaStream_t>(opaque_stream));
 }
 
 namespace {
+int run_fused(const Inputs& in, Geometry geo, int config, void* workspace, cudaStream_t stream) {
+  geo.parallel = parallel_of(config, geo.segment_chunks());
+  return launch_forward_fused(in, geo, static_cast<int*>(workspace), stream);
+}
 int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config, int segments, cudaStream_t stream) {
   if (segments > 1) {
     // Three streams.  The caller's: the first segment's prepare, then its walk, which so follows without an event
@@ -436,12 +445,13 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
 }  // namespace
 
 // --------------------------------------------------------------- forward on raw projection outputs
+// The raw projections are normalised and activated inside the single-launch kernel; the configurations of the two
+// tensor-core families select the same kernel here (they give the same bits), with the split their word carries.
 extern "C" long long actlize_la_sm100_projections_workspace_bytes(int b, int t, int hk, int hv, int config) {
-  if (!geometry_ok(b, t, hk, hv) || !config_ok(config) || (config & 0xf) != 1 || (config & (kStageMask | kWalkFlagMask)))
+  if (!geometry_ok(b, t, hk, hv) || !config_ok(config) || ((config & 0xf) != 1 && !is_fused(config)) ||
+      (config & (kStageMask | kWalkFlagMask)))
     return -1;
-  const Geometry geo{b, t, hk, hv};
-  // the ordinary workspace plus the normalised keys and queries, each [B][T][Hk][128] BF16
-  return ((workspace_bytes(geo, segments_of(config, geo)) + 255) & ~255LL) + 2 * (((long long)b * t * hk * kDim * 2 + 255) & ~255LL);
+  return scratch_bytes(Geometry{b, t, hk, hv}, (config & ~0xf) | kFused, 1);
 }
 
 extern "C" int actlize_la_sm100_forward_projections(
@@ -456,15 +466,7 @@ extern "C" int actlize_la_sm100_forward_projections(
       (reinterpret_cast<uintptr_t>(mixed) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
       (reinterpret_cast<uintptr_t>(output) & 15))
     return int(cudaErrorInvalidValue);
-  Geometry geo{b, t, hk, hv};
-  const int segments = segments_of(config, geo);
-  const Workspace ws = carve_workspace(workspace, geo);
   Inputs in{};
-  char* planes = static_cast<char*>(workspace) + ((workspace_bytes(geo, segments) + 255) & ~255LL);
-  in.k_norm = reinterpret_cast<__nv_bfloat16*>(planes);
-  in.q_norm = reinterpret_cast<__nv_bfloat16*>(planes + (((long long)b * t * hk * kDim * 2 + 255) & ~255LL));
-  in.k = in.k_norm;                 // what the walk reads
-  in.q = in.q_norm;
   in.initial = initial;
   in.output = static_cast<__nv_bfloat16*>(output);
   in.final_state = final_state;
@@ -475,13 +477,13 @@ extern "C" int actlize_la_sm100_forward_projections(
   in.act_b = static_cast<const __nv_bfloat16*>(b_act);
   in.a_log = a_log;
   in.dt_bias = dt_bias;
-  return run_forward(in, geo, ws, config, segments, static_cast<cudaStream_t>(opaque_stream));
+  return run_fused(in, Geometry{b, t, hk, hv}, config, workspace, static_cast<cudaStream_t>(opaque_stream));
 }
 
 // ---------------------------------------------------------------------------------- packed sequences
 namespace {
 long long align256_ll(long long x) { return (x + 255) & ~255LL; }
-long long varlen_table_bytes(int n_seqs) { return align256_ll(2LL * (n_seqs + 1) * (long long)sizeof(int)); }
+long long varlen_table_bytes(int n_seqs) { return align256_ll((n_seqs + 1LL) * (long long)sizeof(int)); }
 }  // namespace
 
 extern "C" long long actlize_la_sm100_varlen_workspace_bytes(long long total_tokens, int n_seqs, int hk, int hv) {
@@ -489,7 +491,7 @@ extern "C" long long actlize_la_sm100_varlen_workspace_bytes(long long total_tok
   // every sequence starts a new chunk, so each may add one partly filled chunk to ceil(total / 64)
   const long long max_chunks = (total_tokens + kChunk - 1) / kChunk + n_seqs;
   if (max_chunks * hv > INT_MAX / kDim || (long long)n_seqs * hv > INT_MAX / 8) return -1;
-  return varlen_table_bytes(n_seqs) + max_chunks * hv * kBlockBytes;
+  return varlen_table_bytes(n_seqs);
 }
 
 extern "C" int actlize_la_sm100_forward_varlen(
@@ -508,27 +510,16 @@ extern "C" int actlize_la_sm100_forward_varlen(
       (reinterpret_cast<uintptr_t>(k) & 15) || (reinterpret_cast<uintptr_t>(v) & 15) ||
       (reinterpret_cast<uintptr_t>(output) & 15))
     return int(cudaErrorInvalidValue);
-  // offsets table: cu_seqlens[0..n] then chunk_prefix[0..n]
-  std::vector<int> table(2 * (n_seqs + 1));
-  int chunks = 0;
-  for (int i = 0; i <= n_seqs; ++i) {
-    table[i] = cu_seqlens_host[i];
-    table[n_seqs + 1 + i] = chunks;
-    if (i < n_seqs) chunks += (cu_seqlens_host[i + 1] - cu_seqlens_host[i] + kChunk - 1) / kChunk;
-  }
   cudaStream_t stream = static_cast<cudaStream_t>(opaque_stream);
-  // pageable source: the runtime has staged the bytes when the call returns, so `table` may go out of scope
-  cudaError_t e = cudaMemcpyAsync(workspace, table.data(), table.size() * sizeof(int), cudaMemcpyHostToDevice, stream);
+  // pageable source: the runtime has staged the bytes when the call returns
+  cudaError_t e = cudaMemcpyAsync(workspace, cu_seqlens_host, (n_seqs + 1) * sizeof(int), cudaMemcpyHostToDevice, stream);
   if (e != cudaSuccess) return int(e);
   Geometry geo{n_seqs, total, hk, hv};
   geo.varlen = static_cast<const int*>(workspace);
-  geo.total_chunks = chunks;
   const Inputs in{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                   static_cast<const __nv_bfloat16*>(v), g, static_cast<const __nv_bfloat16*>(beta),
                   initial_states, static_cast<__nv_bfloat16*>(output), final_states, gate_fp32 ? 1 : 0};
-  const Workspace ws = carve_workspace(static_cast<char*>(workspace) + varlen_table_bytes(n_seqs), geo);
-  if (int rc = launch_prepare_umma(in, geo, ws, stream)) return rc;
-  return launch_walk_umma(in, geo, ws, stream);
+  return launch_forward_fused(in, geo, nullptr, stream);
 }
 
 extern "C" int actlize_la_sm100_forward_varlen_device(
@@ -545,19 +536,12 @@ extern "C" int actlize_la_sm100_forward_varlen_device(
       (reinterpret_cast<uintptr_t>(output) & 15))
     return int(cudaErrorInvalidValue);
   cudaStream_t stream = static_cast<cudaStream_t>(opaque_stream);
-  varlen_table_kernel<<<1, 32, 0, stream>>>(cu_seqlens_device, n_seqs, int(total_tokens), static_cast<int*>(workspace));
-  if (cudaError_t e = cudaGetLastError()) return int(e);
   Geometry geo{n_seqs, int(total_tokens), hk, hv};
-  geo.varlen = static_cast<const int*>(workspace);
-  // the host does not know the lengths: the grids and the workspace indexing use the upper bound (every sequence
-  // may add one partly filled chunk); prepare blocks behind the real chunk count leave at once
-  geo.total_chunks = int((total_tokens + kChunk - 1) / kChunk + n_seqs);
+  geo.varlen = cu_seqlens_device;      // read by the kernel, clamped there into the tensors: no host read, one launch
   const Inputs in{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                   static_cast<const __nv_bfloat16*>(v), g, static_cast<const __nv_bfloat16*>(beta),
                   initial_states, static_cast<__nv_bfloat16*>(output), final_states, gate_fp32 ? 1 : 0};
-  const Workspace ws = carve_workspace(static_cast<char*>(workspace) + varlen_table_bytes(n_seqs), geo);
-  if (int rc = launch_prepare_umma(in, geo, ws, stream)) return rc;
-  return launch_walk_umma(in, geo, ws, stream);
+  return launch_forward_fused(in, geo, nullptr, stream);
 }
 
 namespace {
@@ -587,6 +571,8 @@ struct Arena {
   long long q, k, v, g, beta, initial, output, final_state, workspace, total;
 };
 long long align256(long long x) { return (x + 255) & ~255LL; }
+// (the pipelined host entry walks sequence segments, which the two-kernel family does; the bits are the same)
+int host_config(int config) { return is_fused(config) ? (config & ~0xf) | 1 : config; }
 Arena arena_layout(int b, int t, int hk, int hv, int gate_fp32, int has_initial, int has_final, int config) {
   Arena a{};
   long long off = 0;
@@ -608,7 +594,7 @@ Arena arena_layout(int b, int t, int hk, int hv, int gate_fp32, int has_initial,
 extern "C" long long actlize_la_sm100_host_arena_bytes(int b, int t, int hk, int hv, int gate_fp32,
                                                        int has_initial, int has_final, int config) {
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config)) return -1;
-  return arena_layout(b, t, hk, hv, gate_fp32, has_initial, has_final, config).total;
+  return arena_layout(b, t, hk, hv, gate_fp32, has_initial, has_final, host_config(config)).total;
 }
 
 extern "C" int actlize_la_sm100_forward_host(
@@ -619,6 +605,7 @@ extern "C" int actlize_la_sm100_forward_host(
   if (!q || !k || !v || !g || !beta || !output || !device_arena) return int(cudaErrorInvalidValue);
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config)) return int(cudaErrorInvalidValue);
   if (reinterpret_cast<uintptr_t>(device_arena) & 255) return int(cudaErrorInvalidValue);
+  config = host_config(config);
   const Arena a = arena_layout(b, t, hk, hv, gate_fp32, initial != nullptr, final_state != nullptr, config);
   if (device_arena_bytes < a.total) return int(cudaErrorInvalidValue);
   char* base = static_cast<char*>(device_arena);

@@ -188,6 +188,13 @@ int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaSt
 int launch_prepare_fused(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);   // Inputs::mixed etc. set
 int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int configure_umma();
+// single-launch forward (gdn_fused.cu): Geometry::parallel sub-segments; `flags` is scratch of fused_workspace_bytes
+int configure_fused();
+long long fused_workspace_bytes(const Geometry&, int parallel);
+int launch_forward_fused(const Inputs&, const Geometry&, int* flags, cudaStream_t);
+int read_fused_plan_counts(int* host_out2, int reset);
+int set_status_mirror_fused(int* device_pointer);
+int clear_device_status_fused();
 int read_device_status(int* host_out4, int reset);
 int read_walk_plan_counts(int* host_out2, int reset);
 int launch_wait_timeout_selftest(int tag, cudaStream_t);

@@ -1,0 +1,1227 @@
+// Single-launch form of the tensor-core forward (configuration "fused"): one persistent CTA per SM carries the state
+// of one (batch, value head) chunk walk in tensor memory and prepares the WY factors of the coming chunks beside it.
+// Nothing travels through a workspace: per chunk the CTA reads the Q, K, V tiles, gates and betas and writes the
+// output tile, where the two-kernel path hands 73 KB of factors per chunk through L2 and HBM.
+//
+// The arithmetic is that of prepare_umma_kernel and walk_umma_kernel (gdn_umma.cu), operation for operation and in
+// the same order, so both paths give the same bits; orientation and precision are explained there.
+#include "umma_math.cuh"
+
+namespace gdn_sm100 {
+namespace {
+
+// Heads split into parallel sub-segments [0] / walked by one CTA because a sub-segment does not decay or a token is not
+// a contraction [1]; added to the two-kernel path's counts by read_walk_plan_counts.
+__device__ int g_fused_plan_counts[2];
+
+#ifdef GDN_SM100_PHASE_TIMING
+__device__ long long g_stamps[4][64][16], g_blocks[1024][2];
+#define STAMP(role, n, slot) do { if (blockIdx.x == 0 && (n) < 64) g_stamps[role][n][slot] = clock64(); } while (0)
+#else
+#define STAMP(role, n, slot)
+#endif
+
+// Warps (24):
+//    0      issuer of the chain's tensor-core products
+//    1      planner (work items of this CTA) and TMA producer
+//    2-3    query scaling
+//    4-11   state chain
+//    12-15  W operand (W^T accumulator -> hi/lo tiles) and output
+//    16-19, 20-23  two prepare groups: even and odd chunks of the CTA's stream.  The phases of a chunk's preparation
+//           are serial and latency bound (about two chunk periods long), so two chunks are in preparation at a time.
+// All roles share one instruction cache of some tens of KB: with every loop unrolled (134 KB of code) a chunk took
+// twice as long, bound by instruction fetches from the cache that the SMs of a GPC share.  Loops are therefore rolled
+// unless a loop's registers need otherwise, and waits call one polling routine.
+constexpr int kThreads = 768;
+constexpr int kIssueWarp = 0, kPlanWarp = 1, kScaleWarp = 2, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
+constexpr int kRing = 3;      // Q/K tiles, P tiles, gate vectors: one chunk in the chain, two in preparation
+constexpr int kItems = 4;     // work items announced ahead
+
+struct Smem {
+  static constexpr int kKQStage = 4 * kBox;                       // [Q0 K0 Q1 K1]: Q over K per 64-column half
+  static constexpr int kQ0 = 0, kK0 = kBox, kQ1 = 2 * kBox, kK1 = 3 * kBox;
+  static constexpr int kKQ = 0;
+  static constexpr int kV = kKQ + kRing * kKQStage;               // one V tile: needed by U only, once per period
+  static constexpr int kW = kV + 2 * kBox;                        // W^T hi | lo [128 keys][64 tokens]
+  static constexpr int kWTile = 2 * kBox;
+  static constexpr int kP = kW + 2 * kWTile;                      // ring of P tiles
+  static constexpr int kLd = 68;                                  // row pitch (floats) of the FP32 64x64 matrix
+  static constexpr int kATBytes = 64 * kLd * 4;
+  static constexpr int kAT = kP + kRing * kBox;                   // per group: A, then T in place, then T_u hi | lo
+  static constexpr int kTw = kAT + 2 * kATBytes;                  // T diag(beta exp p) hi | lo
+  static constexpr int kGates = kTw + 2 * kBox;                   // ring of gate vectors (kGateWords floats)
+  static constexpr int kPriv = kGates + kRing * kGateWords * 4;   // per group: pl2, beta, beta exp(p),
+  static constexpr int kPrivWords = 3 * 64 + 32;                  // and the column factors of the block off the diagonal
+  static constexpr int kItem = kPriv + 2 * kPrivWords * 4;        // item ring, 16 words each
+  static constexpr int kBars = kItem + kItems * 64;
+  static constexpr int kTotal = kBars + 512;
+  static_assert(kATBytes % 1024 == 0 && kAT % 1024 == 0 && kTw % 1024 == 0, "swizzled tiles start on 1024 bytes");
+  static_assert(2 * kBox <= kATBytes, "the T_u pair must fit on T");
+};
+constexpr int kSmemBytes = Smem::kTotal + 1024;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of one SM");
+
+// Tensor memory (512 columns): the state accumulator, its hi / lo operands, W S (then the N operands of the update: of the
+// 16-token group ks hi at 16 ks, lo at 16 ks + 8), U, the output accumulator, and one accumulator that serves the prepare
+// groups in turn ([Q;K] K^T, then W^T), guarded by a lock word.  N for P N takes the columns of the lo operand, which the
+// product W S has read by then.
+constexpr uint32_t kAccS = 0, kOpSH = 128, kOpSL = 192, kAccX = 256, kAccU = 320, kAccO = 384, kAccD = 448;
+constexpr uint32_t kIdescN64BT = idesc_bf16(128, 64, false, true);     // B MN-major, N = 64
+
+enum ItemWord { kChunks, kBatch, kHv, kFirst, kEnd, kUnstored, kState, kFlags, kFlagSlot, kOwn };
+constexpr int kHasInitial = 1, kHasFinal = 2;
+
+struct Barriers {
+  uint64_t kq_full[kRing], kq_free[kRing], qs_go[kRing], qs_done[kRing];
+  uint64_t v_full, w, w_ready, ws, s, o, ofree;
+  uint64_t t_ready[2], u[2], d[2], ops[2], opn[2];
+  uint64_t item_full[kItems], item_free[kItems];
+  uint32_t tmem;
+  int abort;
+  int lock, released;
+};
+static_assert(sizeof(Barriers) <= 512, "barrier block");
+constexpr int kItemReaders = kThreads / 32 - 1;      // every warp but the planner reads the items
+
+__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+// Barrier of 128 threads that also tells every thread whether all of them are healthy: whoever leaves a loop that
+// holds such barriers does it on this answer, so that no thread is left waiting in one.
+__device__ __forceinline__ bool group_all(int id, bool ok) {
+  uint32_t all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"(uint32_t(ok)), "r"(id) : "memory");
+  return all != 0;
+}
+
+__device__ __forceinline__ uint8_t* shared_base() {
+  extern __shared__ __align__(1024) uint8_t raw_smem[];
+  return raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);      // (no integer round trip: stays in the shared space)
+}
+// Bounded waits as in umma.cuh, with a polling routine that takes two arguments: a wait is in nearly fifty places of this
+// kernel.  The record names the warp (100 + warp).
+__device__ __noinline__ bool fused_wait_poll(uint32_t bar_addr, uint32_t parity) {
+  const AbortFlag abort{&reinterpret_cast<Barriers*>(shared_base() + Smem::kBars)->abort};
+  const uint32_t limit = g_spin_limit;
+  for (uint32_t spin = 0; spin < limit; ++spin) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(bar_addr), "r"(parity) : "memory");
+    if (done) return true;
+    if ((spin & 255u) == 255u && abort.raised()) return false;
+  }
+  abort.raise(1, 100 + (threadIdx.x >> 5), int(bar_addr));
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return fused_wait_poll(smem_u32(bar), parity);
+}
+// for a place with many live registers: no call (a wait that runs out here is recorded by the roles that then run out too)
+__device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity) {
+  for (uint32_t spin = 0; spin < (1u << 20); ++spin)
+    if (mbar_try_wait(bar, parity)) return true;
+  return false;
+}
+// wait with one answer for the whole warp
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+
+// ACC_D's lock: taken by the thread that issues into it, given back by the last of the four warps that have read it.
+__device__ __noinline__ void acc_lock(Barriers* bar) {
+  const AbortFlag abort{&bar->abort};
+  const uint32_t limit = g_spin_limit;
+  for (uint32_t spin = 0; spin < limit; ++spin) {
+    if (atomicCAS(&bar->lock, 0, 1) == 0) {
+      __threadfence_block();
+      return;
+    }
+    if ((spin & 255u) == 255u && abort.raised()) return;
+  }
+  abort.raise(1, 100 + (threadIdx.x >> 5), 0);
+}
+__device__ __forceinline__ void acc_release(Barriers* bar, int lane) {
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_block();
+    if (atomicAdd(&bar->released, 1) == 3) {
+      bar->released = 0;
+      __threadfence_block();
+      atomicExch(&bar->lock, 0);
+    }
+  }
+}
+
+__device__ __forceinline__ uint32_t bf16_bits(const __nv_bfloat16* p) { return *reinterpret_cast<const unsigned short*>(p); }
+__device__ __forceinline__ float raw_gate(const Inputs& in, uint32_t bits, int hv) {
+  // g = -exp(A_log) softplus(a + dt_bias) (z > 20 branch)
+  const float z = bf16_lo(bits) + in.dt_bias[hv];
+  return -expf(in.a_log[hv]) * (z > 20.f ? z : log1pf(expf(z)));
+}
+// A thread's gate and beta of a chunk as loaded (converted where they are used, so that the loads stay in flight):
+// `gate`, `beta` of token t, `lead` of token t - 32 for the threads of the second half
+struct GateLoads {
+  uint32_t gate = 0, beta = 0, lead = 0;
+  bool loaded = false;
+  __device__ __forceinline__ static float as_gate(uint32_t bits, int fp32) { return fp32 ? __uint_as_float(bits) : bf16_lo(bits); }
+  template <bool kRaw>
+  __device__ __forceinline__ static uint32_t gate_bits(const Inputs& in, long long gi) {
+    if (kRaw) return bf16_bits(in.act_a + gi);
+    return in.gate_fp32 ? static_cast<const uint32_t*>(in.g)[gi] : bf16_bits(static_cast<const __nv_bfloat16*>(in.g) + gi);
+  }
+  template <bool kRaw>
+  __device__ __forceinline__ void load(const Inputs& in, const Geometry& geo, int b, int hv, int t0, int valid, int t) {
+    const long long at = ((long long)b * geo.sequence + t0 + t) * geo.value_heads + hv;
+    if (t < valid) {
+      gate = gate_bits<kRaw>(in, at);
+      beta = bf16_bits((kRaw ? in.act_b : in.beta) + at);
+    }
+    if (t >= 32 && t - 32 < valid) lead = gate_bits<kRaw>(in, at - 32LL * geo.value_heads);
+  }
+};
+
+// First chunk boundary of a range at which the decay accumulated since its start is below exp(-40): number of leading
+// chunks an incoming state still reaches (1..count), or -1 when the decay never gets that far.  Sums the gates
+// themselves, eight chunks (sixteen loads per lane) at a time; it stops at the boundary, so a typical gate costs one
+// step.  Warp-collective; every caller with the same range gets the same answer.
+template <bool kRaw>
+__device__ int gate_reach(const Inputs& in, const Geometry& geo, int b, int hv, int first_token, int count, int t_end, int lane) {
+  float total = 0.f;
+  for (int c0 = 0; c0 < count; c0 += 8) {
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      x[u] = 0.f;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int t = first_token + (c0 + u) * kChunk + half * 32 + lane;
+        if (c0 + u < count && t < t_end) {
+          const long long gi = ((long long)b * geo.sequence + t) * geo.value_heads + hv;
+          x[u] += kRaw ? raw_gate(in, bf16_bits(in.act_a + gi), hv) : load_gate(in.g, gi, in.gate_fp32);
+        }
+      }
+    }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] += __shfl_xor_sync(0xffffffffu, x[u], d);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      total += x[u] * kLog2e;
+      if (c0 + u < count && total < kDecayedLog2) return c0 + u + 1;
+    }
+  }
+  return -1;
+}
+
+// 32 columns of row `row`, scaled per column by `coef`, as BF16 hi/lo pieces of a K-major swizzled tile pair (the lo tile
+// one box behind); `first` = first 16-byte piece of the row
+__device__ __forceinline__ void scaled_row(const float4 (&x)[8], const float* coef, uint8_t* tile_row, int first, int row) {
+#pragma unroll
+  for (int g8 = 0; g8 < 4; ++g8) {
+    float4 f[2];
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int q4 = 0; q4 < 2; ++q4) f[q4] = *reinterpret_cast<const float4*>(coef + g8 * 8 + q4 * 4);
+#pragma unroll
+    for (int q4 = 0; q4 < 2; ++q4) {
+      const float4 y = x[g8 * 2 + q4];
+      float a0, a1, b0, b1;
+      mul2(a0, a1, y.x, y.y, f[q4].x, f[q4].y);
+      mul2(b0, b1, y.z, y.w, f[q4].z, f[q4].w);
+      split_pair(a0, a1, hi[q4 * 2], lo[q4 * 2]);
+      split_pair(b0, b1, hi[q4 * 2 + 1], lo[q4 * 2 + 1]);
+    }
+    const int off = ((first + g8) ^ (row & 7)) << 4;
+    *reinterpret_cast<uint4*>(tile_row + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(tile_row + kBox + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// One read of a work item by a warp; `ring` counts items.
+struct ItemCursor {
+  int ring = 0;
+  __device__ __forceinline__ const int* open(uint8_t* sm, Barriers* bar, bool& ok) {
+    ok = warp_wait(&bar->item_full[ring % kItems], (ring / kItems) & 1);
+    return reinterpret_cast<const int*>(sm + Smem::kItem) + (ring % kItems) * 16;
+  }
+  __device__ __forceinline__ void close(Barriers* bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bar->item_free[ring % kItems]);
+    ++ring;
+  }
+};
+
+// What a launch walks: the units of the grid are (batch or sequence, value head[, sub-segment]); see walk_umma_kernel
+// for the sub-segments.  Here the decay part of the plan is read off the gates up front, while the contraction part
+// (beta |k|^2 in [0, 2]) shows only when a chunk is prepared: every CTA records what it saw in `flags`, and a second
+// launch of the same kernel (`serial_pass`) walks the heads for which some sub-segment saw a violation again, whole,
+// by one CTA each, and leaves at once otherwise.
+struct Plan {
+  int units, parallel, serial_pass;
+  int* flags;      // [batch * value_heads][parallel], written when parallel > 1
+};
+
+// ---------------------------------------------------------------------------------------------------- prepare groups
+// Four warps prepare one chunk; the phases are those of prepare_umma_kernel with half the threads.
+//   row = TMEM lane = warp * 32 + lane: rows 0..63 are Q rows (P), 64..127 K rows (A)
+template <bool kRaw>
+__device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const Inputs& in, const Geometry& geo, int group,
+                                              int n, int b, int hv, int t0, int t_next, int t_end, GateLoads& next,
+                                              bool& not_contraction) {
+  using L = Smem;
+  const int t = threadIdx.x & 127, warp = t >> 5, lane = t & 31, id = 1 + group;
+  const int s = n % kRing, valid = min(kChunk, t_end - t0);
+  uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
+  uint8_t* tile_p = sm + L::kP + s * kBox;
+  float* sAT = reinterpret_cast<float*>(sm + L::kAT + group * L::kATBytes);
+  float* gates = reinterpret_cast<float*>(sm + L::kGates) + s * kGateWords;
+  float* s_pl2 = reinterpret_cast<float*>(sm + L::kPriv) + group * L::kPrivWords;
+  float* s_beta = s_pl2 + 64;
+  float* s_coefw = s_beta + 64;
+  float* s_ecol = s_coefw + 64;
+
+  if (t == 96) STAMP(0, n, 0);
+  // gates and betas: warps 0 and 1 own tokens 0..31 and 32..63; warp 1 also scans the first half, whose total it adds.
+  // They were asked for while the group's previous chunk was prepared (the first of an item: here).
+  if (warp < 2 && !next.loaded) next.load<kRaw>(in, geo, b, hv, t0, valid, t);
+  bool ok = warp_wait(&bar->kq_full[s], (n / kRing) & 1) && !AbortFlag{&bar->abort}.raised();
+  if (t == 96) STAMP(0, n, 1);
+  if (kRaw) {
+    // L2-normalise the 64 Q and 64 K rows in place: 16 lanes per row (one swizzled 16-byte slot each), 8 rows per pass
+    if (ok) {
+      const int lane16 = t & 15;
+#pragma unroll 2
+      for (int pass = 0; pass < 16; ++pass) {
+        const int r = pass * 8 + (t >> 4), row = r & 63;
+        uint8_t* slot = kq + (r < 64 ? (lane16 < 8 ? L::kQ0 : L::kQ1) : (lane16 < 8 ? L::kK0 : L::kK1)) + row * 128 +
+                        (((lane16 & 7) ^ (row & 7)) << 4);
+        const uint4 x = *reinterpret_cast<const uint4*>(slot);
+        const float f[8] = {bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y),
+                            bf16_lo(x.z), bf16_hi(x.z), bf16_lo(x.w), bf16_hi(x.w)};
+        float square = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) square = fmaf(f[e], f[e], square);
+#pragma unroll
+        for (int d = 8; d; d >>= 1) square += __shfl_xor_sync(0xffffffffu, square, d, 16);
+        const float factor = rsqrtf(square + 1e-6f);
+        *reinterpret_cast<uint4*>(slot) = make_uint4(pack_bf16(f[0] * factor, f[1] * factor), pack_bf16(f[2] * factor, f[3] * factor),
+                                                     pack_bf16(f[4] * factor, f[5] * factor), pack_bf16(f[6] * factor, f[7] * factor));
+      }
+      fence_proxy_async_smem();
+    }
+    group_sync(id);
+  }
+  if (warp == 3 && ok) {
+    const uint64_t a = smem_desc(smem_u32(kq) + L::kQ0, 16, 1024), x = smem_desc(smem_u32(kq) + L::kK0, 16, 1024);
+    if (elect_one()) {
+      acc_lock(bar);
+      tc_fence_after();
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        const uint64_t at = (ks >> 2) * (L::kQ1 - L::kQ0) / 16 + (ks & 3) * 2;
+        mma_ss(kAccD, a + at, x + at, kIdescN64, ks > 0);
+      }
+      mma_commit(&bar->d[group]);
+    }
+  }
+  __syncwarp();
+  if (warp < 2) {
+    float gate = 0.f, beta = 0.f, lead = 0.f;
+    if (t < valid) {
+      gate = kRaw ? raw_gate(in, next.gate, hv) : next.as_gate(next.gate, in.gate_fp32);
+      beta = kRaw ? __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-bf16_lo(next.beta))))) : bf16_lo(next.beta);
+    }
+    if (warp == 1 && lane < valid) lead = kRaw ? raw_gate(in, next.lead, hv) : next.as_gate(next.lead, in.gate_fp32);
+    next.loaded = t_next >= 0;
+    if (next.loaded) next.load<kRaw>(in, geo, b, hv, t_next, min(kChunk, t_end - t_next), t);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, gate, d), z = __shfl_up_sync(0xffffffffu, lead, d);
+      if (lane >= d) {
+        gate += y;
+        lead += z;
+      }
+    }
+    const float carry = __shfl_sync(0xffffffffu, lead, 31);
+    if (warp == 1) gate += carry;
+    const float e = exp2f(gate * kLog2e), pl2 = gate * kLog2e;
+    s_pl2[t] = pl2;
+    s_beta[t] = beta;
+    s_coefw[t] = beta * e;
+    gates[kGateQueryScale + t] = e * kScale;
+    const float pl2_31 = __shfl_sync(0xffffffffu, pl2, 31);
+    if (warp == 0) s_ecol[t] = fast_exp2(pl2_31 - pl2);
+  }
+  ok = group_all(id, ok);
+  if (!ok) return false;
+
+  // ---- masks and decays on [Q;K] K^T
+  ok = warp_wait(&bar->d[group], (n >> 1) & 1);
+  if (t == 96) STAMP(0, n, 2);
+  tc_fence_after();
+  if (lane == 0) mbar_arrive(&bar->qs_go[s]);
+  const int i = t & 63;
+  const uint32_t taddr = (uint32_t(warp * 32) << 16) + kAccD;
+  bool bad = false;
+  // Per 32-column half that reaches the diagonal of this warp's rows: all loads, then the arithmetic in place, then the
+  // stores (loads behind stores to the same memory would each wait for them).  Nothing is masked element by element:
+  // of A only what the solves and products read has to be right (they do not read above the diagonal of a 16x16 block),
+  // and of P the one 16-byte piece per row that holds the diagonal is cut afterwards.  In the half that lies off the
+  // diagonal (rows 32.., columns ..31) exp(p_i - p_j) = exp(p_i - p_31) exp(p_31 - p_j): a factor per row and one per
+  // column (an exponential takes the special-function unit eight cycles per warp).
+  const int halves = (warp & 1) + 1;
+  const float pi = s_pl2[i], bi = s_beta[i];
+  // A takes the place of the T_u pair of this group's previous chunk, which U was formed from as that chunk began
+  if (warp >= 2 && n >= 2) ok = warp_wait(&bar->u[group], ((n >> 1) - 1) & 1) && ok;
+  if (t == 96) STAMP(0, n, 3);
+  if (ok) {
+    float* arow = sAT + i * L::kLd;
+    uint8_t* prow = tile_p + i * 128;
+#pragma unroll 1
+    for (int h = 0; h < halves; ++h) {
+      uint32_t d[32];
+      tmem_ld32(taddr + h * 32, d);
+      tmem_wait_ld();
+      if (h == halves - 1) acc_release(bar, lane);
+      const bool diagonal = h == halves - 1;
+      const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 32 : s_ecol);
+      const float last = warp < 2 ? kScale : 1.f, first = warp < 2 ? 1.f : bi;
+      if (diagonal) {
+#pragma unroll
+        for (int q4 = 0; q4 < 8; ++q4) {
+          const float4 p4 = pj[q4];
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            float x0 = __uint_as_float(d[q4 * 4 + e]), x1 = __uint_as_float(d[q4 * 4 + e + 1]), e0, e1;
+            sub2(e0, e1, pi, pi, e ? p4.z : p4.x, e ? p4.w : p4.y);
+            mul2(x0, x1, x0, x1, first, first);
+            mul2(x0, x1, x0, x1, fast_exp2(e0), fast_exp2(e1));
+            mul2(x0, x1, x0, x1, last, last);
+            d[q4 * 4 + e] = __float_as_uint(x0);
+            d[q4 * 4 + e + 1] = __float_as_uint(x1);
+          }
+        }
+      } else {
+        const float f = fast_exp2(pi - s_pl2[31]) * (warp < 2 ? kScale : bi);
+#pragma unroll
+        for (int q4 = 0; q4 < 8; ++q4) {
+          const float4 p4 = pj[q4];
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            float x0 = __uint_as_float(d[q4 * 4 + e]), x1 = __uint_as_float(d[q4 * 4 + e + 1]);
+            mul2(x0, x1, x0, x1, e ? p4.z : p4.x, e ? p4.w : p4.y);
+            mul2(x0, x1, x0, x1, f, f);
+            d[q4 * 4 + e] = __float_as_uint(x0);
+            d[q4 * 4 + e + 1] = __float_as_uint(x1);
+          }
+        }
+      }
+      if (warp < 2) {
+#pragma unroll
+        for (int c8 = 0; c8 < 4; ++c8) {
+          uint32_t packed[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) packed[e] = pack_bf16(__uint_as_float(d[c8 * 8 + 2 * e]), __uint_as_float(d[c8 * 8 + 2 * e + 1]));
+          *reinterpret_cast<uint4*>(prow + (((h * 4 + c8) ^ (i & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        }
+      } else {
+        // the upper right 16x16 block of a 32x32 diagonal block is read as zeros
+        if (diagonal && !(i & 16)) {
+#pragma unroll
+          for (int e = 16; e < 32; ++e) d[e] = 0u;
+        }
+#pragma unroll
+        for (int q4 = 0; q4 < 8; ++q4)
+          *reinterpret_cast<uint4*>(arow + h * 32 + q4 * 4) = make_uint4(d[q4 * 4], d[q4 * 4 + 1], d[q4 * 4 + 2], d[q4 * 4 + 3]);
+      }
+    }
+    if (warp < 2) {
+      uint4* at = reinterpret_cast<uint4*>(prow + (((i >> 3) ^ (i & 7)) << 4));
+      uint4 x = *at;
+      const int keep = (i & 7) + 1;                       // columns of the piece on or below the diagonal, two to a word
+      x.x &= keep > 1 ? ~0u : 0xffffu;
+      x.y &= keep > 3 ? ~0u : (keep == 3 ? 0xffffu : 0u);
+      x.z &= keep > 5 ? ~0u : (keep == 5 ? 0xffffu : 0u);
+      x.w &= keep > 7 ? ~0u : (keep == 7 ? 0xffffu : 0u);
+      *at = x;
+#pragma unroll 1
+      for (int c8 = (i >> 3) + 1; c8 < 8; ++c8) *reinterpret_cast<uint4*>(prow + ((c8 ^ (i & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
+    // (the diagonal of A as stored is beta_i |k_i|^2 exp(0))
+    if (warp >= 2) bad = !(bi >= 0.f && arow[i] <= 2.f);
+  }
+  not_contraction |= __any_sync(0xffffffffu, bad);
+  if (warp < 2) {
+    const float last = s_pl2[valid - 1];
+    gates[t] = (t < valid) ? fast_exp2(last - s_pl2[t]) : 0.f;
+    if (t == 0) gates[kChunk] = fast_exp2(last);
+  }
+  if (t == 96) STAMP(0, n, 4);
+
+  // ---- T = (I+A)^-1 in place, blocked 16 -> 32 -> 64
+  // diagonal 16x16 solves, a column per thread (left-looking, in registers); the 16 threads of a block sit in one warp and
+  // overwrite the block only after all of them have read it
+  // (warp 2 wrote rows 0..31 of A, warp 3 rows 32..63: each solves its own two blocks)
+  __syncwarp();
+  if (ok && warp >= 2) {
+    const int col = lane & 15;
+    float* a0 = sAT + (t & 48) * L::kLd + (t & 48);
+    float x[16];
+    float4 cur[4], nxt[4] = {};
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+#pragma unroll
+      for (int j4 = 0; j4 < r + 1 && r + 1 < 16; j4 += 4)
+        nxt[j4 >> 2] = *reinterpret_cast<const float4*>(a0 + (r + 1) * L::kLd + j4);
+      float acc0 = (r == col) ? 1.f : 0.f, acc1 = 0.f;
+#pragma unroll
+      for (int j4 = 0; j4 < r; j4 += 4) {
+        const float4 a = cur[j4 >> 2];
+        if (j4 + 0 < r) acc0 = fmaf(-a.x, x[j4 + 0], acc0);
+        if (j4 + 1 < r) acc1 = fmaf(-a.y, x[j4 + 1], acc1);
+        if (j4 + 2 < r) acc0 = fmaf(-a.z, x[j4 + 2], acc0);
+        if (j4 + 3 < r) acc1 = fmaf(-a.w, x[j4 + 3], acc1);
+      }
+      x[r] = acc0 + acc1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cur[q] = nxt[q];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 16; ++r) a0[r * L::kLd + col] = x[r];
+  }
+  group_sync(id);
+  if (t == 96) STAMP(0, n, 5);
+  // block products T21 = -T22 (A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
+  // above the diagonal, which holds nothing
+  {
+    const int g = lane >> 2, tq = lane & 3;
+    const int big = warp >> 1, o = big * 32, col16 = (warp & 1) * 8;
+    float* x16 = sAT + (big * 16) * L::kLd + 32 + col16;
+    const uint32_t frag = smem_u32(sAT) + fragment_row(lane, L::kLd) * 4;
+#pragma unroll 1
+    for (int step = 0; step < 2; ++step) {
+      const uint32_t left = frag + ((o + 16) * L::kLd + o + step * 16) * 4;
+      const float* right = (step ? x16 : sAT + o * L::kLd + o + col16) + tq * L::kLd + g;
+      float* out = (step ? sAT + (o + 16) * L::kLd + o + col16 : x16) + g * L::kLd + 2 * tq;
+      const float sign = step ? -1.f : 1.f;
+      float c[1][4] = {};
+      if (ok) {
+        tile_row_tf32x3(c, left, right, L::kLd, 16);
+        *reinterpret_cast<float2*>(out) = make_float2(sign * c[0][0], sign * c[0][1]);
+        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(sign * c[0][2], sign * c[0][3]);
+      }
+      group_sync(id);
+    }
+    // 32 wide: a warp takes one row half and sixteen columns
+    const int row16 = big * 16, col32 = (warp & 1) * 16;
+#pragma unroll 1
+    for (int step = 0; step < 2; ++step) {
+      const uint32_t left = frag + ((32 + row16) * L::kLd + step * 32) * 4;
+      const float* right = sAT + step * 32 + col32 + tq * L::kLd + g;
+      float* out = (step ? sAT + (32 + row16) * L::kLd + col32 : sAT + row16 * L::kLd + 32 + col32) + g * L::kLd + 2 * tq;
+      const float sign = step ? -1.f : 1.f;
+      float c[2][4] = {};
+      if (ok) {
+        tile_row_tf32x3(c, left, right, L::kLd, 32);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          *reinterpret_cast<float2*>(out + q * 8) = make_float2(sign * c[q][0], sign * c[q][1]);
+          *reinterpret_cast<float2*>(out + q * 8 + 8 * L::kLd) = make_float2(sign * c[q][2], sign * c[q][3]);
+        }
+      }
+      if (step == 0) group_sync(id);
+    }
+  }
+  if (t == 96) STAMP(0, n, 6);
+  // T_w has one place: free once the previous chunk's W^T has been formed from it
+  if (n >= 1) ok = warp_wait(&bar->w, (n - 1) & 1) && ok;
+  group_sync(id);
+  if (t == 96) STAMP(0, n, 7);
+  // ---- T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row, 32 columns
+  {
+    const int row = t & 63, c0 = (t >> 6) * 32;
+    const bool empty = c0 == 32 && row < 32;          // above the diagonal
+    const float* trow = sAT + row * L::kLd + c0;
+    float4 x[8];
+#pragma unroll
+    for (int q4 = 0; q4 < 8; ++q4) {
+      x[q4] = *reinterpret_cast<const float4*>(trow + q4 * 4);
+      if (empty) x[q4] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      if (pass) group_sync(id);          // every thread holds its part of T: the U pair may take its place
+      scaled_row(x, (pass ? s_beta : s_coefw) + c0, sm + (pass ? L::kAT + group * L::kATBytes : L::kTw) + row * 128, c0 >> 3, row);
+    }
+    fence_proxy_async_smem();
+  }
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&bar->t_ready[group]);       // P, the gate vector and T_u of this chunk
+  ok = group_all(id, ok);
+  if (!ok) return false;
+  if (t == 96) STAMP(0, n, 8);
+
+  // ---- W^T = K^T (T diag(beta exp p))^T: the output warps turn it into the hi/lo operand, this group goes on
+  if (warp == 3) {
+    const uint64_t a = smem_desc(smem_u32(kq) + L::kK0, L::kK1 - L::kK0, 1024), x = smem_desc(smem_u32(sm + L::kTw), 16, 1024);
+    if (elect_one()) {
+      acc_lock(bar);
+      tc_fence_after();
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks)
+        mma_ss(kAccD, a + uint64_t((ks & 3) * 128), x + uint64_t((ks >> 2) * (kBox / 16) + (ks & 3) * 2), kIdescN64AT, ks != 0);
+      mma_commit(&bar->w);
+    }
+  }
+  __syncwarp();
+  if (t == 96) STAMP(0, n, 9);
+  return true;      // the same answer for the whole group; a wait that gave up shows at the next chunk's group_all
+}
+
+template <bool kRaw>
+__global__ void __launch_bounds__(kThreads, 1)
+forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                    const __grid_constant__ CUtensorMap tm_v, const Inputs in, const Geometry geo, const Plan plan) {
+  uint8_t* sm = shared_base();
+  using L = Smem;
+  Barriers* bar = reinterpret_cast<Barriers*>(sm + L::kBars);
+  const AbortFlag abort{&bar->abort};
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+#ifdef GDN_SM100_PHASE_TIMING
+  if (!plan.serial_pass && tid == 0) g_blocks[blockIdx.x][0] = clock64();
+#endif
+  if (plan.serial_pass) {
+    // nothing to repair for this CTA's heads: leave before anything is set up
+    bool any = false;
+    for (int unit = blockIdx.x; unit < plan.units; unit += gridDim.x)
+      for (int r = 1; r < plan.parallel; ++r) any |= plan.flags[unit * plan.parallel + r] != 0;
+    if (!any) return;
+  }
+  if (tid == 0) {
+    for (int i = 0; i < kRing; ++i) {
+      mbar_init(&bar->kq_full[i], 1);
+      mbar_init(&bar->kq_free[i], 1);
+      mbar_init(&bar->qs_go[i], 4);
+      mbar_init(&bar->qs_done[i], 2);
+    }
+    mbar_init(&bar->v_full, 1);
+    mbar_init(&bar->w, 1);
+    mbar_init(&bar->w_ready, 4);
+    mbar_init(&bar->ws, 1);
+    mbar_init(&bar->s, 1);
+    mbar_init(&bar->o, 1);
+    mbar_init(&bar->ofree, 4);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar->t_ready[i], 4);
+      mbar_init(&bar->u[i], 1);
+      mbar_init(&bar->d[i], 1);
+      mbar_init(&bar->ops[i], 8);
+      mbar_init(&bar->opn[i], 8);
+    }
+    for (int i = 0; i < kItems; ++i) {
+      mbar_init(&bar->item_full[i], 1);
+      mbar_init(&bar->item_free[i], kItemReaders);
+    }
+    bar->abort = bar->lock = bar->released = 0;
+    fence_barrier_init();
+  }
+  if (warp == kIssueWarp) {
+    tmem_alloc(&bar->tmem, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // all 512 columns were allocated, so tensor memory is addressed from column 0
+  if (tid == 0 && bar->tmem != 0) abort.raise(2, 90, 0);
+
+  if (warp == kPlanWarp) {
+    // ------------------------------------------------------------------ work items and TMA loads
+    if (lane == 0) {
+      prefetch_tensormap(&tm_q);
+      prefetch_tensormap(&tm_k);
+      prefetch_tensormap(&tm_v);
+    }
+    int ring = 0, n = 0;
+    bool ok = true;
+    // The V tile of a chunk is asked for one step behind its Q and K tiles: its single buffer is given back at the start
+    // of the previous chunk's chain step, ring stages at the end of one.
+    int v_n = -1, v_row = 0, v_t0 = 0, v_b = 0, v_hv = 0;
+    auto load_v = [&]() -> bool {
+      if (v_n >= 1 && !mbar_wait(&bar->u[(v_n - 1) & 1], ((v_n - 1) >> 1) & 1)) return false;
+      uint8_t* sv = sm + L::kV;
+      mbar_arrive_expect_tx(&bar->v_full, 2 * kBox);
+      if (kRaw) {
+        tma_load_2d(sv, &tm_q, &bar->v_full, (2 * geo.key_heads + v_hv) * kDim, v_row);
+        tma_load_2d(sv + kBox, &tm_q, &bar->v_full, (2 * geo.key_heads + v_hv) * kDim + 64, v_row);
+      } else {
+        tma_load_4d(sv, &tm_v, &bar->v_full, 0, v_hv, v_t0, v_b);
+        tma_load_4d(sv + kBox, &tm_v, &bar->v_full, 64, v_hv, v_t0, v_b);
+      }
+      return true;
+    };
+#pragma unroll 1
+    for (int unit = blockIdx.x; ok; unit += gridDim.x) {
+      const bool end = unit >= plan.units;
+      int bh = 0, b = 0, hv = 0, sub = 0, chunks = -1, t_first = 0, t_end = 0, unstored = 0, flags = 0, own = 0, slot = -1;
+      if (!end) {
+        const int parallel = plan.serial_pass ? 1 : plan.parallel;
+        bh = unit / parallel;
+        sub = unit % parallel;
+        b = bh / geo.value_heads;
+        hv = bh % geo.value_heads;
+        flags = (in.initial ? kHasInitial : 0) | (in.final_state ? kHasFinal : 0);
+        if (geo.varlen) {
+          // offsets forced into 0 <= ... <= total and non-decreasing: no index can leave the tensors
+          int most = 0;
+          for (int i = lane; i <= b; i += 32) most = max(most, i ? geo.varlen[i] : 0);
+#pragma unroll
+          for (int d = 16; d; d >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, d));
+          t_first = min(most, geo.sequence);
+          t_end = min(max(geo.varlen[b + 1], most), geo.sequence);
+          chunks = (t_end - t_first + kChunk - 1) / kChunk;
+          b = 0;
+        } else {
+          chunks = geo.segment_chunks();
+          t_first = geo.chunk_begin * kChunk;
+          t_end = geo.sequence;
+        }
+        if (plan.serial_pass) {
+          bool any = false;
+          for (int r = 1; r < plan.parallel; ++r) any |= plan.flags[bh * plan.parallel + r] != 0;
+          if (!any) continue;
+          if (lane == 0) {
+            atomicAdd(&g_fused_plan_counts[0], -1);
+            atomicAdd(&g_fused_plan_counts[1], 1);
+          }
+        } else if (parallel > 1) {
+          bool serial = false;
+          int mine = 0, next = 0;
+          for (int r = 1; r < parallel && !serial; ++r) {
+            const int c0 = sub_segment_begin(chunks, r, parallel), c1 = sub_segment_begin(chunks, r + 1, parallel);
+            const int reach = gate_reach<kRaw>(in, geo, b, hv, t_first + c0 * kChunk, c1 - c0, t_end, lane);
+            serial = reach < 0;
+            if (r == sub) mine = reach;
+            if (r == sub + 1) next = reach;
+          }
+          if (lane == 0) {
+            if (sub == 0) atomicAdd(&g_fused_plan_counts[serial ? 1 : 0], 1);
+            plan.flags[bh * parallel + sub] = 0;
+          }
+          if (serial) {
+            if (sub) continue;
+          } else {
+            const int c0 = sub_segment_begin(chunks, sub, parallel), c1 = sub_segment_begin(chunks, sub + 1, parallel);
+            own = c1 - c0;
+            chunks = own + next;
+            t_first += c0 * kChunk;
+            unstored = mine;
+            if (sub) {
+              flags &= ~kHasInitial;
+              slot = bh * parallel + sub;
+            }
+            if (sub + 1 < parallel) flags &= ~kHasFinal;
+          }
+        }
+      }
+      const int at = ring % kItems;
+      if (ring >= kItems) ok = warp_wait(&bar->item_free[at], ((ring / kItems) - 1) & 1);
+      if (!ok) break;
+      const int hk = hv / geo.group();
+      if (lane == 0) {
+        int* item = reinterpret_cast<int*>(sm + L::kItem) + at * 16;
+        item[kChunks] = chunks;
+        item[kBatch] = b;
+        item[kHv] = hv;
+        item[kFirst] = t_first;
+        item[kEnd] = t_end;
+        item[kUnstored] = unstored;
+        item[kState] = bh;
+        item[kFlags] = flags;
+        item[kFlagSlot] = slot;
+        item[kOwn] = own;
+        mbar_arrive(&bar->item_full[at]);
+        if (end && v_n >= 0) load_v();
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c, ++n) {
+          const int s = n % kRing, t0 = t_first + c * kChunk;
+          if (n >= kRing && !mbar_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1)) break;
+          uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
+          mbar_arrive_expect_tx(&bar->kq_full[s], 4 * kBox);
+          if (kRaw) {
+            // packed rows [q heads | k heads | v heads]; rows behind the batch element's end belong to the next one (or
+            // read as zero behind the last) and are neutralised by beta = 0 / zero gate weights
+            const int row = b * geo.sequence + t0;
+            tma_load_2d(kq + L::kQ0, &tm_q, &bar->kq_full[s], hk * kDim, row);
+            tma_load_2d(kq + L::kQ1, &tm_q, &bar->kq_full[s], hk * kDim + 64, row);
+            tma_load_2d(kq + L::kK0, &tm_q, &bar->kq_full[s], (geo.key_heads + hk) * kDim, row);
+            tma_load_2d(kq + L::kK1, &tm_q, &bar->kq_full[s], (geo.key_heads + hk) * kDim + 64, row);
+          } else {
+            tma_load_4d(kq + L::kQ0, &tm_q, &bar->kq_full[s], 0, hk, t0, b);
+            tma_load_4d(kq + L::kQ1, &tm_q, &bar->kq_full[s], 64, hk, t0, b);
+            tma_load_4d(kq + L::kK0, &tm_k, &bar->kq_full[s], 0, hk, t0, b);
+            tma_load_4d(kq + L::kK1, &tm_k, &bar->kq_full[s], 64, hk, t0, b);
+          }
+          if (n >= 1 && !load_v()) break;
+          v_row = b * geo.sequence + t0;
+          v_t0 = t0;
+          v_b = b;
+          v_hv = hv;
+          ++v_n;
+        }
+      }
+      __syncwarp();
+      n = __shfl_sync(0xffffffffu, n, 0);
+      ok = __all_sync(0xffffffffu, !abort.raised());
+      ++ring;
+      if (end) break;
+    }
+  } else if (warp == kIssueWarp) {
+    // ------------------------------------------------------------------ issuer of the chain's products
+    // The whole warp waits and forms descriptors, one elected lane issues.
+    const uint32_t base = smem_u32(sm);
+    const uint64_t dW = smem_desc(base + L::kW, 16, 1024), dV = smem_desc(base + L::kV, kBox, 1024);
+    ItemCursor cursor;
+    int n = 0;
+#pragma unroll 1
+    for (bool ok = true; ok;) {
+      const int* item = cursor.open(sm, bar, ok);
+      if (!ok) break;
+      const int chunks = item[kChunks];
+      cursor.close(bar, lane);
+      if (chunks < 0) break;
+#pragma unroll 1
+      for (int c = 0; c < chunks && ok; ++c, ++n) {
+        const int s = n % kRing, par = n & 1;
+        const uint32_t kq = base + L::kKQ + s * L::kKQStage;
+        // U^T = V^T (T diag(beta))^T, while the chain warps split the state
+        ok = mbar_wait(&bar->t_ready[par], (n >> 1) & 1);
+        ok &= mbar_wait(&bar->v_full, par);
+        STAMP(3, n, 0);
+        tc_fence_after();
+        const uint64_t dU = smem_desc(base + L::kAT + par * L::kATBytes, 16, 1024);
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            mma_ss(kAccU, dV + uint64_t((ks & 3) * 128), dU + uint64_t((ks >> 2) * (kBox >> 4) + (ks & 3) * 2), kIdescN64AT, ks != 0);
+          mma_commit(&bar->u[par]);
+        }
+        ok &= mbar_wait(&bar->w_ready, par);
+        // (W S)^T with St ~ SH + SL and W ~ W_hi + W_lo (not lo lo); K steps {0,1,4,5} of the split become available
+        // first, {2,3,6,7} second
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          ok &= mbar_wait(&bar->ops[half], par);
+          STAMP(3, n, 1 + half);
+          tc_fence_after();
+          const uint64_t dw = dW + uint64_t(half * 256);
+          const uint32_t op = half * 16;
+          if (elect_one()) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int ks = (q >> 1) * 4 + (q & 1);
+              mma_ts(kAccX, kOpSH + ks * 8 + op, dw + uint64_t(ks * 128), kIdescN64BT, q != 0 || half != 0);
+              mma_ts(kAccX, kOpSL + ks * 8 + op, dw + uint64_t(ks * 128), kIdescN64BT, 1);
+              mma_ts(kAccX, kOpSH + ks * 8 + op, dw + uint64_t(L::kWTile / 16 + ks * 128), kIdescN64BT, 1);
+            }
+            if (half) mma_commit(&bar->ws);
+          }
+        }
+        STAMP(3, n, 3);
+        ok &= mbar_wait(&bar->qs_done[s], (n / kRing) & 1);
+        if (n > 0) ok &= mbar_wait(&bar->ofree, (n - 1) & 1);
+        STAMP(3, n, 4);
+        tc_fence_after();
+        const uint64_t qd = smem_desc(kq + L::kQ0, 16, 1024);
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            mma_ts(kAccO, kOpSH + ks * 8, qd + uint64_t((ks >> 2) * (L::kQ1 - L::kQ0) / 16 + (ks & 3) * 2), kIdescN64, ks != 0);
+        }
+        // St += (N*rel)^T K (the accumulator already holds gamma * St); token groups {0,2} first, {1,3} second
+        const uint64_t kd = smem_desc(kq + L::kK0, L::kK1 - L::kK0, 1024), pd = smem_desc(base + L::kP + s * kBox, 16, 1024);
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          ok &= mbar_wait(&bar->opn[half], par);
+          STAMP(3, n, 5 + half);
+          tc_fence_after();
+          const uint64_t dk = kd + uint64_t(half * 128);
+          const uint32_t op = kAccX + half * 16;
+          if (elect_one()) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              mma_ts(kAccS, op + h * 32, dk + uint64_t(h * 256), kIdescN128BT, 1);
+              mma_ts(kAccS, op + h * 32 + 8, dk + uint64_t(h * 256), kIdescN128BT, 1);
+            }
+            if (half) {
+              mma_commit(&bar->s);
+              // O^T += N^T P^T behind the state update: the next chunk's split waits for that, not for the output
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) mma_ts(kAccO, kOpSL + ks * 8, pd + uint64_t(ks * 2), kIdescN64, 1);
+              mma_commit(&bar->o);
+              mma_commit(&bar->kq_free[s]);
+            }
+          }
+        }
+        STAMP(3, n, 7);
+      }
+      ok = __all_sync(0xffffffffu, ok);
+    }
+  } else if (warp < kChainWarp) {
+    // ------------------------------------------------------------------ query scaling
+    ItemCursor cursor;
+    int n = 0;
+    const int t64 = tid - kScaleWarp * 32;
+#pragma unroll 1
+    for (bool ok = true; ok;) {
+      const int* item = cursor.open(sm, bar, ok);
+      if (!ok) break;
+      const int chunks = item[kChunks];
+      cursor.close(bar, lane);
+      if (chunks < 0) break;
+#pragma unroll 1
+      for (int c = 0; c < chunks && ok; ++c, ++n) {
+        const int s = n % kRing;
+        ok = warp_wait(&bar->qs_go[s], (n / kRing) & 1);
+        if (!ok) break;
+        uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
+        const float* scale = reinterpret_cast<const float*>(sm + L::kGates) + s * kGateWords + kGateQueryScale;
+#pragma unroll 2
+        for (int it = 0; it < 16; ++it) {
+          const int piece = it * 64 + t64, row = piece >> 4, col16 = piece & 15;
+          uint4* at = reinterpret_cast<uint4*>(kq + (col16 < 8 ? L::kQ0 : L::kQ1) + row * 128 + (((col16 & 7) ^ (row & 7)) << 4));
+          const float f = scale[row];
+          const uint4 x = *at;
+          uint4 o;
+          o.x = pack_bf16(bf16_lo(x.x) * f, bf16_hi(x.x) * f);
+          o.y = pack_bf16(bf16_lo(x.y) * f, bf16_hi(x.y) * f);
+          o.z = pack_bf16(bf16_lo(x.z) * f, bf16_hi(x.z) * f);
+          o.w = pack_bf16(bf16_lo(x.w) * f, bf16_hi(x.w) * f);
+          *at = o;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar->qs_done[s]);
+      }
+    }
+  } else if (warp < kOutWarp) {
+    // ------------------------------------------------------------------ state chain
+    const int quarter = warp & 3, half = (warp - kChainWarp) >> 2;
+    const int v = quarter * 32 + lane;                     // value row = TMEM lane
+    const uint32_t taddr = uint32_t(quarter * 32) << 16;
+    ItemCursor cursor;
+    int n = 0;
+#pragma unroll 1
+    for (bool ok = true; ok;) {
+      const int* item = cursor.open(sm, bar, ok);
+      if (!ok) break;
+      const int chunks = item[kChunks], flags = item[kFlags], bh = item[kState];
+      cursor.close(bar, lane);
+      if (chunks < 0) break;
+      {
+        const float* init = (flags & kHasInitial) ? in.initial + (long long)bh * kDim * kDim + v : nullptr;
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          uint32_t vals[32];
+          const int k0 = half * 64 + part * 32;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) vals[j] = init ? __float_as_uint(init[(k0 + j) * kDim]) : 0u;
+          tmem_st32(taddr + kAccS + k0, vals);
+        }
+        tmem_wait_st();
+      }
+#pragma unroll 1
+      for (int c = 0; c < chunks && ok; ++c, ++n) {
+        const int par = n & 1;
+        const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + (n % kRing) * kGateWords;
+        ok = mbar_wait(&bar->w_ready, par);            // (the gate vector comes with it)
+        if (tid == 128) STAMP(1, n, 0);
+        if (n > 0) ok = ok && mbar_wait(&bar->s, (n - 1) & 1);
+        if (tid == 128) STAMP(1, n, 1);
+        if (!ok) break;
+        tc_fence_after();
+        const float gamma = gates[kChunk];
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          uint32_t d[32], hi[16], lo[16];
+          const int k0 = half * 64 + part * 32;
+          tmem_ld32(taddr + kAccS + k0, d);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float s0 = __uint_as_float(d[j]), s1 = __uint_as_float(d[j + 1]);
+            split_pair(s0, s1, hi[j >> 1], lo[j >> 1]);
+            float g0, g1;
+            mul2(g0, g1, s0, s1, gamma, gamma);
+            d[j] = __float_as_uint(g0);
+            d[j + 1] = __float_as_uint(g1);
+          }
+          tmem_st16(taddr + kOpSH + (k0 >> 1), hi);
+          tmem_st32(taddr + kAccS + k0, d);
+          // P N of the previous chunk reads its N from the columns of the lo operand
+          if (n > 0 && part == 0) ok = mbar_wait_inline(&bar->o, (n - 1) & 1);
+          tmem_st16(taddr + kOpSL + (k0 >> 1), lo);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar->ops[part]);
+        }
+        if (tid == 128) STAMP(1, n, 2);
+        ok = ok && mbar_wait(&bar->ws, par);
+        if (tid == 128) STAMP(1, n, 3);
+        ok = ok && mbar_wait(&bar->u[par], (n >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          const int ks = half * 2 + part;                     // 16-token group
+          uint32_t x[16], u[16], nh[8], nl[8], n16[8];
+          tmem_ld16(taddr + kAccX + ks * 16, x);
+          tmem_ld16(taddr + kAccU + ks * 16, u);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            const int i = ks * 16 + j;
+            float n0, n1, r0, r1;
+            sub2(n0, n1, __uint_as_float(u[j]), __uint_as_float(u[j + 1]), __uint_as_float(x[j]), __uint_as_float(x[j + 1]));
+            mul2(r0, r1, n0, n1, gates[i], gates[i + 1]);
+            split_pair(r0, r1, nh[j >> 1], nl[j >> 1]);
+            n16[j >> 1] = pack_bf16(n0, n1);
+          }
+          tmem_st8(taddr + kAccX + ks * 16, nh);
+          tmem_st8(taddr + kAccX + ks * 16 + 8, nl);
+          tmem_st8(taddr + kOpSL + ks * 8, n16);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar->opn[part]);
+        }
+        if (tid == 128) STAMP(1, n, 4);
+      }
+      if (ok && n > 0) ok = mbar_wait(&bar->s, (n - 1) & 1);
+      if (ok && (flags & kHasFinal)) {
+        tc_fence_after();
+        float* fin = in.final_state + (long long)bh * kDim * kDim + v;
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          uint32_t d[32];
+          const int k0 = half * 64 + part * 32;
+          tmem_ld32(taddr + kAccS + k0, d);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) fin[(k0 + j) * kDim] = __uint_as_float(d[j]);
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+    }
+  } else if (warp < kPrepWarp) {
+    // ------------------------------------------------------------------ W operand and output
+    // Every chunk's W^T accumulator becomes the hi/lo operand of the chain here, one chunk ahead of the output tile: these
+    // four warps are idle most of a chunk, the prepare groups are what a chunk waits for.
+    const int quarter = warp - kOutWarp;
+    const uint32_t lanes = uint32_t(quarter * 32) << 16;
+    const int row_stride = geo.value_heads * kDim;
+    ItemCursor cursor;
+    int n = 0;                                  // chunks whose W has been converted; the output of chunk n - 1 is due
+    __nv_bfloat16* o_at = nullptr;              // its first row at this lane's place
+    int o_rows = 0;                             // rows of it to be stored
+    int chunks = 0, c = 0, b = 0, hv = 0, t_first = 0, t_end = 0, unstored = 0;
+#pragma unroll 1
+    for (bool ok = true; ok;) {
+      if (c == chunks) {
+        const int* item = cursor.open(sm, bar, ok);
+        if (!ok) break;
+        c = 0;
+        chunks = item[kChunks];
+        b = item[kBatch];
+        hv = item[kHv];
+        t_first = item[kFirst];
+        t_end = item[kEnd];
+        unstored = item[kUnstored];
+        cursor.close(bar, lane);
+        if (chunks == 0) continue;
+      }
+      const bool end = chunks < 0;
+      if (!end) {
+        ok = warp_wait(&bar->w, n & 1);
+        ok = warp_wait(&bar->t_ready[n & 1], (n >> 1) & 1) && ok;         // what it announces is passed on with W
+        if (n > 0) ok = warp_wait(&bar->ws, (n - 1) & 1) && ok;            // W of the previous chunk has been read
+        tc_fence_after();
+        if (!ok) break;
+        const int key = quarter * 32 + lane;
+        uint8_t* wt = sm + L::kW + key * 128;
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          uint32_t dw[32];
+          tmem_ld32(lanes + kAccD + h * 32, dw);
+          tmem_wait_ld();
+          if (h == 1) acc_release(bar, lane);
+#pragma unroll
+          for (int c8 = 0; c8 < 4; ++c8) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              split_pair(__uint_as_float(dw[c8 * 8 + 2 * e]), __uint_as_float(dw[c8 * 8 + 2 * e + 1]), hi[e], lo[e]);
+            const int slot = ((h * 4 + c8) ^ (key & 7)) << 4;
+            *reinterpret_cast<uint4*>(wt + slot) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(wt + L::kWTile + slot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar->w_ready);
+      }
+      if (n > 0) {
+        // The output tile leaves straight from registers: neighbouring lanes (value columns) swap halves of a token pair,
+        // so that an even lane holds two columns of the first token and an odd lane of the second, and a warp writes
+        // two 64-byte pieces.  (No staging tile: its 16 KB are what lets T_w have a place of its own.)
+        ok = warp_wait(&bar->o, (n - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        __nv_bfloat16* at = o_at;
+        int rows = o_rows - (lane & 1);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          uint32_t d[32];
+          tmem_ld32(lanes + kAccO + h * 32, d);
+          tmem_wait_ld();
+          if (h == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar->ofree);
+          }
+          if (o_rows > 0) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const uint32_t x = pack_bf16(__uint_as_float(d[2 * j]), __uint_as_float(d[2 * j + 1]));
+              const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1);
+              const uint32_t pair = __byte_perm(x, y, (lane & 1) ? 0x3276 : 0x5410);
+              if (2 * j < rows) *reinterpret_cast<uint32_t*>(at) = pair;
+              at += 2 * row_stride;
+            }
+          }
+          rows -= 32;
+        }
+      }
+      if (end) break;
+      const int t0 = t_first + c * kChunk;
+      o_at = in.output + (((long long)b * geo.sequence + t0 + (lane & 1)) * geo.value_heads + hv) * kDim + quarter * 32 + (lane & 30);
+      o_rows = c >= unstored ? min(kChunk, t_end - t0) : 0;
+      ++c;
+      ++n;
+    }
+  } else {
+    // ------------------------------------------------------------------ prepare groups
+    const int group = (warp - kPrepWarp) >> 2;
+    ItemCursor cursor;
+    int n = 0;
+#pragma unroll 1
+    for (bool ok = true; ok;) {
+      const int* item = cursor.open(sm, bar, ok);
+      ok = group_all(1 + group, ok);
+      if (!ok) break;
+      const int chunks = item[kChunks], b = item[kBatch], hv = item[kHv], t_first = item[kFirst], t_end = item[kEnd];
+      const int slot = item[kFlagSlot], own = item[kOwn];
+      cursor.close(bar, lane);
+      if (chunks < 0) break;
+      bool violation = false;
+      GateLoads next;
+#pragma unroll 1
+      for (int c = 0; c < chunks && ok; ++c, ++n) {
+        if ((n & 1) != group) continue;
+        bool not_contraction = false;
+        const int t0 = t_first + c * kChunk;
+        ok = prepare_chunk<kRaw>(sm, bar, in, geo, group, n, b, hv, t0, c + 2 < chunks ? t0 + 2 * kChunk : -1, t_end, next,
+                                 not_contraction);
+        violation |= not_contraction && c < own;
+      }
+      if (slot >= 0 && violation && lane == 0) plan.flags[slot] = 1;
+      ok = group_all(1 + group, ok);
+    }
+  }
+  if (abort.raised()) {
+    for (int i = 0; i < 20; ++i) __nanosleep(100000);   // let copies in flight land before the CTA leaves
+  }
+  tc_fence_before();
+  __syncthreads();
+#ifdef GDN_SM100_PHASE_TIMING
+  if (!plan.serial_pass && tid == 0) g_blocks[blockIdx.x][1] = clock64();
+#endif
+  if (warp == kIssueWarp) tmem_dealloc(bar->tmem, 512);
+}
+#undef STAMP
+
+template <bool kRaw>
+int launch(const Inputs& in, const Geometry& geo, const Plan& plan, int grid, cudaStream_t stream) {
+  TensorMapEncoder& enc = tensor_map_encoder();
+  if (int rc = enc.init()) return rc;
+  CUtensorMap tm_q, tm_k, tm_v;
+  const uint64_t batch = geo.varlen ? 1 : geo.batch;
+  if (kRaw) {
+    // one 2-D map over the packed projection rows serves Q, K and V
+    if (int rc = enc.bf16_2d(&tm_q, in.mixed, uint64_t(in.mixed_stride), batch * geo.sequence, kChunk)) return rc;
+    tm_k = tm_v = tm_q;
+  } else {
+    if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, batch, kChunk)) return rc;
+  }
+  forward_umma_kernel<kRaw><<<grid, kThreads, kSmemBytes, stream>>>(tm_q, tm_k, tm_v, in, geo, plan);
+  return int(cudaGetLastError());
+}
+int sm_count() {
+  static int counts[64] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 1;
+  if (!counts[device] && cudaDeviceGetAttribute(&counts[device], cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 1;
+  return counts[device];
+}
+}  // namespace
+
+int configure_fused() {
+  cudaError_t e = cudaFuncSetAttribute(forward_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(forward_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  return int(e);
+}
+
+long long fused_workspace_bytes(const Geometry& geo, int parallel) {
+  return parallel > 1 ? ((long long)geo.batch * geo.value_heads * parallel * (long long)sizeof(int) + 255) & ~255LL : 0;
+}
+
+// `flags`: fused_workspace_bytes(geo, geo.parallel) bytes of scratch (may be null when that is 0)
+int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cudaStream_t stream) {
+  Plan plan{};
+  plan.parallel = geo.parallel > 1 ? geo.parallel : 1;
+  plan.flags = flags;
+  const int heads = geo.batch * geo.value_heads, sms = sm_count();
+  if (plan.parallel > 1 && (geo.varlen || !flags || plan.parallel > geo.segment_chunks())) return int(cudaErrorInvalidValue);
+  plan.units = heads * plan.parallel;
+  const auto go = in.mixed ? launch<true> : launch<false>;
+  if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
+  if (plan.parallel == 1) return 0;
+  plan.serial_pass = 1;
+  plan.units = heads;
+  return go(in, geo, plan, heads < sms ? heads : sms, stream);
+}
+
+GDN_SM100_DEFINE_STATUS_HOOKS(fused)
+
+int read_fused_plan_counts(int* host_out2, int reset) {
+  cudaError_t e = cudaMemcpyFromSymbol(host_out2, g_fused_plan_counts, 2 * sizeof(int));
+  if (e != cudaSuccess) return int(e);
+  if (reset) {
+    const int zero[2] = {0, 0};
+    e = cudaMemcpyToSymbol(g_fused_plan_counts, zero, sizeof(zero));
+  }
+  return int(e);
+}
+
+}  // namespace gdn_sm100
+#ifdef GDN_SM100_PHASE_TIMING
+extern "C" int gdn_read_stamps(void* host) { return int(cudaMemcpyFromSymbol(host, gdn_sm100::g_stamps, sizeof(gdn_sm100::g_stamps))); }
+extern "C" int gdn_read_blocks(void* host) { return int(cudaMemcpyFromSymbol(host, gdn_sm100::g_blocks, sizeof(gdn_sm100::g_blocks))); }
+#endif

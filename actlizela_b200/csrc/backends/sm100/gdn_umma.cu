@@ -17,7 +17,7 @@
 // Math reference: the WY chunk form of the reference project (tests/wy_cpu.py:44-88;
 // prepare/state/output kernels csrc/gdn_chunk/gdn_wy_ppu.cu:7-292), re-derived in transposed form.
 #include "gdn_common.cuh"
-#include "umma.cuh"
+#include "umma_math.cuh"
 
 namespace gdn_sm100 {
 using namespace ptx;
@@ -81,73 +81,6 @@ namespace {
 // because a sub-segment does not decay or a token is not a contraction [1]; read by read_walk_plan_counts.
 __device__ int g_walk_plan_counts[2];
 
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kBox = 8192;            // one TMA box: 64 rows x 128 bytes
-constexpr uint32_t kIdescN64 = idesc_bf16(128, 64, false, false);      // A K-major (smem or TMEM), B K-major
-constexpr uint32_t kIdescN64AT = idesc_bf16(128, 64, true, false);     // A MN-major (transposed smem tile)
-constexpr uint32_t kIdescN128BT = idesc_bf16(128, 128, false, true);   // B MN-major
-
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// Packed FP32 pairs (two IEEE round-to-nearest operations per instruction on sm_100): the arithmetic of the walk's
-// chain warps is bound by instruction issue, and these halve its floating-point instruction count bit for bit.
-#define GDN_F32X2(name, op)                                                                                      \
-  __device__ __forceinline__ void name(float& x0, float& x1, float a0, float a1, float b0, float b1) {          \
-    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" op                       \
-        ".rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"                                                       \
-        : "=f"(x0), "=f"(x1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));                                              \
-  }
-GDN_F32X2(add2, "add")
-GDN_F32X2(sub2, "sub")
-GDN_F32X2(mul2, "mul")
-#undef GDN_F32X2
-// d += a b for one m16n8k8 tile with FP32-grade accuracy from TF32 tensor-core products: a ~ ah + al, b ~ bh + bl
-// (both parts TF32), d += ah bh + ah bl + al bh (the 3xTF32 scheme the reference uses for these merges,
-// tests/wy_cpu.py:10-18).  Fragment layout of mma.m16n8k8: g = lane / 4, t = lane % 4;
-// a = {A[g][t], A[g+8][t], A[g][t+4], A[g+8][t+4]}, b = {B[t][g], B[t+4][g]}, d = {D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1]}.
-__device__ __forceinline__ void mma_tf32x3(float (&d)[4], const float (&a)[4], const float (&b)[2]) {
-  // The high part is the operand with its 13 low mantissa bits cleared (a TF32 value), the low part the exact FP32
-  // remainder, of which the tensor core reads the leading TF32 bits: about 2^-20 relative in all, below the
-  // 16 significant bits the inverse is later stored with.  Logic and add instructions: the conversion unit, the
-  // kernel's busiest pipe, stays free for the BF16 packing.
-  uint32_t ah[4], al[4], bh[2], bl[2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    ah[i] = __float_as_uint(a[i]) & 0xffffe000u;
-    al[i] = __float_as_uint(a[i] - __uint_as_float(ah[i]));
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    bh[i] = __float_as_uint(b[i]) & 0xffffe000u;
-    bl[i] = __float_as_uint(b[i] - __uint_as_float(bh[i]));
-  }
-#define GDN_MMA_TF32(A, B)                                                                              \
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, " \
-               "{%8, %9}, {%0, %1, %2, %3};"                                                             \
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])                                          \
-               : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(B[0]), "r"(B[1]))
-  GDN_MMA_TF32(al, bh);
-  GDN_MMA_TF32(ah, bl);
-  GDN_MMA_TF32(ah, bh);
-#undef GDN_MMA_TF32
-}
-// One m16n8 tile of D = A B over k in [0, kdim): A row-major with pitch lda (rows a_row0 + {g, g+8}), B row-major with
-// pitch ldb (column b_col0 + g); both in shared memory.
-__device__ __forceinline__ void tile_product_tf32x3(float (&d)[4], const float* a, int lda, const float* b, int ldb,
-                                                    int kdim, int g, int t) {
-#pragma unroll
-  for (int k0 = 0; k0 < kdim; k0 += 8) {
-    const float av[4] = {a[g * lda + k0 + t], a[(g + 8) * lda + k0 + t], a[g * lda + k0 + t + 4], a[(g + 8) * lda + k0 + t + 4]};
-    const float bv[2] = {b[(k0 + t) * ldb + g], b[(k0 + t + 4) * ldb + g]};
-    mma_tf32x3(d, av, bv);
-  }
-}
-__device__ __forceinline__ float bf16_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }
-
 // ================================================================================= prepare kernel
 // One CTA per (batch, value head, chunk) block, 256 threads, THREE CTAs per SM (at most 80 registers, 67 KB of
 // shared memory, 128 tensor-memory columns): the phases of a block are serial and latency bound, so the
@@ -179,7 +112,7 @@ struct PrepLayout {
   static constexpr int kStageWH = 0, kStageWL = 2 * kBox;  // phase 6: W^T hi / lo tiles [128][64] over the Q/K boxes
   static constexpr int kLdX = 20, kLdX3 = 36;
   static constexpr int kVec = kAT + 64 * kLd * 4;          // float [4][64]: pl2, beta, beta*exp(p), exp(p)/sqrt(128)
-  static constexpr int kBars = kVec + 4 * 64 * 4;          // 2 mbarriers, tmem slot, abort flag, carry
+  static constexpr int kBars = kVec + (4 * 64 + 32) * 4;   // (and 32 column factors) 2 mbarriers, tmem slot, abort flag, carry
   static constexpr int kTotal = kBars + 64;
   static_assert(2 * kBox <= 64 * kLd * 4 && kAT % 1024 == 0, "the U pair of T tiles must fit on T, box aligned");
   static_assert(32 * kLdX3 * 4 <= kBox && 32 * kLdX * 4 <= kBox, "block-product scratch must fit in one Q box");
@@ -214,6 +147,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   float* s_beta = s_pl2 + 64;
   float* s_coefw = s_beta + 64;
   float* s_qscale = s_coefw + 64;
+  float* s_ecol = s_qscale + 64;
   uint64_t* bar_tma = reinterpret_cast<uint64_t*>(sm + L::kBars);
   uint64_t* bar_mma = bar_tma + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tma + 2);
@@ -319,6 +253,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     s_beta[tid] = beta;
     s_coefw[tid] = beta * e;
     s_qscale[tid] = e * kScale;
+    const float pl2_31 = __shfl_sync(0xffffffffu, prefix * kLog2e, 31);
+    if (tid < 32) s_ecol[tid] = fast_exp2(pl2_31 - prefix * kLog2e);
   }
   __syncthreads();
 
@@ -404,10 +340,13 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
         continue;
       }
+      // in the 32x32 block off the diagonal exp(p_i - p_j) = exp(p_i - p_31) exp(p_31 - p_j): a factor per row, one per column
+      const bool off = quarter & 1 && chalf == 0;
+      const float row_factor = off ? fast_exp2(pi - s_pl2[31]) * (lrow < 64 ? kScale : bi) : 0.f;
       float pj[16];
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4) {
-        const float4 t = *reinterpret_cast<const float4*>(s_pl2 + j0 + q4 * 4);
+        const float4 t = *reinterpret_cast<const float4*>((off ? s_ecol : s_pl2) + j0 + q4 * 4);
         pj[q4 * 4] = t.x; pj[q4 * 4 + 1] = t.y; pj[q4 * 4 + 2] = t.z; pj[q4 * 4 + 3] = t.w;
       }
       if (lrow < 64) {
@@ -415,9 +354,15 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
         for (int jj = 0; jj < 16; jj += 2) {
           const int j = j0 + jj;
-          const float a0 = (j <= i) ? __uint_as_float(d[piece][jj]) * fast_exp2(pi - pj[jj]) * kScale : 0.f;
-          const float a1 = (j + 1 <= i) ? __uint_as_float(d[piece][jj + 1]) * fast_exp2(pi - pj[jj + 1]) * kScale : 0.f;
-          packed[jj >> 1] = pack_bf16(a0, a1);
+          float a0 = __uint_as_float(d[piece][jj]), a1 = __uint_as_float(d[piece][jj + 1]);
+          if (off) {
+            a0 = a0 * pj[jj] * row_factor;
+            a1 = a1 * pj[jj + 1] * row_factor;
+          } else {
+            a0 = a0 * fast_exp2(pi - pj[jj]) * kScale;
+            a1 = a1 * fast_exp2(pi - pj[jj + 1]) * kScale;
+          }
+          packed[jj >> 1] = pack_bf16(j <= i ? a0 : 0.f, j + 1 <= i ? a1 : 0.f);
         }
         uint4* dst = reinterpret_cast<uint4*>(ws.p + (block * kChunk + i) * kChunk + j0);
         dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
@@ -430,8 +375,10 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int jj = q4 * 4 + e;
-            a[e] = (j0 + jj < i) ? bi * __uint_as_float(d[piece][jj]) * fast_exp2(pi - pj[jj]) : 0.f;
-            if (j0 + jj == i) kk = __uint_as_float(d[piece][jj]);
+            const float x = __uint_as_float(d[piece][jj]);
+            const float y = off ? x * pj[jj] * row_factor : bi * x * fast_exp2(pi - pj[jj]);
+            a[e] = j0 + jj < i ? y : 0.f;
+            kk = j0 + jj == i ? x : kk;
           }
           *reinterpret_cast<float4*>(arow + q4 * 4) = make_float4(a[0], a[1], a[2], a[3]);
         }
@@ -669,13 +616,12 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 // kernel; 512 threads, one CTA per SM.  Tensor memory (512 columns):
 //   ACC_S [  0,128)  St FP32 accumulator (pre-scaled by the chunk decay before the update MMA)
 //   OP_SH [128,192)  St BF16 hi, packed pairs      OP_SL [192,256)  St BF16 lo
-//   ACC_X [256,384)  S_hi^T [W_hi ; W_lo]^T, with S_lo^T W_hi^T added to the first half:
-//           [256,320) (W_hi S)^T   [320,384) (W_lo S_hi)^T
+//   ACC_X [256,320)  (W S)^T = S_hi^T W_hi^T + S_lo^T W_hi^T + S_hi^T W_lo^T;
 //         after N = U - W S has been formed, the columns are reused for the N operands of the
 //         16-token group ks:  (N*rel) hi at 256+16ks, lo at 256+16ks+8,  N (BF16) at 320+16ks
 //   ACC_O [384,448) and [448,512)  O^T = S_hi^T Qs^T + N^T P^T, alternating by chunk: the epilogue drains one
 //         while the next chunk's products fill the other
-// Per chunk: 16 instructions for W S (N = 128 and 64), on which the chain waits; 8 for S Qs and 4 for P N, issued
+// Per chunk: 24 instructions for W S (N = 64), on which the chain waits; 8 for S Qs and 4 for P N, issued
 // behind the commits the chain waits for; 8 for the state update (N = 128).
 // Roles: warp 0 MMA issuer and warp 1 TMA producer (the lowest warp ids: their short instruction streams
 //        sit on the critical path and must not queue behind the arithmetic of the chain warps);
@@ -1037,16 +983,14 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         const int ks = half * 2 + part;                     // 16-token group
-        uint32_t dh[16], dl[16], nh[8], nl[8], n16[8];
-        tmem_ld16(taddr + kAccX + ks * 16, dh);
-        tmem_ld16(taddr + kAccX + 64 + ks * 16, dl);
+        uint32_t x[16], nh[8], nl[8], n16[8];
+        tmem_ld16(taddr + kAccX + ks * 16, x);
         tmem_wait_ld();
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
           const int i = ks * 16 + j;
-          float z0, z1, n0, n1, r0, r1, e0, e1;
-          add2(z0, z1, __uint_as_float(dh[j]), __uint_as_float(dh[j + 1]), __uint_as_float(dl[j]), __uint_as_float(dl[j + 1]));
-          sub2(n0, n1, u[part * 16 + j], u[part * 16 + j + 1], z0, z1);
+          float n0, n1, r0, r1, e0, e1;
+          sub2(n0, n1, u[part * 16 + j], u[part * 16 + j + 1], __uint_as_float(x[j]), __uint_as_float(x[j + 1]));
           mul2(r0, r1, n0, n1, gates[i], gates[i + 1]);
           const uint32_t h = pack_bf16(r0, r1);
           nh[j >> 1] = h;
@@ -1212,14 +1156,14 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       bool ok = true;
       // Descriptors of ring stage 0; stage 1 is a constant further on (the start-address field counts 16-byte units).
       static_assert(L::kStages == 2 && L::kStage % 16 == 0, "descriptor arithmetic below assumes a two-stage ring");
-      const uint64_t dW = smem_desc(st0 + L::kWH, L::kWL - L::kWH, 1024);      // MN-major: 64-token groups hi | lo
+      const uint64_t dW = smem_desc(st0 + L::kWH, 16, 1024);      // MN-major, one 64-token group; the lo tile is one tile behind
       const uint64_t dQ0 = smem_desc(st0 + L::kQS0, 16, 1024), dQ1 = smem_desc(st0 + L::kQS1, 16, 1024);
       const uint64_t dK = smem_desc(st0 + L::kK, kBox, 1024), dP = smem_desc(st0 + L::kP, 16, 1024);
       for (int c = 0; c < chunks && ok; ++c) {
         const uint64_t stage = uint64_t((c & 1) * (L::kStage >> 4));
         const uint64_t wd = dW + stage, q0 = dQ0 + stage, q1 = dQ1 + stage, kd = dK + stage, pd = dP + stage;
         const uint32_t acc_o = tm + kAccO + (c & 1) * 64;
-        // St [W_hi | W_lo] with St ~ SH + SL (the SL pass only against W_hi, added to the first half).  The B
+        // (W S)^T with St ~ SH + SL and W ~ W_hi + W_lo (not lo lo), one accumulator.  The B
         // operand is the transposed W tile: key index on the 128-byte lines (K), tokens contiguous (N); one K
         // step of 16 keys is 2048 bytes.  K steps {0,1,4,5} of the split become available first, {2,3,6,7}
         // second.  The chain waits for this product only; the state part of the output, St Qs^T, reads the same
@@ -1230,8 +1174,9 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         for (int q = 0; q < 4; ++q) {
           const int ks = (q >> 1) * 4 + (q & 1);
           const uint64_t bdesc = wd + uint64_t(ks * 128);
-          mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc, kIdescN128BT, q != 0);
+          mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc, kIdescN64BT, q != 0);
           mma_ts(tm + kAccX, tm + kOpSL + ks * 8, bdesc, kIdescN64BT, 1);
+          mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc + uint64_t((L::kWL - L::kWH) >> 4), kIdescN64BT, 1);
         }
         ok &= mbar_wait(bar_ops + 1, c & 1, abort, 41, c);
         tc_fence_after();
@@ -1239,8 +1184,9 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         for (int q = 0; q < 4; ++q) {
           const int ks = (q >> 1) * 4 + 2 + (q & 1);
           const uint64_t bdesc = wd + uint64_t(ks * 128);
-          mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc, kIdescN128BT, 1);
+          mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc, kIdescN64BT, 1);
           mma_ts(tm + kAccX, tm + kOpSL + ks * 8, bdesc, kIdescN64BT, 1);
+          mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc + uint64_t((L::kWL - L::kWH) >> 4), kIdescN64BT, 1);
         }
         mma_commit(bar_ws);
         ok &= mbar_wait(bar_qs + (c & 1), (c >> 1) & 1, abort, 44, c);     // scaled long ago: the tile landed a chunk ahead

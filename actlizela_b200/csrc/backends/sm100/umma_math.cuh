@@ -1,0 +1,111 @@
+// Device arithmetic shared by the tensor-core kernels of this backend (two-kernel path and single-launch forward):
+// both produce the same bits, so the operations and their order live in one place.
+#pragma once
+#include "gdn_common.cuh"
+#include "umma.cuh"
+
+namespace gdn_sm100 {
+using namespace ptx;
+namespace {
+
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kBox = 8192;            // one TMA box: 64 rows x 128 bytes
+constexpr uint32_t kIdescN64 = idesc_bf16(128, 64, false, false);      // A K-major (smem or TMEM), B K-major
+constexpr uint32_t kIdescN64AT = idesc_bf16(128, 64, true, false);     // A MN-major (transposed smem tile)
+constexpr uint32_t kIdescN128BT = idesc_bf16(128, 128, false, true);   // B MN-major
+
+__device__ __forceinline__ float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Packed FP32 pairs (two IEEE round-to-nearest operations per instruction on sm_100): the arithmetic of the walk's
+// chain warps is bound by instruction issue, and these halve its floating-point instruction count bit for bit.
+#define GDN_F32X2(name, op)                                                                                      \
+  __device__ __forceinline__ void name(float& x0, float& x1, float a0, float a1, float b0, float b1) {          \
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" op                       \
+        ".rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"                                                       \
+        : "=f"(x0), "=f"(x1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));                                              \
+  }
+GDN_F32X2(sub2, "sub")
+GDN_F32X2(mul2, "mul")
+#undef GDN_F32X2
+// d += a b for one m16n8k8 tile with FP32-grade accuracy from TF32 tensor-core products: a ~ ah + al, b ~ bh + bl
+// (both parts TF32), d += ah bh + ah bl + al bh (the 3xTF32 scheme the reference uses for these merges,
+// tests/wy_cpu.py:10-18).  Fragment layout of mma.m16n8k8: g = lane / 4, t = lane % 4;
+// a = {A[g][t], A[g+8][t], A[g][t+4], A[g+8][t+4]}, b = {B[t][g], B[t+4][g]}, d = {D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1]}.
+// The high part is the operand with its 13 low mantissa bits cleared (a TF32 value), the low part the exact FP32
+// remainder, of which the tensor core reads the leading TF32 bits: about 2^-20 relative in all, below the 16 significant
+// bits the inverse is later stored with.  Logic and add instructions: the conversion unit stays free for BF16 packing.
+template <int kN>
+__device__ __forceinline__ void split_tf32(const float (&x)[kN], uint32_t (&hi)[kN], uint32_t (&lo)[kN]) {
+#pragma unroll
+  for (int i = 0; i < kN; ++i) {
+    hi[i] = __float_as_uint(x[i]) & 0xffffe000u;
+    lo[i] = __float_as_uint(x[i] - __uint_as_float(hi[i]));
+  }
+}
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// The A fragment {A[g][t], A[g+8][t], A[g][t+4], A[g+8][t+4]} of a row-major FP32 matrix in shared memory in one instruction:
+// a 16-byte row piece of an 8x8 16-bit matrix holds four floats.  `addr` is this lane's row piece (fragment_row).
+__device__ __forceinline__ void load_fragment_a(float (&a)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]) : "r"(addr) : "memory");
+}
+// row piece of a lane: rows 0..15, columns 0 or 4 (floats, pitch lda)
+__device__ __forceinline__ int fragment_row(int lane, int lda) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * lda + (lane >> 4) * 4; }
+// kN m16n8 tiles side by side, D[i] = A B[:, 8 i .. 8 i + 8) over k in [0, kdim): A at this lane's `a_addr`, B row-major with
+// pitch ldb, b = this lane's B[t][g].  Same products in the same order as tile_product_tf32x3, one A fragment for all tiles.
+template <int kN>
+__device__ __forceinline__ void tile_row_tf32x3(float (&d)[kN][4], uint32_t a_addr, const float* b, int ldb, int kdim) {
+#pragma unroll
+  for (int k0 = 0; k0 < kdim; k0 += 8) {
+    float av[4];
+    uint32_t ah[4], al[4], bh[kN][2], bl[kN][2];
+    load_fragment_a(av, a_addr + k0 * 4);
+    split_tf32(av, ah, al);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      const float bv[2] = {b[k0 * ldb + i * 8], b[(k0 + 4) * ldb + i * 8]};
+      split_tf32(bv, bh[i], bl[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kN; ++i) mma_tf32(d[i], al, bh[i]);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) mma_tf32(d[i], ah, bl[i]);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) mma_tf32(d[i], ah, bh[i]);
+  }
+}
+// One m16n8 tile of D = A B over k in [0, kdim): A row-major with pitch lda (rows {g, g+8}), B row-major with pitch ldb
+// (column g); both in shared memory.
+__device__ __forceinline__ void tile_product_tf32x3(float (&d)[4], const float* a, int lda, const float* b, int ldb,
+                                                    int kdim, int g, int t) {
+#pragma unroll
+  for (int k0 = 0; k0 < kdim; k0 += 8) {
+    const float av[4] = {a[g * lda + k0 + t], a[(g + 8) * lda + k0 + t], a[g * lda + k0 + t + 4], a[(g + 8) * lda + k0 + t + 4]};
+    const float bv[2] = {b[(k0 + t) * ldb + g], b[(k0 + t + 4) * ldb + g]};
+    uint32_t ah[4], al[4], bh[2], bl[2];
+    split_tf32(av, ah, al);
+    split_tf32(bv, bh, bl);
+    mma_tf32(d, al, bh);
+    mma_tf32(d, ah, bl);
+    mma_tf32(d, ah, bh);
+  }
+}
+__device__ __forceinline__ float bf16_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }
+// (x0, x1) ~ hi + lo as packed BF16 pairs
+__device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  hi = pack_bf16(x0, x1);
+  float l0, l1;
+  sub2(l0, l1, x0, x1, bf16_lo(hi), bf16_hi(hi));
+  lo = pack_bf16(l0, l1);
+}
+
+}  // namespace
+}  // namespace gdn_sm100

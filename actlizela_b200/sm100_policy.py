@@ -52,7 +52,7 @@ class Selection:
         """Native configuration word: kernel family in the low bits, segment count in bits 8..15, parallel
         sub-segments of the walk in bits 16..19."""
         family = policy()["configuration_ids"][self.configuration]
-        return family | (self.segments << 8) | ((self.parallel << 16) if family == 1 else 0)
+        return family | (self.segments << 8) | ((self.parallel << 16) if family in (1, 4) else 0)
 
 
 def default_parallel(batch, length, value_heads):
@@ -63,9 +63,9 @@ def default_parallel(batch, length, value_heads):
 
 
 def default_segments(batch, length, value_heads):
-    """Segment count for a shape without a measured row.  Overlapping the prepare of a later segment with the walk
-    of an earlier one only pays while the walk leaves SMs idle, i.e. when it is not split into parallel
-    sub-segments: then up to 64 heads -> isqrt(chunks/8) clamped to 1..8, more -> 1.  The native selector computes
+    """Segment count of the two-kernel family for a shape without a measured row (the single-launch form has one
+    segment).  Overlapping the prepare of a later segment with the walk of an earlier one only pays while the walk leaves SMs idle,
+    i.e. when it is not split into parallel sub-segments: then up to 64 heads -> isqrt(chunks/8) clamped to 1..8, more -> 1.  The native selector computes
     the same."""
     from math import isqrt
     heads, chunks = batch * value_heads, (length + 63) // 64
@@ -106,7 +106,7 @@ def select(shape, profile):
             return Selection(row["configuration"], "b200-measured-shape", data["id"],
                              int(row.get("segments", 1)), int(row.get("parallel", 1)))
     return Selection(data["default"], "unmeasured-shape-default", data["id"],
-                     default_segments(shape[0], shape[1], shape[3]), default_parallel(shape[0], shape[1], shape[3]))
+                     default_segments(shape[0], shape[1], shape[3]) if data["default"] == "umma" else 1, default_parallel(shape[0], shape[1], shape[3]))
 
 
 _SELECTIONS = {}

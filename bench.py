@@ -669,8 +669,12 @@ def main():
     for _ in range(args.warmup):
         forward()
     ms_step, spread = timed(forward, args.steps)
-    ms_walk, _ = timed(lambda: forward(0x20), args.steps)
-    ms_prepare, _ = timed(lambda: forward(0x10), args.steps)
+    # the two-kernel family can be timed stage by stage; the single-launch form is one kernel (and, where the walk is
+    # split, a second launch that leaves at once)
+    single = (config & 0xf) == 4
+    kernels_ms = dict(forward=ms_step)
+    if not single:
+        kernels_ms.update(walk=timed(lambda: forward(0x20), args.steps)[0], prepare=timed(lambda: forward(0x10), args.steps)[0])
     forward()
 
     # end to end through the host-buffer entry: pinned host tensors in, output + state back
@@ -718,14 +722,16 @@ def main():
         return
 
     alg_bytes, alg_flops = algorithmic_bytes(shard), algorithmic_flops(shard)
-    # the roofline object describes the longer of the two kernels of a forward; both see the whole problem, so the
-    # algorithmic bytes of the path (each tensor once) are set against that kernel's own time
-    top, ms_top = ("prepare", ms_prepare) if ms_prepare > ms_walk else ("walk", ms_walk)
+    # the roofline object describes the kernel of the single-launch form, or the longer of the two kernels of the
+    # two-kernel family; each sees the whole problem, so the algorithmic bytes of the path (each tensor once) are set
+    # against that kernel's own time
+    top, ms_top = ("forward", ms_step) if single else max(((k2, kernels_ms[k2]) for k2 in ("prepare", "walk")), key=lambda x: x[1])
     achieved = alg_bytes / (ms_top * 1e-3) / 1e9
-    # DRAM traffic per launch from the committed ncu captures of a smaller case (profiles/; caches flushed before the
-    # captured launch, so an upper bound), per (chunk, value head) block and scaled by the blocks of one launch
+    # DRAM traffic of the two-kernel family per launch from the committed ncu captures of a smaller case (profiles/;
+    # caches flushed before the captured launch, so an upper bound), per (chunk, value head) block and scaled by the
+    # blocks of one launch; the single-launch form moves each tensor once
     blocks = shard.batch * shard.value_heads * ((shard.length + 63) // 64)
-    traffic = {"walk": 108.3e3, "prepare": 52.3e3}[top] * blocks if config_name == "umma" else None
+    traffic = {"walk": 108.3e3, "prepare": 52.3e3}[top] * blocks if config_name == "umma" else (alg_bytes if single else None)
     whole_ms = max(alg_bytes / (hbm_peak * 1e9), alg_flops / (tensor_peak * 1e12)) * 1e3
     line = dict(
         metric=METRIC, value=workload.tokens * world / (ms_step * 1e-3), unit=UNIT, n_gpus=world,
@@ -734,11 +740,12 @@ def main():
         data="synthetic", config=config_dict(workload, world),
         kernel_configuration=dict(family=config_name, segments=(config >> 8) & 0xff, parallel=max(1, (config >> 16) & 0xf)),
         gpu_launches=args.steps * lib.actlize_la_sm100_launches_per_forward(config),
-        kernels_ms=dict(prepare=ms_prepare, walk=ms_walk, forward=ms_step),
+        kernels_ms=kernels_ms,
         step_spread=spread,
         roofline=dict(bound="hbm", kernel=top, achieved=achieved, peak=hbm_peak, unit="GB/s",
                       frac=achieved / hbm_peak, traffic=traffic,
-                      traffic_note=("dram bytes read + written of one launch in the ncu capture of cfg0 (caches flushed "
+                      traffic_note=("every tensor once: no workspace" if single else
+                                    "dram bytes read + written of one launch in the ncu capture of cfg0 (caches flushed "
                                     "before the launch; workspace lines still dirty in L2 at its end are not in it), "
                                     "per block, scaled by the blocks of this launch" if traffic else None),
                       peak_source=peak_source, algorithmic_bytes=alg_bytes, algorithmic_flops=alg_flops,
