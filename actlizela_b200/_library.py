@@ -17,10 +17,12 @@ import json
 import os
 from pathlib import Path
 
+from . import _host
 from .backends.registry import require_implementation
 
 ABI_VERSION = 1
 LIBRARY_NAME = "libactlize_la_sm100.so"
+HOST_MODULE_NAME = "actlize_la_sm100_host.so"
 NATIVE_DIRECTORY = Path(__file__).resolve().parent / "_native"
 ENVIRONMENT_OVERRIDE = "ACTLIZE_LA_SM100_LIBRARY"
 
@@ -128,6 +130,11 @@ class NativeLibrary:
             raise LibraryError("native library ABI/target/numerical-contract identity mismatch")
         self.numerical_contract = contract
         self._configured = set()
+        # the host side of the entry points: built beside the default library, whichever library it is bound to
+        host = NATIVE_DIRECTORY / HOST_MODULE_NAME
+        if not host.is_file():
+            raise LibraryError(f"native host extension not built: {host}; run python -m actlizela_b200.build_sm100")
+        _host.bind(self.lib, str(host), os.environ.get(ENVIRONMENT_OVERRIDE))
 
     def configure(self, device):
         """Per-device function attributes; once per device, before any capture."""
@@ -138,7 +145,11 @@ class NativeLibrary:
                 if torch.cuda.is_current_stream_capturing():
                     raise RuntimeError("configure the cuda_sm100 library before stream capture")
                 self.check(self.lib.actlize_la_sm100_configure())
+                index = torch.cuda.current_device()
             self._configured.add(key)
+            from .sm100_policy import is_policy_device
+            if is_policy_device(index):
+                _host.configured(index)
 
     @staticmethod
     def current_stream_handle(device_index):

@@ -13,6 +13,7 @@ current stream.
 """
 from __future__ import annotations
 
+from . import _host
 from ._library import load_library
 
 
@@ -44,6 +45,9 @@ def _operands(*specs):
 def gdn_prepare_inputs(mixed, a, b, a_log, dt_bias, key_heads, value_heads):
     """mixed [N, (2Hk+Hv)*128] BF16, a,b [N,Hv] BF16, a_log, dt_bias [Hv] FP32 ->
     (q [N,Hk,128], k [N,Hk,128], v [N,Hv,128] BF16, g [N,Hv] FP32, beta [N,Hv] BF16)."""
+    result = _host.prepare_inputs(mixed, a, b, a_log, dt_bias, key_heads, value_heads)
+    if result is not None:
+        return result
     import torch
     bf16, fp32 = (torch.bfloat16,), (torch.float32,)
     if type(key_heads) is not int or type(value_heads) is not int or key_heads < 1 or value_heads % key_heads:
@@ -74,6 +78,9 @@ def gdn_prepare_inputs(mixed, a, b, a_log, dt_bias, key_heads, value_heads):
 def gdn_decode_step(q, k, v, g, beta, state):
     """q,k [B,Hk,128], v [B,Hv,128] BF16, g [B,Hv] (BF16/FP32 natural-log decay), beta [B,Hv] BF16,
     state FP32 [B,Hv,128,128] updated IN PLACE.  Returns the BF16 output [B,Hv,128]."""
+    result = _host.decode_step(q, k, v, g, beta, state)
+    if result is not None:
+        return result
     import torch
     bf16, fp32 = (torch.bfloat16,), (torch.float32,)
     if q.ndim != 3 or v.ndim != 3:
@@ -100,6 +107,9 @@ def gdn_forward_projections(mixed, a, b, a_log, dt_bias, key_heads, value_heads,
     [q heads | k heads | v heads], ``a``, ``b`` BF16 [B,T,Hv], ``a_log``, ``dt_bias`` FP32 [Hv].  Normalisation
     and gate activation happen inside the prepare kernel; the result equals ``gdn_prepare_inputs`` followed by
     ``gdn_forward`` bit for bit.  Returns (out [B,T,Hv,128] BF16, final state or None)."""
+    result = _host.projections(mixed, a, b, a_log, dt_bias, key_heads, value_heads, initial_state, output_final_state)
+    if result is not None:
+        return result
     import torch
     from .sm100 import load_sm100
     from .sm100_policy import select
@@ -162,6 +172,9 @@ def gdn_verify_step(q, k, v, g, beta, state):
     [B,Hv,128,128] is READ ONLY.  Returns (out [B,W,Hv,128] BF16, delta [B,W,Hv,128] FP32); ``gdn_commit_step``
     applies the accepted prefix (the reference's verify/commit pair, csrc/serving/gdn.cu:152-217,255-300,
     without its slot pool)."""
+    result = _host.verify_step(q, k, v, g, beta, state)
+    if result is not None:
+        return result
     import torch
     b_, w, hk, hv = _check_step_inputs(q, k, v, g, beta, state)
     lib = load_library()
@@ -178,6 +191,9 @@ def gdn_verify_step(q, k, v, g, beta, state):
 def gdn_commit_step(k, g, delta, counts, state):
     """Apply the first ``counts[b]`` (int32 device tensor [B], 0..W) recorded updates of a verify step to ``state``
     in place: S <- e^{g_t} S + k_t delta_t^T."""
+    result = _host.commit_step(k, g, delta, counts, state)
+    if result is not None:
+        return result
     import torch
     b_, w, hk, hv = _check_step_inputs(None, k, None, g, None, state, delta, counts)
     lib = load_library()
@@ -190,6 +206,9 @@ def gdn_commit_step(k, g, delta, counts, state):
 
 def rmsnorm_gated(y, z, weight):
     """y, z [..., 128] BF16, weight [128] BF16 -> BF16 tensor shaped like y."""
+    result = _host.rmsnorm_gated(y, z, weight)
+    if result is not None:
+        return result
     import torch
     if y.ndim < 1 or y.shape[-1] != 128:
         raise ValueError("y must have a last dimension of 128")
@@ -207,6 +226,9 @@ def rmsnorm_gated(y, z, weight):
 def out_proj_gemm(a, w):
     """C = A @ W^T: A [M,K] BF16 row-major, W [N,K] BF16 (Linear weight layout), FP32 accumulation, C [M,N] BF16.
     K and N must be multiples of 8.  One tcgen05 kernel on the caller's current stream."""
+    result = _host.out_proj_gemm(a, w)
+    if result is not None:
+        return result
     import torch
     if a.ndim != 2 or w.ndim != 2:
         raise ValueError("A must be [M,K] and W [N,K]")

@@ -3,6 +3,9 @@
 
     python -m actlizela_b200.build_sm100 [--out DIR] [--compiler NVCC] [--verbose-ptxas]
 
+Also builds ``actlize_la_sm100_host``, the extension that carries the host side of the Python entry points
+(``torch_host.cpp``, g++ against torch's headers; it calls the C ABI through addresses bound at load).
+
 One nvcc invocation compiles every kernel for sm_100a only
 (``-gencode arch=compute_100a,code=sm_100a``) and links ``libactlize_la_sm100.so``.  The static
 shape table ``sm100_policy.json`` is rendered into a C++ include so that the native
@@ -28,6 +31,7 @@ ROOT = PACKAGE.parent
 SOURCE = PACKAGE / "csrc" / "backends" / "sm100"
 INCLUDE = ROOT / "include"
 UNITS = ("abi.cu", "gdn_simt.cu", "gdn_umma.cu", "gdn_fused.cu", "gdn_aux.cu", "out_proj.cu", "static_scratch.cu")
+HOST_UNIT, HOST_MODULE = "torch_host.cpp", "actlize_la_sm100_host"
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
          "-DNDEBUG", *ARCH_FLAGS]
@@ -52,6 +56,20 @@ def render_policy_table(policy_path, out_path):
         % (data["id"], ids[data["default"]], rows))
 
 
+def host_command(out):
+    """g++ line of the host extension; torch's libraries are resolved from the process that has imported torch."""
+    import sysconfig
+    import torch
+    torch_root = Path(torch.__file__).parent
+    cuda = Path(os.getenv("CUDA_HOME", "/usr/local/cuda"))
+    includes = [torch_root / "include", torch_root / "include" / "torch" / "csrc" / "api" / "include",
+                sysconfig.get_paths()["include"], cuda / "include"]
+    return ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-DNDEBUG",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{x}" for x in includes),
+            str(SOURCE / HOST_UNIT), f"-L{torch_root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+            "-ltorch_python", "-o", str(out)]
+
+
 def build(out=None, compiler=None, verbose_ptxas=False, quiet=False, defines=()):
     out = Path(out) if out else PACKAGE / "_native"
     out.mkdir(parents=True, exist_ok=True)
@@ -62,7 +80,7 @@ def build(out=None, compiler=None, verbose_ptxas=False, quiet=False, defines=())
         raise RuntimeError(f"compiler missing: {compiler}")
     policy_path = PACKAGE / "sm100_policy.json"
     render_policy_table(policy_path, generated / "sm100_policy_table.inc")
-    sources = sorted(p for p in SOURCE.iterdir() if p.suffix in (".cu", ".cuh", ".h"))
+    sources = sorted(p for p in SOURCE.iterdir() if p.suffix in (".cu", ".cuh", ".h", ".cpp"))
     identity = dict(
         target="cuda_sm100", arch="sm_100a", abi_version=1, complete=False,
         compiler=str(compiler),
@@ -77,18 +95,25 @@ def build(out=None, compiler=None, verbose_ptxas=False, quiet=False, defines=())
                *(str(SOURCE / unit) for unit in UNITS), "-o", str(library)]
     if not quiet:
         print("[sm100 build]", shlex.join(command), flush=True)
+    host = out / f"{HOST_MODULE}.so"
     log = out / "build.log"
-    with log.open("w") as stream:
+    with log.open("w") as stream, (out / "build_host.log").open("w") as host_stream:
+        host_build = subprocess.Popen(host_command(host), stdout=host_stream, stderr=subprocess.STDOUT)
         stream.write(shlex.join(command) + "\n")
         stream.flush()
         result = subprocess.run(command, stdout=stream, stderr=subprocess.STDOUT)
+        host_build.wait()
     if result.returncode:
         sys.stderr.write(log.read_text()[-6000:])
         raise RuntimeError(f"nvcc failed rc={result.returncode}; see {log}")
+    if host_build.returncode:
+        sys.stderr.write((out / "build_host.log").read_text()[-6000:])
+        raise RuntimeError(f"g++ failed rc={host_build.returncode}; see {out / 'build_host.log'}")
     after = {str(p.relative_to(ROOT)): sha(p) for p in [*sources, INCLUDE / "actlize_la_sm100.h"]}
     if after != identity["source_sha256"]:
         raise RuntimeError("source changed during build; do not use this binary")
-    identity.update(library=library.name, library_sha256=sha(library), complete=True)
+    identity.update(library=library.name, library_sha256=sha(library), host_module=host.name, host_sha256=sha(host),
+                    complete=True)
     receipt.write_text(json.dumps(identity, indent=2) + "\n")
     if not quiet:
         print(f"[sm100 build] PASS scope=COMPILE_LINK_ONLY library={library} device=NOT_RUN")

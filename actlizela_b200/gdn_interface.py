@@ -9,6 +9,7 @@ unsupported device or a missing binary is an error, never a fallback.
 """
 from importlib import import_module
 
+from . import _host
 from .backends.registry import require_implementation
 from .device import validate_profile_options
 
@@ -49,6 +50,11 @@ def gdn_forward(q, k, v, g, beta, initial_state=None, output_final_state=True,
     1/sqrt(128) query scale are built in; no hidden Q/K normalisation, gate activation,
     rescaling or state conversion takes place.
     """
+    if (algorithm == "auto" and mode == "device" and backend is None and delivery is None and configuration is None
+            and sm_count is None):
+        result = _host.forward(q, k, v, g, beta, initial_state, output_final_state)
+        if result is not None:
+            return result
     route = _resolve_forward(q, initial_state, algorithm=algorithm, backend=backend,
                              delivery=delivery, configuration=configuration,
                              mode=mode, sm_count=sm_count)

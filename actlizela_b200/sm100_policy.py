@@ -85,6 +85,13 @@ def tensor_backend(q):
     raise ValueError("automatic GDN target unsupported; this build admits sm_100 devices only")
 
 
+def is_policy_device(index):
+    """Whether the table (and the native selector, which reads shapes only) applies to a CUDA device."""
+    expected, profile = policy()["device"], device_profile(index)
+    return (profile.capability == tuple(expected["capability"]) and expected["name_contains"] in profile.name
+            and profile.sm_count == expected["sm_count"])
+
+
 def select(shape, profile):
     """shape=(B,T,Hk,Hv,K,V); metadata only."""
     data = policy()

@@ -11,6 +11,8 @@ bits and the second exists as a cross-check.
 """
 from __future__ import annotations
 
+from . import _host
+
 
 def gdn_forward_varlen(q, k, v, g, beta, cu_seqlens, initial_states=None, output_final_state=True, *,
                        per_sequence=False, forward_fn=None, **forward_options):
@@ -18,6 +20,10 @@ def gdn_forward_varlen(q, k, v, g, beta, cu_seqlens, initial_states=None, output
 
     ``initial_states`` is FP32 ``[N,Hv,128,128]`` or None; sequences of length 0 keep their state.
     """
+    if not per_sequence and forward_fn is None and not forward_options:
+        result = _host.varlen(q, k, v, g, beta, cu_seqlens, initial_states, output_final_state)
+        if result is not None:
+            return result
     import torch
     if isinstance(cu_seqlens, torch.Tensor) and cu_seqlens.is_cuda and not per_sequence and forward_fn is None:
         # int32 offsets in device memory go to the native entry untouched (no host read; capturable)
