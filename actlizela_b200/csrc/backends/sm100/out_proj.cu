@@ -128,18 +128,182 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   if (warp == 1) tmem_dealloc(tmem, kTileN);
 }
 
+// ------------------------------------------------------------------------------------------- few rows: split over K
+// With few rows of A (a decode step) the 128 x 128 tiles above are fewer than the SMs, and a CTA walks all of K alone: at
+// M 4, K 4096, N 2560 twenty CTAs streamed W, 21 MB, at 0.7 TB/s.  Here the roles are swapped (128 rows of W on the
+// tensor-memory lanes, kM rows of A as the N dimension, so that nothing but kM rows is multiplied) and a cluster of CTAs
+// splits K: each accumulates its range, leaves its partial tile in its own shared memory, and sums a share of the rows
+// over the cluster, in rank order, through distributed shared memory.  Bound by the stream of W (L2 or HBM).
+constexpr int kSkinnyThreads = 192;
+template <int kM> struct SkinnyLayout {
+  static constexpr int kStage = kOperandBytes + kM * kTileK * 2;             // W tile, A tile
+  static constexpr int kStages = kM <= 32 ? 5 : (kM == 64 ? 4 : 3);          // two CTAs per SM
+  static constexpr int kBars = kStages * kStage;
+  static constexpr int kBytes = kBars + 128 + 1024;
+  static_assert(kM * 128 * 4 <= kBars, "the partial tile must fit on the stages");
+  static_assert(2 * (kBytes + 1024) <= 227 * 1024, "two CTAs per SM");
+};
+
+template <int kM>
+__global__ void __launch_bounds__(kSkinnyThreads, 2)
+out_proj_skinny_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
+                       __nv_bfloat16* __restrict__ c, int m, int n, int k) {
+  using L = SkinnyLayout<kM>;
+  extern __shared__ __align__(1024) uint8_t raw_smem[];
+  uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + L::kBars);        // [stages] tiles landed
+  uint64_t* empty = full + L::kStages;                                // [stages] tiles consumed
+  uint64_t* done = empty + L::kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const AbortFlag abort{abort_word};
+  constexpr uint32_t kColumns = kM < 32 ? 32 : kM;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = blockIdx.x, split = gridDim.x;                      // the cluster spans the first grid dimension
+  const int n0 = blockIdx.y * kTileM, m0 = blockIdx.z * kM;
+  const int k_tiles = (k + kTileK - 1) / kTileK;
+  const int kt0 = k_tiles * rank / split, kt1 = k_tiles * (rank + 1) / split;
+
+  if (tid == 0) {
+    for (int s = 0; s < L::kStages; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    mbar_init(done, 1);
+    *abort_word = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, kColumns);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kt = kt0; kt < kt1; ++kt) {
+        const int i = kt - kt0, s = i % L::kStages;
+        if (i >= L::kStages && !mbar_wait(empty + s, ((i / L::kStages) - 1) & 1, abort, 63, kt)) break;
+        uint8_t* stage = sm + s * L::kStage;
+        mbar_arrive_expect_tx(full + s, L::kStage);
+        tma_load_2d(stage, &tm_w, full + s, kt * kTileK, n0);
+        tma_load_2d(stage + kOperandBytes, &tm_a, full + s, kt * kTileK, m0);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t base = smem_u32(sm);
+      bool ok = true;
+      for (int kt = kt0; kt < kt1 && ok; ++kt) {
+        const int i = kt - kt0, s = i % L::kStages;
+        ok = mbar_wait(full + s, (i / L::kStages) & 1, abort, 64, kt);
+        tc_fence_after();
+        const uint64_t dw = smem_desc(base + s * L::kStage, 16, 1024), da = smem_desc(base + s * L::kStage + kOperandBytes, 16, 1024);
+#pragma unroll
+        for (int ks = 0; ks < kTileK / 16; ++ks)
+          mma_ss(tmem, dw + uint64_t(ks * 2), da + uint64_t(ks * 2), idesc_bf16(128, kM, false, false), (i | ks) != 0);
+        mma_commit(empty + s);
+      }
+      mma_commit(done);
+    }
+    __syncwarp();
+  } else if (mbar_wait(done, 0, abort, 65, 0)) {
+    // the partial tile as [row of A][row of W], over the stages (every tile has been consumed)
+    tc_fence_after();
+    const int quarter = warp & 3;
+    float* part = reinterpret_cast<float*>(sm) + quarter * 32 + lane;
+#pragma unroll
+    for (int piece = 0; piece < kM / 16; ++piece) {
+      uint32_t d[16];
+      tmem_ld16(tmem + (uint32_t(quarter * 32) << 16) + piece * 16, d);
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) part[(piece * 16 + j) * 128] = __uint_as_float(d[j]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, kColumns);
+  // every CTA of the cluster comes here, also one that gave up a wait
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  {
+    // rank r sums rows r, r + split, ...: 64 threads take a row's 128 columns in pairs
+    const int pair = tid & 63;
+    const bool inside = n0 + pair * 2 < n;
+    for (int row = rank + (tid >> 6) * split; row < kM && m0 + row < m; row += 3 * split) {
+      const uint32_t at = smem_u32(sm) + (row * 128 + pair * 2) * 4;
+      float x = 0.f, y = 0.f;
+      for (int r = 0; r < split; ++r) {
+        uint32_t remote;
+        float px, py;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(r));
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(px), "=f"(py) : "r"(remote) : "memory");
+        x += px;
+        y += py;
+      }
+      if (inside) *reinterpret_cast<uint32_t*>(c + (long long)(m0 + row) * n + n0 + pair * 2) = pack_bf16(x, y);
+    }
+  }
+  if (abort.raised()) {
+    for (int i = 0; i < 20; ++i) __nanosleep(100000);   // let copies in flight land before the CTA leaves
+  }
+  // nobody leaves while its partial tile may still be read
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int kM>
+int launch_skinny(TensorMapEncoder& enc, const void* a, const void* w, void* c, int m, int n, int k, int split, cudaStream_t stream) {
+  CUtensorMap tm_a, tm_w;
+  if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kM)) return rc;
+  if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kTileM)) return rc;
+  cudaLaunchConfig_t launch{};
+  launch.gridDim = dim3(split, (n + kTileM - 1) / kTileM, (m + kM - 1) / kM);
+  launch.blockDim = dim3(kSkinnyThreads);
+  launch.dynamicSmemBytes = SkinnyLayout<kM>::kBytes;
+  launch.stream = stream;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = split;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  launch.attrs = &cluster;
+  launch.numAttrs = 1;
+  return int(cudaLaunchKernelEx(&launch, out_proj_skinny_kernel<kM>, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k));
+}
+
 }  // namespace
 
 GDN_SM100_DEFINE_STATUS_HOOKS(gemm)
 
 int configure_out_proj() {
   if (int rc = tensor_map_encoder().init()) return rc;
-  return int(cudaFuncSetAttribute(out_proj_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(out_proj_umma_kernel, smem, kGemmSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<16>, smem, SkinnyLayout<16>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<32>, smem, SkinnyLayout<32>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<64>, smem, SkinnyLayout<64>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<128>, smem, SkinnyLayout<128>::kBytes);
+  return int(e);
 }
 
 int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, cudaStream_t stream) {
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
+  // Fewer 128 x 128 tiles than half the CTA slots (two per SM): split K over a cluster, by the largest power of two up to 8
+  // that keeps the CTAs within the slots and at least two K steps in each.
+  const long long tiles = ((n + kTileM - 1LL) / kTileM) * ((m + 127LL) / 128), k_tiles = (k + kTileK - 1LL) / kTileK;
+  int split = 1;
+  while (split < 8 && tiles * split * 2 <= 2 * 148 && k_tiles >= 4 * split) split *= 2;
+  if (split > 1) {
+    if (m <= 16) return launch_skinny<16>(enc, a, w, c, m, n, k, split, stream);
+    if (m <= 32) return launch_skinny<32>(enc, a, w, c, m, n, k, split, stream);
+    if (m <= 64) return launch_skinny<64>(enc, a, w, c, m, n, k, split, stream);
+    return launch_skinny<128>(enc, a, w, c, m, n, k, split, stream);
+  }
   CUtensorMap tm_a, tm_w;
   if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM)) return rc;
   if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kTileN)) return rc;

@@ -1,0 +1,48 @@
+"""Kernel variants chosen by a rule on sizes, at the edges of their ranges, against the oracle or the two-kernel path."""
+import ctypes
+
+import pytest
+import torch
+
+from actlizela_b200.workloads import WORKLOADS, make_inputs
+from oracle import gdn_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 256, 8), (16, 264, 128), (17, 4096, 136), (32, 512, 2560), (33, 264, 264), (64, 4096, 128),
+                                   (65, 1032, 2560), (128, 4096, 2560), (129, 4096, 1288), (300, 512, 2560), (896, 4096, 2560),
+                                   (897, 4096, 2560)])
+def test_out_proj_with_few_rows(m, k, n):
+    """K split over a cluster: row counts at the edges of the 16/32/64/128-row tiles, ragged columns and K tails, and
+    both sides of the rule that goes back to one CTA per tile."""
+    from actlizela_b200 import out_proj_gemm
+    gen = torch.Generator().manual_seed(m * 1000 + n)
+    a = torch.randn(m, k, generator=gen).to(torch.bfloat16).cuda()
+    w = (torch.randn(n, k, generator=gen) * k ** -0.5).to(torch.bfloat16).cuda()
+    want = a.float() @ w.float().t()
+    got = out_proj_gemm(a, w)
+    assert got.shape == (m, n)
+    assert oracle.rel_frobenius(got.float().cpu(), want.cpu()) < 3e-3
+    assert oracle.max_abs(got.float(), want) <= 2 ** -8 * float(want.abs().max()) + 1e-6
+    assert torch.equal(got, out_proj_gemm(a, w))                  # the sum over the cluster has one order
+
+
+@pytest.mark.parametrize("batch,length,hk,hv,parallel", [(1, 1, 1, 1, 1), (1, 64, 2, 6, 1), (3, 129, 1, 2, 1), (2, 193, 1, 4, 3),
+                                                         (5, 700, 8, 32, 1), (1, 64 * 40 + 1, 1, 2, 8), (300, 65, 1, 1, 1)])
+def test_single_launch_form_equals_the_two_kernels_bitwise(batch, length, hk, hv, parallel, native_library):
+    """One chunk, two, odd and even chunk counts, tails, several work items per CTA (more heads than SMs), more
+    sub-segments than chunks would allow; the states and every output row have the bits of the two-kernel path."""
+    from actlizela_b200.sm100 import Sm100Forward
+    forward = Sm100Forward(native_library)
+    w = WORKLOADS["cfg1"].sliced(batch=batch, length=length, key_heads=hk, value_heads=hv, seed=4000 + length)
+    dev = [x.cuda() for x in make_inputs(w)]
+    suffix = "" if parallel == 1 else f"-par{parallel}"
+    want_out, want_state = forward(*dev, True, configuration="umma" + suffix)
+    out, state = forward(*dev, True, configuration="fused" + suffix)
+    torch.cuda.synchronize()
+    status = (ctypes.c_int * 4)()
+    assert native_library.lib.actlize_la_sm100_device_status(status, 1) == 0 and status[0] == 0
+    assert torch.equal(out, want_out) and torch.equal(state, want_state)
+    out_only, none = forward(*dev, False, configuration="fused" + suffix)
+    assert none is None and torch.equal(out_only, want_out)
