@@ -21,18 +21,19 @@ __device__ long long g_stamps[4][64][16], g_blocks[1024][2];
 #define STAMP(role, n, slot)
 #endif
 
-// Warps (24):
+// Warps (32, 64 registers a thread):
 //    0      issuer of the chain's tensor-core products
 //    1      planner (work items of this CTA) and TMA producer
-//    2-3    query scaling
+//    2      query scaling
+//    3      gates: prefix sums and exponentials of the coming chunks
 //    4-11   state chain
 //    12-15  W operand (W^T accumulator -> hi/lo tiles) and output
-//    16-19, 20-23  two prepare groups: even and odd chunks of the CTA's stream.  The phases of a chunk's preparation
+//    16-23, 24-31  two prepare groups: even and odd chunks of the CTA's stream.  The phases of a chunk's preparation
 //           are serial and latency bound (about two chunk periods long), so two chunks are in preparation at a time.
 // All roles share one instruction cache of some tens of KB: with every loop unrolled (134 KB of code) a chunk took
 // twice as long, bound by instruction fetches from the cache that the SMs of a GPC share.  Loops are therefore rolled
 // unless a loop's registers need otherwise, and waits call one polling routine.
-constexpr int kThreads = 768;
+constexpr int kThreads = 1024, kPrepThreads = 256;
 constexpr int kIssueWarp = 0, kPlanWarp = 1, kScaleWarp = 2, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
 constexpr int kRing = 3;      // Q/K tiles, P tiles, gate vectors: one chunk in the chain, two in preparation
 constexpr int kItems = 4;     // work items announced ahead
@@ -49,10 +50,11 @@ struct Smem {
   static constexpr int kATBytes = 64 * kLd * 4;
   static constexpr int kAT = kP + kRing * kBox;                   // per group: A, then T in place, then T_u hi | lo
   static constexpr int kTw = kAT + 2 * kATBytes;                  // T diag(beta exp p) hi | lo
-  static constexpr int kGates = kTw + 2 * kBox;                   // ring of gate vectors (kGateWords floats)
-  static constexpr int kPriv = kGates + kRing * kGateWords * 4;   // per group: pl2, beta, beta exp(p),
-  static constexpr int kPrivWords = 3 * 64 + 32;                  // and the column factors of the block off the diagonal
-  static constexpr int kItem = kPriv + 2 * kPrivWords * 4;        // item ring, 16 words each
+  // ring of gate vectors: exp(p_last - p_i), exp(p_last), [kGateQueryScale, +64) exp(p_i) / sqrt(128), then p_i log2(e),
+  // beta, beta exp(p), and the column factors exp(p_31 - p_j) of the block off the diagonal
+  static constexpr int kGates = kTw + 2 * kBox;
+  static constexpr int kPl2 = kGateWords, kBeta = kPl2 + 64, kCoefW = kBeta + 64, kECol = kCoefW + 64, kGateStage = kECol + 32;
+  static constexpr int kItem = kGates + kRing * kGateStage * 4;   // item ring, 16 words each
   static constexpr int kBars = kItem + kItems * 64;
   static constexpr int kTotal = kBars + 512;
   static_assert(kATBytes % 1024 == 0 && kAT % 1024 == 0 && kTw % 1024 == 0, "swizzled tiles start on 1024 bytes");
@@ -72,24 +74,25 @@ enum ItemWord { kChunks, kBatch, kHv, kFirst, kEnd, kUnstored, kState, kFlags, k
 constexpr int kHasInitial = 1, kHasFinal = 2;
 
 struct Barriers {
-  uint64_t kq_full[kRing], kq_free[kRing], qs_go[kRing], qs_done[kRing];
+  uint64_t kq_full[kRing], kq_free[kRing], g_ready[kRing], qs_go[kRing], qs_done[kRing];
   uint64_t v_full, w, w_ready, ws, s, o, ofree;
   uint64_t t_ready[2], u[2], d[2], ops[2], opn[2];
   uint64_t item_full[kItems], item_free[kItems];
   uint32_t tmem;
   int abort;
   int lock, released;
+  int reach[8];
 };
 static_assert(sizeof(Barriers) <= 512, "barrier block");
 constexpr int kItemReaders = kThreads / 32 - 1;      // every warp but the planner reads the items
 
-__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
-// Barrier of 128 threads that also tells every thread whether all of them are healthy: whoever leaves a loop that
+__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kPrepThreads) : "memory"); }
+// Barrier of a prepare group that also tells every thread whether all of them are healthy: whoever leaves a loop that
 // holds such barriers does it on this answer, so that no thread is left waiting in one.
 __device__ __forceinline__ bool group_all(int id, bool ok) {
   uint32_t all;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-               : "=r"(all) : "r"(uint32_t(ok)), "r"(id) : "memory");
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"(uint32_t(ok)), "r"(id), "n"(kPrepThreads) : "memory");
   return all != 0;
 }
 
@@ -97,12 +100,13 @@ __device__ __forceinline__ uint8_t* shared_base() {
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   return raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);      // (no integer round trip: stays in the shared space)
 }
-// Bounded waits as in umma.cuh, with a polling routine that takes two arguments: a wait is in nearly fifty places of this
-// kernel.  The record names the warp (100 + warp).
+// Bounded waits as in umma.cuh, with a polling routine that takes two arguments and loads nothing: a wait is in nearly
+// fifty places of this kernel.  The record names the warp (100 + warp).
+constexpr uint32_t kPolls = 1u << 20;
 __device__ __noinline__ bool fused_wait_poll(uint32_t bar_addr, uint32_t parity) {
   const AbortFlag abort{&reinterpret_cast<Barriers*>(shared_base() + Smem::kBars)->abort};
-  const uint32_t limit = g_spin_limit;
-  for (uint32_t spin = 0; spin < limit; ++spin) {
+#pragma unroll 1
+  for (uint32_t spin = 0; spin < kPolls; ++spin) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(bar_addr), "r"(parity) : "memory");
@@ -118,18 +122,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 }
 // for a place with many live registers: no call (a wait that runs out here is recorded by the roles that then run out too)
 __device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spin = 0; spin < (1u << 20); ++spin)
+  for (uint32_t spin = 0; spin < kPolls; ++spin)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
 // wait with one answer for the whole warp
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
-// ACC_D's lock: taken by the thread that issues into it, given back by the last of the four warps that have read it.
+// ACC_D's lock: taken by the thread that issues into it, given back by the last of the `readers` warps that read it.
 __device__ __noinline__ void acc_lock(Barriers* bar) {
   const AbortFlag abort{&bar->abort};
-  const uint32_t limit = g_spin_limit;
-  for (uint32_t spin = 0; spin < limit; ++spin) {
+#pragma unroll 1
+  for (uint32_t spin = 0; spin < kPolls; ++spin) {
     if (atomicCAS(&bar->lock, 0, 1) == 0) {
       __threadfence_block();
       return;
@@ -138,12 +142,12 @@ __device__ __noinline__ void acc_lock(Barriers* bar) {
   }
   abort.raise(1, 100 + (threadIdx.x >> 5), 0);
 }
-__device__ __forceinline__ void acc_release(Barriers* bar, int lane) {
+__device__ __forceinline__ void acc_release(Barriers* bar, int lane, int readers) {
   tc_fence_before();
   __syncwarp();
   if (lane == 0) {
     __threadfence_block();
-    if (atomicAdd(&bar->released, 1) == 3) {
+    if (atomicAdd(&bar->released, 1) == readers - 1) {
       bar->released = 0;
       __threadfence_block();
       atomicExch(&bar->lock, 0);
@@ -157,34 +161,12 @@ __device__ __forceinline__ float raw_gate(const Inputs& in, uint32_t bits, int h
   const float z = bf16_lo(bits) + in.dt_bias[hv];
   return -expf(in.a_log[hv]) * (z > 20.f ? z : log1pf(expf(z)));
 }
-// A thread's gate and beta of a chunk as loaded (converted where they are used, so that the loads stay in flight):
-// `gate`, `beta` of token t, `lead` of token t - 32 for the threads of the second half
-struct GateLoads {
-  uint32_t gate = 0, beta = 0, lead = 0;
-  bool loaded = false;
-  __device__ __forceinline__ static float as_gate(uint32_t bits, int fp32) { return fp32 ? __uint_as_float(bits) : bf16_lo(bits); }
-  template <bool kRaw>
-  __device__ __forceinline__ static uint32_t gate_bits(const Inputs& in, long long gi) {
-    if (kRaw) return bf16_bits(in.act_a + gi);
-    return in.gate_fp32 ? static_cast<const uint32_t*>(in.g)[gi] : bf16_bits(static_cast<const __nv_bfloat16*>(in.g) + gi);
-  }
-  template <bool kRaw>
-  __device__ __forceinline__ void load(const Inputs& in, const Geometry& geo, int b, int hv, int t0, int valid, int t) {
-    const long long at = ((long long)b * geo.sequence + t0 + t) * geo.value_heads + hv;
-    if (t < valid) {
-      gate = gate_bits<kRaw>(in, at);
-      beta = bf16_bits((kRaw ? in.act_b : in.beta) + at);
-    }
-    if (t >= 32 && t - 32 < valid) lead = gate_bits<kRaw>(in, at - 32LL * geo.value_heads);
-  }
-};
-
 // First chunk boundary of a range at which the decay accumulated since its start is below exp(-40): number of leading
 // chunks an incoming state still reaches (1..count), or -1 when the decay never gets that far.  Sums the gates
 // themselves, eight chunks (sixteen loads per lane) at a time; it stops at the boundary, so a typical gate costs one
 // step.  Warp-collective; every caller with the same range gets the same answer.
 template <bool kRaw>
-__device__ int gate_reach(const Inputs& in, const Geometry& geo, int b, int hv, int first_token, int count, int t_end, int lane) {
+__device__ __noinline__ int gate_reach(const Inputs& in, const Geometry& geo, int b, int hv, int first_token, int count, int t_end, int lane) {
   float total = 0.f;
   for (int c0 = 0; c0 < count; c0 += 8) {
     float x[8];
@@ -214,21 +196,21 @@ __device__ int gate_reach(const Inputs& in, const Geometry& geo, int b, int hv, 
   return -1;
 }
 
-// 32 columns of row `row`, scaled per column by `coef`, as BF16 hi/lo pieces of a K-major swizzled tile pair (the lo tile
+// 16 columns of row `row`, scaled per column by `coef`, as BF16 hi/lo pieces of a K-major swizzled tile pair (the lo tile
 // one box behind); `first` = first 16-byte piece of the row
-__device__ __forceinline__ void scaled_row(const float4 (&x)[8], const float* coef, uint8_t* tile_row, int first, int row) {
+__device__ __forceinline__ void scaled_row(const float4 (&x)[4], const float* coef, uint8_t* tile_row, int first, int row) {
+  float4 f[4];
 #pragma unroll
-  for (int g8 = 0; g8 < 4; ++g8) {
-    float4 f[2];
+  for (int q4 = 0; q4 < 4; ++q4) f[q4] = *reinterpret_cast<const float4*>(coef + q4 * 4);
+#pragma unroll
+  for (int g8 = 0; g8 < 2; ++g8) {
     uint32_t hi[4], lo[4];
 #pragma unroll
-    for (int q4 = 0; q4 < 2; ++q4) f[q4] = *reinterpret_cast<const float4*>(coef + g8 * 8 + q4 * 4);
-#pragma unroll
     for (int q4 = 0; q4 < 2; ++q4) {
-      const float4 y = x[g8 * 2 + q4];
+      const float4 y = x[g8 * 2 + q4], c = f[g8 * 2 + q4];
       float a0, a1, b0, b1;
-      mul2(a0, a1, y.x, y.y, f[q4].x, f[q4].y);
-      mul2(b0, b1, y.z, y.w, f[q4].z, f[q4].w);
+      mul2(a0, a1, y.x, y.y, c.x, c.y);
+      mul2(b0, b1, y.z, y.w, c.z, c.w);
       split_pair(a0, a1, hi[q4 * 2], lo[q4 * 2]);
       split_pair(b0, b1, hi[q4 * 2 + 1], lo[q4 * 2 + 1]);
     }
@@ -263,37 +245,30 @@ struct Plan {
 };
 
 // ---------------------------------------------------------------------------------------------------- prepare groups
-// Four warps prepare one chunk; the phases are those of prepare_umma_kernel with half the threads.
-//   row = TMEM lane = warp * 32 + lane: rows 0..63 are Q rows (P), 64..127 K rows (A)
+// Eight warps prepare one chunk; the phases are those of prepare_umma_kernel.  A warp owns the TMEM lane quarter
+// (warp & 3) and the column half (warp >> 2): quarters 0, 1 are Q rows (P), 2, 3 K rows (A).
 template <bool kRaw>
-__device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const Inputs& in, const Geometry& geo, int group,
-                                              int n, int b, int hv, int t0, int t_next, int t_end, GateLoads& next,
-                                              bool& not_contraction) {
+__device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int group,
+                                              int n, bool& not_contraction) {
   using L = Smem;
-  const int t = threadIdx.x & 127, warp = t >> 5, lane = t & 31, id = 1 + group;
-  const int s = n % kRing, valid = min(kChunk, t_end - t0);
+  const int t = threadIdx.x & (kPrepThreads - 1), warp = t >> 5, lane = t & 31, id = 1 + group;
+  const int s = n % kRing;
   uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
   uint8_t* tile_p = sm + L::kP + s * kBox;
   float* sAT = reinterpret_cast<float*>(sm + L::kAT + group * L::kATBytes);
-  float* gates = reinterpret_cast<float*>(sm + L::kGates) + s * kGateWords;
-  float* s_pl2 = reinterpret_cast<float*>(sm + L::kPriv) + group * L::kPrivWords;
-  float* s_beta = s_pl2 + 64;
-  float* s_coefw = s_beta + 64;
-  float* s_ecol = s_coefw + 64;
+  const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + s * L::kGateStage;
+  const float *s_pl2 = gates + L::kPl2, *s_beta = gates + L::kBeta, *s_coefw = gates + L::kCoefW, *s_ecol = gates + L::kECol;
 
-  if (t == 96) STAMP(0, n, 0);
-  // gates and betas: warps 0 and 1 own tokens 0..31 and 32..63; warp 1 also scans the first half, whose total it adds.
-  // They were asked for while the group's previous chunk was prepared (the first of an item: here).
-  if (warp < 2 && !next.loaded) next.load<kRaw>(in, geo, b, hv, t0, valid, t);
+  if (t == 224) STAMP(0, n, 0);
   bool ok = warp_wait(&bar->kq_full[s], (n / kRing) & 1) && !AbortFlag{&bar->abort}.raised();
-  if (t == 96) STAMP(0, n, 1);
+  if (t == 224) STAMP(0, n, 1);
   if (kRaw) {
-    // L2-normalise the 64 Q and 64 K rows in place: 16 lanes per row (one swizzled 16-byte slot each), 8 rows per pass
+    // L2-normalise the 64 Q and 64 K rows in place: 16 lanes per row (one swizzled 16-byte slot each), 16 rows per pass
     if (ok) {
       const int lane16 = t & 15;
-#pragma unroll 2
-      for (int pass = 0; pass < 16; ++pass) {
-        const int r = pass * 8 + (t >> 4), row = r & 63;
+#pragma unroll 1
+      for (int pass = 0; pass < 8; ++pass) {
+        const int r = pass * 16 + (t >> 4), row = r & 63;
         uint8_t* slot = kq + (r < 64 ? (lane16 < 8 ? L::kQ0 : L::kQ1) : (lane16 < 8 ? L::kK0 : L::kK1)) + row * 128 +
                         (((lane16 & 7) ^ (row & 7)) << 4);
         const uint4 x = *reinterpret_cast<const uint4*>(slot);
@@ -312,84 +287,59 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
     }
     group_sync(id);
   }
-  if (warp == 3 && ok) {
+  if (warp == 7 && ok) {
     const uint64_t a = smem_desc(smem_u32(kq) + L::kQ0, 16, 1024), x = smem_desc(smem_u32(kq) + L::kK0, 16, 1024);
     if (elect_one()) {
       acc_lock(bar);
       tc_fence_after();
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const uint64_t at = h * (L::kQ1 - L::kQ0) / 16;
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint64_t at = (ks >> 2) * (L::kQ1 - L::kQ0) / 16 + (ks & 3) * 2;
-        mma_ss(kAccD, a + at, x + at, kIdescN64, ks > 0);
+        for (int ks = 0; ks < 4; ++ks) mma_ss(kAccD, a + at + uint64_t(ks * 2), x + at + uint64_t(ks * 2), kIdescN64, (h | ks) != 0);
       }
       mma_commit(&bar->d[group]);
     }
   }
   __syncwarp();
-  if (warp < 2) {
-    float gate = 0.f, beta = 0.f, lead = 0.f;
-    if (t < valid) {
-      gate = kRaw ? raw_gate(in, next.gate, hv) : next.as_gate(next.gate, in.gate_fp32);
-      beta = kRaw ? __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-bf16_lo(next.beta))))) : bf16_lo(next.beta);
-    }
-    if (warp == 1 && lane < valid) lead = kRaw ? raw_gate(in, next.lead, hv) : next.as_gate(next.lead, in.gate_fp32);
-    next.loaded = t_next >= 0;
-    if (next.loaded) next.load<kRaw>(in, geo, b, hv, t_next, min(kChunk, t_end - t_next), t);
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const float y = __shfl_up_sync(0xffffffffu, gate, d), z = __shfl_up_sync(0xffffffffu, lead, d);
-      if (lane >= d) {
-        gate += y;
-        lead += z;
-      }
-    }
-    const float carry = __shfl_sync(0xffffffffu, lead, 31);
-    if (warp == 1) gate += carry;
-    const float e = exp2f(gate * kLog2e), pl2 = gate * kLog2e;
-    s_pl2[t] = pl2;
-    s_beta[t] = beta;
-    s_coefw[t] = beta * e;
-    gates[kGateQueryScale + t] = e * kScale;
-    const float pl2_31 = __shfl_sync(0xffffffffu, pl2, 31);
-    if (warp == 0) s_ecol[t] = fast_exp2(pl2_31 - pl2);
-  }
+  ok = warp_wait(&bar->g_ready[s], (n / kRing) & 1) && ok;
   ok = group_all(id, ok);
   if (!ok) return false;
 
   // ---- masks and decays on [Q;K] K^T
   ok = warp_wait(&bar->d[group], (n >> 1) & 1);
-  if (t == 96) STAMP(0, n, 2);
+  if (t == 224) STAMP(0, n, 2);
   tc_fence_after();
   if (lane == 0) mbar_arrive(&bar->qs_go[s]);
-  const int i = t & 63;
-  const uint32_t taddr = (uint32_t(warp * 32) << 16) + kAccD;
+  const int quarter = warp & 3, half = warp >> 2, i = (quarter & 1) * 32 + lane;
+  const uint32_t taddr = (uint32_t(quarter * 32) << 16) + kAccD;
   bool bad = false;
-  // Per 32-column half that reaches the diagonal of this warp's rows: all loads, then the arithmetic in place, then the
-  // stores (loads behind stores to the same memory would each wait for them).  Nothing is masked element by element:
-  // of A only what the solves and products read has to be right (they do not read above the diagonal of a 16x16 block),
-  // and of P the one 16-byte piece per row that holds the diagonal is cut afterwards.  In the half that lies off the
-  // diagonal (rows 32.., columns ..31) exp(p_i - p_j) = exp(p_i - p_31) exp(p_31 - p_j): a factor per row and one per
-  // column (an exponential takes the special-function unit eight cycles per warp).
-  const int halves = (warp & 1) + 1;
+  // Per 16-column piece: all loads, then the arithmetic in place, then the stores (loads behind stores to the same memory
+  // would each wait for them).  Nothing is masked element by element: of A only what the solves and products read has to
+  // be right (they do not read above the diagonal of a 16x16 block), and of P the one 16-byte piece per row that holds
+  // the diagonal is cut afterwards.  In the block off the diagonal (rows 32.., columns ..31)
+  // exp(p_i - p_j) = exp(p_i - p_31) exp(p_31 - p_j): a factor per row and one per column (an exponential takes the
+  // special-function unit eight cycles per warp).
+  const bool diagonal = half == (quarter & 1), below = half < (quarter & 1);      // else above: nothing there
   const float pi = s_pl2[i], bi = s_beta[i];
   // A takes the place of the T_u pair of this group's previous chunk, which U was formed from as that chunk began
-  if (warp >= 2 && n >= 2) ok = warp_wait(&bar->u[group], ((n >> 1) - 1) & 1) && ok;
-  if (t == 96) STAMP(0, n, 3);
-  if (ok) {
-    float* arow = sAT + i * L::kLd;
+  if (quarter >= 2 && n >= 2) ok = warp_wait(&bar->u[group], ((n >> 1) - 1) & 1) && ok;
+  if (t == 224) STAMP(0, n, 3);
+  float* arow = sAT + i * L::kLd;
+  if (ok && (diagonal || below)) {
     uint8_t* prow = tile_p + i * 128;
+    const float f = below ? fast_exp2(pi - s_pl2[31]) * (quarter < 2 ? kScale : bi) : 0.f;
 #pragma unroll 1
-    for (int h = 0; h < halves; ++h) {
-      uint32_t d[32];
-      tmem_ld32(taddr + h * 32, d);
+    for (int h = half * 2; h < half * 2 + 2; ++h) {
+      uint32_t d[16];
+      tmem_ld16(taddr + h * 16, d);
       tmem_wait_ld();
-      if (h == halves - 1) acc_release(bar, lane);
-      const bool diagonal = h == halves - 1;
-      const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 32 : s_ecol);
-      const float last = warp < 2 ? kScale : 1.f, first = warp < 2 ? 1.f : bi;
+      if (h & 1) acc_release(bar, lane, 6);      // (the two warps above the diagonal read nothing)
+      const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 16 : s_ecol + h * 16);
+      const float last = quarter < 2 ? kScale : 1.f, first = quarter < 2 ? 1.f : bi;
       if (diagonal) {
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {
+        for (int q4 = 0; q4 < 4; ++q4) {
           const float4 p4 = pj[q4];
 #pragma unroll
           for (int e = 0; e < 4; e += 2) {
@@ -403,9 +353,8 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
           }
         }
       } else {
-        const float f = fast_exp2(pi - s_pl2[31]) * (warp < 2 ? kScale : bi);
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {
+        for (int q4 = 0; q4 < 4; ++q4) {
           const float4 p4 = pj[q4];
 #pragma unroll
           for (int e = 0; e < 4; e += 2) {
@@ -417,26 +366,26 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
           }
         }
       }
-      if (warp < 2) {
+      if (quarter < 2) {
 #pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8) {
+        for (int c8 = 0; c8 < 2; ++c8) {
           uint32_t packed[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) packed[e] = pack_bf16(__uint_as_float(d[c8 * 8 + 2 * e]), __uint_as_float(d[c8 * 8 + 2 * e + 1]));
-          *reinterpret_cast<uint4*>(prow + (((h * 4 + c8) ^ (i & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+          *reinterpret_cast<uint4*>(prow + (((h * 2 + c8) ^ (i & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
       } else {
         // the upper right 16x16 block of a 32x32 diagonal block is read as zeros
-        if (diagonal && !(i & 16)) {
+        if (diagonal && (h & 1) && !(i & 16)) {
 #pragma unroll
-          for (int e = 16; e < 32; ++e) d[e] = 0u;
+          for (int e = 0; e < 16; ++e) d[e] = 0u;
         }
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4)
-          *reinterpret_cast<uint4*>(arow + h * 32 + q4 * 4) = make_uint4(d[q4 * 4], d[q4 * 4 + 1], d[q4 * 4 + 2], d[q4 * 4 + 3]);
+        for (int q4 = 0; q4 < 4; ++q4)
+          *reinterpret_cast<uint4*>(arow + h * 16 + q4 * 4) = make_uint4(d[q4 * 4], d[q4 * 4 + 1], d[q4 * 4 + 2], d[q4 * 4 + 3]);
       }
     }
-    if (warp < 2) {
+    if (quarter < 2 && diagonal) {
       uint4* at = reinterpret_cast<uint4*>(prow + (((i >> 3) ^ (i & 7)) << 4));
       uint4 x = *at;
       const int keep = (i & 7) + 1;                       // columns of the piece on or below the diagonal, two to a word
@@ -450,24 +399,20 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
     }
     // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
     // (the diagonal of A as stored is beta_i |k_i|^2 exp(0))
-    if (warp >= 2) bad = !(bi >= 0.f && arow[i] <= 2.f);
+    if (quarter >= 2 && diagonal) bad = !(bi >= 0.f && arow[i] <= 2.f);
   }
   not_contraction |= __any_sync(0xffffffffu, bad);
-  if (warp < 2) {
-    const float last = s_pl2[valid - 1];
-    gates[t] = (t < valid) ? fast_exp2(last - s_pl2[t]) : 0.f;
-    if (t == 0) gates[kChunk] = fast_exp2(last);
-  }
-  if (t == 96) STAMP(0, n, 4);
+  if (t == 224) STAMP(0, n, 4);
 
   // ---- T = (I+A)^-1 in place, blocked 16 -> 32 -> 64
   // diagonal 16x16 solves, a column per thread (left-looking, in registers); the 16 threads of a block sit in one warp and
   // overwrite the block only after all of them have read it
-  // (warp 2 wrote rows 0..31 of A, warp 3 rows 32..63: each solves its own two blocks)
+  // (the two warps that wrote the diagonal 32x32 blocks of A solve the two 16x16 blocks in theirs)
   __syncwarp();
-  if (ok && warp >= 2) {
+  if (ok && quarter >= 2 && diagonal) {
     const int col = lane & 15;
-    float* a0 = sAT + (t & 48) * L::kLd + (t & 48);
+    const int o = (quarter & 1) * 32 + (lane & 16);
+    float* a0 = sAT + o * L::kLd + o;
     float x[16];
     float4 cur[4], nxt[4] = {};
 #pragma unroll
@@ -493,12 +438,12 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
     for (int r = 0; r < 16; ++r) a0[r * L::kLd + col] = x[r];
   }
   group_sync(id);
-  if (t == 96) STAMP(0, n, 5);
+  if (t == 224) STAMP(0, n, 5);
   // block products T21 = -T22 (A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
   // above the diagonal, which holds nothing
   {
     const int g = lane >> 2, tq = lane & 3;
-    const int big = warp >> 1, o = big * 32, col16 = (warp & 1) * 8;
+    const int big = (warp >> 1) & 1, o = big * 32, col16 = (warp & 1) * 8;
     float* x16 = sAT + (big * 16) * L::kLd + 32 + col16;
     const uint32_t frag = smem_u32(sAT) + fragment_row(lane, L::kLd) * 4;
 #pragma unroll 1
@@ -507,47 +452,44 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
       const float* right = (step ? x16 : sAT + o * L::kLd + o + col16) + tq * L::kLd + g;
       float* out = (step ? sAT + (o + 16) * L::kLd + o + col16 : x16) + g * L::kLd + 2 * tq;
       const float sign = step ? -1.f : 1.f;
-      float c[1][4] = {};
-      if (ok) {
+      float c[4];
+      if (ok && warp < 4) {
         tile_row_tf32x3(c, left, right, L::kLd, 16);
-        *reinterpret_cast<float2*>(out) = make_float2(sign * c[0][0], sign * c[0][1]);
-        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(sign * c[0][2], sign * c[0][3]);
+        *reinterpret_cast<float2*>(out) = make_float2(sign * c[0], sign * c[1]);
+        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(sign * c[2], sign * c[3]);
       }
       group_sync(id);
     }
-    // 32 wide: a warp takes one row half and sixteen columns
-    const int row16 = big * 16, col32 = (warp & 1) * 16;
+    // 32 wide: eight tiles, one per warp
+    const int row16 = (warp & 1) * 16, col32 = (warp >> 1) * 8;
 #pragma unroll 1
     for (int step = 0; step < 2; ++step) {
       const uint32_t left = frag + ((32 + row16) * L::kLd + step * 32) * 4;
       const float* right = sAT + step * 32 + col32 + tq * L::kLd + g;
       float* out = (step ? sAT + (32 + row16) * L::kLd + col32 : sAT + row16 * L::kLd + 32 + col32) + g * L::kLd + 2 * tq;
       const float sign = step ? -1.f : 1.f;
-      float c[2][4] = {};
+      float c[4];
       if (ok) {
         tile_row_tf32x3(c, left, right, L::kLd, 32);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          *reinterpret_cast<float2*>(out + q * 8) = make_float2(sign * c[q][0], sign * c[q][1]);
-          *reinterpret_cast<float2*>(out + q * 8 + 8 * L::kLd) = make_float2(sign * c[q][2], sign * c[q][3]);
-        }
+        *reinterpret_cast<float2*>(out) = make_float2(sign * c[0], sign * c[1]);
+        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(sign * c[2], sign * c[3]);
       }
       if (step == 0) group_sync(id);
     }
   }
-  if (t == 96) STAMP(0, n, 6);
+  if (t == 224) STAMP(0, n, 6);
   // T_w has one place: free once the previous chunk's W^T has been formed from it
   if (n >= 1) ok = warp_wait(&bar->w, (n - 1) & 1) && ok;
   group_sync(id);
-  if (t == 96) STAMP(0, n, 7);
-  // ---- T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row, 32 columns
+  if (t == 224) STAMP(0, n, 7);
+  // ---- T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row, 16 columns
   {
-    const int row = t & 63, c0 = (t >> 6) * 32;
-    const bool empty = c0 == 32 && row < 32;          // above the diagonal
+    const int row = t & 63, c0 = (t >> 6) * 16;
+    const bool empty = c0 >= 32 && row < 32;          // above the diagonal
     const float* trow = sAT + row * L::kLd + c0;
-    float4 x[8];
+    float4 x[4];
 #pragma unroll
-    for (int q4 = 0; q4 < 8; ++q4) {
+    for (int q4 = 0; q4 < 4; ++q4) {
       x[q4] = *reinterpret_cast<const float4*>(trow + q4 * 4);
       if (empty) x[q4] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -559,25 +501,9 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, const 
     fence_proxy_async_smem();
   }
   __syncwarp();
-  if (lane == 0) mbar_arrive(&bar->t_ready[group]);       // P, the gate vector and T_u of this chunk
-  ok = group_all(id, ok);
-  if (!ok) return false;
-  if (t == 96) STAMP(0, n, 8);
+  if (lane == 0) mbar_arrive(&bar->t_ready[group]);       // P, the gate vector, T_u and T_w of this chunk
+  if (t == 224) STAMP(0, n, 8);
 
-  // ---- W^T = K^T (T diag(beta exp p))^T: the output warps turn it into the hi/lo operand, this group goes on
-  if (warp == 3) {
-    const uint64_t a = smem_desc(smem_u32(kq) + L::kK0, L::kK1 - L::kK0, 1024), x = smem_desc(smem_u32(sm + L::kTw), 16, 1024);
-    if (elect_one()) {
-      acc_lock(bar);
-      tc_fence_after();
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        mma_ss(kAccD, a + uint64_t((ks & 3) * 128), x + uint64_t((ks >> 2) * (kBox / 16) + (ks & 3) * 2), kIdescN64AT, ks != 0);
-      mma_commit(&bar->w);
-    }
-  }
-  __syncwarp();
-  if (t == 96) STAMP(0, n, 9);
   return true;      // the same answer for the whole group; a wait that gave up shows at the next chunk's group_all
 }
 
@@ -595,18 +521,22 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (!plan.serial_pass && tid == 0) g_blocks[blockIdx.x][0] = clock64();
 #endif
   if (plan.serial_pass) {
+    // (launched while the first launch still ran: its flags and outputs are complete behind this wait)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     // nothing to repair for this CTA's heads: leave before anything is set up
     bool any = false;
     for (int unit = blockIdx.x; unit < plan.units; unit += gridDim.x)
       for (int r = 1; r < plan.parallel; ++r) any |= plan.flags[unit * plan.parallel + r] != 0;
     if (!any) return;
   }
+  if (plan.parallel > 1) asm volatile("griddepcontrol.launch_dependents;");
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) {
       mbar_init(&bar->kq_full[i], 1);
       mbar_init(&bar->kq_free[i], 1);
-      mbar_init(&bar->qs_go[i], 4);
-      mbar_init(&bar->qs_done[i], 2);
+      mbar_init(&bar->qs_go[i], 8);
+      mbar_init(&bar->qs_done[i], 1);
+      mbar_init(&bar->g_ready[i], 1);
     }
     mbar_init(&bar->v_full, 1);
     mbar_init(&bar->w, 1);
@@ -616,7 +546,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     mbar_init(&bar->o, 1);
     mbar_init(&bar->ofree, 4);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bar->t_ready[i], 4);
+      mbar_init(&bar->t_ready[i], 8);
       mbar_init(&bar->u[i], 1);
       mbar_init(&bar->d[i], 1);
       mbar_init(&bar->ops[i], 8);
@@ -632,6 +562,14 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (warp == kIssueWarp) {
     tmem_alloc(&bar->tmem, 512);
     tmem_relinquish();
+  }
+  if (!plan.serial_pass && warp >= kChainWarp && warp - kChainWarp + 1 < plan.parallel) {
+    // the decay reaches of the first item's sub-segments, one warp each (usually the CTA's only item)
+    const int r = warp - kChainWarp + 1, bh = blockIdx.x / plan.parallel, n = geo.segment_chunks();
+    const int c0 = sub_segment_begin(n, r, plan.parallel), c1 = sub_segment_begin(n, r + 1, plan.parallel);
+    const int reach = gate_reach<kRaw>(in, geo, bh / geo.value_heads, bh % geo.value_heads, (geo.chunk_begin + c0) * kChunk,
+                                       c1 - c0, geo.sequence, lane);
+    if (lane == 0) bar->reach[r] = reach;
   }
   tc_fence_before();
   __syncthreads();
@@ -703,7 +641,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           int mine = 0, next = 0;
           for (int r = 1; r < parallel && !serial; ++r) {
             const int c0 = sub_segment_begin(chunks, r, parallel), c1 = sub_segment_begin(chunks, r + 1, parallel);
-            const int reach = gate_reach<kRaw>(in, geo, b, hv, t_first + c0 * kChunk, c1 - c0, t_end, lane);
+            const int reach = unit == blockIdx.x ? bar->reach[r] :
+                              gate_reach<kRaw>(in, geo, b, hv, t_first + c0 * kChunk, c1 - c0, t_end, lane);
             serial = reach < 0;
             if (r == sub) mine = reach;
             if (r == sub + 1) next = reach;
@@ -805,9 +744,12 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         const uint64_t dU = smem_desc(base + L::kAT + par * L::kATBytes, 16, 1024);
         if (elect_one()) {
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            mma_ss(kAccU, dV + uint64_t((ks & 3) * 128), dU + uint64_t((ks >> 2) * (kBox >> 4) + (ks & 3) * 2), kIdescN64AT, ks != 0);
+            for (int ks = 0; ks < 4; ++ks)
+              mma_ss(kAccU, dV + uint64_t(ks * 128), dU + uint64_t(h * (kBox >> 4) + ks * 2), kIdescN64AT, (h | ks) != 0);
+          }
           mma_commit(&bar->u[par]);
         }
         ok &= mbar_wait(&bar->w_ready, par);
@@ -838,9 +780,12 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         const uint64_t qd = smem_desc(kq + L::kQ0, 16, 1024);
         if (elect_one()) {
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            mma_ts(kAccO, kOpSH + ks * 8, qd + uint64_t((ks >> 2) * (L::kQ1 - L::kQ0) / 16 + (ks & 3) * 2), kIdescN64, ks != 0);
+            for (int ks = 0; ks < 4; ++ks)
+              mma_ts(kAccO, kOpSH + h * 32 + ks * 8, qd + uint64_t(h * (L::kQ1 - L::kQ0) / 16 + ks * 2), kIdescN64, (h | ks) != 0);
+          }
         }
         // St += (N*rel)^T K (the accumulator already holds gamma * St); token groups {0,2} first, {1,3} second
         const uint64_t kd = smem_desc(kq + L::kK0, L::kK1 - L::kK0, 1024), pd = smem_desc(base + L::kP + s * kBox, 16, 1024);
@@ -872,41 +817,88 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp < kChainWarp) {
-    // ------------------------------------------------------------------ query scaling
+    // ------------------------------------------------------------------ query scaling; gates
     ItemCursor cursor;
     int n = 0;
-    const int t64 = tid - kScaleWarp * 32;
 #pragma unroll 1
     for (bool ok = true; ok;) {
       const int* item = cursor.open(sm, bar, ok);
       if (!ok) break;
-      const int chunks = item[kChunks];
+      const int chunks = item[kChunks], b = item[kBatch], hv = item[kHv], t_first = item[kFirst], t_end = item[kEnd];
       cursor.close(bar, lane);
       if (chunks < 0) break;
 #pragma unroll 1
       for (int c = 0; c < chunks && ok; ++c, ++n) {
         const int s = n % kRing;
-        ok = warp_wait(&bar->qs_go[s], (n / kRing) & 1);
-        if (!ok) break;
-        uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
-        const float* scale = reinterpret_cast<const float*>(sm + L::kGates) + s * kGateWords + kGateQueryScale;
+        float* gates = reinterpret_cast<float*>(sm + L::kGates) + s * L::kGateStage;
+        if (warp == kScaleWarp) {
+          ok = warp_wait(&bar->qs_go[s], (n / kRing) & 1);
+          if (!ok) break;
+          uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
+          const float* scale = gates + kGateQueryScale;
 #pragma unroll 2
-        for (int it = 0; it < 16; ++it) {
-          const int piece = it * 64 + t64, row = piece >> 4, col16 = piece & 15;
-          uint4* at = reinterpret_cast<uint4*>(kq + (col16 < 8 ? L::kQ0 : L::kQ1) + row * 128 + (((col16 & 7) ^ (row & 7)) << 4));
-          const float f = scale[row];
-          const uint4 x = *at;
-          uint4 o;
-          o.x = pack_bf16(bf16_lo(x.x) * f, bf16_hi(x.x) * f);
-          o.y = pack_bf16(bf16_lo(x.y) * f, bf16_hi(x.y) * f);
-          o.z = pack_bf16(bf16_lo(x.z) * f, bf16_hi(x.z) * f);
-          o.w = pack_bf16(bf16_lo(x.w) * f, bf16_hi(x.w) * f);
-          *at = o;
+          for (int it = 0; it < 32; ++it) {
+            const int piece = it * 32 + lane, row = piece >> 4, col16 = piece & 15;
+            uint4* at = reinterpret_cast<uint4*>(kq + (col16 < 8 ? L::kQ0 : L::kQ1) + row * 128 + (((col16 & 7) ^ (row & 7)) << 4));
+            const float f = scale[row];
+            const uint4 x = *at;
+            uint4 o;
+            o.x = pack_bf16(bf16_lo(x.x) * f, bf16_hi(x.x) * f);
+            o.y = pack_bf16(bf16_lo(x.y) * f, bf16_hi(x.y) * f);
+            o.z = pack_bf16(bf16_lo(x.z) * f, bf16_hi(x.z) * f);
+            o.w = pack_bf16(bf16_lo(x.w) * f, bf16_hi(x.w) * f);
+            *at = o;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar->qs_done[s]);
+        } else {
+          // tokens lane and lane + 32: two scans, the second half then adds the first half's total
+          const int t0 = t_first + c * kChunk, valid = min(kChunk, t_end - t0);
+          const long long at = ((long long)b * geo.sequence + t0 + lane) * geo.value_heads + hv;
+          float g[2], beta[2], p[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            g[h] = beta[h] = 0.f;
+            if (h * 32 + lane < valid) {
+              const long long gi = at + h * 32LL * geo.value_heads;
+              g[h] = kRaw ? raw_gate(in, bf16_bits(in.act_a + gi), hv) : load_gate(in.g, gi, in.gate_fp32);
+              beta[h] = __bfloat162float(kRaw ? __float2bfloat16_rn(1.f / (1.f + expf(-__bfloat162float(in.act_b[gi])))) : in.beta[gi]);
+            }
+          }
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const float y = __shfl_up_sync(0xffffffffu, g[0], d), z = __shfl_up_sync(0xffffffffu, g[1], d);
+            if (lane >= d) {
+              g[0] += y;
+              g[1] += z;
+            }
+          }
+          g[1] += __shfl_sync(0xffffffffu, g[0], 31);
+          p[0] = g[0] * kLog2e;
+          p[1] = g[1] * kLog2e;
+          const float last = __shfl_sync(0xffffffffu, valid > 32 ? p[1] : p[0], (valid - 1) & 31);
+          const float p31 = __shfl_sync(0xffffffffu, p[0], 31);
+          // the stage is free once the chain has left the chunk that used it
+          if (n >= kRing) ok = warp_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1);
+          if (!ok) break;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int t = h * 32 + lane;
+            const float e = exp2f(p[h]);
+            gates[t] = t < valid ? fast_exp2(last - p[h]) : 0.f;
+            gates[kGateQueryScale + t] = e * kScale;
+            gates[L::kPl2 + t] = p[h];
+            gates[L::kBeta + t] = beta[h];
+            gates[L::kCoefW + t] = beta[h] * e;
+          }
+          gates[L::kECol + lane] = fast_exp2(p31 - p[0]);
+          if (lane == 0) gates[kChunk] = fast_exp2(last);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar->g_ready[s]);
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar->qs_done[s]);
       }
+      ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp < kOutWarp) {
     // ------------------------------------------------------------------ state chain
@@ -925,19 +917,19 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       {
         const float* init = (flags & kHasInitial) ? in.initial + (long long)bh * kDim * kDim + v : nullptr;
 #pragma unroll 1
-        for (int part = 0; part < 2; ++part) {
-          uint32_t vals[32];
-          const int k0 = half * 64 + part * 32;
+        for (int part = 0; part < 4; ++part) {
+          uint32_t vals[16];
+          const int k0 = half * 64 + part * 16;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) vals[j] = init ? __float_as_uint(init[(k0 + j) * kDim]) : 0u;
-          tmem_st32(taddr + kAccS + k0, vals);
+          for (int j = 0; j < 16; ++j) vals[j] = init ? __float_as_uint(init[(k0 + j) * kDim]) : 0u;
+          tmem_st16(taddr + kAccS + k0, vals);
         }
         tmem_wait_st();
       }
 #pragma unroll 1
       for (int c = 0; c < chunks && ok; ++c, ++n) {
         const int par = n & 1;
-        const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + (n % kRing) * kGateWords;
+        const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + (n % kRing) * L::kGateStage;
         ok = mbar_wait(&bar->w_ready, par);            // (the gate vector comes with it)
         if (tid == 128) STAMP(1, n, 0);
         if (n > 0) ok = ok && mbar_wait(&bar->s, (n - 1) & 1);
@@ -946,13 +938,13 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         const float gamma = gates[kChunk];
 #pragma unroll 1
-        for (int part = 0; part < 2; ++part) {
-          uint32_t d[32], hi[16], lo[16];
-          const int k0 = half * 64 + part * 32;
-          tmem_ld32(taddr + kAccS + k0, d);
+        for (int part = 0; part < 4; ++part) {
+          uint32_t d[16], hi[8], lo[8];
+          const int k0 = half * 64 + part * 16;
+          tmem_ld16(taddr + kAccS + k0, d);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
+          for (int j = 0; j < 16; j += 2) {
             const float s0 = __uint_as_float(d[j]), s1 = __uint_as_float(d[j + 1]);
             split_pair(s0, s1, hi[j >> 1], lo[j >> 1]);
             float g0, g1;
@@ -960,15 +952,17 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             d[j] = __float_as_uint(g0);
             d[j + 1] = __float_as_uint(g1);
           }
-          tmem_st16(taddr + kOpSH + (k0 >> 1), hi);
-          tmem_st32(taddr + kAccS + k0, d);
+          tmem_st8(taddr + kOpSH + (k0 >> 1), hi);
+          tmem_st16(taddr + kAccS + k0, d);
           // P N of the previous chunk reads its N from the columns of the lo operand
           if (n > 0 && part == 0) ok = mbar_wait_inline(&bar->o, (n - 1) & 1);
-          tmem_st16(taddr + kOpSL + (k0 >> 1), lo);
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar->ops[part]);
+          tmem_st8(taddr + kOpSL + (k0 >> 1), lo);
+          if (part & 1) {
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar->ops[part >> 1]);
+          }
         }
         if (tid == 128) STAMP(1, n, 2);
         ok = ok && mbar_wait(&bar->ws, par);
@@ -1007,13 +1001,13 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         float* fin = in.final_state + (long long)bh * kDim * kDim + v;
 #pragma unroll 1
-        for (int part = 0; part < 2; ++part) {
-          uint32_t d[32];
-          const int k0 = half * 64 + part * 32;
-          tmem_ld32(taddr + kAccS + k0, d);
+        for (int part = 0; part < 4; ++part) {
+          uint32_t d[16];
+          const int k0 = half * 64 + part * 16;
+          tmem_ld16(taddr + kAccS + k0, d);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) fin[(k0 + j) * kDim] = __uint_as_float(d[j]);
+          for (int j = 0; j < 16; ++j) fin[(k0 + j) * kDim] = __uint_as_float(d[j]);
         }
       }
       ok = __all_sync(0xffffffffu, ok);
@@ -1047,26 +1041,43 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       const bool end = chunks < 0;
       if (!end) {
-        ok = warp_wait(&bar->w, n & 1);
-        ok = warp_wait(&bar->t_ready[n & 1], (n >> 1) & 1) && ok;         // what it announces is passed on with W
+        ok = warp_wait(&bar->t_ready[n & 1], (n >> 1) & 1);                // (what it announces is passed on with W)
+        if (warp == kOutWarp) {
+          // W^T = K^T (T diag(beta exp p))^T; issued here so that the prepare group does not wait for the accumulator
+          const uint64_t a = smem_desc(smem_u32(sm) + L::kKQ + (n % kRing) * L::kKQStage + L::kK0, L::kK1 - L::kK0, 1024);
+          const uint64_t x = smem_desc(smem_u32(sm) + L::kTw, 16, 1024);
+          if (elect_one()) {
+            acc_lock(bar);
+            tc_fence_after();
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks)
+                mma_ss(kAccD, a + uint64_t(ks * 128), x + uint64_t(h * (kBox / 16) + ks * 2), kIdescN64AT, (h | ks) != 0);
+            }
+            mma_commit(&bar->w);
+          }
+          __syncwarp();
+        }
+        ok = warp_wait(&bar->w, n & 1) && ok;
         if (n > 0) ok = warp_wait(&bar->ws, (n - 1) & 1) && ok;            // W of the previous chunk has been read
         tc_fence_after();
         if (!ok) break;
         const int key = quarter * 32 + lane;
         uint8_t* wt = sm + L::kW + key * 128;
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          uint32_t dw[32];
-          tmem_ld32(lanes + kAccD + h * 32, dw);
+        for (int h = 0; h < 4; ++h) {
+          uint32_t dw[16];
+          tmem_ld16(lanes + kAccD + h * 16, dw);
           tmem_wait_ld();
-          if (h == 1) acc_release(bar, lane);
+          if (h == 3) acc_release(bar, lane, 4);
 #pragma unroll
-          for (int c8 = 0; c8 < 4; ++c8) {
+          for (int c8 = 0; c8 < 2; ++c8) {
             uint32_t hi[4], lo[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               split_pair(__uint_as_float(dw[c8 * 8 + 2 * e]), __uint_as_float(dw[c8 * 8 + 2 * e + 1]), hi[e], lo[e]);
-            const int slot = ((h * 4 + c8) ^ (key & 7)) << 4;
+            const int slot = ((h * 2 + c8) ^ (key & 7)) << 4;
             *reinterpret_cast<uint4*>(wt + slot) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             *reinterpret_cast<uint4*>(wt + L::kWTile + slot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
@@ -1085,18 +1096,18 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __nv_bfloat16* at = o_at;
         int rows = o_rows - (lane & 1);
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          uint32_t d[32];
-          tmem_ld32(lanes + kAccO + h * 32, d);
+        for (int h = 0; h < 4; ++h) {
+          uint32_t d[16];
+          tmem_ld16(lanes + kAccO + h * 16, d);
           tmem_wait_ld();
-          if (h == 1) {
+          if (h == 3) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar->ofree);
           }
           if (o_rows > 0) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < 8; ++j) {
               const uint32_t x = pack_bf16(__uint_as_float(d[2 * j]), __uint_as_float(d[2 * j + 1]));
               const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1);
               const uint32_t pair = __byte_perm(x, y, (lane & 1) ? 0x3276 : 0x5410);
@@ -1104,7 +1115,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
               at += 2 * row_stride;
             }
           }
-          rows -= 32;
+          rows -= 16;
         }
       }
       if (end) break;
@@ -1116,7 +1127,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   } else {
     // ------------------------------------------------------------------ prepare groups
-    const int group = (warp - kPrepWarp) >> 2;
+    const int group = (warp - kPrepWarp) >> 3;
     ItemCursor cursor;
     int n = 0;
 #pragma unroll 1
@@ -1124,19 +1135,15 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int* item = cursor.open(sm, bar, ok);
       ok = group_all(1 + group, ok);
       if (!ok) break;
-      const int chunks = item[kChunks], b = item[kBatch], hv = item[kHv], t_first = item[kFirst], t_end = item[kEnd];
-      const int slot = item[kFlagSlot], own = item[kOwn];
+      const int chunks = item[kChunks], slot = item[kFlagSlot], own = item[kOwn];
       cursor.close(bar, lane);
       if (chunks < 0) break;
       bool violation = false;
-      GateLoads next;
 #pragma unroll 1
       for (int c = 0; c < chunks && ok; ++c, ++n) {
         if ((n & 1) != group) continue;
         bool not_contraction = false;
-        const int t0 = t_first + c * kChunk;
-        ok = prepare_chunk<kRaw>(sm, bar, in, geo, group, n, b, hv, t0, c + 2 < chunks ? t0 + 2 * kChunk : -1, t_end, next,
-                                 not_contraction);
+        ok = prepare_chunk<kRaw>(sm, bar, group, n, not_contraction);
         violation |= not_contraction && c < own;
       }
       if (slot >= 0 && violation && lane == 0) plan.flags[slot] = 1;
@@ -1170,8 +1177,18 @@ int launch(const Inputs& in, const Geometry& geo, const Plan& plan, int grid, cu
     if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, batch, kChunk)) return rc;
   }
-  forward_umma_kernel<kRaw><<<grid, kThreads, kSmemBytes, stream>>>(tm_q, tm_k, tm_v, in, geo, plan);
-  return int(cudaGetLastError());
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kSmemBytes;
+  config.stream = stream;
+  // the serial pass may start before the first launch has ended (it waits for it in the kernel): its launch latency is hidden
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &early;
+  config.numAttrs = plan.serial_pass ? 1 : 0;
+  return int(cudaLaunchKernelEx(&config, forward_umma_kernel<kRaw>, tm_q, tm_k, tm_v, in, geo, plan));
 }
 int sm_count() {
   static int counts[64] = {};

@@ -58,33 +58,30 @@ __device__ __forceinline__ void load_fragment_a(float (&a)[4], uint32_t addr) {
 }
 // row piece of a lane: rows 0..15, columns 0 or 4 (floats, pitch lda)
 __device__ __forceinline__ int fragment_row(int lane, int lda) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * lda + (lane >> 4) * 4; }
-// kN m16n8 tiles side by side, D[i] = A B[:, 8 i .. 8 i + 8) over k in [0, kdim): A at this lane's `a_addr`, B row-major with
-// pitch ldb, b = this lane's B[t][g].  Same products in the same order as tile_product_tf32x3, one A fragment for all tiles.
-template <int kN>
-__device__ __forceinline__ void tile_row_tf32x3(float (&d)[kN][4], uint32_t a_addr, const float* b, int ldb, int kdim) {
+// One m16n8 tile D = A B over k in [0, kdim): A at this lane's `a_addr`, B row-major with pitch ldb, b = this lane's
+// B[t][g].  The three TF32 products of the split run as three chains that are added at the end (one chain of dependent
+// products would be three times as long, some 25 cycles each).
+__device__ __forceinline__ void tile_row_tf32x3(float (&d)[4], uint32_t a_addr, const float* b, int ldb, int kdim) {
+  float lh[4] = {}, hl[4] = {}, hh[4] = {};
 #pragma unroll
   for (int k0 = 0; k0 < kdim; k0 += 8) {
     float av[4];
-    uint32_t ah[4], al[4], bh[kN][2], bl[kN][2];
+    uint32_t ah[4], al[4], bh[2], bl[2];
     load_fragment_a(av, a_addr + k0 * 4);
+    const float bv[2] = {b[k0 * ldb], b[(k0 + 4) * ldb]};
     split_tf32(av, ah, al);
-#pragma unroll
-    for (int i = 0; i < kN; ++i) {
-      const float bv[2] = {b[k0 * ldb + i * 8], b[(k0 + 4) * ldb + i * 8]};
-      split_tf32(bv, bh[i], bl[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < kN; ++i) mma_tf32(d[i], al, bh[i]);
-#pragma unroll
-    for (int i = 0; i < kN; ++i) mma_tf32(d[i], ah, bl[i]);
-#pragma unroll
-    for (int i = 0; i < kN; ++i) mma_tf32(d[i], ah, bh[i]);
+    split_tf32(bv, bh, bl);
+    mma_tf32(lh, al, bh);
+    mma_tf32(hl, ah, bl);
+    mma_tf32(hh, ah, bh);
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) d[i] = (lh[i] + hl[i]) + hh[i];
 }
-// One m16n8 tile of D = A B over k in [0, kdim): A row-major with pitch lda (rows {g, g+8}), B row-major with pitch ldb
-// (column g); both in shared memory.
+// The same with both operands read word by word: A row-major with pitch lda (rows {g, g+8}).
 __device__ __forceinline__ void tile_product_tf32x3(float (&d)[4], const float* a, int lda, const float* b, int ldb,
                                                     int kdim, int g, int t) {
+  float lh[4] = {}, hl[4] = {}, hh[4] = {};
 #pragma unroll
   for (int k0 = 0; k0 < kdim; k0 += 8) {
     const float av[4] = {a[g * lda + k0 + t], a[(g + 8) * lda + k0 + t], a[g * lda + k0 + t + 4], a[(g + 8) * lda + k0 + t + 4]};
@@ -92,10 +89,12 @@ __device__ __forceinline__ void tile_product_tf32x3(float (&d)[4], const float* 
     uint32_t ah[4], al[4], bh[2], bl[2];
     split_tf32(av, ah, al);
     split_tf32(bv, bh, bl);
-    mma_tf32(d, al, bh);
-    mma_tf32(d, ah, bl);
-    mma_tf32(d, ah, bh);
+    mma_tf32(lh, al, bh);
+    mma_tf32(hl, ah, bl);
+    mma_tf32(hh, ah, bh);
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) d[i] = (lh[i] + hl[i]) + hh[i];
 }
 __device__ __forceinline__ float bf16_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }
