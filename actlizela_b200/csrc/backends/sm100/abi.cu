@@ -44,7 +44,8 @@ bool geometry_ok(int b, int t, int hk, int hv) {
 constexpr int kStageMask = 0x30, kPrepareOnly = 0x10, kWalkOnly = 0x20, kSegmentShift = 8, kMaxSegments = 16;
 constexpr int kWalkFlagMask = 0xc0, kHomogeneousBit = 0x40, kUntilDecayedBit = 0x80;
 constexpr int kParallelShift = 16, kMaxParallel = 8, kOffsetTailBit = 0x100000, kPairBit = 0x200000;
-// kernel family 4: the single-launch tensor-core forward (gdn_fused.cu): one segment, no stage restriction
+// kernel family 4: the single-launch tensor-core forward (gdn_fused.cu): one segment, no stage restriction; its
+// sub-segment field says only whether heads may be cut (0, 1: no), the kernel's launcher chooses the cuts
 constexpr int kFused = 4;
 bool is_fused(int config) { return (config & 0xf) == kFused; }
 bool config_ok(int config) {
@@ -74,8 +75,7 @@ int segments_of(int config, const Geometry& geo) {
 // workspace a call needs: the factors of every block, or (single-launch form) the flag words of the sub-segments
 long long scratch_bytes(const Geometry& geo, int config, int segments) {
   if (!is_fused(config)) return workspace_bytes(geo, segments);
-  const long long flags = fused_workspace_bytes(geo, parallel_of(config, geo.chunks()));
-  return flags > 256 ? flags : 256;
+  return fused_workspace_bytes();
 }
 
 // Second stream and events of the segmented forward, created by configure() for the current device.

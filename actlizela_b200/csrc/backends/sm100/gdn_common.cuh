@@ -188,9 +188,10 @@ int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaSt
 int launch_prepare_fused(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);   // Inputs::mixed etc. set
 int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int configure_umma();
-// single-launch forward (gdn_fused.cu): Geometry::parallel sub-segments; `flags` is scratch of fused_workspace_bytes
+// single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces; `flags` is scratch of
+// fused_workspace_bytes
 int configure_fused();
-long long fused_workspace_bytes(const Geometry&, int parallel);
+long long fused_workspace_bytes();
 int launch_forward_fused(const Inputs&, const Geometry&, int* flags, cudaStream_t);
 int read_fused_plan_counts(int* host_out2, int reset);
 int set_status_mirror_fused(int* device_pointer);

@@ -37,6 +37,7 @@ constexpr int kThreads = 1024, kPrepThreads = 256;
 constexpr int kIssueWarp = 0, kPlanWarp = 1, kScaleWarp = 2, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
 constexpr int kRing = 3;      // Q/K tiles, P tiles, gate vectors: one chunk in the chain, two in preparation
 constexpr int kItems = 4;     // work items announced ahead
+constexpr int kMaxSms = 256;  // CTAs of a launch at most: the flag words
 
 struct Smem {
   static constexpr int kKQStage = 4 * kBox;                       // [Q0 K0 Q1 K1]: Q over K per 64-column half
@@ -56,7 +57,7 @@ struct Smem {
   static constexpr int kPl2 = kGateWords, kBeta = kPl2 + 64, kCoefW = kBeta + 64, kECol = kCoefW + 64, kGateStage = kECol + 32;
   static constexpr int kItem = kGates + kRing * kGateStage * 4;   // item ring, 16 words each
   static constexpr int kBars = kItem + kItems * 64;
-  static constexpr int kTotal = kBars + 512;
+  static constexpr int kTotal = kBars + 640;
   static_assert(kATBytes % 1024 == 0 && kAT % 1024 == 0 && kTw % 1024 == 0, "swizzled tiles start on 1024 bytes");
   static_assert(2 * kBox <= kATBytes, "the T_u pair must fit on T");
 };
@@ -81,9 +82,11 @@ struct Barriers {
   uint32_t tmem;
   int abort;
   int lock, released;
-  int reach[8];
+  // split heads: decay reach of this CTA's sub-segment and of the next one; does some sub-segment of the head not decay
+  // (one word per scanning warp)
+  int reach[2], slow[32];
 };
-static_assert(sizeof(Barriers) <= 512, "barrier block");
+static_assert(sizeof(Barriers) <= 640, "barrier block");
 constexpr int kItemReaders = kThreads / 32 - 1;      // every warp but the planner reads the items
 
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kPrepThreads) : "memory"); }
@@ -234,15 +237,24 @@ struct ItemCursor {
   }
 };
 
-// What a launch walks: the units of the grid are (batch or sequence, value head[, sub-segment]); see walk_umma_kernel
-// for the sub-segments.  Here the decay part of the plan is read off the gates up front, while the contraction part
-// (beta |k|^2 in [0, 2]) shows only when a chunk is prepared: every CTA records what it saw in `flags`, and a second
-// launch of the same kernel (`serial_pass`) walks the heads for which some sub-segment saw a violation again, whole,
-// by one CTA each, and leaves at once otherwise.
+// What a launch walks: the units of the grid, a (batch or sequence, value head) each, or with `pieces` > 1 one of its
+// sub-segments (see walk_umma_kernel), at most one per CTA.  The decay part of the sub-segments' conditions is read off
+// the gates up front, while the contraction part (beta |k|^2 in [0, 2]) shows only when a chunk is prepared: every CTA
+// records what it saw in `flags`, and a second launch of the same kernel (`serial_pass`) walks the heads for which some
+// sub-segment saw a violation again, whole, by one CTA each, and leaves at once otherwise.
 struct Plan {
-  int units, parallel, serial_pass;
-  int* flags;      // [batch * value_heads][parallel], written when parallel > 1
+  int units, pieces, serial_pass;
+  int* flags;      // [batch * value_heads][pieces], written when pieces > 1
 };
+constexpr int kLeastPiece = 8;       // chunks: a piece has to outlast the decay, which takes about four at typical gates
+
+// did a CTA that walked a piece of head h see a token that is no contraction?
+__device__ __forceinline__ bool violated(const Plan& plan, int h) {
+  bool any = false;
+#pragma unroll 1
+  for (int r = 1; r < plan.pieces; ++r) any |= plan.flags[h * plan.pieces + r] != 0;
+  return any;
+}
 
 // ---------------------------------------------------------------------------------------------------- prepare groups
 // Eight warps prepare one chunk; the phases are those of prepare_umma_kernel.  A warp owns the TMEM lane quarter
@@ -510,7 +522,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
 template <bool kRaw>
 __global__ void __launch_bounds__(kThreads, 1)
 forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_v, const Inputs in, const Geometry geo, const Plan plan) {
+                    const __grid_constant__ CUtensorMap tm_v, const Inputs in, const Geometry geo, const __grid_constant__ Plan plan) {
   uint8_t* sm = shared_base();
   using L = Smem;
   Barriers* bar = reinterpret_cast<Barriers*>(sm + L::kBars);
@@ -525,11 +537,10 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // nothing to repair for this CTA's heads: leave before anything is set up
     bool any = false;
-    for (int unit = blockIdx.x; unit < plan.units; unit += gridDim.x)
-      for (int r = 1; r < plan.parallel; ++r) any |= plan.flags[unit * plan.parallel + r] != 0;
+    for (int unit = blockIdx.x; unit < plan.units; unit += gridDim.x) any |= violated(plan, unit);
     if (!any) return;
   }
-  if (plan.parallel > 1) asm volatile("griddepcontrol.launch_dependents;");
+  if (plan.pieces > 1) asm volatile("griddepcontrol.launch_dependents;");
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) {
       mbar_init(&bar->kq_full[i], 1);
@@ -563,13 +574,18 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tmem_alloc(&bar->tmem, 512);
     tmem_relinquish();
   }
-  if (!plan.serial_pass && warp >= kChainWarp && warp - kChainWarp + 1 < plan.parallel) {
-    // the decay reaches of the first item's sub-segments, one warp each (usually the CTA's only item)
-    const int r = warp - kChainWarp + 1, bh = blockIdx.x / plan.parallel, n = geo.segment_chunks();
-    const int c0 = sub_segment_begin(n, r, plan.parallel), c1 = sub_segment_begin(n, r + 1, plan.parallel);
-    const int reach = gate_reach<kRaw>(in, geo, bh / geo.value_heads, bh % geo.value_heads, (geo.chunk_begin + c0) * kChunk,
-                                       c1 - c0, geo.sequence, lane);
-    if (lane == 0) bar->reach[r] = reach;
+  if (plan.pieces > 1 && !plan.serial_pass && warp >= kChainWarp) {
+    const int n = geo.chunks(), head = blockIdx.x / plan.pieces, sub = blockIdx.x % plan.pieces;
+    int slow = 0;
+#pragma unroll 1
+    for (int r = 1 + warp - kChainWarp; r < plan.pieces; r += kThreads / 32 - kChainWarp) {
+      const int c0 = sub_segment_begin(n, r, plan.pieces), c1 = sub_segment_begin(n, r + 1, plan.pieces);
+      const int reach = gate_reach<kRaw>(in, geo, head / geo.value_heads, head % geo.value_heads, c0 * kChunk, c1 - c0,
+                                         geo.sequence, lane);
+      if (reach < 0) slow = 1;
+      if (lane == 0 && (r == sub || r == sub + 1)) bar->reach[r - sub] = reach;
+    }
+    if (lane == 0) bar->slow[warp] = slow;
   }
   tc_fence_before();
   __syncthreads();
@@ -602,16 +618,15 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       return true;
     };
+    const bool split = plan.pieces > 1 && !plan.serial_pass;
 #pragma unroll 1
     for (int unit = blockIdx.x; ok; unit += gridDim.x) {
       const bool end = unit >= plan.units;
-      int bh = 0, b = 0, hv = 0, sub = 0, chunks = -1, t_first = 0, t_end = 0, unstored = 0, flags = 0, own = 0, slot = -1;
+      const int head = split ? unit / plan.pieces : unit;
+      int b = 0, hv = 0, chunks = -1, t_first = 0, t_end = 0, unstored = 0, flags = 0, own = 0, slot = -1;
       if (!end) {
-        const int parallel = plan.serial_pass ? 1 : plan.parallel;
-        bh = unit / parallel;
-        sub = unit % parallel;
-        b = bh / geo.value_heads;
-        hv = bh % geo.value_heads;
+        b = head / geo.value_heads;
+        hv = head % geo.value_heads;
         flags = (in.initial ? kHasInitial : 0) | (in.final_state ? kHasFinal : 0);
         if (geo.varlen) {
           // offsets forced into 0 <= ... <= total and non-decreasing: no index can leave the tensors
@@ -629,41 +644,34 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           t_end = geo.sequence;
         }
         if (plan.serial_pass) {
-          bool any = false;
-          for (int r = 1; r < plan.parallel; ++r) any |= plan.flags[bh * plan.parallel + r] != 0;
-          if (!any) continue;
+          if (!violated(plan, unit)) continue;
           if (lane == 0) {
             atomicAdd(&g_fused_plan_counts[0], -1);
             atomicAdd(&g_fused_plan_counts[1], 1);
           }
-        } else if (parallel > 1) {
-          bool serial = false;
-          int mine = 0, next = 0;
-          for (int r = 1; r < parallel && !serial; ++r) {
-            const int c0 = sub_segment_begin(chunks, r, parallel), c1 = sub_segment_begin(chunks, r + 1, parallel);
-            const int reach = unit == blockIdx.x ? bar->reach[r] :
-                              gate_reach<kRaw>(in, geo, b, hv, t_first + c0 * kChunk, c1 - c0, t_end, lane);
-            serial = reach < 0;
-            if (r == sub) mine = reach;
-            if (r == sub + 1) next = reach;
-          }
+        } else if (split) {
+          const int sub = unit % plan.pieces;
+          const bool serial = __ballot_sync(0xffffffffu, lane >= kChainWarp && bar->slow[lane]);
           if (lane == 0) {
             if (sub == 0) atomicAdd(&g_fused_plan_counts[serial ? 1 : 0], 1);
-            plan.flags[bh * parallel + sub] = 0;
+            plan.flags[unit] = 0;
           }
           if (serial) {
             if (sub) continue;
           } else {
-            const int c0 = sub_segment_begin(chunks, sub, parallel), c1 = sub_segment_begin(chunks, sub + 1, parallel);
+            const int c0 = sub_segment_begin(chunks, sub, plan.pieces), c1 = sub_segment_begin(chunks, sub + 1, plan.pieces);
             own = c1 - c0;
-            chunks = own + next;
+            chunks = own;
             t_first += c0 * kChunk;
-            unstored = mine;
             if (sub) {
+              unstored = bar->reach[0];
               flags &= ~kHasInitial;
-              slot = bh * parallel + sub;
+              slot = unit;
             }
-            if (sub + 1 < parallel) flags &= ~kHasFinal;
+            if (sub + 1 < plan.pieces) {
+              chunks += bar->reach[1];
+              flags &= ~kHasFinal;
+            }
           }
         }
       }
@@ -679,7 +687,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         item[kFirst] = t_first;
         item[kEnd] = t_end;
         item[kUnstored] = unstored;
-        item[kState] = bh;
+        item[kState] = head;
         item[kFlags] = flags;
         item[kFlagSlot] = slot;
         item[kOwn] = own;
@@ -1195,7 +1203,7 @@ int sm_count() {
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 1;
   if (!counts[device] && cudaDeviceGetAttribute(&counts[device], cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 1;
-  return counts[device];
+  return counts[device] < kMaxSms ? counts[device] : kMaxSms;
 }
 }  // namespace
 
@@ -1205,21 +1213,29 @@ int configure_fused() {
   return int(e);
 }
 
-long long fused_workspace_bytes(const Geometry& geo, int parallel) {
-  return parallel > 1 ? ((long long)geo.batch * geo.value_heads * parallel * (long long)sizeof(int) + 255) & ~255LL : 0;
-}
+long long fused_workspace_bytes() { return kMaxSms * (long long)sizeof(int); }
 
-// `flags`: fused_workspace_bytes(geo, geo.parallel) bytes of scratch (may be null when that is 0)
+// `flags`: fused_workspace_bytes() bytes of scratch (may be null for an unsplit walk)
 int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cudaStream_t stream) {
   Plan plan{};
-  plan.parallel = geo.parallel > 1 ? geo.parallel : 1;
+  const int heads = geo.batch * geo.value_heads, sms = sm_count(), chunks = geo.segment_chunks();
+  const bool split = geo.parallel > 1 && heads > 0;
+  if (split && (geo.varlen || !flags || geo.chunk_begin || geo.chunk_count)) return int(cudaErrorInvalidValue);
   plan.flags = flags;
-  const int heads = geo.batch * geo.value_heads, sms = sm_count();
-  if (plan.parallel > 1 && (geo.varlen || !flags || plan.parallel > geo.segment_chunks())) return int(cudaErrorInvalidValue);
-  plan.units = heads * plan.parallel;
+  plan.units = heads;
+  plan.pieces = 1;
+  if (split) {
+    // A head in as many pieces as give every SM one, none shorter than kLeastPiece (8 heads of 30000 tokens: 250 us in
+    // the two-kernel form with its at most eight pieces, 156 in eighteen).  Equal ranges of the line of all heads'
+    // chunks, one per SM, were tried as well: a CTA with the ends of two heads pays the walk-on twice and the long
+    // launches are at the board's power limit anyway (B1 T8192, 32 heads: 194 us against 171; T131072: 2155 against 2210).
+    plan.pieces = sms / heads < chunks / kLeastPiece ? sms / heads : chunks / kLeastPiece;
+    if (plan.pieces < 1) plan.pieces = 1;
+    plan.units = heads * plan.pieces;
+  }
   const auto go = in.mixed ? launch<true> : launch<false>;
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
-  if (plan.parallel == 1) return 0;
+  if (plan.pieces == 1) return 0;
   plan.serial_pass = 1;
   plan.units = heads;
   return go(in, geo, plan, heads < sms ? heads : sms, stream);

@@ -15,9 +15,8 @@ from .sm100_policy import policy, selection_for
 
 MATH_CONTRACT = "wy-splitbf16-state-bf16-out-sm100-v1"
 _DIAGNOSTIC_IDS = {"simt": 0, "umma": 1, "simt-prepare+umma-walk": 2, "umma-prepare+simt-walk": 3,
-                   # the single-launch form, alone and with parallel sub-segments of the walk
-                   "fused": 4, "fused-par2": 4 | (2 << 16), "fused-par3": 4 | (3 << 16), "fused-par4": 4 | (4 << 16),
-                   "fused-par8": 4 | (8 << 16),
+                   # the single-launch form, unsplit and with its heads cut into pieces over the SMs
+                   "fused": 4, "fused-split": 4 | (2 << 16),
                    "umma-seg2": 1 | (2 << 8), "umma-seg4": 1 | (4 << 8), "umma-seg8": 1 | (8 << 8), "umma-seg16": 1 | (16 << 8),
                    # parallel sub-segments of the walk (bits 16..19), alone and with sequence segments
                    "umma-par2": 1 | (2 << 16), "umma-par3": 1 | (3 << 16), "umma-par4": 1 | (4 << 16),

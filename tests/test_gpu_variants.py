@@ -28,21 +28,58 @@ def test_out_proj_with_few_rows(m, k, n):
     assert torch.equal(got, out_proj_gemm(a, w))                  # the sum over the cluster has one order
 
 
-@pytest.mark.parametrize("batch,length,hk,hv,parallel", [(1, 1, 1, 1, 1), (1, 64, 2, 6, 1), (3, 129, 1, 2, 1), (2, 193, 1, 4, 3),
-                                                         (5, 700, 8, 32, 1), (1, 64 * 40 + 1, 1, 2, 8), (300, 65, 1, 1, 1)])
-def test_single_launch_form_equals_the_two_kernels_bitwise(batch, length, hk, hv, parallel, native_library):
-    """One chunk, two, odd and even chunk counts, tails, several work items per CTA (more heads than SMs), more
-    sub-segments than chunks would allow; the states and every output row have the bits of the two-kernel path."""
+@pytest.mark.parametrize("batch,length,hk,hv", [(1, 1, 1, 1), (1, 64, 2, 6), (3, 129, 1, 2), (2, 193, 1, 4), (5, 700, 8, 32),
+                                                (300, 65, 1, 1)])
+def test_single_launch_form_equals_the_two_kernels_bitwise(batch, length, hk, hv, native_library):
+    """One chunk, two, odd and even chunk counts, tails, several work items per CTA (more heads than SMs): the states
+    and every output row have the bits of the two-kernel path."""
     from actlizela_b200.sm100 import Sm100Forward
     forward = Sm100Forward(native_library)
     w = WORKLOADS["cfg1"].sliced(batch=batch, length=length, key_heads=hk, value_heads=hv, seed=4000 + length)
     dev = [x.cuda() for x in make_inputs(w)]
-    suffix = "" if parallel == 1 else f"-par{parallel}"
-    want_out, want_state = forward(*dev, True, configuration="umma" + suffix)
-    out, state = forward(*dev, True, configuration="fused" + suffix)
+    want_out, want_state = forward(*dev, True, configuration="umma")
+    out, state = forward(*dev, True, configuration="fused")
     torch.cuda.synchronize()
-    status = (ctypes.c_int * 4)()
-    assert native_library.lib.actlize_la_sm100_device_status(status, 1) == 0 and status[0] == 0
+    assert _healthy(native_library)
     assert torch.equal(out, want_out) and torch.equal(state, want_state)
-    out_only, none = forward(*dev, False, configuration="fused" + suffix)
+    out_only, none = forward(*dev, False, configuration="fused")
     assert none is None and torch.equal(out_only, want_out)
+
+
+def _healthy(native_library):
+    status = (ctypes.c_int * 4)()
+    return native_library.lib.actlize_la_sm100_device_status(status, 1) == 0 and status[0] == 0
+
+
+@pytest.mark.parametrize("batch,length,hk,hv", [(1, 64 * 16, 1, 2), (1, 64 * 17 + 5, 2, 6), (2, 64 * 40 + 1, 1, 2), (1, 64 * 300 + 1, 1, 1),
+                                                (1, 64 * 1300, 1, 2), (1, 64 * 20 + 63, 37, 74)])
+@pytest.mark.parametrize("stress", ["none", "slow-head", "long-key"])
+def test_heads_cut_over_the_sms(batch, length, hk, hv, stress, native_library):
+    """Heads cut into two pieces up to one for every SM, of the least length and of many chunks: agreement with the
+    unsplit walk to exp(-40) of the state, and a head whose gates hardly decay or that holds a token that is no
+    contraction comes out with the unsplit walk's bits."""
+    from actlizela_b200.sm100 import Sm100Forward
+    forward = Sm100Forward(native_library)
+    w = WORKLOADS["cfg1"].sliced(batch=batch, length=length, key_heads=hk, value_heads=hv, seed=5000 + length)
+    q, k, v, g, beta, init = make_inputs(w)
+    lone = hv - 1
+    if stress == "slow-head":
+        g[:, :, lone] *= 1e-3
+    elif stress == "long-key":
+        beta[:, length - 3, lone] = -0.25
+    dev = [x.cuda() for x in (q, k, v, g, beta, init)]
+    want_out, want_state = forward(*dev, True, configuration="fused")
+    counts = (ctypes.c_int * 2)()
+    assert native_library.lib.actlize_la_sm100_walk_plan_counts(counts, 1) == 0
+    out, state = forward(*dev, True, configuration="fused-split")
+    torch.cuda.synchronize()
+    assert _healthy(native_library)
+    assert native_library.lib.actlize_la_sm100_walk_plan_counts(counts, 1) == 0
+    alone = 0 if stress == "none" else batch
+    assert list(counts) == [batch * hv - alone, alone]
+    assert oracle.max_abs(out.float(), want_out.float()) < 1e-5
+    assert oracle.rel_frobenius(state.cpu(), want_state.cpu()) < 1e-6
+    if stress != "none":
+        assert torch.equal(out[:, :, lone], want_out[:, :, lone]) and torch.equal(state[:, lone], want_state[:, lone])
+    again_out, again_state = forward(*dev, True, configuration="fused-split")
+    assert torch.equal(again_out, out) and torch.equal(again_state, state)
