@@ -116,12 +116,6 @@ int create_segment_streams() {
 // 0 = simt/simt, 1 = umma/umma, 2 = simt prepare + umma walk, 3 = umma prepare + simt walk
 bool prepare_is_umma(int config) { return (config & 0xf) == 1 || (config & 0xf) == 3; }
 bool walk_is_umma(int config) { return (config & 0xf) == 1 || (config & 0xf) == 2; }
-int launch_prepare_tc(int, const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream) {
-  return in.mixed ? launch_prepare_fused(in, geo, ws, stream) : launch_prepare_umma(in, geo, ws, stream);
-}
-int launch_walk_tc(int, const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream) {
-  return launch_walk_umma(in, geo, ws, stream);
-}
 
 // One affine step of a 128x128 state block, out = M @ S + b, by the 256 threads of a CTA (each 64 outputs).
 // `s_in` and `s_out` may be the same block: every read of s_in is finished before the first write.
@@ -416,17 +410,17 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
       geo.chunk_count = int((long long)chunks * (i + 1) / segments) - geo.chunk_begin;
       geo.parallel = parallel_of(config, geo.chunk_count);
       if (i == 0) {
-        if (int rc = launch_prepare_tc(config, in, geo, ws, stream)) return rc;
+        if (int rc = launch_prepare_umma(in, geo, ws, stream)) return rc;
         if ((e = cudaEventRecord(ss.start, stream)) != cudaSuccess) return int(e);
         if ((e = cudaStreamWaitEvent(ss.prepare, ss.start, 0)) != cudaSuccess) return int(e);
-        if (int rc = launch_walk_tc(config, in, geo, ws, stream)) return rc;
+        if (int rc = launch_walk_umma(in, geo, ws, false, stream)) return rc;
         if ((e = cudaEventRecord(ss.walked[0], stream)) != cudaSuccess) return int(e);
         if ((e = cudaStreamWaitEvent(ss.walk, ss.walked[0], 0)) != cudaSuccess) return int(e);
       } else {
-        if (int rc = launch_prepare_tc(config, in, geo, ws, ss.prepare)) return rc;
+        if (int rc = launch_prepare_umma(in, geo, ws, ss.prepare)) return rc;
         if ((e = cudaEventRecord(ss.prepared[i], ss.prepare)) != cudaSuccess) return int(e);
         if ((e = cudaStreamWaitEvent(ss.walk, ss.prepared[i], 0)) != cudaSuccess) return int(e);
-        if (int rc = launch_walk_tc(config, in, geo, ws, ss.walk)) return rc;
+        if (int rc = launch_walk_umma(in, geo, ws, false, ss.walk)) return rc;
       }
     }
     if ((e = cudaEventRecord(ss.done, ss.walk)) != cudaSuccess) return int(e);
@@ -434,13 +428,12 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
   }
   geo.parallel = parallel_of(config, geo.segment_chunks());
   if (!(config & kWalkOnly)) {
-    if (int rc = in.mixed                  ? launch_prepare_fused(in, geo, ws, stream)
-                 : prepare_is_umma(config) ? launch_prepare_umma(in, geo, ws, stream)
-                                           : launch_prepare_simt(in, geo, ws, stream))
+    if (int rc = prepare_is_umma(config) ? launch_prepare_umma(in, geo, ws, stream) : launch_prepare_simt(in, geo, ws, stream))
       return rc;
   }
   if (config & kPrepareOnly) return 0;
-  return walk_is_umma(config) ? launch_walk_umma(in, geo, ws, stream) : launch_walk_simt(in, geo, ws, stream);
+  return walk_is_umma(config) ? launch_walk_umma(in, geo, ws, !(config & kWalkOnly) && prepare_is_umma(config), stream)
+                              : launch_walk_simt(in, geo, ws, stream);
 }
 }  // namespace
 
@@ -665,10 +658,10 @@ extern "C" int actlize_la_sm100_forward_host(
         }
         if ((e = cudaEventRecord(ss.arrived[i], ss.copy_in)) != cudaSuccess) return int(e);
         if ((e = cudaStreamWaitEvent(stream, ss.arrived[i], 0)) != cudaSuccess) return int(e);
-        if (int rc = launch_prepare_tc(config, in, geo, ws, stream)) return rc;
+        if (int rc = launch_prepare_umma(in, geo, ws, stream)) return rc;
         if ((e = cudaEventRecord(ss.prepared[i], stream)) != cudaSuccess) return int(e);
         if ((e = cudaStreamWaitEvent(ss.walk, ss.prepared[i], 0)) != cudaSuccess) return int(e);
-        if (int rc = launch_walk_tc(config, in, geo, ws, ss.walk)) return rc;
+        if (int rc = launch_walk_umma(in, geo, ws, false, ss.walk)) return rc;
         if ((e = cudaEventRecord(ss.walked[i], ss.walk)) != cudaSuccess) return int(e);
         if ((e = cudaStreamWaitEvent(ss.copy_out, ss.walked[i], 0)) != cudaSuccess) return int(e);
         for (int bb = 0; bb < b; ++bb) {

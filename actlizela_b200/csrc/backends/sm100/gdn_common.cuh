@@ -19,23 +19,18 @@ struct Geometry {
   int batch, sequence, key_heads, value_heads;
   // A launch may cover a contiguous range of chunks only (sequence segment); 0 chunks = the whole sequence.
   int chunk_begin = 0, chunk_count = 0;
-  // tcgen05 walk only: the launch's chunk range is cut into `parallel` sub-segments per (batch, value head), walked by
+  // tensor-core kernels only: the launch's chunk range is cut into `parallel` sub-segments per (batch, value head), walked by
   // as many CTAs at the same time (0 or 1 = one CTA walks the whole range); see walk_umma_kernel.
   int parallel = 0;
-  // Packed variable-length mode (tcgen05 kernels only): the tensors are [1, sequence = total tokens, H, ...],
-  // `batch` is the number of sequences and `varlen` points at 2 (batch + 1) device integers: the token offsets
-  // cu_seqlens[0..batch] followed by the chunk offsets chunk_prefix[0..batch] (every sequence starts a new chunk);
-  // `total_chunks` = chunk_prefix[batch].  Workspace blocks are then indexed hv * total_chunks + global chunk.
+  // Packed variable-length mode (single-launch kernel only): the tensors are [1, sequence = total tokens, H, ...],
+  // `batch` is the number of sequences and `varlen` points at the token offsets cu_seqlens[0..batch] on the device.
   const int* varlen = nullptr;
-  int total_chunks = 0;
-  __host__ __device__ int chunks() const { return varlen ? total_chunks : (sequence + kChunk - 1) / kChunk; }
+  __host__ __device__ int chunks() const { return (sequence + kChunk - 1) / kChunk; }
   __host__ __device__ int segment_chunks() const { return chunk_count ? chunk_count : chunks(); }
   __host__ __device__ bool first_segment() const { return chunk_begin == 0; }
   __host__ __device__ bool last_segment() const { return chunk_begin + segment_chunks() == chunks(); }
   __host__ __device__ int group() const { return value_heads / key_heads; }
-  __host__ __device__ long long blocks() const {
-    return varlen ? (long long)value_heads * total_chunks : (long long)batch * value_heads * chunks();
-  }
+  __host__ __device__ long long blocks() const { return (long long)batch * value_heads * chunks(); }
 };
 
 // Parallel sub-segments of a walk over `chunks` chunks: sub-segment r covers [sub_segment_begin(r), sub_segment_begin(r + 1)).
@@ -48,17 +43,6 @@ __host__ __device__ inline int sub_segment_begin(int chunks, int r, int parallel
   if (r >= parallel) return chunks;
   const int body = chunks - kNominalReach;
   return int((long long)(body >= parallel * kNominalReach ? body : chunks) * r / parallel);
-}
-
-// Packed mode: the sequence that owns global chunk `gchunk` (largest s with chunk_prefix[s] <= gchunk; empty
-// sequences share their successor's offset and are skipped by the search).
-__device__ __forceinline__ int varlen_sequence_of(const int* chunk_prefix, int count, int gchunk) {
-  int lo = 0, hi = count;          // invariant: chunk_prefix[lo] <= gchunk < chunk_prefix[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (chunk_prefix[mid] <= gchunk) lo = mid; else hi = mid;
-  }
-  return lo;
 }
 
 // Workspace: structure-of-arrays planes, one entry per (batch, value head, chunk) block,
@@ -129,18 +113,15 @@ struct Inputs {
   //   kWalkPair         kWalkTail and kWalkHomogeneous (from an identity state made in the kernel) in one launch,
   //                     two CTAs per (batch, value head); final_state is then [2][B][Hv][128][128] = (M, b)
   int walk_flags = 0;
-  // Fused input preparation (tcgen05 prepare kernel only): q, k, v are then read from the packed projection
-  // rows `mixed` [B*T][mixed_stride] = [q heads | k heads | v heads] x 128, normalised in shared memory; the gate and
-  // beta come from the raw activations `act_a`, `act_b` [B*T][Hv] with the per-head constants `a_log`, `dt_bias`;
-  // the normalised keys are written to `k_norm` [B][T][Hk][128] for the walk (which gets it as its `k`).
+  // Raw projections (single-launch forward only): q, k, v are then read from the packed projection rows `mixed`
+  // [B*T][mixed_stride] = [q heads | k heads | v heads] x 128 and normalised in shared memory; the gate and beta come
+  // from the raw activations `act_a`, `act_b` [B*T][Hv] with the per-head constants `a_log`, `dt_bias`.
   const __nv_bfloat16* mixed = nullptr;
   long long mixed_stride = 0;
   const __nv_bfloat16* act_a = nullptr;
   const __nv_bfloat16* act_b = nullptr;
   const float* a_log = nullptr;
   const float* dt_bias = nullptr;
-  __nv_bfloat16* k_norm = nullptr;
-  __nv_bfloat16* q_norm = nullptr;      // likewise the normalised queries [B][T][Hk][128] (the walk gets it as its `q`)
 };
 constexpr int kWalkHomogeneous = 1, kWalkUntilDecayed = 2;
 constexpr int kWalkTail = 8;              // offset pass: walk, from zero, only the suffix that decides the outgoing state
@@ -185,8 +166,8 @@ int launch_prepare_simt(const Inputs&, const Geometry&, const Workspace&, cudaSt
 int launch_walk_simt(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int configure_simt();
 int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
-int launch_prepare_fused(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);   // Inputs::mixed etc. set
-int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
+// `early`: the kernel in front of it on the stream is this call's prepare kernel, which lets it set itself up beside it
+int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, bool early, cudaStream_t);
 int configure_umma();
 // single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces; `flags` is scratch of
 // fused_workspace_bytes

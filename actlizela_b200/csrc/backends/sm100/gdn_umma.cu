@@ -129,10 +129,6 @@ static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit
 #define GDN_PSTAMP(slot)
 #endif
 
-// Fused variant (kFused): the tiles come from the packed projection rows (tm_q is a 2-D map over them, tm_k the 4-D
-// map of the normalised-key plane that the walk reads); Q and K rows are L2-normalised in shared memory with the
-// arithmetic of the separate input-preparation kernel (16 lanes per row), gate and beta are activated on load.
-template <bool kFused>
 __global__ void __launch_bounds__(kPrepThreads, 3)
 prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_wh,
@@ -157,45 +153,29 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int chunks = geo.chunks(), seg_chunks = geo.segment_chunks();
-  int chunk = geo.chunk_begin + blockIdx.x % seg_chunks;      // chunk index inside its sequence
-  int bh = blockIdx.x / seg_chunks;
-  if (!geo.varlen) {
-    // Block order = reverse of the order in which the walk consumes the blocks: the walk's CTAs (one per
-    // (batch, head) and parallel sub-segment) all start at the first chunk of their sub-segment, so the blocks
-    // prepared LAST are the leading chunks of every sub-segment of every head, and the walk finds them in L2.
-    // The grid covers heads x sub-segments x longest sub-segment; a slot behind a shorter sub-segment's end is empty.
-    const int parallel = geo.parallel > 1 ? geo.parallel : 1;
-    // (The cut is an even one; the walk's own cut, sub_segment_begin, differs from it by a few chunks at most.)
-    const int longest = (seg_chunks + parallel - 1) / parallel;
-    const int units = geo.batch * geo.value_heads * parallel;
-    const int offset = longest - 1 - int(blockIdx.x) / units, unit = int(blockIdx.x) % units;
-    const int sub = unit % parallel;
-    const int sub_begin = int((long long)seg_chunks * sub / parallel), sub_end = int((long long)seg_chunks * (sub + 1) / parallel);
-    if (sub_begin + offset >= sub_end) return;
-    bh = unit / parallel;
-    chunk = geo.chunk_begin + sub_begin + offset;
-  }
-  const int b = bh / geo.value_heads, hv = bh % geo.value_heads;     // packed mode: bh = hv, b = 0
+  // Block order = reverse of the order in which the walk consumes the blocks: the walk's CTAs (one per
+  // (batch, head) and parallel sub-segment) all start at the first chunk of their sub-segment, so the blocks
+  // prepared LAST are the leading chunks of every sub-segment of every head, and the walk finds them in L2.
+  // The grid covers heads x sub-segments x longest sub-segment; a slot behind a shorter sub-segment's end is empty.
+  const int parallel = geo.parallel > 1 ? geo.parallel : 1;
+  // (The cut is an even one; the walk's own cut, sub_segment_begin, differs from it by a few chunks at most.)
+  const int longest = (seg_chunks + parallel - 1) / parallel;
+  const int units = geo.batch * geo.value_heads * parallel;
+  const int offset = longest - 1 - int(blockIdx.x) / units, unit = int(blockIdx.x) % units;
+  const int sub = unit % parallel;
+  const int sub_begin = int((long long)seg_chunks * sub / parallel), sub_end = int((long long)seg_chunks * (sub + 1) / parallel);
+  if (sub_begin + offset >= sub_end) return;
+  const int bh = unit / parallel, chunk = geo.chunk_begin + sub_begin + offset;
+  const int b = bh / geo.value_heads, hv = bh % geo.value_heads;
   const int hk = hv / geo.group();
-  int t0 = chunk * kChunk, t_end = geo.sequence;
-  long long block = (long long)bh * chunks + chunk;
-  if (geo.varlen) {
-    // packed sequences: the grid runs over (value head, global chunk); rows behind the sequence end belong to the
-    // next sequence and are neutralised by beta = 0 / zero gate weights exactly like zero-filled padding rows
-    const int gchunk = chunk;
-    const int* prefix = geo.varlen + geo.batch + 1;
-    if (gchunk >= prefix[geo.batch]) return;     // grid sized by an upper bound of the chunk count (device offsets)
-    const int seq = varlen_sequence_of(prefix, geo.batch, gchunk);
-    chunk = gchunk - prefix[seq];
-    t0 = geo.varlen[seq] + chunk * kChunk;
-    t_end = geo.varlen[seq + 1];
-    block = (long long)hv * chunks + gchunk;
-  }
+  const int t0 = chunk * kChunk, t_end = geo.sequence;
+  const long long block = (long long)bh * chunks + chunk;
   const int valid = min(kChunk, t_end - t0);
 #ifdef GDN_SM100_PHASE_TIMING
   const long long t_begin = clock64();
 #endif
 
+  asm volatile("griddepcontrol.launch_dependents;");      // the walk sets itself up as SMs fall free
   if (tid == 0) {
     mbar_init(bar_tma, 1);
     mbar_init(bar_mma, 1);
@@ -203,25 +183,12 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     fence_barrier_init();
     // the input tiles do not depend on tensor memory: start them before the allocation
     mbar_arrive_expect_tx(bar_tma, 6 * kBox);
-    if (kFused) {
-      // packed rows [q heads | k heads | v heads]; rows behind the batch element's end belong to the next one
-      // (or read as zero behind the last) and are neutralised by beta = 0 / zero gate weights
-      const int row = b * geo.sequence + t0;
-      const int xq = hk * kDim, xk = (geo.key_heads + hk) * kDim, xv = (2 * geo.key_heads + hv) * kDim;
-      tma_load_2d(sm + L::kQ0, &tm_q, bar_tma, xq, row);
-      tma_load_2d(sm + L::kQ1, &tm_q, bar_tma, xq + 64, row);
-      tma_load_2d(sm + L::kK0, &tm_q, bar_tma, xk, row);
-      tma_load_2d(sm + L::kK1, &tm_q, bar_tma, xk + 64, row);
-      tma_load_2d(sm + L::kV0, &tm_q, bar_tma, xv, row);
-      tma_load_2d(sm + L::kV1, &tm_q, bar_tma, xv + 64, row);
-    } else {
-      tma_load_4d(sm + L::kQ0, &tm_q, bar_tma, 0, hk, t0, b);
-      tma_load_4d(sm + L::kQ1, &tm_q, bar_tma, 64, hk, t0, b);
-      tma_load_4d(sm + L::kK0, &tm_k, bar_tma, 0, hk, t0, b);
-      tma_load_4d(sm + L::kK1, &tm_k, bar_tma, 64, hk, t0, b);
-      tma_load_4d(sm + L::kV0, &tm_v, bar_tma, 0, hv, t0, b);
-      tma_load_4d(sm + L::kV1, &tm_v, bar_tma, 64, hv, t0, b);
-    }
+    tma_load_4d(sm + L::kQ0, &tm_q, bar_tma, 0, hk, t0, b);
+    tma_load_4d(sm + L::kQ1, &tm_q, bar_tma, 64, hk, t0, b);
+    tma_load_4d(sm + L::kK0, &tm_k, bar_tma, 0, hk, t0, b);
+    tma_load_4d(sm + L::kK1, &tm_k, bar_tma, 64, hk, t0, b);
+    tma_load_4d(sm + L::kV0, &tm_v, bar_tma, 0, hv, t0, b);
+    tma_load_4d(sm + L::kV1, &tm_v, bar_tma, 64, hv, t0, b);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kPrepTmemCols);
@@ -230,15 +197,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   float gate = 0.f, beta = 0.f;
   if (tid < valid) {
     const long long gi = ((long long)b * geo.sequence + t0 + tid) * geo.value_heads + hv;
-    if (kFused) {
-      // g = -exp(A_log) softplus(a + dt_bias) (z > 20 branch), beta = sigmoid(b) rounded to BF16
-      const float z = __bfloat162float(in.act_a[gi]) + in.dt_bias[hv];
-      gate = -expf(in.a_log[hv]) * (z > 20.f ? z : log1pf(expf(z)));
-      beta = __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-__bfloat162float(in.act_b[gi])))));
-    } else {
-      gate = load_gate(in.g, gi, in.gate_fp32);
-      beta = __bfloat162float(in.beta[gi]);
-    }
+    gate = load_gate(in.g, gi, in.gate_fp32);
+    beta = __bfloat162float(in.beta[gi]);
   }
   tc_fence_before();
   __syncthreads();
@@ -261,44 +221,9 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   // ---- phase 2: D1 = [Q;K] K^T
   bool ok = mbar_wait(bar_tma, 0, abort, 1, chunk);
   GDN_PSTAMP(1);
-  if (kFused) {
-    // L2-normalise the 64 Q and 64 K rows in place: 16 lanes per row (8 BF16 = one swizzled 16-byte slot each),
-    // 16 rows per pass; x * rsqrt(sum x^2 + 1e-6) rounded to BF16
-    if (ok) {
-      const int lane16 = tid & 15;
-#pragma unroll
-      for (int pass = 0; pass < 8; ++pass) {
-        const int r = pass * 16 + (tid >> 4), row = r & 63;
-        uint8_t* slot = sm + (r < 64 ? (lane16 < 8 ? L::kQ0 : L::kQ1) : (lane16 < 8 ? L::kK0 : L::kK1)) + row * 128 +
-                        (((lane16 & 7) ^ (row & 7)) << 4);
-        const uint4 x = *reinterpret_cast<const uint4*>(slot);
-        const float f[8] = {bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y),
-                            bf16_lo(x.z), bf16_hi(x.z), bf16_lo(x.w), bf16_hi(x.w)};
-        float square = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) square = fmaf(f[e], f[e], square);
-#pragma unroll
-        for (int d = 8; d; d >>= 1) square += __shfl_xor_sync(0xffffffffu, square, d, 16);
-        const float factor = rsqrtf(square + 1e-6f);
-        *reinterpret_cast<uint4*>(slot) = make_uint4(pack_bf16(f[0] * factor, f[1] * factor), pack_bf16(f[2] * factor, f[3] * factor),
-                                                     pack_bf16(f[4] * factor, f[5] * factor), pack_bf16(f[6] * factor, f[7] * factor));
-      }
-      fence_proxy_async_smem();
-    }
-    __syncthreads();
-    // the walk reads the normalised queries and keys: one CTA per key-head group stores the tiles (rows behind T
-    // are clipped); tm_v doubles as the map of the normalised-query plane in this variant
-    if (tid == 0 && ok && hv % geo.group() == 0) {
-      tma_store_4d(&tm_k, sm + L::kK0, 0, hk, t0, b);
-      tma_store_4d(&tm_k, sm + L::kK1, 64, hk, t0, b);
-      tma_store_4d(&tm_v, sm + L::kQ0, 0, hk, t0, b);
-      tma_store_4d(&tm_v, sm + L::kQ1, 64, hk, t0, b);
-      tma_store_commit();
-    }
-  }
-  if (tid == 0 && ok) {
+  const uint32_t base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);       // warp-uniform, for the descriptors
+  if (warp == 0 && __all_sync(0xffffffffu, ok) && elect_one()) {
     tc_fence_after();
-    const uint32_t base = smem_u32(sm);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       const uint32_t a = base + (ks < 4 ? L::kQ0 : L::kQ1) + (ks & 3) * 32;
@@ -388,8 +313,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
     if (lrow >= 64) not_contraction = !(bi >= 0.f && bi * kk <= 2.f);
   }
-  if (kFused && tid == 0) tma_store_wait_read();     // the Q and K tiles' stores have left shared memory: the
-                                                     // inverse's scratch and the T tiles reuse the Q boxes from here on
   const int chunk_not_contraction = __syncthreads_or(not_contraction);
   ok = __syncthreads_and(ok);                  // uniform from here on: the warp-level barrier below needs that
   GDN_PSTAMP(3);
@@ -522,9 +445,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   GDN_PSTAMP(4);
 
   // ---- phase 5: W^T (into D1's columns, which every thread has read) and U^T
-  if (tid == 0 && ok) {
+  if (warp == 0 && ok && elect_one()) {
     tc_fence_after();
-    const uint32_t base = smem_u32(sm);
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
 #pragma unroll
@@ -776,22 +698,12 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   const int unit = blockIdx.x / parallel, sub = blockIdx.x % parallel;
   const int bh = pair_pass ? unit % heads : unit;
   const int flags = pair_pass ? (unit >= heads ? kWalkHomogeneous : kWalkTail) : in.walk_flags;
-  int b = bh / geo.value_heads;
+  const int b = bh / geo.value_heads;
   const int hv = bh % geo.value_heads;
   const int hk = hv / geo.group();
   int chunks = geo.segment_chunks();                 // this launch walks `chunks` chunks from token t_first on
-  int t_first = geo.chunk_begin * kChunk, tail_valid = kChunk;
+  int t_first = geo.chunk_begin * kChunk;
   long long block0 = (long long)bh * geo.chunks() + geo.chunk_begin;
-  if (geo.varlen) {
-    // packed sequences: one CTA per (sequence, value head); states are indexed by bh = sequence * Hv + hv
-    const int seq = b;
-    const int* prefix = geo.varlen + geo.batch + 1;
-    chunks = prefix[seq + 1] - prefix[seq];
-    t_first = geo.varlen[seq];
-    tail_valid = geo.varlen[seq + 1] - t_first - (chunks - 1) * kChunk;     // rows of the sequence's last chunk
-    block0 = (long long)hv * geo.total_chunks + prefix[seq];
-    b = 0;
-  }
   const float* state_in = geo.first_segment() ? in.initial : ws.carry;
   float* state_out = geo.last_segment() ? in.final_state : ws.carry;
   if (sub > 0) state_in = nullptr;
@@ -831,6 +743,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched early behind prepare: its planes are complete from here on
   if ((flags & kWalkUntilDecayed) && warp == kTmaWarp) {
     // first chunk boundary at which the accumulated decay is below exp(-40): 32 chunks per step, the per-chunk
     // decay exp(p_last) is word 64 of the chunk's gate vector
@@ -1052,16 +965,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       GDN_OSTAMP(1);
       if (c < unstored) continue;
       const int cs = c - unstored;           // count of stored tiles: staging buffers and their barriers follow it
-      if (geo.varlen && c == chunks - 1 && tail_valid < kChunk) {
-        // packed mode, ragged end of a sequence: the rows behind it belong to the next sequence, so the tile
-        // cannot leave through a clipping TMA store; this is the sequence's last chunk, nothing follows it
-        __nv_bfloat16* out = in.output + ((long long)(t_first + c * kChunk) * geo.value_heads + hv) * kDim + v;
-        const long long row = (long long)geo.value_heads * kDim;
-#pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (i < tail_valid) out[i * row] = __float2bfloat16_rn(__uint_as_float(o[i]));
-        break;
-      }
       // stage the tile as two 128-byte-swizzled boxes [token][64 values] and hand it to a TMA store,
       // which also clips the rows of a tail chunk at the sequence end
       uint8_t* stage = sm + L::kOut + (cs & 1) * 2 * kBox + (v >> 6) * kBox + ((v & 7) << 1);
@@ -1152,7 +1055,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     // the compiler knows they are warp-uniform.
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     const uint32_t st0 = __shfl_sync(0xffffffffu, smem_u32(sm), 0);
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       // Descriptors of ring stage 0; stage 1 is a constant further on (the start-address field counts 16-byte units).
       static_assert(L::kStages == 2 && L::kStage % 16 == 0, "descriptor arithmetic below assumes a two-stage ring");
@@ -1240,9 +1143,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 // ======================================================================================= launchers
 int configure_umma() {
   if (int rc = tensor_map_encoder().init()) return rc;
-  cudaError_t e = cudaFuncSetAttribute(prepare_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
-  if (e != cudaSuccess) return int(e);
-  e = cudaFuncSetAttribute(prepare_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
+  cudaError_t e = cudaFuncSetAttribute(prepare_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
   if (e != cudaSuccess) return int(e);
   e = cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
   return int(e);
@@ -1252,62 +1153,51 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
   CUtensorMap tm_q, tm_k, tm_v;
-  const bool fused = in.mixed != nullptr;
-  if (fused) {
-    if (geo.varlen) return int(cudaErrorInvalidValue);
-    // one 2-D map over the packed projection rows; the 4-D map of the normalised-key plane is the store target
-    if (int rc = enc.bf16_2d(&tm_q, in.mixed, uint64_t(in.mixed_stride), uint64_t(geo.batch) * geo.sequence, kChunk)) return rc;
-    if (int rc = enc.bf16_4d(&tm_k, in.k_norm, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-    if (int rc = enc.bf16_4d(&tm_v, in.q_norm, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-  } else {
-    if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.varlen ? 1 : geo.batch, kChunk)) return rc;
-    if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.varlen ? 1 : geo.batch, kChunk)) return rc;
-    if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, geo.varlen ? 1 : geo.batch, kChunk)) return rc;
-  }
+  if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, geo.batch, kChunk)) return rc;
   // W^T planes: [blocks * 128 key rows][64 tokens], one 128-row box per block (the walk loads the same boxes)
   CUtensorMap tm_wh, tm_wl;
   const uint64_t plane_rows = uint64_t(geo.blocks()) * kDim;
   if (int rc = enc.bf16_2d(&tm_wh, ws.w_hi, kChunk, plane_rows, kDim)) return rc;
   if (int rc = enc.bf16_2d(&tm_wl, ws.w_lo, kChunk, plane_rows, kDim)) return rc;
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
-  const unsigned grid = geo.varlen
-      ? (unsigned)((long long)geo.value_heads * geo.segment_chunks())
-      : (unsigned)((long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel));
-  if (fused)
-    prepare_umma_kernel<true><<<grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws);
-  else
-    prepare_umma_kernel<false><<<grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws);
+  const long long grid = (long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel);
+  prepare_umma_kernel<<<(unsigned)grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws);
   return int(cudaGetLastError());
 }
-int launch_prepare_fused(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream) {
-  if (!in.mixed || !in.act_a || !in.act_b || !in.a_log || !in.dt_bias || !in.k_norm || !in.q_norm)
-    return int(cudaErrorInvalidValue);
-  return launch_prepare_umma(in, geo, ws, stream);
-}
 
-int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream) {
+int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, bool early, cudaStream_t stream) {
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
   const uint64_t rows = uint64_t(geo.blocks()) * kChunk;
   CUtensorMap tm_wh, tm_wl, tm_q, tm_k, tm_p, tm_out;
-  if (int rc = enc.bf16_4d(&tm_out, in.output, kDim, geo.value_heads, geo.sequence, geo.varlen ? 1 : geo.batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_out, in.output, kDim, geo.value_heads, geo.sequence, geo.batch, kChunk)) return rc;
   // W^T planes: [blocks * 128 key rows][64 tokens], one 128-row box per block
   if (int rc = enc.bf16_2d(&tm_wh, ws.w_hi, kChunk, 2 * rows, kDim)) return rc;
   if (int rc = enc.bf16_2d(&tm_wl, ws.w_lo, kChunk, 2 * rows, kDim)) return rc;
-  if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.varlen ? 1 : geo.batch, kChunk)) return rc;
-  if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.varlen ? 1 : geo.batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
   if (int rc = enc.bf16_2d(&tm_p, ws.p, kChunk, rows, kChunk)) return rc;
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
-  if (parallel > 1 && (geo.varlen || in.walk_flags || parallel > geo.segment_chunks())) return int(cudaErrorInvalidValue);
-  if ((in.walk_flags & kWalkSelftestStall) && (in.walk_flags != kWalkSelftestStall || geo.varlen)) return int(cudaErrorInvalidValue);
+  if (parallel > 1 && (in.walk_flags || parallel > geo.segment_chunks())) return int(cudaErrorInvalidValue);
+  if ((in.walk_flags & kWalkSelftestStall) && in.walk_flags != kWalkSelftestStall) return int(cudaErrorInvalidValue);
   if ((in.walk_flags & (kWalkTail | kWalkPair)) &&
-      ((in.walk_flags != kWalkTail && in.walk_flags != kWalkPair) || parallel > 1 || geo.varlen || !geo.first_segment() ||
+      ((in.walk_flags != kWalkTail && in.walk_flags != kWalkPair) || parallel > 1 || !geo.first_segment() ||
        !geo.last_segment() || !in.final_state))
     return int(cudaErrorInvalidValue);
   const int per_head = (in.walk_flags & kWalkPair) ? 2 : parallel;
-  walk_umma_kernel<<<geo.batch * geo.value_heads * per_head, kWalkThreads, kWalkSmem, stream>>>(
-      tm_wh, tm_wl, tm_q, tm_k, tm_p, tm_out, in, geo, ws);
-  return int(cudaGetLastError());
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(geo.batch * geo.value_heads * per_head);
+  config.blockDim = dim3(kWalkThreads);
+  config.dynamicSmemBytes = kWalkSmem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = early ? 1 : 0;
+  return int(cudaLaunchKernelEx(&config, walk_umma_kernel, tm_wh, tm_wl, tm_q, tm_k, tm_p, tm_out, in, geo, ws));
 }
 
 namespace {
@@ -1353,7 +1243,7 @@ int launch_walk_stall_selftest(const Inputs& in, const Geometry& geo, const Work
   stalled.walk_flags = kWalkSelftestStall;
   Geometry one = geo;
   one.parallel = 0;
-  const int launched = launch_walk_umma(stalled, one, ws, stream);
+  const int launched = launch_walk_umma(stalled, one, ws, false, stream);
   const int restored = set_spin_limit_on(stream, kProductionPolls);
   return launched ? launched : restored;
 }
