@@ -270,23 +270,18 @@ extern "C" int actlize_la_sm100_select(int b, int t, int hk, int hv, int gate_fp
   for (const PolicyRow& row : kPolicyRows)
     if (row.b == b && row.t == t && row.hk == hk && row.hv == hv)
       return row.config | (row.segments << kSegmentShift) | (row.parallel << kParallelShift);
-  // no measured row: integer rules (sm100_policy.py::default_parallel / default_segments are the same).  Parallel
+  // no measured row: integer rules (sm100_policy.py::default_configuration / default_parallel are the same).  Parallel
   // sub-segments: as many as fill the 148 SMs with one walk CTA each, at least 8 chunks per sub-segment, at most 8.
-  // Sequence segments (prepare of a later segment next to the walk of an earlier one) only pay while the walk
-  // leaves SMs idle, i.e. when the walk is not split.
+  // Family: the two-kernel form for few (head, chunk) blocks, which its prepare kernel has done in two to three waves
+  // and whose walk is the faster one per chunk; at most three chunks are over before its second launch, and with many
+  // blocks its factors' way through memory costs more than the slower chunk period of the single launch.
   const long long heads = (long long)b * hv, chunks = (t + kChunk - 1) / kChunk;
   long long parallel = 148 / heads;
   if (parallel > chunks / 8) parallel = chunks / 8;
   if (parallel > kMaxParallel) parallel = kMaxParallel;
   if (parallel < 1) parallel = 1;
-  int segments = 1;
-  if (heads <= 64 && parallel == 1) {
-    int root = 0;
-    while ((long long)(root + 1) * (root + 1) <= chunks / 8) ++root;
-    segments = root < 1 ? 1 : (root > 8 ? 8 : root);
-  }
-  if (kPolicyDefault == kFused) segments = 1;
-  return kPolicyDefault | (segments << kSegmentShift) | (int(parallel) << kParallelShift);
+  const int family = heads < 64 && chunks > 3 && heads * chunks < 1024 ? 1 : kFused;
+  return family | (1 << kSegmentShift) | (int(parallel) << kParallelShift);
 }
 
 extern "C" long long actlize_la_sm100_workspace_bytes(int b, int t, int hk, int hv, int config) {

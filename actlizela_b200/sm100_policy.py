@@ -74,6 +74,16 @@ def default_segments(batch, length, value_heads):
     return max(1, min(8, isqrt(chunks // 8)))
 
 
+def default_configuration(batch, length, value_heads):
+    """Kernel family for a shape without a measured row.  Few (head, chunk) blocks: the two-kernel form, whose prepare
+    kernel takes them all at once (444 fit on the device) and whose walk then needs 4.4k cycles a chunk; the single-launch
+    form has a period of 7.1k but no second launch, no factors through memory and no prepare time that grows with the blocks.
+    The two meet near 1024 blocks (6, 16, 32, 48 heads: at 7000, 3900, 1950, 1500 tokens), up to three chunks the
+    second launch is all that counts, and from 64 heads on prepare is never short.  The native selector computes the same."""
+    heads, chunks = batch * value_heads, (length + 63) // 64
+    return "umma" if heads < 64 and chunks > 3 and heads * chunks < 1024 else "fused"
+
+
 def tensor_backend(q):
     """Device tensor -> backend name; only capability (10,0) is admitted, nothing is guessed."""
     device = getattr(q, "device", None)
@@ -112,8 +122,8 @@ def select(shape, profile):
         if tuple(row["shape"]) == tuple(shape[:4]):
             return Selection(row["configuration"], "b200-measured-shape", data["id"],
                              int(row.get("segments", 1)), int(row.get("parallel", 1)))
-    return Selection(data["default"], "unmeasured-shape-default", data["id"],
-                     default_segments(shape[0], shape[1], shape[3]) if data["default"] == "umma" else 1, default_parallel(shape[0], shape[1], shape[3]))
+    return Selection(default_configuration(shape[0], shape[1], shape[3]), "unmeasured-shape-default", data["id"], 1,
+                     default_parallel(shape[0], shape[1], shape[3]))
 
 
 _SELECTIONS = {}

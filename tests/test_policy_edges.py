@@ -1,0 +1,15 @@
+"""The rule that chooses between the two tensor-core forms, at its edges, on both sides of the library boundary."""
+import pytest
+
+from actlizela_b200 import sm100_policy
+
+from test_host_contract import B200
+
+
+@pytest.mark.parametrize("shape,family", [((1, 192, 2, 4), "fused"), ((1, 193, 2, 4), "umma"), ((1, 449, 9, 63), "umma"),
+                                          ((1, 449, 16, 64), "fused"), ((1, 64 * 255, 2, 4), "umma"), ((1, 64 * 255 + 1, 2, 4), "fused"),
+                                          ((31, 64 * 33, 1, 1), "umma"), ((31, 64 * 33 + 1, 1, 1), "fused")])
+def test_family_rule(shape, family, native_library):
+    choice = sm100_policy.select((*shape, 128, 128), B200)
+    assert choice.configuration == family and choice.segments == 1
+    assert native_library.lib.actlize_la_sm100_select(*shape, 1) == choice.configuration_id
