@@ -1,9 +1,9 @@
 """The rule that chooses between the two tensor-core forms, at its edges, on both sides of the library boundary."""
 import pytest
 
-from actlizela_b200 import sm100_policy
+from actlizela_b200 import device, sm100_policy
 
-from test_host_contract import B200
+B200 = device.DeviceProfile("NVIDIA B200", 148, (10, 0))
 
 
 @pytest.mark.parametrize("shape,family", [((1, 192, 2, 4), "fused"), ((1, 193, 2, 4), "umma"), ((1, 449, 9, 63), "umma"),
