@@ -5,6 +5,9 @@
 //
 // The arithmetic is that of prepare_umma_kernel and walk_umma_kernel (gdn_umma.cu), operation for operation and in
 // the same order, so both paths give the same bits; orientation and precision are explained there.
+//
+// Bound: the chunk period, 7.1k cycles (B1 T8192, 32 value heads on 128 CTAs: 172 us, 228 as prepare + walk; B8 T4096: 566
+// us, 855).  Of it the state chain takes 5k; the rest is the latency of the preparation, of which two are in flight.
 #include "umma_math.cuh"
 
 namespace gdn_sm100 {

@@ -32,7 +32,8 @@ extern "C" {
 
 /* Kernel configurations of the static shape table (see sm100_policy.json). */
 #define ACTLIZE_LA_SM100_CONFIG_SIMT 0      /* FP32 CUDA-core kernels: diagnostic / cross-check */
-#define ACTLIZE_LA_SM100_CONFIG_UMMA 1      /* tcgen05 + TMEM + TMA kernels */
+#define ACTLIZE_LA_SM100_CONFIG_UMMA 1      /* tcgen05 + TMEM + TMA: prepare kernel, then chunk walk */
+#define ACTLIZE_LA_SM100_CONFIG_FUSED 4     /* the same arithmetic in a single launch: no factors through memory */
 /* ids 2 and 3 mix the stages (2: CUDA-core prepare + tcgen05 walk, 3: the reverse) for diagnosis.
  * OR-ing one of the following into `config` restricts forward_prepared to a single stage
  * (per-kernel timing; the walk-only form needs a workspace filled by an earlier call). */
@@ -84,13 +85,16 @@ int actlize_la_sm100_configure(void);
 int actlize_la_sm100_select(int batch, int sequence, int key_heads, int value_heads, int gate_fp32);
 
 /* Bytes of caller-owned scratch that forward_prepared needs for this geometry and
- * configuration (the WY factors of every chunk); negative for an unsupported geometry.
+ * configuration (the WY factors of every chunk; for the single-launch form flag words only); negative for an unsupported geometry.
  * Replaces the Python-side workspace table gdn_core_workspace_specs
  * (actlize_la/serving/gdn_core.py:14-22). */
 long long actlize_la_sm100_workspace_bytes(int batch, int sequence, int key_heads, int value_heads,
                                            int config);
 
-/* Complete forward on caller-owned buffers: prepare kernel (per-chunk gate prefix, decay-masked
+/* Complete forward on caller-owned buffers.  Configuration 4: one kernel, in which every CTA prepares the chunks of a head
+ * and walks them (one segment, no stage bits; the sub-segment field says only whether heads may be cut into pieces, 0 or
+ * 1 = no, and the launcher chooses how many; a second launch walks again the heads for which a piece met a token that is
+ * no contraction, and leaves at once when there is none).  The others: prepare kernel (per-chunk gate prefix, decay-masked
  * K.K^T, unit-lower-triangular inverse, WY factors) followed by the sequential chunk walk.
  * `config` is the value returned by actlize_la_sm100_select: kernel family in bits 0..3, number of
  * sequence segments in bits 8..15, number of parallel sub-segments of the walk in bits 16..19 (tcgen05 family only;
@@ -234,12 +238,12 @@ int actlize_la_sm100_selftest_walk_stall(
 
 /* The forward on the raw projection outputs of the layer: the step before the path (Q/K L2-normalisation, gate
  * activation g = -exp(A_log) softplus(a + dt_bias), beta = sigmoid(b); csrc/serving/prefill.cu:45-70,
- * csrc/serving/runtime.cuh:48-52) is done inside the tcgen05 prepare kernel instead of by a kernel of its own
+ * csrc/serving/runtime.cuh:48-52) is done inside the single-launch kernel instead of by a kernel of its own
  * (actlize_la_sm100_prepare_inputs): `mixed` is BF16 [B*T][mixed_row_stride] with the row layout
  * [Hk q vectors | Hk k vectors | Hv v vectors] x 128, `a` and `b` are BF16 [B*T][Hv], `a_log`, `dt_bias` FP32 [Hv].
  * Same results, bit for bit, as prepare_inputs followed by forward_prepared with an FP32 gate.  `config` as returned
- * by actlize_la_sm100_select (tcgen05 configuration, segments allowed, no stage bits); the workspace
- * (actlize_la_sm100_projections_workspace_bytes) also holds the normalised queries and keys for the walk.  Rows behind a batch
+ * by actlize_la_sm100_select (a tensor-core configuration, no stage bits; both families run the single-launch kernel
+ * here); workspace: actlize_la_sm100_projections_workspace_bytes, flag words only.  Rows behind a batch
  * element's end inside its last chunk are the next element's tokens and meet exact zeros: inputs must be finite. */
 long long actlize_la_sm100_projections_workspace_bytes(int b, int t, int hk, int hv, int config);
 int actlize_la_sm100_forward_projections(
@@ -253,11 +257,11 @@ int actlize_la_sm100_forward_projections(
  * marks the boundaries; initial_states / final_states are FP32 [n_seqs,Hv,128,128] (nullable).  Every sequence
  * is chunked from its own start, an empty sequence passes its state through.  The reference has no such entry:
  * its serving prefill pads the requests into a fixed [R,W] batch first (csrc/serving/prefill.cu:196-255,
- * csrc/serving/abi.h:48-56); this entry removes the padding.  Two launches (tcgen05 prepare + walk) on `stream`
- * plus one small host-to-device copy of the offsets table (from pageable memory: not for stream capture).
+ * csrc/serving/abi.h:48-56); this entry removes the padding.  One launch on `stream`
+ * plus one small host-to-device copy of the offsets (from pageable memory: not for stream capture).
  * Rows behind a sequence's end inside its last chunk are the next sequence's tokens; they are multiplied by
  * exact zeros, so all inputs must be finite.  `workspace` needs actlize_la_sm100_varlen_workspace_bytes(...)
- * bytes, 256-byte aligned.  Returns 0 or a cudaError_t value. */
+ * bytes (the offsets), 256-byte aligned.  Returns 0 or a cudaError_t value. */
 long long actlize_la_sm100_varlen_workspace_bytes(long long total_tokens, int n_seqs, int hk, int hv);
 int actlize_la_sm100_forward_varlen(
     const void* q, const void* k, const void* v, const void* g, const void* beta,
@@ -266,12 +270,9 @@ int actlize_la_sm100_forward_varlen(
     const int* cu_seqlens_host, int n_seqs, int hk, int hv, int gate_fp32, void* stream);
 
 /* The packed forward with the offsets on the DEVICE: cu_seqlens_device[0..n_seqs] are int32 in device memory, as a
- * serving scheduler produces them; nothing is read on the host, nothing is allocated, and the call consists of kernel
- * launches only (a one-thread kernel builds the offsets table, then the two tcgen05 kernels), so it can be captured
- * in a CUDA graph.  `total_tokens` is the token dimension of the tensors.  Offsets are forced into
- * 0 <= ... <= total_tokens and made non-decreasing on the device; tokens behind the last offset are not written.
- * Grids and workspace are sized for the upper bound ceil(total/64) + n_seqs chunks
- * (actlize_la_sm100_varlen_workspace_bytes already returns that). */
+ * serving scheduler produces them; nothing is read on the host, nothing is allocated, and the call is one kernel
+ * launch, so it can be captured in a CUDA graph.  `total_tokens` is the token dimension of the tensors.  Offsets are forced into
+ * 0 <= ... <= total_tokens and made non-decreasing on the device; tokens behind the last offset are not written. */
 int actlize_la_sm100_forward_varlen_device(
     const void* q, const void* k, const void* v, const void* g, const void* beta,
     const float* initial_states, void* output, float* final_states,
