@@ -72,10 +72,11 @@ int segments_of(int config, const Geometry& geo) {
   return segments > chunks ? chunks : segments;
 }
 
-// workspace a call needs: the factors of every block, or (single-launch form) the flag words of the sub-segments
-long long scratch_bytes(const Geometry& geo, int config, int segments) {
+// workspace a call needs: the factors of every block; single-launch form: its flag words and, when heads may be cut, room
+// for the factors of those that turn out not to decay (not on raw projections, where that kernel walks them itself)
+long long scratch_bytes(const Geometry& geo, int config, int segments, bool raw = false) {
   if (!is_fused(config)) return workspace_bytes(geo, segments);
-  return fused_workspace_bytes();
+  return fused_workspace_bytes() + (raw || parallel_of(config, geo.chunks()) == 1 ? 0 : workspace_bytes(geo, 1));
 }
 
 // Second stream and events of the segmented forward, created by configure() for the current device.
@@ -293,7 +294,7 @@ extern "C" long long actlize_la_sm100_workspace_bytes(int b, int t, int hk, int 
 extern "C" int actlize_la_sm100_launches_per_forward(int config) {
   if (!config_ok(config)) return -1;
   if (config & kStageMask) return 1;
-  if (is_fused(config)) return ((config >> kParallelShift) & 0xf) > 1 ? 2 : 1;
+  if (is_fused(config)) return ((config >> kParallelShift) & 0xf) > 1 ? 3 : 1;
   const int segments = (config >> kSegmentShift) & 0xff;
   return ((config & 0xf) == 1 && segments > 1) ? 2 * segments : 2;
 }
@@ -385,7 +386,8 @@ extern "C" int actlize_la_sm100_forward_prepared(
 namespace {
 int run_fused(const Inputs& in, Geometry geo, int config, void* workspace, cudaStream_t stream) {
   geo.parallel = parallel_of(config, geo.segment_chunks());
-  return launch_forward_fused(in, geo, static_cast<int*>(workspace), stream);
+  const Workspace ws = carve_workspace(static_cast<char*>(workspace) + fused_workspace_bytes(), geo);
+  return launch_forward_fused(in, geo, static_cast<int*>(workspace), ws, stream);
 }
 int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config, int segments, cudaStream_t stream) {
   if (segments > 1) {
@@ -439,7 +441,7 @@ extern "C" long long actlize_la_sm100_projections_workspace_bytes(int b, int t, 
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config) || ((config & 0xf) != 1 && !is_fused(config)) ||
       (config & (kStageMask | kWalkFlagMask)))
     return -1;
-  return scratch_bytes(Geometry{b, t, hk, hv}, (config & ~0xf) | kFused, 1);
+  return scratch_bytes(Geometry{b, t, hk, hv}, (config & ~0xf) | kFused, 1, true);
 }
 
 extern "C" int actlize_la_sm100_forward_projections(
@@ -507,7 +509,7 @@ extern "C" int actlize_la_sm100_forward_varlen(
   const Inputs in{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                   static_cast<const __nv_bfloat16*>(v), g, static_cast<const __nv_bfloat16*>(beta),
                   initial_states, static_cast<__nv_bfloat16*>(output), final_states, gate_fp32 ? 1 : 0};
-  return launch_forward_fused(in, geo, nullptr, stream);
+  return launch_forward_fused(in, geo, nullptr, Workspace{}, stream);
 }
 
 extern "C" int actlize_la_sm100_forward_varlen_device(
@@ -529,7 +531,7 @@ extern "C" int actlize_la_sm100_forward_varlen_device(
   const Inputs in{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                   static_cast<const __nv_bfloat16*>(v), g, static_cast<const __nv_bfloat16*>(beta),
                   initial_states, static_cast<__nv_bfloat16*>(output), final_states, gate_fp32 ? 1 : 0};
-  return launch_forward_fused(in, geo, nullptr, stream);
+  return launch_forward_fused(in, geo, nullptr, Workspace{}, stream);
 }
 
 namespace {

@@ -165,15 +165,22 @@ __device__ __forceinline__ float chunk_prefix64(float x, int tid, float* carry) 
 int launch_prepare_simt(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int launch_walk_simt(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int configure_simt();
-int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
+// Heads that a single-launch forward with cut heads left for the two kernels: flags[head * pieces + piece] != 0 for some
+// piece > 0.  flags == nullptr: every head, the ordinary launch.
+constexpr int kMaxSms = 256;       // CTAs of a single-launch forward at most: its flag words
+struct Repair {
+  const int* flags = nullptr;
+  int pieces = 0, sms = 0;
+};
+int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaStream_t, const Repair& = {});
 // `early`: the kernel in front of it on the stream is this call's prepare kernel, which lets it set itself up beside it
-int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, bool early, cudaStream_t);
+int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, bool early, cudaStream_t, const Repair& = {});
 int configure_umma();
 // single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces; `flags` is scratch of
-// fused_workspace_bytes
+// fused_workspace_bytes, the workspace (unless the inputs are raw projections) takes the factors of heads it cannot cut
 int configure_fused();
 long long fused_workspace_bytes();
-int launch_forward_fused(const Inputs&, const Geometry&, int* flags, cudaStream_t);
+int launch_forward_fused(const Inputs&, const Geometry&, int* flags, const Workspace&, cudaStream_t);
 int read_fused_plan_counts(int* host_out2, int reset);
 int set_status_mirror_fused(int* device_pointer);
 int clear_device_status_fused();

@@ -40,7 +40,7 @@ constexpr int kThreads = 1024, kPrepThreads = 256;
 constexpr int kIssueWarp = 0, kPlanWarp = 1, kScaleWarp = 2, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
 constexpr int kRing = 3;      // Q/K tiles, P tiles, gate vectors: one chunk in the chain, two in preparation
 constexpr int kItems = 4;     // work items announced ahead
-constexpr int kMaxSms = 256;  // CTAs of a launch at most: the flag words
+
 
 struct Smem {
   static constexpr int kKQStage = 4 * kBox;                       // [Q0 K0 Q1 K1]: Q over K per 64-column half
@@ -243,10 +243,11 @@ struct ItemCursor {
 // What a launch walks: the units of the grid, a (batch or sequence, value head) each, or with `pieces` > 1 one of its
 // sub-segments (see walk_umma_kernel), at most one per CTA.  The decay part of the sub-segments' conditions is read off
 // the gates up front, while the contraction part (beta |k|^2 in [0, 2]) shows only when a chunk is prepared: every CTA
-// records what it saw in `flags`, and a second launch of the same kernel (`serial_pass`) walks the heads for which some
-// sub-segment saw a violation again, whole, by one CTA each, and leaves at once otherwise.
+// records what it saw in `flags`.  The heads that could not be cut are left to the two kernels of gdn_umma.cu (`leave`; a
+// flag word of 2), which also repair those with a violation; on raw projections, which only this kernel reads, their first
+// CTA walks them whole and a second launch of this kernel (`serial_pass`) repairs.
 struct Plan {
-  int units, pieces, serial_pass;
+  int units, pieces, serial_pass, leave;
   int* flags;      // [batch * value_heads][pieces], written when pieces > 1
 };
 constexpr int kLeastPiece = 8;       // chunks: a piece has to outlast the decay, which takes about four at typical gates
@@ -657,10 +658,10 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           const bool serial = __ballot_sync(0xffffffffu, lane >= kChainWarp && bar->slow[lane]);
           if (lane == 0) {
             if (sub == 0) atomicAdd(&g_fused_plan_counts[serial ? 1 : 0], 1);
-            plan.flags[unit] = 0;
+            plan.flags[unit] = serial && plan.leave ? 2 : 0;
           }
           if (serial) {
-            if (sub) continue;
+            if (sub || plan.leave) continue;
           } else {
             const int c0 = sub_segment_begin(chunks, sub, plan.pieces), c1 = sub_segment_begin(chunks, sub + 1, plan.pieces);
             own = c1 - c0;
@@ -1219,7 +1220,7 @@ int configure_fused() {
 long long fused_workspace_bytes() { return kMaxSms * (long long)sizeof(int); }
 
 // `flags`: fused_workspace_bytes() bytes of scratch (may be null for an unsplit walk)
-int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cudaStream_t stream) {
+int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, const Workspace& ws, cudaStream_t stream) {
   Plan plan{};
   const int heads = geo.batch * geo.value_heads, sms = sm_count(), chunks = geo.segment_chunks();
   const bool split = geo.parallel > 1 && heads > 0;
@@ -1236,9 +1237,19 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cuda
     if (plan.pieces < 1) plan.pieces = 1;
     plan.units = heads * plan.pieces;
   }
+  plan.leave = plan.pieces > 1 && !in.mixed;
   const auto go = in.mixed ? launch<true> : launch<false>;
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
   if (plan.pieces == 1) return 0;
+  if (plan.leave) {
+    // Heads that may not be cut: their chunks prepared by all SMs, then walked at 4.4k cycles a chunk instead of 7.1k by one
+    // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now @@).  Two launches that leave at once otherwise.
+    Geometry whole = geo;
+    whole.parallel = 0;
+    const Repair left{flags, plan.pieces, sms};
+    if (int rc = launch_prepare_umma(in, whole, ws, stream, left)) return rc;
+    return launch_walk_umma(in, whole, ws, true, stream, left);
+  }
   plan.serial_pass = 1;
   plan.units = heads;
   return go(in, geo, plan, heads < sms ? heads : sms, stream);

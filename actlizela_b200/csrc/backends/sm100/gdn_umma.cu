@@ -129,10 +129,13 @@ static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit
 #define GDN_PSTAMP(slot)
 #endif
 
+// kRepair: behind a single-launch forward that left some heads (Repair::flags); a grid that just fills the device takes
+// the chunks of those heads in turn, and leaves at once when there are none.
+template <bool kRepair>
 __global__ void __launch_bounds__(kPrepThreads, 3)
 prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_wh,
-                    const __grid_constant__ CUtensorMap tm_wl, Inputs in, Geometry geo, Workspace ws) {
+                    const __grid_constant__ CUtensorMap tm_wl, Inputs in, Geometry geo, Workspace ws, Repair left) {
   // Indexing the declared array (no integer round trip) keeps these accesses in the shared state space.
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
@@ -153,19 +156,51 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int chunks = geo.chunks(), seg_chunks = geo.segment_chunks();
-  // Block order = reverse of the order in which the walk consumes the blocks: the walk's CTAs (one per
-  // (batch, head) and parallel sub-segment) all start at the first chunk of their sub-segment, so the blocks
-  // prepared LAST are the leading chunks of every sub-segment of every head, and the walk finds them in L2.
-  // The grid covers heads x sub-segments x longest sub-segment; a slot behind a shorter sub-segment's end is empty.
-  const int parallel = geo.parallel > 1 ? geo.parallel : 1;
-  // (The cut is an even one; the walk's own cut, sub_segment_begin, differs from it by a few chunks at most.)
-  const int longest = (seg_chunks + parallel - 1) / parallel;
-  const int units = geo.batch * geo.value_heads * parallel;
-  const int offset = longest - 1 - int(blockIdx.x) / units, unit = int(blockIdx.x) % units;
-  const int sub = unit % parallel;
-  const int sub_begin = int((long long)seg_chunks * sub / parallel), sub_end = int((long long)seg_chunks * (sub + 1) / parallel);
-  if (sub_begin + offset >= sub_end) return;
-  const int bh = unit / parallel, chunk = geo.chunk_begin + sub_begin + offset;
+  __shared__ int s_left[kRepair ? kMaxSms : 1], s_count;
+  asm volatile("griddepcontrol.launch_dependents;");      // the walk sets itself up as SMs fall free
+  if constexpr (kRepair) {
+    const int heads = geo.batch * geo.value_heads;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!__syncthreads_or(tid < heads * left.pieces && tid % left.pieces && left.flags[tid])) return;
+    if (warp == 0) {
+      int n = 0;
+      for (int h0 = 0; h0 < heads; h0 += 32) {
+        const int h = h0 + tid;
+        bool mine = false;
+        if (h < heads)
+          for (int r = 1; r < left.pieces; ++r) mine |= left.flags[h * left.pieces + r] != 0;
+        const unsigned all = __ballot_sync(0xffffffffu, mine);
+        if (mine) s_left[n + __popc(all & ((1u << tid) - 1))] = h;
+        n += __popc(all);
+      }
+      if (tid == 0) s_count = n;
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int round = 0;; ++round) {
+  int bh, chunk;
+  if constexpr (kRepair) {
+    const int at = int(blockIdx.x) + round * int(gridDim.x);
+    if (at >= s_count * chunks) break;
+    bh = s_left[at % s_count];
+    chunk = chunks - 1 - at / s_count;
+  } else {
+    // Block order = reverse of the order in which the walk consumes the blocks: the walk's CTAs (one per
+    // (batch, head) and parallel sub-segment) all start at the first chunk of their sub-segment, so the blocks
+    // prepared LAST are the leading chunks of every sub-segment of every head, and the walk finds them in L2.
+    // The grid covers heads x sub-segments x longest sub-segment; a slot behind a shorter sub-segment's end is empty.
+    const int parallel = geo.parallel > 1 ? geo.parallel : 1;
+    // (The cut is an even one; the walk's own cut, sub_segment_begin, differs from it by a few chunks at most.)
+    const int longest = (seg_chunks + parallel - 1) / parallel;
+    const int units = geo.batch * geo.value_heads * parallel;
+    const int offset = longest - 1 - int(blockIdx.x) / units, unit = int(blockIdx.x) % units;
+    const int sub = unit % parallel;
+    const int sub_begin = int((long long)seg_chunks * sub / parallel), sub_end = int((long long)seg_chunks * (sub + 1) / parallel);
+    if (sub_begin + offset >= sub_end) return;
+    bh = unit / parallel;
+    chunk = geo.chunk_begin + sub_begin + offset;
+  }
   const int b = bh / geo.value_heads, hv = bh % geo.value_heads;
   const int hk = hv / geo.group();
   const int t0 = chunk * kChunk, t_end = geo.sequence;
@@ -175,12 +210,13 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const long long t_begin = clock64();
 #endif
 
-  asm volatile("griddepcontrol.launch_dependents;");      // the walk sets itself up as SMs fall free
   if (tid == 0) {
-    mbar_init(bar_tma, 1);
-    mbar_init(bar_mma, 1);
-    *abort_word = 0;
-    fence_barrier_init();
+    if (!kRepair || round == 0) {
+      mbar_init(bar_tma, 1);
+      mbar_init(bar_mma, 1);
+      *abort_word = 0;
+      fence_barrier_init();
+    }
     // the input tiles do not depend on tensor memory: start them before the allocation
     mbar_arrive_expect_tx(bar_tma, 6 * kBox);
     tma_load_4d(sm + L::kQ0, &tm_q, bar_tma, 0, hk, t0, b);
@@ -190,7 +226,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tma_load_4d(sm + L::kV0, &tm_v, bar_tma, 0, hv, t0, b);
     tma_load_4d(sm + L::kV1, &tm_v, bar_tma, 64, hv, t0, b);
   }
-  if (warp == 1) {
+  if (warp == 1 && (!kRepair || round == 0)) {
     tmem_alloc(tmem_slot, kPrepTmemCols);
     tmem_relinquish();
   }
@@ -219,7 +255,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
 
   // ---- phase 2: D1 = [Q;K] K^T
-  bool ok = mbar_wait(bar_tma, 0, abort, 1, chunk);
+  bool ok = mbar_wait(bar_tma, kRepair ? round & 1 : 0, abort, 1, chunk);
   GDN_PSTAMP(1);
   const uint32_t base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);       // warp-uniform, for the descriptors
   if (warp == 0 && __all_sync(0xffffffffu, ok) && elect_one()) {
@@ -529,7 +565,11 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, kPrepTmemCols);
+  if (!kRepair || !ok) break;
+  tc_fence_after();
+  }
+  // (a repair CTA without a block of its own has allocated nothing)
+  if (warp == 1 && (!kRepair || int(blockIdx.x) < s_count * chunks)) tmem_dealloc(*tmem_slot, kPrepTmemCols);
 }
 #undef GDN_PSTAMP
 
@@ -667,7 +707,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1)
 walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constant__ CUtensorMap tm_wl,
                  const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_out,
-                 Inputs in, Geometry geo, Workspace ws) {
+                 Inputs in, Geometry geo, Workspace ws, Repair left) {
   // Indexing the declared array (no integer round trip) keeps these accesses in the shared state space.
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
@@ -698,6 +738,16 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   const int unit = blockIdx.x / parallel, sub = blockIdx.x % parallel;
   const int bh = pair_pass ? unit % heads : unit;
   const int flags = pair_pass ? (unit >= heads ? kWalkHomogeneous : kWalkTail) : in.walk_flags;
+  if (left.flags) {
+    // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: it does not decay)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int mark = tid > 0 && tid < left.pieces ? left.flags[bh * left.pieces + tid] : 0;
+    if (!__syncthreads_or(mark)) return;
+    if (!__syncthreads_or(mark == 2) && tid == 0) {
+      atomicAdd(&g_walk_plan_counts[0], -1);
+      atomicAdd(&g_walk_plan_counts[1], 1);
+    }
+  }
   const int b = bh / geo.value_heads;
   const int hv = bh % geo.value_heads;
   const int hk = hv / geo.group();
@@ -1143,13 +1193,33 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 // ======================================================================================= launchers
 int configure_umma() {
   if (int rc = tensor_map_encoder().init()) return rc;
-  cudaError_t e = cudaFuncSetAttribute(prepare_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
+  cudaError_t e = cudaFuncSetAttribute(prepare_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
+  if (e != cudaSuccess) return int(e);
+  e = cudaFuncSetAttribute(prepare_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
   if (e != cudaSuccess) return int(e);
   e = cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
   return int(e);
 }
 
-int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream) {
+namespace {
+// a launch that may start before the kernel in front of it has ended (it waits for it inside)
+template <typename... Params, typename... Args>
+int launch_early(void (*kernel)(Params...), unsigned grid, int threads, int smem, bool early, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = early ? 1 : 0;
+  return int(cudaLaunchKernelEx(&config, kernel, args...));
+}
+}  // namespace
+
+int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream, const Repair& left) {
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
   CUtensorMap tm_q, tm_k, tm_v;
@@ -1163,11 +1233,16 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   if (int rc = enc.bf16_2d(&tm_wl, ws.w_lo, kChunk, plane_rows, kDim)) return rc;
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
   const long long grid = (long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel);
-  prepare_umma_kernel<<<(unsigned)grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws);
-  return int(cudaGetLastError());
+  if (!left.flags) {
+    prepare_umma_kernel<false><<<(unsigned)grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
+    return int(cudaGetLastError());
+  }
+  const long long resident = 3LL * left.sms;
+  return launch_early(prepare_umma_kernel<true>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
+                      tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
 }
 
-int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, bool early, cudaStream_t stream) {
+int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, bool early, cudaStream_t stream, const Repair& left) {
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
   const uint64_t rows = uint64_t(geo.blocks()) * kChunk;
@@ -1187,17 +1262,8 @@ int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws,
        !geo.last_segment() || !in.final_state))
     return int(cudaErrorInvalidValue);
   const int per_head = (in.walk_flags & kWalkPair) ? 2 : parallel;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(geo.batch * geo.value_heads * per_head);
-  config.blockDim = dim3(kWalkThreads);
-  config.dynamicSmemBytes = kWalkSmem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &attribute;
-  config.numAttrs = early ? 1 : 0;
-  return int(cudaLaunchKernelEx(&config, walk_umma_kernel, tm_wh, tm_wl, tm_q, tm_k, tm_p, tm_out, in, geo, ws));
+  return launch_early(walk_umma_kernel, geo.batch * geo.value_heads * per_head, kWalkThreads, kWalkSmem, early, stream,
+                      tm_wh, tm_wl, tm_q, tm_k, tm_p, tm_out, in, geo, ws, left);
 }
 
 namespace {
