@@ -281,7 +281,7 @@ extern "C" int actlize_la_sm100_select(int b, int t, int hk, int hv, int gate_fp
   if (parallel > chunks / 8) parallel = chunks / 8;
   if (parallel > kMaxParallel) parallel = kMaxParallel;
   if (parallel < 1) parallel = 1;
-  const int family = heads < 64 && chunks > 3 && heads * chunks < 1024 ? 1 : kFused;
+  const int family = heads < 64 && chunks > 3 && heads * chunks < 1280 ? 1 : kFused;
   return family | (1 << kSegmentShift) | (int(parallel) << kParallelShift);
 }
 

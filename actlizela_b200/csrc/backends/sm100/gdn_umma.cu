@@ -157,10 +157,10 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5;
   const int chunks = geo.chunks(), seg_chunks = geo.segment_chunks();
   __shared__ int s_left[kRepair ? kMaxSms : 1], s_count;
+  if (kRepair) asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");      // the walk sets itself up as SMs fall free
   if constexpr (kRepair) {
     const int heads = geo.batch * geo.value_heads;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!__syncthreads_or(tid < heads * left.pieces && tid % left.pieces && left.flags[tid])) return;
     if (warp == 0) {
       int n = 0;
@@ -740,8 +740,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   const int flags = pair_pass ? (unit >= heads ? kWalkHomogeneous : kWalkTail) : in.walk_flags;
   if (left.flags) {
     // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: it does not decay)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int mark = tid > 0 && tid < left.pieces ? left.flags[bh * left.pieces + tid] : 0;
+    // (the repairing prepare kernel lets this one start when the flags are final, so they need no further wait)
+    const int mark = tid > 0 && tid < left.pieces ? *reinterpret_cast<const volatile int*>(left.flags + bh * left.pieces + tid) : 0;
     if (!__syncthreads_or(mark)) return;
     if (!__syncthreads_or(mark == 2) && tid == 0) {
       atomicAdd(&g_walk_plan_counts[0], -1);

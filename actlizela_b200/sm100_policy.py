@@ -78,10 +78,10 @@ def default_configuration(batch, length, value_heads):
     """Kernel family for a shape without a measured row.  Few (head, chunk) blocks: the two-kernel form, whose prepare
     kernel takes them all at once (444 fit on the device) and whose walk then needs 4.4k cycles a chunk; the single-launch
     form has a period of 7.1k but no second launch, no factors through memory and no prepare time that grows with the blocks.
-    The two meet near 1024 blocks (6, 16, 32, 48 heads: at 7000, 3900, 1950, 1500 tokens), up to three chunks the
+    The two meet near 1280 blocks (16, 32, 48 heads: at 4700, 2800, 1750 tokens), up to three chunks the
     second launch is all that counts, and from 64 heads on prepare is never short.  The native selector computes the same."""
     heads, chunks = batch * value_heads, (length + 63) // 64
-    return "umma" if heads < 64 and chunks > 3 and heads * chunks < 1024 else "fused"
+    return "umma" if heads < 64 and chunks > 3 and heads * chunks < 1280 else "fused"
 
 
 def tensor_backend(q):

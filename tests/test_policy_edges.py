@@ -7,8 +7,8 @@ B200 = device.DeviceProfile("NVIDIA B200", 148, (10, 0))
 
 
 @pytest.mark.parametrize("shape,family", [((1, 192, 2, 4), "fused"), ((1, 193, 2, 4), "umma"), ((1, 449, 9, 63), "umma"),
-                                          ((1, 449, 16, 64), "fused"), ((1, 64 * 255, 2, 4), "umma"), ((1, 64 * 255 + 1, 2, 4), "fused"),
-                                          ((31, 64 * 33, 1, 1), "umma"), ((31, 64 * 33 + 1, 1, 1), "fused")])
+                                          ((1, 449, 16, 64), "fused"), ((1, 64 * 319, 2, 4), "umma"), ((1, 64 * 319 + 1, 2, 4), "fused"),
+                                          ((31, 64 * 41, 1, 1), "umma"), ((31, 64 * 41 + 1, 1, 1), "fused")])
 def test_family_rule(shape, family, native_library):
     choice = sm100_policy.select((*shape, 128, 128), B200)
     assert choice.configuration == family and choice.segments == 1
