@@ -29,6 +29,8 @@ prepare_inputs_kernel(const __nv_bfloat16* __restrict__ mixed, long long mixed_s
                       const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                       __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v,
                       float* __restrict__ g, __nv_bfloat16* __restrict__ beta, long long tokens, int hk, int hv) {
+  wait_for_previous_kernel();
+  dependents_may_start();
   const int heads = 2 * hk + hv;
   const int lane = threadIdx.x & 15;
   const long long first = (long long)blockIdx.x * (16 * kPrepSweeps) + (threadIdx.x >> 4);
@@ -86,6 +88,8 @@ decode_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
                    const __nv_bfloat16* __restrict__ beta, float* __restrict__ state,
                    __nv_bfloat16* __restrict__ out, int hk, int hv, int gate_fp32) {
   __shared__ float sk[kDim], sq[kDim], partial[2][kDim];
+  wait_for_previous_kernel();
+  dependents_may_start();
   const int bh = blockIdx.x, col = threadIdx.x & (kDim - 1), half = threadIdx.x >> 7;
   const int bidx = bh / hv, vh = bh % hv;
   const long long qk_at = ((long long)bidx * hk + vh / (hv / hk)) * kDim;
@@ -131,6 +135,8 @@ verify_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
                    __nv_bfloat16* __restrict__ out, float* __restrict__ delta_out, int width, int hk, int hv,
                    int gate_fp32) {
   __shared__ float sk[2][kDim], sq[2][kDim], partial[2][kDim];
+  wait_for_previous_kernel();
+  dependents_may_start();
   const int bh = blockIdx.x, col = threadIdx.x & (kDim - 1), half = threadIdx.x >> 7;
   const int bidx = bh / hv, vh = bh % hv, kh = vh / (hv / hk);
   const float* column = state + ((long long)bh * kDim + half * 64) * kDim + col;
@@ -181,6 +187,8 @@ commit_step_kernel(const __nv_bfloat16* __restrict__ k, const void* __restrict__
                    const float* __restrict__ delta, const int* __restrict__ counts, float* __restrict__ state,
                    int width, int hk, int hv, int gate_fp32) {
   __shared__ float sk[2][kDim];
+  wait_for_previous_kernel();
+  dependents_may_start();
   const int bh = blockIdx.x, col = threadIdx.x & (kDim - 1), half = threadIdx.x >> 7;
   const int bidx = bh / hv, vh = bh % hv, kh = vh / (hv / hk);
   const int count = min(max(counts[bidx], 0), width);
@@ -211,6 +219,8 @@ constexpr int kNormSweeps = 4;
 __global__ void __launch_bounds__(256)
 rmsnorm_gated_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ z,
                      const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long rows) {
+  wait_for_previous_kernel();
+  dependents_may_start();
   const int lane = threadIdx.x & 15;
   const long long first = (long long)blockIdx.x * (16 * kNormSweeps) + (threadIdx.x >> 4);
   uint4 yy[kNormSweeps], zz[kNormSweeps];
@@ -266,11 +276,10 @@ extern "C" int actlize_la_sm100_prepare_inputs(
   const long long vectors = tokens * (2LL * hk + hv);
   const long long ctas = (vectors + 16 * kPrepSweeps - 1) / (16 * kPrepSweeps);
   if (ctas > INT_MAX) return int(cudaErrorInvalidValue);
-  prepare_inputs_kernel<<<(unsigned)ctas, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return launch_early(prepare_inputs_kernel, dim3((unsigned)ctas), 256, 0, true, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(mixed), mixed_row_stride, static_cast<const __nv_bfloat16*>(a),
       static_cast<const __nv_bfloat16*>(b), a_log, dt_bias, static_cast<__nv_bfloat16*>(q),
       static_cast<__nv_bfloat16*>(k), static_cast<__nv_bfloat16*>(v), g, static_cast<__nv_bfloat16*>(beta), tokens, hk, hv);
-  return int(cudaGetLastError());
 }
 
 extern "C" int actlize_la_sm100_decode_step(
@@ -278,10 +287,9 @@ extern "C" int actlize_la_sm100_decode_step(
     int batch, int hk, int hv, int gate_fp32, void* stream) {
   if (!q || !k || !v || !g || !beta || !state || !output) return int(cudaErrorInvalidValue);
   if (batch <= 0 || hk <= 0 || hv <= 0 || hv % hk || (long long)batch * hv > INT_MAX) return int(cudaErrorInvalidValue);
-  decode_step_kernel<<<batch * hv, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return launch_early(decode_step_kernel, dim3(batch * hv), 256, 0, true, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
       g, static_cast<const __nv_bfloat16*>(beta), state, static_cast<__nv_bfloat16*>(output), hk, hv, gate_fp32 ? 1 : 0);
-  return int(cudaGetLastError());
 }
 
 extern "C" int actlize_la_sm100_verify_step(
@@ -290,11 +298,10 @@ extern "C" int actlize_la_sm100_verify_step(
   if (!q || !k || !v || !g || !beta || !state || !output || !delta) return int(cudaErrorInvalidValue);
   if (batch <= 0 || width <= 0 || width > 64 || hk <= 0 || hv <= 0 || hv % hk || (long long)batch * hv > INT_MAX)
     return int(cudaErrorInvalidValue);
-  verify_step_kernel<<<batch * hv, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return launch_early(verify_step_kernel, dim3(batch * hv), 256, 0, true, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
       g, static_cast<const __nv_bfloat16*>(beta), state, static_cast<__nv_bfloat16*>(output), delta, width, hk, hv,
       gate_fp32 ? 1 : 0);
-  return int(cudaGetLastError());
 }
 
 extern "C" int actlize_la_sm100_commit_step(const void* k, const void* g, const float* delta, const int* counts,
@@ -303,9 +310,8 @@ extern "C" int actlize_la_sm100_commit_step(const void* k, const void* g, const 
   if (!k || !g || !delta || !counts || !state) return int(cudaErrorInvalidValue);
   if (batch <= 0 || width <= 0 || width > 64 || hk <= 0 || hv <= 0 || hv % hk || (long long)batch * hv > INT_MAX)
     return int(cudaErrorInvalidValue);
-  commit_step_kernel<<<batch * hv, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return launch_early(commit_step_kernel, dim3(batch * hv), 256, 0, true, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(k), g, delta, counts, state, width, hk, hv, gate_fp32 ? 1 : 0);
-  return int(cudaGetLastError());
 }
 
 extern "C" int actlize_la_sm100_rmsnorm_gated(const void* y, const void* z, const void* weight, void* out,
@@ -314,8 +320,7 @@ extern "C" int actlize_la_sm100_rmsnorm_gated(const void* y, const void* z, cons
   if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(weight) |
        reinterpret_cast<uintptr_t>(out)) & 15)
     return int(cudaErrorInvalidValue);
-  rmsnorm_gated_kernel<<<(unsigned)((rows + 16 * kNormSweeps - 1) / (16 * kNormSweeps)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  return launch_early(rmsnorm_gated_kernel, dim3((unsigned)((rows + 16 * kNormSweeps - 1) / (16 * kNormSweeps))), 256, 0, true, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(z),
       static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(out), rows);
-  return int(cudaGetLastError());
 }

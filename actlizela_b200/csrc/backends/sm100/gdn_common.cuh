@@ -161,6 +161,27 @@ __device__ __forceinline__ float chunk_prefix64(float x, int tid, float* carry) 
   return x;
 }
 
+// Programmatic launch: a kernel launched by launch_early may start when every CTA of the kernel in front of it on the
+// stream has called dependents_may_start() (or ended), sets itself up, and touches global memory only behind
+// wait_for_previous_kernel(), which waits until that kernel has ended and its writes are visible.  Every kernel that is
+// launched so waits in all its CTAs, so the end of one implies the end of all in front of it.
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... Params, typename... Args>
+int launch_early(void (*kernel)(Params...), dim3 grid, int threads, int smem, bool early, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = early ? 1 : 0;
+  return int(cudaLaunchKernelEx(&config, kernel, Params(args)...));
+}
+
 // Launchers implemented by the kernel translation units; each returns a cudaError_t value.
 int launch_prepare_simt(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int launch_walk_simt(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);

@@ -538,13 +538,13 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #endif
   if (plan.serial_pass) {
     // (launched while the first launch still ran: its flags and outputs are complete behind this wait)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    wait_for_previous_kernel();
     // nothing to repair for this CTA's heads: leave before anything is set up
     bool any = false;
     for (int unit = blockIdx.x; unit < plan.units; unit += gridDim.x) any |= violated(plan, unit);
     if (!any) return;
   }
-  if (plan.pieces > 1) asm volatile("griddepcontrol.launch_dependents;");
+  dependents_may_start();
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) {
       mbar_init(&bar->kq_full[i], 1);
@@ -1189,18 +1189,8 @@ int launch(const Inputs& in, const Geometry& geo, const Plan& plan, int grid, cu
     if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, batch, kChunk)) return rc;
   }
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(grid);
-  config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = kSmemBytes;
-  config.stream = stream;
   // the serial pass may start before the first launch has ended (it waits for it in the kernel): its launch latency is hidden
-  cudaLaunchAttribute early{};
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &early;
-  config.numAttrs = plan.serial_pass ? 1 : 0;
-  return int(cudaLaunchKernelEx(&config, forward_umma_kernel<kRaw>, tm_q, tm_k, tm_v, in, geo, plan));
+  return launch_early(forward_umma_kernel<kRaw>, dim3(grid), kThreads, kSmemBytes, plan.serial_pass, stream, tm_q, tm_k, tm_v, in, geo, plan);
 }
 int sm_count() {
   static int counts[64] = {};

@@ -157,8 +157,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5;
   const int chunks = geo.chunks(), seg_chunks = geo.segment_chunks();
   __shared__ int s_left[kRepair ? kMaxSms : 1], s_count;
-  if (kRepair) asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");      // the walk sets itself up as SMs fall free
+  if (kRepair) wait_for_previous_kernel();
+  dependents_may_start();                                 // the walk sets itself up as SMs fall free
   if constexpr (kRepair) {
     const int heads = geo.batch * geo.value_heads;
     if (!__syncthreads_or(tid < heads * left.pieces && tid % left.pieces && left.flags[tid])) return;
@@ -738,6 +738,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   const int unit = blockIdx.x / parallel, sub = blockIdx.x % parallel;
   const int bh = pair_pass ? unit % heads : unit;
   const int flags = pair_pass ? (unit >= heads ? kWalkHomogeneous : kWalkTail) : in.walk_flags;
+  dependents_may_start();
   if (left.flags) {
     // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: it does not decay)
     // (the repairing prepare kernel lets this one start when the flags are final, so they need no further wait)
@@ -793,7 +794,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");      // launched early behind prepare: its planes are complete from here on
+  wait_for_previous_kernel();      // launched early behind prepare: its planes are complete from here on
   if ((flags & kWalkUntilDecayed) && warp == kTmaWarp) {
     // first chunk boundary at which the accumulated decay is below exp(-40): 32 chunks per step, the per-chunk
     // decay exp(p_last) is word 64 of the chunk's gate vector
@@ -1200,24 +1201,6 @@ int configure_umma() {
   e = cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
   return int(e);
 }
-
-namespace {
-// a launch that may start before the kernel in front of it has ended (it waits for it inside)
-template <typename... Params, typename... Args>
-int launch_early(void (*kernel)(Params...), unsigned grid, int threads, int smem, bool early, cudaStream_t stream, const Args&... args) {
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(grid);
-  config.blockDim = dim3(threads);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &attribute;
-  config.numAttrs = early ? 1 : 0;
-  return int(cudaLaunchKernelEx(&config, kernel, args...));
-}
-}  // namespace
 
 int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream, const Repair& left) {
   TensorMapEncoder& enc = tensor_map_encoder();

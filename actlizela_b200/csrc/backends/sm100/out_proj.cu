@@ -57,6 +57,8 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  wait_for_previous_kernel();
+  dependents_may_start();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -182,6 +184,8 @@ out_proj_skinny_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  wait_for_previous_kernel();
+  dependents_may_start();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -266,12 +270,14 @@ int launch_skinny(TensorMapEncoder& enc, const void* a, const void* w, void* c, 
   launch.blockDim = dim3(kSkinnyThreads);
   launch.dynamicSmemBytes = SkinnyLayout<kM>::kBytes;
   launch.stream = stream;
-  cudaLaunchAttribute cluster{};
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = split;
-  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-  launch.attrs = &cluster;
-  launch.numAttrs = 1;
+  cudaLaunchAttribute attributes[2] = {};
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = split;
+  attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_early
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  launch.attrs = attributes;
+  launch.numAttrs = 2;
   return int(cudaLaunchKernelEx(&launch, out_proj_skinny_kernel<kM>, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k));
 }
 
@@ -308,8 +314,7 @@ int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, 
   if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM)) return rc;
   if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kTileN)) return rc;
   const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
-  out_proj_umma_kernel<<<grid, kGemmThreads, kGemmSmem, stream>>>(tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k);
-  return int(cudaGetLastError());
+  return launch_early(out_proj_umma_kernel, grid, kGemmThreads, kGemmSmem, true, stream, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k);
 }
 
 }  // namespace gdn_sm100
