@@ -124,51 +124,78 @@ decode_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   if (half == 0) out[(long long)bh * kDim + col] = __float2bfloat16_rn((partial[0][col] + partial[1][col]) * kScale);
 }
 
+// The head's 64 KB of state towards L2 while the kernel in front still runs (a prefetch reads nothing into the SM, so what that
+// kernel may yet write to the state is not missed).
+__device__ __forceinline__ void prefetch_state(const float* state) {
+  const char* line = reinterpret_cast<const char*>(state + (long long)blockIdx.x * kDim * kDim) + threadIdx.x * 128;
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(line + 256 * 128));
+}
 // Verify step (speculative decoding): `width` draft tokens per request run through the same recurrence with the
 // state held in registers and NOT written back; besides the outputs it records delta_t = beta_t (v_t - k_t^T S),
 // from which commit_step_kernel later applies the accepted prefix.  Thread layout as in decode_step_kernel; the
-// arithmetic per token is the decode step's, operation for operation.
+// arithmetic per token is the decode step's, operation for operation.  Bound: the latency of a token's two reductions and
+// the state's way from HBM.  A token's operands come one token ahead (behind the barriers their latency was most of a
+// token's time), k and q are read 16 bytes at a time, the state is on its way to L2 before the launch's turn: 16 requests
+// x 4 tokens with the commit 32.2 -> 26.1 us, 90 x 8 249 -> 188.  (One barrier a token instead of four, with three k/q buffers,
+// was slower from 16 requests on: 26.3 and 193.)
 __global__ void __launch_bounds__(256)
 verify_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                    const __nv_bfloat16* __restrict__ v, const void* __restrict__ g,
                    const __nv_bfloat16* __restrict__ beta, const float* __restrict__ state,
                    __nv_bfloat16* __restrict__ out, float* __restrict__ delta_out, int width, int hk, int hv,
                    int gate_fp32) {
-  __shared__ float sk[2][kDim], sq[2][kDim], partial[2][kDim];
+  __shared__ __align__(16) float sk[2][kDim], sq[2][kDim];
+  __shared__ float partial[2][kDim];
+  prefetch_state(state);
   wait_for_previous_kernel();
   dependents_may_start();
   const int bh = blockIdx.x, col = threadIdx.x & (kDim - 1), half = threadIdx.x >> 7;
   const int bidx = bh / hv, vh = bh % hv, kh = vh / (hv / hk);
   const float* column = state + ((long long)bh * kDim + half * 64) * kDim + col;
+  // a token's operands are loaded one token ahead: behind the reduction's barriers their latency was most of a token's time
+  struct Token { __nv_bfloat16 qk, beta, value; float gate; };
+  const __nv_bfloat16* qk = half == 0 ? k : q;
+  const auto load_token = [&](int t) {
+    const long long token = (long long)bidx * width + t, head = token * hv + vh;
+    return Token{qk[(token * hk + kh) * kDim + col], beta[head], v[head * kDim + col], load_gate(g, head, gate_fp32)};
+  };
+  Token next = load_token(0);
   float s[64];
 #pragma unroll
   for (int r = 0; r < 64; ++r) s[r] = column[r * kDim];
   for (int t = 0; t < width; ++t) {
-    const long long token = (long long)bidx * width + t;
-    const long long qk_at = (token * hk + kh) * kDim, head = token * hv + vh;
+    const long long head = ((long long)bidx * width + t) * hv + vh;
     float* skt = sk[t & 1];
     float* sqt = sq[t & 1];
-    if (half == 0) skt[col] = __bfloat162float(k[qk_at + col]);
-    else sqt[col] = __bfloat162float(q[qk_at + col]);
-    const float decay = expf(load_gate(g, head, gate_fp32));
-    const float bt = __bfloat162float(beta[head]);
-    const float value = __bfloat162float(v[head * kDim + col]);
+    (half == 0 ? skt : sqt)[col] = __bfloat162float(next.qk);
+    const float decay = expf(next.gate);
+    const float bt = __bfloat162float(next.beta);
+    const float value = __bfloat162float(next.value);
+    if (t + 1 < width) next = load_token(t + 1);
 #pragma unroll
     for (int r = 0; r < 64; ++r) s[r] *= decay;
     __syncthreads();
-    const float* kk = skt + half * 64;
-    const float* qq = sqt + half * 64;
+    const float4* kk = reinterpret_cast<const float4*>(skt + half * 64);
+    const float4* qq = reinterpret_cast<const float4*>(sqt + half * 64);
     float kv = 0.f;
 #pragma unroll
-    for (int r = 0; r < 64; ++r) kv = fmaf(kk[r], s[r], kv);
+    for (int r = 0; r < 64; r += 4) {
+      const float4 x = kk[r >> 2];
+      kv = fmaf(x.w, s[r + 3], fmaf(x.z, s[r + 2], fmaf(x.y, s[r + 1], fmaf(x.x, s[r], kv))));
+    }
     partial[half][col] = kv;
     __syncthreads();
     const float delta = bt * (value - (partial[0][col] + partial[1][col]));
     float o = 0.f;
 #pragma unroll
-    for (int r = 0; r < 64; ++r) {
-      s[r] = fmaf(kk[r], delta, s[r]);
-      o = fmaf(qq[r], s[r], o);
+    for (int r = 0; r < 64; r += 4) {
+      const float4 x = kk[r >> 2], y = qq[r >> 2];
+      s[r] = fmaf(x.x, delta, s[r]);
+      s[r + 1] = fmaf(x.y, delta, s[r + 1]);
+      s[r + 2] = fmaf(x.z, delta, s[r + 2]);
+      s[r + 3] = fmaf(x.w, delta, s[r + 3]);
+      o = fmaf(y.w, s[r + 3], fmaf(y.z, s[r + 2], fmaf(y.y, s[r + 1], fmaf(y.x, s[r], o))));
     }
     __syncthreads();
     partial[half][col] = o;
@@ -186,7 +213,7 @@ __global__ void __launch_bounds__(256)
 commit_step_kernel(const __nv_bfloat16* __restrict__ k, const void* __restrict__ g,
                    const float* __restrict__ delta, const int* __restrict__ counts, float* __restrict__ state,
                    int width, int hk, int hv, int gate_fp32) {
-  __shared__ float sk[2][kDim];
+  __shared__ __align__(16) float sk[2][kDim];
   wait_for_previous_kernel();
   dependents_may_start();
   const int bh = blockIdx.x, col = threadIdx.x & (kDim - 1), half = threadIdx.x >> 7;
@@ -194,19 +221,29 @@ commit_step_kernel(const __nv_bfloat16* __restrict__ k, const void* __restrict__
   const int count = min(max(counts[bidx], 0), width);
   if (count == 0) return;
   float* column = state + ((long long)bh * kDim + half * 64) * kDim + col;
+  struct Token { __nv_bfloat16 key; float gate, delta; };      // loaded one token ahead
+  const auto load_token = [&](int t) {
+    const long long token = (long long)bidx * width + t, head = token * hv + vh;
+    return Token{k[(token * hk + kh) * kDim + col], load_gate(g, head, gate_fp32), delta[head * kDim + col]};
+  };
+  Token next = load_token(0);
   float s[64];
 #pragma unroll
   for (int r = 0; r < 64; ++r) s[r] = column[r * kDim];
   for (int t = 0; t < count; ++t) {
-    const long long token = (long long)bidx * width + t;
-    const long long head = token * hv + vh;
-    if (half == 0) sk[t & 1][col] = __bfloat162float(k[(token * hk + kh) * kDim + col]);
-    const float decay = expf(load_gate(g, head, gate_fp32));
-    const float d = delta[head * kDim + col];
+    if (half == 0) sk[t & 1][col] = __bfloat162float(next.key);
+    const float decay = expf(next.gate), d = next.delta;
+    if (t + 1 < count) next = load_token(t + 1);
     __syncthreads();
-    const float* kk = sk[t & 1] + half * 64;
+    const float4* kk = reinterpret_cast<const float4*>(sk[t & 1] + half * 64);
 #pragma unroll
-    for (int r = 0; r < 64; ++r) s[r] = fmaf(kk[r], d, s[r] * decay);
+    for (int r = 0; r < 64; r += 4) {
+      const float4 x = kk[r >> 2];
+      s[r] = fmaf(x.x, d, s[r] * decay);
+      s[r + 1] = fmaf(x.y, d, s[r + 1] * decay);
+      s[r + 2] = fmaf(x.z, d, s[r + 2] * decay);
+      s[r + 3] = fmaf(x.w, d, s[r + 3] * decay);
+    }
   }
 #pragma unroll
   for (int r = 0; r < 64; ++r) column[r * kDim] = s[r];

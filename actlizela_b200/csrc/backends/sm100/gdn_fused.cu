@@ -1233,7 +1233,7 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cons
   if (plan.pieces == 1) return 0;
   if (plan.leave) {
     // Heads that may not be cut: their chunks prepared by all SMs, then walked at 4.4k cycles a chunk instead of 7.1k by one
-    // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now @@).  Two launches that leave at once otherwise.
+    // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now 450).  Two launches that leave at once otherwise.
     Geometry whole = geo;
     whole.parallel = 0;
     const Repair left{flags, plan.pieces, sms};
