@@ -83,3 +83,25 @@ def test_heads_cut_over_the_sms(batch, length, hk, hv, stress, native_library):
         assert torch.equal(out[:, :, lone], want_out[:, :, lone]) and torch.equal(state[:, lone], want_state[:, lone])
     again_out, again_state = forward(*dev, True, configuration="fused-split")
     assert torch.equal(again_out, out) and torch.equal(again_state, state)
+
+
+@pytest.mark.parametrize("sequences,hv", [(149, 1), (75, 2), (256, 1), (257, 1)])
+def test_packed_sequences_dealt_longest_first(sequences, hv, native_library):
+    """More packed sequences than SMs, up to the most that are ordered and one more, some empty: the bits of calls that hold
+    too few sequences to be ordered."""
+    from actlizela_b200 import gdn_forward_varlen
+    lengths = [(37 * i * i + 11 * i) % 190 for i in range(sequences)]
+    bounds = [0]
+    for n in lengths:
+        bounds.append(bounds[-1] + n)
+    w = WORKLOADS["cfg1"].sliced(batch=1, length=bounds[-1], key_heads=1, value_heads=hv, seed=6000 + sequences)
+    q, k, v, g, beta, _ = (x.cuda() if x is not None else None for x in make_inputs(w))
+    init = torch.randn(sequences, hv, 128, 128, device="cuda") * 0.05
+    out, state = gdn_forward_varlen(q, k, v, g, beta, torch.tensor(bounds, dtype=torch.int32, device="cuda"), init, True)
+    for first in range(0, sequences, 70):
+        last = min(first + 70, sequences)
+        a, b = bounds[first], bounds[last]
+        part = [x[:, a:b].contiguous() for x in (q, k, v, g, beta)]
+        offsets = torch.tensor([x - a for x in bounds[first:last + 1]], dtype=torch.int32, device="cuda")
+        want_out, want_state = gdn_forward_varlen(*part, offsets, init[first:last].contiguous(), True)
+        assert torch.equal(out[:, a:b], want_out) and torch.equal(state[first:last], want_state)
