@@ -93,8 +93,8 @@ long long actlize_la_sm100_workspace_bytes(int batch, int sequence, int key_head
 
 /* Complete forward on caller-owned buffers.  Configuration 4: one kernel, in which every CTA prepares the chunks of a head
  * and walks them (one segment, no stage bits; the sub-segment field says only whether heads may be cut into pieces, 0 or
- * 1 = no, and the launcher chooses how many; a second launch walks again the heads for which a piece met a token that is
- * no contraction, and leaves at once when there is none).  The others: prepare kernel (per-chunk gate prefix, decay-masked
+ * 1 = no, and the launcher chooses how many; heads that do not decay, or hold a token that is no contraction, are left to the
+ * two kernels of configuration 1, launched behind it, which leave at once when there are none).  The others: prepare kernel (per-chunk gate prefix, decay-masked
  * K.K^T, unit-lower-triangular inverse, WY factors) followed by the sequential chunk walk.
  * `config` is the value returned by actlize_la_sm100_select: kernel family in bits 0..3, number of
  * sequence segments in bits 8..15, number of parallel sub-segments of the walk in bits 16..19 (tcgen05 family only;
