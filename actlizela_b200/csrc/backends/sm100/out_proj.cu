@@ -15,33 +15,40 @@ namespace gdn_sm100 {
 using namespace ptx;
 namespace {
 
-constexpr int kTileM = 128, kTileN = 128, kTileK = 64, kGemmStages = 3;
-constexpr int kOperandBytes = kTileM * kTileK * 2;                 // 16 KB per operand tile
-constexpr int kGemmStageBytes = 2 * kOperandBytes;
-constexpr int kGemmBars = kGemmStages * kGemmStageBytes;
-constexpr int kGemmSmem = kGemmBars + 128 + 1024;
-constexpr int kGemmThreads = 192;
-constexpr uint32_t kIdescGemm = idesc_bf16(kTileM, kTileN, false, false);
-static_assert(2 * (kGemmSmem + 1024) <= 227 * 1024, "two GEMM CTAs must fit in one SM's shared memory");
+constexpr int kTileM = 128, kTileK = 64, kGemmThreads = 192;
+constexpr int kOperandBytes = kTileM * kTileK * 2;                 // 16 KB per 128-row operand tile
+// Tiles of 128 x kN.  Bound by the operands' way into shared memory (about 64 bytes a cycle and SM): a 128 x 128 step takes in
+// 32 KB, a 128 x 256 step 48 KB for twice the products.  Two CTAs of the narrow tile share an SM, the wide one has it alone.
+// (M 8192, K 4096, N 2560: 165 us with 128 columns, 145 with 256, 1.18 PFLOP/s; M 3000: 68 and 62.)
+template <int kN> struct GemmLayout {
+  static constexpr int kStage = kOperandBytes * (1 + kN / 128);
+  static constexpr int kStages = kN == 256 ? 4 : 3, kPerSm = kN == 256 ? 1 : 2;
+  static constexpr int kBars = kStages * kStage;
+  static constexpr int kBytes = kBars + 128 + 1024;
+  static constexpr uint32_t kIdesc = idesc_bf16(kTileM, kN, false, false);
+  static_assert(kPerSm * (kBytes + 1024) <= 227 * 1024, "shared memory of one SM");
+};
 
-__global__ void __launch_bounds__(kGemmThreads, 2)
+template <int kN>
+__global__ void __launch_bounds__(kGemmThreads, GemmLayout<kN>::kPerSm)
 out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                      __nv_bfloat16* __restrict__ c, int m, int n, int k) {
+  using L = GemmLayout<kN>;
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
-  uint64_t* full = reinterpret_cast<uint64_t*>(sm + kGemmBars);       // [stages] tiles landed
-  uint64_t* empty = full + kGemmStages;                               // [stages] tiles consumed
-  uint64_t* done = empty + kGemmStages;                               // accumulator complete
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + L::kBars);       // [stages] tiles landed
+  uint64_t* empty = full + L::kStages;                               // [stages] tiles consumed
+  uint64_t* done = empty + L::kStages;                               // accumulator complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const AbortFlag abort{abort_word};
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * kTileN, m0 = blockIdx.y * kTileM;
+  const int n0 = blockIdx.x * kN, m0 = blockIdx.y * kTileM;
   const int k_tiles = (k + kTileK - 1) / kTileK;
 
   if (tid == 0) {
-    for (int s = 0; s < kGemmStages; ++s) {
+    for (int s = 0; s < L::kStages; ++s) {
       mbar_init(full + s, 1);
       mbar_init(empty + s, 1);
     }
@@ -50,7 +57,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, kTileN);
+    tmem_alloc(tmem_slot, kN);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -65,28 +72,28 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       prefetch_tensormap(&tm_a);
       prefetch_tensormap(&tm_w);
       for (int kt = 0; kt < k_tiles; ++kt) {
-        const int s = kt % kGemmStages;
-        if (kt >= kGemmStages && !mbar_wait(empty + s, ((kt / kGemmStages) - 1) & 1, abort, 60, kt)) break;
-        uint8_t* stage = sm + s * kGemmStageBytes;
-        mbar_arrive_expect_tx(full + s, kGemmStageBytes);
+        const int s = kt % L::kStages;
+        if (kt >= L::kStages && !mbar_wait(empty + s, ((kt / L::kStages) - 1) & 1, abort, 60, kt)) break;
+        uint8_t* stage = sm + s * L::kStage;
+        mbar_arrive_expect_tx(full + s, L::kStage);
         tma_load_2d(stage, &tm_a, full + s, kt * kTileK, m0);
         tma_load_2d(stage + kOperandBytes, &tm_w, full + s, kt * kTileK, n0);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t base = smem_u32(sm);
+    const uint32_t base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);
+    if (elect_one()) {
       bool ok = true;
       for (int kt = 0; kt < k_tiles && ok; ++kt) {
-        const int s = kt % kGemmStages;
-        ok = mbar_wait(full + s, (kt / kGemmStages) & 1, abort, 61, kt);
+        const int s = kt % L::kStages;
+        ok = mbar_wait(full + s, (kt / L::kStages) & 1, abort, 61, kt);
         tc_fence_after();
-        const uint64_t da = smem_desc(base + s * kGemmStageBytes, 16, 1024);
-        const uint64_t db = smem_desc(base + s * kGemmStageBytes + kOperandBytes, 16, 1024);
+        const uint64_t da = smem_desc(base + s * L::kStage, 16, 1024);
+        const uint64_t db = smem_desc(base + s * L::kStage + kOperandBytes, 16, 1024);
 #pragma unroll
         for (int ks = 0; ks < kTileK / 16; ++ks)          // 16 BF16 (32 bytes) along K per instruction
-          mma_ss(tmem, da + uint64_t(ks * 2), db + uint64_t(ks * 2), kIdescGemm, (kt | ks) != 0);
+          mma_ss(tmem, da + uint64_t(ks * 2), db + uint64_t(ks * 2), L::kIdesc, (kt | ks) != 0);
         mma_commit(empty + s);
       }
       mma_commit(done);
@@ -101,7 +108,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     if (ok) {
       const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16);
 #pragma unroll
-      for (int piece = 0; piece < kTileN / 32; ++piece) {
+      for (int piece = 0; piece < kN / 32; ++piece) {
         uint32_t d[32];
         tmem_ld32(taddr + piece * 32, d);        // warp-collective: every lane takes part, also rows beyond M
         tmem_wait_ld();
@@ -127,7 +134,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, kTileN);
+  if (warp == 1) tmem_dealloc(tmem, kN);
 }
 
 // ------------------------------------------------------------------------------------------- few rows: split over K
@@ -281,6 +288,15 @@ int launch_skinny(TensorMapEncoder& enc, const void* a, const void* w, void* c, 
   return int(cudaLaunchKernelEx(&launch, out_proj_skinny_kernel<kM>, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k));
 }
 
+
+template <int kN>
+int launch_tiles(TensorMapEncoder& enc, const void* a, const void* w, void* c, int m, int n, int k, cudaStream_t stream) {
+  CUtensorMap tm_a, tm_w;
+  if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM)) return rc;
+  if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kN)) return rc;
+  return launch_early(out_proj_umma_kernel<kN>, dim3((n + kN - 1) / kN, (m + kTileM - 1) / kTileM), kGemmThreads,
+                      GemmLayout<kN>::kBytes, true, stream, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k);
+}
 }  // namespace
 
 GDN_SM100_DEFINE_STATUS_HOOKS(gemm)
@@ -288,7 +304,8 @@ GDN_SM100_DEFINE_STATUS_HOOKS(gemm)
 int configure_out_proj() {
   if (int rc = tensor_map_encoder().init()) return rc;
   const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(out_proj_umma_kernel, smem, kGemmSmem);
+  cudaError_t e = cudaFuncSetAttribute(out_proj_umma_kernel<128>, smem, GemmLayout<128>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<256>, smem, GemmLayout<256>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<16>, smem, SkinnyLayout<16>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<32>, smem, SkinnyLayout<32>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<64>, smem, SkinnyLayout<64>::kBytes);
@@ -310,11 +327,10 @@ int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, 
     if (m <= 64) return launch_skinny<64>(enc, a, w, c, m, n, k, split, stream);
     return launch_skinny<128>(enc, a, w, c, m, n, k, split, stream);
   }
-  CUtensorMap tm_a, tm_w;
-  if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM)) return rc;
-  if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kTileN)) return rc;
-  const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
-  return launch_early(out_proj_umma_kernel, grid, kGemmThreads, kGemmSmem, true, stream, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k);
+  // a K step of all tiles of an SM's turn takes 512 cycles of operand traffic for a 128 x 128 tile, 768 for a 128 x 256 one
+  const long long wide = ((n + 255LL) / 256) * ((m + 127LL) / 128);
+  return (wide + 147) / 148 * 768 < (tiles + 147) / 148 * 512 ? launch_tiles<256>(enc, a, w, c, m, n, k, stream)
+                                                              : launch_tiles<128>(enc, a, w, c, m, n, k, stream);
 }
 
 }  // namespace gdn_sm100

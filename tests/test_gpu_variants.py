@@ -28,6 +28,20 @@ def test_out_proj_with_few_rows(m, k, n):
     assert torch.equal(got, out_proj_gemm(a, w))                  # the sum over the cluster has one order
 
 
+@pytest.mark.parametrize("m,k,n", [(1100, 264, 2560), (1930, 136, 2312), (2049, 72, 5128), (3000, 4096, 2560), (1999, 64, 5000)])
+def test_out_proj_tile_widths(m, k, n):
+    """Tiles of 128 and 256 columns, both sides of the rule: ragged rows, columns that end in either half of a wide tile,
+    K of one step and with a tail."""
+    from actlizela_b200 import out_proj_gemm
+    gen = torch.Generator().manual_seed(m + n)
+    a = torch.randn(m, k, generator=gen).to(torch.bfloat16).cuda()
+    w = (torch.randn(n, k, generator=gen) * k ** -0.5).to(torch.bfloat16).cuda()
+    want = a.float() @ w.float().t()
+    got = out_proj_gemm(a, w)
+    assert oracle.rel_frobenius(got.float().cpu(), want.cpu()) < 3e-3
+    assert oracle.max_abs(got.float(), want) <= 2 ** -8 * float(want.abs().max()) + 1e-6
+
+
 @pytest.mark.parametrize("batch,length,hk,hv", [(1, 1, 1, 1), (1, 64, 2, 6), (3, 129, 1, 2), (2, 193, 1, 4), (5, 700, 8, 32),
                                                 (300, 65, 1, 1)])
 def test_single_launch_form_equals_the_two_kernels_bitwise(batch, length, hk, hv, native_library):
