@@ -58,18 +58,6 @@ int TensorMapEncoder::bf16_4d(CUtensorMap* map, const void* base, uint64_t d0, u
   return r == CUDA_SUCCESS ? 0 : int(cudaErrorInvalidValue);
 }
 
-int TensorMapEncoder::f32_2d(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows,
-                             uint32_t box_rows) const {
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 4};
-  const cuuint32_t box[2] = {32, box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
-                      elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : int(cudaErrorInvalidValue);
-}
-
 TensorMapEncoder& tensor_map_encoder() {
   static TensorMapEncoder encoder;
   return encoder;

@@ -292,8 +292,6 @@ struct TensorMapEncoder {
   int bf16_2d(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint32_t box_rows) const;
   int bf16_4d(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
               uint32_t box_rows_d2) const;
-  // FP32 matrix, box = 32 columns (128 bytes) x box_rows, no swizzle (dense box in shared memory)
-  int f32_2d(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint32_t box_rows) const;
 };
 TensorMapEncoder& tensor_map_encoder();
 
