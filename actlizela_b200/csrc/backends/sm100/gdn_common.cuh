@@ -164,7 +164,8 @@ __device__ __forceinline__ float chunk_prefix64(float x, int tid, float* carry) 
 // Programmatic launch: a kernel launched by launch_early may start when every CTA of the kernel in front of it on the
 // stream has called dependents_may_start() (or ended), sets itself up, and touches global memory only behind
 // wait_for_previous_kernel(), which waits until that kernel has ended and its writes are visible.  Every kernel that is
-// launched so waits in all its CTAs, so the end of one implies the end of all in front of it.
+// launched so waits in all its CTAs, those that find nothing to do among them, so the end of one implies the end of all in
+// front of it: what an earlier kernel of the stream still reads is never written by a later one.
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... Params, typename... Args>

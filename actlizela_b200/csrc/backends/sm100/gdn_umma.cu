@@ -729,8 +729,10 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   dependents_may_start();
   if (left.flags) {
     // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: it does not decay)
-    // (the repairing prepare kernel lets this one start when the flags are final, so they need no further wait)
-    const int mark = tid > 0 && tid < left.pieces ? *reinterpret_cast<const volatile int*>(left.flags + bh * left.pieces + tid) : 0;
+    // (the wait comes first: the flags live in scratch that is given back behind this call, and a CTA that left without it
+    // would let this launch end, and the next one begin, while a late CTA of the repairing prepare kernel still reads them)
+    wait_for_previous_kernel();
+    const int mark = tid > 0 && tid < left.pieces ? left.flags[bh * left.pieces + tid] : 0;
     if (!__syncthreads_or(mark)) return;
     if (!__syncthreads_or(mark == 2) && tid == 0) {
       atomicAdd(&g_walk_plan_counts[0], -1);
