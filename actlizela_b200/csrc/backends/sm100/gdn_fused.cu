@@ -274,6 +274,7 @@ struct Plan {
   int* flags;      // [batch * value_heads][pieces], written when pieces > 1
 };
 constexpr int kLeastPiece = 8;       // chunks: a piece has to outlast the decay, which takes about four at typical gates
+constexpr int kWalkPieces = 8;       // pieces at most in the two-kernel form: longer than those here when there are few heads
 
 // did a CTA that walked a piece of head h see a token that is no contraction?
 __device__ __forceinline__ bool violated(const Plan& plan, int h) {
@@ -1282,13 +1283,15 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cons
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
   if (plan.pieces == 1) return 0;
   if (plan.leave) {
-    // Heads that may not be cut: their chunks prepared by all SMs, then walked at 4.4k cycles a chunk instead of 7.1k by one
-    // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now 450).  Two launches that leave at once otherwise.
-    Geometry whole = geo;
-    whole.parallel = 0;
+    // Heads that may not be cut: their chunks prepared by all SMs, then walked at 4.1k cycles a chunk instead of 7.5k by one
+    // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now 440).  Two launches that leave at once otherwise.
+    // Where this launch's pieces are shorter than an eighth of a head, the walk tries again with eight: gates too slow for the
+    // one are often fast enough for the other (B1, 8 heads, T32768, mean gate -0.02: 1279 us walked uncut, now 372).
+    Geometry again = geo;
+    again.parallel = plan.pieces > kWalkPieces ? kWalkPieces : 0;
     const Repair left{flags, plan.pieces, sms};
-    if (int rc = launch_prepare_umma(in, whole, ws, stream, left)) return rc;
-    return launch_walk_umma(in, whole, ws, true, stream, left);
+    if (int rc = launch_prepare_umma(in, again, ws, stream, left)) return rc;
+    return launch_walk_umma(in, again, ws, true, stream, left);
   }
   plan.serial_pass = 1;
   plan.units = heads;

@@ -727,6 +727,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   const int bh = pair_pass ? unit % heads : unit;
   const int flags = pair_pass ? (unit >= heads ? kWalkHomogeneous : kWalkTail) : in.walk_flags;
   dependents_may_start();
+  bool counted_cut = false;                  // how the single-launch forward counted a head it left
   if (left.flags) {
     // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: it does not decay)
     // (the wait comes first: the flags live in scratch that is given back behind this call, and a CTA that left without it
@@ -734,10 +735,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     wait_for_previous_kernel();
     const int mark = tid > 0 && tid < left.pieces ? left.flags[bh * left.pieces + tid] : 0;
     if (!__syncthreads_or(mark)) return;
-    if (!__syncthreads_or(mark == 2) && tid == 0) {
-      atomicAdd(&g_walk_plan_counts[0], -1);
-      atomicAdd(&g_walk_plan_counts[1], 1);
-    }
+    counted_cut = !__syncthreads_or(mark == 2);
   }
   const int b = bh / geo.value_heads;
   const int hv = bh % geo.value_heads;
@@ -834,6 +832,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     state_in = nullptr;           // zeros go into tensor memory and straight out as the transition matrix
     identity_in = false;
   }
+  bool is_cut = false;
   int unstored = 0;                          // leading chunks whose output rows the previous sub-segment's CTA writes
   if (flags & kWalkTail) {
     // offset pass: only the suffix that determines the outgoing state, from zero, no output rows
@@ -847,7 +846,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     const int n = chunks;
     bool serial = false;
     for (int r = 1; r < parallel; ++r) serial |= reach_slot[r] < 0;
-    if (tid == 0 && sub == 0) atomicAdd(&g_walk_plan_counts[serial ? 1 : 0], 1);
+    is_cut = !serial;
+    if (tid == 0 && sub == 0 && !left.flags) atomicAdd(&g_walk_plan_counts[serial ? 1 : 0], 1);
     if (serial) {
       chunks = sub == 0 ? n : 0;             // the head's first CTA walks the whole range alone
       if (sub != 0) state_out = nullptr;
@@ -859,6 +859,10 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       unstored = sub == 0 ? 0 : reach_slot[sub];
       if (sub != parallel - 1) state_out = nullptr;
     }
+  }
+  if (left.flags && is_cut != counted_cut && tid == 0 && sub == 0) {
+    atomicAdd(&g_walk_plan_counts[0], is_cut ? 1 : -1);
+    atomicAdd(&g_walk_plan_counts[1], is_cut ? -1 : 1);
   }
 
   if (warp >= kChainWarp0 && warp < kChainWarp0 + kChainWarps) {

@@ -119,3 +119,40 @@ def test_packed_sequences_dealt_longest_first(sequences, hv, native_library):
         offsets = torch.tensor([x - a for x in bounds[first:last + 1]], dtype=torch.int32, device="cuda")
         want_out, want_state = gdn_forward_varlen(*part, offsets, init[first:last].contiguous(), True)
         assert torch.equal(out[:, a:b], want_out) and torch.equal(state[first:last], want_state)
+
+
+@pytest.mark.parametrize("chunks,reach,split", [
+    (300, (4, 20, 60), 2),                   # one for the single launch's 37 pieces, one for eight, one for neither
+    (300, (30, 20, 12, 36, 1000), 4),
+    (131, (9, 17, 25), 1),                   # pieces of 8, and of 16 chunks: the first just too slow for the former
+    (130, (2, 3, 64, 65), 2)])
+def test_cuts_follow_the_gates(chunks, reach, split, native_library):
+    """Heads whose state outlives the shortest pieces, each by another factor: cut into as many pieces as the single launch
+    has CTAs for, into eight in the two kernels, or walked whole with the unsplit walk's bits.  Under slow gates a piece's own rounding (16-bit operand pairs: the
+    state is good to 4e-6) is not forgotten within the piece: both walks' errors in the state, and single BF16 flips in the
+    output, which has 2^-9 per flipped value (a sixteenth of them is 5e-4)."""
+    from actlizela_b200.sm100 import Sm100Forward
+    forward = Sm100Forward(native_library)
+    length, hv = 64 * chunks - 7, len(reach)
+    w = WORKLOADS["cfg1"].sliced(batch=1, length=length, key_heads=1, value_heads=hv, seed=7000 + chunks)
+    q, k, v, g, beta, init = make_inputs(w)
+    gen = torch.Generator().manual_seed(chunks)
+    for h, r in enumerate(reach):            # 40 nats within r chunks, with half a chunk to spare
+        g[:, :, h] = -40.0 / (64 * (r - 0.5)) * (0.9 + 0.2 * torch.rand(1, length, generator=gen))
+    dev = [x.cuda() for x in (q, k, v, g, beta, init)]
+    want_out, want_state = forward(*dev, True, configuration="fused")
+    counts = (ctypes.c_int * 2)()
+    assert native_library.lib.actlize_la_sm100_walk_plan_counts(counts, 1) == 0
+    out, state = forward(*dev, True, configuration="fused-split")
+    torch.cuda.synchronize()
+    assert _healthy(native_library)
+    assert native_library.lib.actlize_la_sm100_walk_plan_counts(counts, 1) == 0
+    assert list(counts) == [split, hv - split]
+    for h in range(hv):
+        assert oracle.rel_frobenius(out[:, :, h].float().cpu(), want_out[:, :, h].float().cpu()) < 5e-4
+        assert oracle.rel_frobenius(state[:, h].cpu(), want_state[:, h].cpu()) < 8e-6
+    for h, r in enumerate(reach):
+        if r > chunks:
+            assert torch.equal(out[:, :, h], want_out[:, :, h]) and torch.equal(state[:, h], want_state[:, h])
+    again_out, again_state = forward(*dev, True, configuration="fused-split")
+    assert torch.equal(again_out, out) and torch.equal(again_state, state)
