@@ -266,14 +266,15 @@ struct ItemCursor {
 // What a launch walks: the units of the grid, a (batch or sequence, value head) each, or with `pieces` > 1 one of its
 // sub-segments (see walk_umma_kernel), at most one per CTA.  The decay part of the sub-segments' conditions is read off
 // the gates up front, while the contraction part (beta |k|^2 in [0, 2]) shows only when a chunk is prepared: every CTA
-// records what it saw in `flags`.  The heads that could not be cut are left to the two kernels of gdn_umma.cu (`leave`; a
-// flag word of 2), which also repair those with a violation; on raw projections, which only this kernel reads, their first
-// CTA walks them whole and a second launch of this kernel (`serial_pass`) repairs.
+// records what it saw in `flags`, and the two kernels of gdn_umma.cu, launched behind, repair the heads with a violation.
+// Heads that could not be cut are left to them as well (`leave`; a flag word of 2), or walked whole by their first CTA: with
+// many heads, and on raw projections, which only this kernel reads and a second launch of it (`serial_pass`) repairs.
 struct Plan {
   int units, pieces, serial_pass, leave;
   int* flags;      // [batch * value_heads][pieces], written when pieces > 1
 };
 constexpr int kLeastPiece = 8;       // chunks: a piece has to outlast the decay, which takes about four at typical gates
+constexpr int kMostLeft = 56;        // heads: more are never left
 constexpr int kWalkPieces = 8;       // pieces at most in the two-kernel form: longer than those here when there are few heads
 
 // did a CTA that walked a piece of head h see a token that is no contraction?
@@ -1278,11 +1279,14 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cons
     if (plan.pieces < 1) plan.pieces = 1;
     plan.units = heads * plan.pieces;
   }
-  plan.leave = plan.pieces > 1 && !in.mixed;
+  // A head that is walked whole takes 3.8 us a chunk here; the two kernels take 2.1 us a chunk of the longest head and 31 ns for
+  // every chunk they prepare, which is less up to 56 heads (B1, all heads undecayed, T1024 / T8192: 64 heads 103 / 558 us
+  // left, 95 / 550 walked here; 48 heads at T8192 499 left, 515 walked here).
+  plan.leave = plan.pieces > 1 && !in.mixed && heads <= kMostLeft;
   const auto go = in.mixed ? launch<true> : launch<false>;
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
   if (plan.pieces == 1) return 0;
-  if (plan.leave) {
+  if (!in.mixed) {
     // Heads that may not be cut: their chunks prepared by all SMs, then walked at 4.1k cycles a chunk instead of 7.5k by one
     // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now 440).  Two launches that leave at once otherwise.
     // Where this launch's pieces are shorter than an eighth of a head, the walk tries again with eight: gates too slow for the
