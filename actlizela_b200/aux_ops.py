@@ -105,7 +105,7 @@ def gdn_forward_projections(mixed, a, b, a_log, dt_bias, key_heads, value_heads,
                             output_final_state=True):
     """The forward straight from the layer's projection outputs: ``mixed`` BF16 [B,T,(2Hk+Hv)*128] laid out
     [q heads | k heads | v heads], ``a``, ``b`` BF16 [B,T,Hv], ``a_log``, ``dt_bias`` FP32 [Hv].  Normalisation
-    and gate activation happen inside the prepare kernel; the result equals ``gdn_prepare_inputs`` followed by
+    and gate activation happen inside the forward's kernels; the result equals ``gdn_prepare_inputs`` followed by
     ``gdn_forward`` bit for bit.  Returns (out [B,T,Hv,128] BF16, final state or None)."""
     result = _host.projections(mixed, a, b, a_log, dt_bias, key_heads, value_heads, initial_state, output_final_state)
     if result is not None:

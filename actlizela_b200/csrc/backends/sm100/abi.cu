@@ -72,11 +72,15 @@ int segments_of(int config, const Geometry& geo) {
   return segments > chunks ? chunks : segments;
 }
 
-// workspace a call needs: the factors of every block; single-launch form: its flag words and, when heads may be cut, room
-// for the factors of those that turn out not to decay (not on raw projections, where that kernel walks them itself)
+// raw projections: the planes of normalised queries and keys the walk reads, each [B][T][Hk][128] BF16
+long long norm_plane_bytes(const Geometry& geo) { return ((long long)geo.batch * geo.sequence * geo.key_heads * kDim * 2 + 255) & ~255LL; }
+long long factor_bytes(const Geometry& geo, int segments) { return (workspace_bytes(geo, segments) + 255) & ~255LL; }
+// workspace a call needs: the factors of every block, with raw projections the normalised planes behind them; single-launch
+// form: its flag words in front and, when heads may be cut, room for the factors of those that turn out not to decay
 long long scratch_bytes(const Geometry& geo, int config, int segments, bool raw = false) {
-  if (!is_fused(config)) return workspace_bytes(geo, segments);
-  return fused_workspace_bytes() + (raw || parallel_of(config, geo.chunks()) == 1 ? 0 : workspace_bytes(geo, 1));
+  const long long factors = raw ? factor_bytes(geo, segments) + 2 * norm_plane_bytes(geo) : workspace_bytes(geo, segments);
+  if (!is_fused(config)) return factors;
+  return fused_workspace_bytes() + (parallel_of(config, geo.chunks()) == 1 ? 0 : factors);
 }
 
 // Second stream and events of the segmented forward, created by configure() for the current device.
@@ -435,13 +439,23 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
 }  // namespace
 
 // --------------------------------------------------------------- forward on raw projection outputs
-// The raw projections are normalised and activated inside the single-launch kernel; the configurations of the two
-// tensor-core families select the same kernel here (they give the same bits), with the split their word carries.
+// The raw projections are normalised and activated inside the prepare kernel, which stores the normalised queries and keys for
+// the walk, or inside the single-launch kernel.  The two kernels take every shape whose heads can be cut: a layer's heads
+// decay at very different speeds, and where the single launch has to leave some to the two kernels, one follows the other
+// (B1 T4000, 32 heads, slow gates: 226 us in the two kernels, 374 in the single launch; 8 heads, T1000, ordinary gates: 44
+// and 85).  Only where the sequence is long and every head decays within a piece the single launch would be ahead (32 heads,
+// T16000: 435 and 378).  One chunk is over before a second launch (B1 T50: 23.6 and 20.4), and with more heads than half
+// the SMs nothing is cut and preparing them all first is never cheap (128 heads, T1000: 128 and 106).
+int projections_config(const Geometry& geo, int config) {
+  return 2LL * geo.batch * geo.value_heads <= 148 && geo.chunks() > 1 ? (config & ~0xf) | 1 : kFused;
+}
 extern "C" long long actlize_la_sm100_projections_workspace_bytes(int b, int t, int hk, int hv, int config) {
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config) || ((config & 0xf) != 1 && !is_fused(config)) ||
       (config & (kStageMask | kWalkFlagMask)))
     return -1;
-  return scratch_bytes(Geometry{b, t, hk, hv}, (config & ~0xf) | kFused, 1, true);
+  const Geometry geo{b, t, hk, hv};
+  config = projections_config(geo, config);
+  return scratch_bytes(geo, config, segments_of(config, geo), true);
 }
 
 extern "C" int actlize_la_sm100_forward_projections(
@@ -467,7 +481,15 @@ extern "C" int actlize_la_sm100_forward_projections(
   in.act_b = static_cast<const __nv_bfloat16*>(b_act);
   in.a_log = a_log;
   in.dt_bias = dt_bias;
-  return run_fused(in, Geometry{b, t, hk, hv}, config, workspace, static_cast<cudaStream_t>(opaque_stream));
+  const Geometry geo{b, t, hk, hv};
+  config = projections_config(geo, config);
+  const cudaStream_t stream = static_cast<cudaStream_t>(opaque_stream);
+  if (is_fused(config)) return run_fused(in, geo, config, workspace, stream);
+  const int segments = segments_of(config, geo);
+  const char* planes = static_cast<const char*>(workspace) + factor_bytes(geo, segments);
+  in.q = reinterpret_cast<const __nv_bfloat16*>(planes);
+  in.k = reinterpret_cast<const __nv_bfloat16*>(planes + norm_plane_bytes(geo));
+  return run_forward(in, geo, carve_workspace(workspace, geo), config, segments, stream);
 }
 
 // ---------------------------------------------------------------------------------- packed sequences

@@ -113,9 +113,11 @@ struct Inputs {
   //   kWalkPair         kWalkTail and kWalkHomogeneous (from an identity state made in the kernel) in one launch,
   //                     two CTAs per (batch, value head); final_state is then [2][B][Hv][128][128] = (M, b)
   int walk_flags = 0;
-  // Raw projections (single-launch forward only): q, k, v are then read from the packed projection rows `mixed`
-  // [B*T][mixed_stride] = [q heads | k heads | v heads] x 128 and normalised in shared memory; the gate and beta come
-  // from the raw activations `act_a`, `act_b` [B*T][Hv] with the per-head constants `a_log`, `dt_bias`.
+  // Raw projections (tensor-core kernels): the single-launch forward and the prepare kernel then read q, k, v from the packed
+  // projection rows `mixed` [B*T][mixed_stride] = [q heads | k heads | v heads] x 128 and normalise them in shared memory;
+  // the gate and beta come from the raw activations `act_a`, `act_b` [B*T][Hv] with the per-head constants `a_log`,
+  // `dt_bias`.  `q` and `k` are then planes of scratch [B][T][Hk][128]: the prepare kernel stores the normalised tiles there,
+  // for the walk.
   const __nv_bfloat16* mixed = nullptr;
   long long mixed_stride = 0;
   const __nv_bfloat16* act_a = nullptr;
@@ -133,6 +135,16 @@ constexpr float kDecayedLog2 = -40.f * 1.4426950408889634f;
 __device__ __forceinline__ float load_gate(const void* g, long long index, int gate_fp32) {
   return gate_fp32 ? static_cast<const float*>(g)[index]
                    : __bfloat162float(static_cast<const __nv_bfloat16*>(g)[index]);
+}
+// gate and beta of a token from the raw activations: g = -exp(A_log) softplus(a + dt_bias) (z > 20 branch), `bits` = a;
+// beta = sigmoid(b) rounded to BF16
+__device__ __forceinline__ float raw_gate(const Inputs& in, uint32_t bits, int hv) {
+  const float z = __uint_as_float(bits << 16) + in.dt_bias[hv];
+  return -expf(in.a_log[hv]) * (z > 20.f ? z : log1pf(expf(z)));
+}
+__device__ __forceinline__ uint32_t bf16_bits(const __nv_bfloat16* p) { return *reinterpret_cast<const unsigned short*>(p); }
+__device__ __forceinline__ float raw_beta(const Inputs& in, long long index) {
+  return __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-__bfloat162float(in.act_b[index])))));
 }
 
 // x ~= hi + lo with both parts BF16 (16 significant bits in total).
@@ -198,8 +210,8 @@ int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaSt
 // `early`: the kernel in front of it on the stream is this call's prepare kernel, which lets it set itself up beside it
 int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, bool early, cudaStream_t, const Repair& = {});
 int configure_umma();
-// single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces; `flags` is scratch of
-// fused_workspace_bytes, the workspace (unless the inputs are raw projections) takes the factors of heads it cannot cut
+// single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces (not on raw projections); `flags`
+// is scratch of fused_workspace_bytes, the workspace takes the factors of heads it cannot cut
 int configure_fused();
 long long fused_workspace_bytes();
 int launch_forward_fused(const Inputs&, const Geometry&, int* flags, const Workspace&, cudaStream_t);

@@ -117,9 +117,12 @@ static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit
 #define GDN_PSTAMP(slot)
 #endif
 
+// kRaw: the tiles come from the packed projection rows (tm_q is a 2-D map over them, tm_k and tm_v the 4-D maps of the planes
+// of normalised keys and queries, which the walk reads); Q and K rows are L2-normalised in shared memory, gate and beta
+// activated on load.
 // kRepair: behind a single-launch forward that left some heads (Repair::flags); a grid that just fills the device takes
 // the chunks of those heads in turn, and leaves at once when there are none.
-template <bool kRepair>
+template <bool kRaw, bool kRepair>
 __global__ void __launch_bounds__(kPrepThreads, 3)
 prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_wh,
@@ -207,12 +210,25 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     // the input tiles do not depend on tensor memory: start them before the allocation
     mbar_arrive_expect_tx(bar_tma, 6 * kBox);
-    tma_load_4d(sm + L::kQ0, &tm_q, bar_tma, 0, hk, t0, b);
-    tma_load_4d(sm + L::kQ1, &tm_q, bar_tma, 64, hk, t0, b);
-    tma_load_4d(sm + L::kK0, &tm_k, bar_tma, 0, hk, t0, b);
-    tma_load_4d(sm + L::kK1, &tm_k, bar_tma, 64, hk, t0, b);
-    tma_load_4d(sm + L::kV0, &tm_v, bar_tma, 0, hv, t0, b);
-    tma_load_4d(sm + L::kV1, &tm_v, bar_tma, 64, hv, t0, b);
+    if (kRaw) {
+      // packed rows [q heads | k heads | v heads]; rows behind the batch element's end belong to the next one
+      // (or read as zero behind the last) and are neutralised by beta = 0 / zero gate weights
+      const int row = b * geo.sequence + t0;
+      const int xq = hk * kDim, xk = (geo.key_heads + hk) * kDim, xv = (2 * geo.key_heads + hv) * kDim;
+      tma_load_2d(sm + L::kQ0, &tm_q, bar_tma, xq, row);
+      tma_load_2d(sm + L::kQ1, &tm_q, bar_tma, xq + 64, row);
+      tma_load_2d(sm + L::kK0, &tm_q, bar_tma, xk, row);
+      tma_load_2d(sm + L::kK1, &tm_q, bar_tma, xk + 64, row);
+      tma_load_2d(sm + L::kV0, &tm_q, bar_tma, xv, row);
+      tma_load_2d(sm + L::kV1, &tm_q, bar_tma, xv + 64, row);
+    } else {
+      tma_load_4d(sm + L::kQ0, &tm_q, bar_tma, 0, hk, t0, b);
+      tma_load_4d(sm + L::kQ1, &tm_q, bar_tma, 64, hk, t0, b);
+      tma_load_4d(sm + L::kK0, &tm_k, bar_tma, 0, hk, t0, b);
+      tma_load_4d(sm + L::kK1, &tm_k, bar_tma, 64, hk, t0, b);
+      tma_load_4d(sm + L::kV0, &tm_v, bar_tma, 0, hv, t0, b);
+      tma_load_4d(sm + L::kV1, &tm_v, bar_tma, 64, hv, t0, b);
+    }
   }
   if (warp == 1 && (!kRepair || round == 0)) {
     tmem_alloc(tmem_slot, kPrepTmemCols);
@@ -221,8 +237,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   float gate = 0.f, beta = 0.f;
   if (tid < valid) {
     const long long gi = ((long long)b * geo.sequence + t0 + tid) * geo.value_heads + hv;
-    gate = load_gate(in.g, gi, in.gate_fp32);
-    beta = __bfloat162float(in.beta[gi]);
+    gate = kRaw ? raw_gate(in, bf16_bits(in.act_a + gi), hv) : load_gate(in.g, gi, in.gate_fp32);
+    beta = kRaw ? raw_beta(in, gi) : __bfloat162float(in.beta[gi]);
   }
   tc_fence_before();
   __syncthreads();
@@ -245,6 +261,23 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   // ---- phase 2: D1 = [Q;K] K^T
   bool ok = mbar_wait(bar_tma, kRepair ? round & 1 : 0, abort, 1, chunk);
   GDN_PSTAMP(1);
+  if (kRaw) {
+    static_assert(L::kQ0 == 0 && L::kK0 == kBox && L::kQ1 == 2 * kBox && L::kK1 == 3 * kBox, "tiles as normalise_rows takes them");
+    if (ok) {
+#pragma unroll
+      for (int pass = 0; pass < 8; ++pass) normalise_rows(sm, pass, tid);
+      fence_proxy_async_smem();
+    }
+    __syncthreads();
+    // the walk reads the normalised queries and keys: one CTA per key head stores the tiles (rows behind T are clipped)
+    if (tid == 0 && ok && hv % geo.group() == 0) {
+      tma_store_4d(&tm_k, sm + L::kK0, 0, hk, t0, b);
+      tma_store_4d(&tm_k, sm + L::kK1, 64, hk, t0, b);
+      tma_store_4d(&tm_v, sm + L::kQ0, 0, hk, t0, b);
+      tma_store_4d(&tm_v, sm + L::kQ1, 64, hk, t0, b);
+      tma_store_commit();
+    }
+  }
   const uint32_t base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);       // warp-uniform, for the descriptors
   if (warp == 0 && __all_sync(0xffffffffu, ok) && elect_one()) {
     tc_fence_after();
@@ -337,6 +370,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
     if (lrow >= 64) not_contraction = !(bi >= 0.f && bi * kk <= 2.f);
   }
+  if (kRaw && tid == 0) tma_store_wait_read();     // the inverse's scratch and the T tiles reuse the Q boxes from here on
   const int chunk_not_contraction = __syncthreads_or(not_contraction);
   ok = __syncthreads_and(ok);                  // uniform from here on: the warp-level barrier below needs that
   GDN_PSTAMP(3);
@@ -1188,21 +1222,26 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 // ======================================================================================= launchers
 int configure_umma() {
   if (int rc = tensor_map_encoder().init()) return rc;
-  cudaError_t e = cudaFuncSetAttribute(prepare_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
-  if (e != cudaSuccess) return int(e);
-  e = cudaFuncSetAttribute(prepare_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
-  if (e != cudaSuccess) return int(e);
-  e = cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
-  return int(e);
+  for (const auto prepare : {prepare_umma_kernel<false, false>, prepare_umma_kernel<false, true>, prepare_umma_kernel<true, false>})
+    if (cudaError_t e = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem)) return int(e);
+  return int(cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem));
 }
 
 int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream, const Repair& left) {
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
   CUtensorMap tm_q, tm_k, tm_v;
-  if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-  if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-  if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  if (in.mixed) {
+    // one 2-D map over the packed projection rows; the 4-D maps of the normalised planes are store targets
+    if (!in.q || !in.k || left.flags) return int(cudaErrorInvalidValue);
+    if (int rc = enc.bf16_2d(&tm_q, in.mixed, uint64_t(in.mixed_stride), uint64_t(geo.batch) * geo.sequence, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_v, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  } else {
+    if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  }
   // W^T planes: [blocks * 128 key rows][64 tokens], one 128-row box per block (the walk loads the same boxes)
   CUtensorMap tm_wh, tm_wl;
   const uint64_t plane_rows = uint64_t(geo.blocks()) * kDim;
@@ -1211,11 +1250,12 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
   const long long grid = (long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel);
   if (!left.flags) {
-    prepare_umma_kernel<false><<<(unsigned)grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
+    const auto prepare = in.mixed ? prepare_umma_kernel<true, false> : prepare_umma_kernel<false, false>;
+    prepare<<<(unsigned)grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
     return int(cudaGetLastError());
   }
   const long long resident = 3LL * left.sms;
-  return launch_early(prepare_umma_kernel<true>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
+  return launch_early(prepare_umma_kernel<false, true>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
                       tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
 }
 

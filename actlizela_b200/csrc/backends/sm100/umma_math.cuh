@@ -98,6 +98,23 @@ __device__ __forceinline__ void tile_product_tf32x3(float (&d)[4], const float* 
 }
 __device__ __forceinline__ float bf16_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }
+// L2-normalises 16 of the 128 rows of a [Q0 K0 Q1 K1] tile group in place, the pass-th sixteen of the 64 Q rows and then the 64 K
+// rows: 256 threads, 16 per row (one swizzled 16-byte slot each); x rsqrt(sum x^2 + 1e-6) rounded to BF16.
+__device__ __forceinline__ void normalise_rows(uint8_t* tiles, int pass, int t) {
+  const int lane16 = t & 15, r = pass * 16 + (t >> 4), row = r & 63;
+  uint8_t* slot = tiles + ((r < 64 ? 0 : 1) + (lane16 < 8 ? 0 : 2)) * kBox + row * 128 + (((lane16 & 7) ^ (row & 7)) << 4);
+  const uint4 x = *reinterpret_cast<const uint4*>(slot);
+  const float f[8] = {bf16_lo(x.x), bf16_hi(x.x), bf16_lo(x.y), bf16_hi(x.y),
+                      bf16_lo(x.z), bf16_hi(x.z), bf16_lo(x.w), bf16_hi(x.w)};
+  float square = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) square = fmaf(f[e], f[e], square);
+#pragma unroll
+  for (int d = 8; d; d >>= 1) square += __shfl_xor_sync(0xffffffffu, square, d, 16);
+  const float factor = rsqrtf(square + 1e-6f);
+  *reinterpret_cast<uint4*>(slot) = make_uint4(pack_bf16(f[0] * factor, f[1] * factor), pack_bf16(f[2] * factor, f[3] * factor),
+                                               pack_bf16(f[4] * factor, f[5] * factor), pack_bf16(f[6] * factor, f[7] * factor));
+}
 // (x0, x1) ~ hi + lo as packed BF16 pairs
 __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
   hi = pack_bf16(x0, x1);

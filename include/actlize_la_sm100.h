@@ -238,12 +238,12 @@ int actlize_la_sm100_selftest_walk_stall(
 
 /* The forward on the raw projection outputs of the layer: the step before the path (Q/K L2-normalisation, gate
  * activation g = -exp(A_log) softplus(a + dt_bias), beta = sigmoid(b); csrc/serving/prefill.cu:45-70,
- * csrc/serving/runtime.cuh:48-52) is done inside the single-launch kernel instead of by a kernel of its own
+ * csrc/serving/runtime.cuh:48-52) is done inside the forward's kernels instead of by a kernel of its own
  * (actlize_la_sm100_prepare_inputs): `mixed` is BF16 [B*T][mixed_row_stride] with the row layout
  * [Hk q vectors | Hk k vectors | Hv v vectors] x 128, `a` and `b` are BF16 [B*T][Hv], `a_log`, `dt_bias` FP32 [Hv].
  * Same results, bit for bit, as prepare_inputs followed by forward_prepared with an FP32 gate.  `config` as returned
- * by actlize_la_sm100_select (a tensor-core configuration, no stage bits; both families run the single-launch kernel
- * here); workspace: actlize_la_sm100_projections_workspace_bytes, flag words only.  Rows behind a batch
+ * by actlize_la_sm100_select (a tensor-core configuration, no stage bits; the entry chooses between the two families by
+ * a rule of its own); workspace: actlize_la_sm100_projections_workspace_bytes.  Rows behind a batch
  * element's end inside its last chunk are the next element's tokens and meet exact zeros: inputs must be finite. */
 long long actlize_la_sm100_projections_workspace_bytes(int b, int t, int hk, int hv, int config);
 int actlize_la_sm100_forward_projections(

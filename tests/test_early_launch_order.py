@@ -28,8 +28,10 @@ def _body(code, kernel):
 def _early_kernels():
     for path in sorted(SOURCES.glob("*.cu")):
         code = _code(path)
-        for name in re.findall(r"launch_early\((\w+_kernel)\b", code) + (
-                ["out_proj_skinny_kernel"] if "attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization" in code else []):
+        names = {name for m in re.finditer(r"return launch_early\(", code) for name in re.findall(r"\b\w+_kernel\b", code[m.end():m.end() + 100])}
+        if "attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization" in code:
+            names.add("out_proj_skinny_kernel")
+        for name in sorted(names):
             yield pytest.param(code, name, id=name)
 
 

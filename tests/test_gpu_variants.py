@@ -1,5 +1,6 @@
 """Kernel variants chosen by a rule on sizes, at the edges of their ranges, against the oracle or the two-kernel path."""
 import ctypes
+import math
 
 import pytest
 import torch
@@ -156,3 +157,46 @@ def test_cuts_follow_the_gates(chunks, reach, split, native_library):
             assert torch.equal(out[:, :, h], want_out[:, :, h]) and torch.equal(state[:, h], want_state[:, h])
     again_out, again_state = forward(*dev, True, configuration="fused-split")
     assert torch.equal(again_out, out) and torch.equal(again_state, state)
+
+
+@pytest.mark.parametrize("batch,length,hk,hv,slow,split", [
+    (1, 64, 1, 2, {}, None),                             # one chunk: single launch
+    (1, 65, 1, 2, {}, None),
+    (1, 700, 2, 8, {}, None),                            # few heads: two kernels, walked whole
+    (3, 64 * 9 + 1, 1, 2, {}, None),                     # rows behind a batch element's end are the next one's
+    (1, 64 * 180 + 9, 2, 8, {}, 8),                      # cut into eight
+    (1, 64 * 180 + 9, 2, 8, {3: 18, 5: 1000}, 7),        # one head that just allows that, one that does not
+    (2, 64 * 16 + 3, 37, 37, {3: 1000}, 72),             # the most heads that can be cut, into two
+    (5, 64 * 2 + 3, 5, 15, {}, None)])                   # one head more: single launch
+def test_projections_in_every_form(batch, length, hk, hv, slow, split, native_library):
+    """Raw projections in the two kernels (one CTA per key head stores its normalised queries and keys), walked whole and cut, and
+    in the single launch: the outputs of prepare_inputs + forward, bit for bit where that walks them alike.  ``slow``:
+    chunks that a head's state outlives."""
+    from actlizela_b200 import gdn_forward_projections, gdn_prepare_inputs
+    from actlizela_b200.sm100 import Sm100Forward
+    gen = torch.Generator().manual_seed(9000 + length)
+    mixed = torch.randn(batch, length, (2 * hk + hv) * 128, generator=gen).to(torch.bfloat16).cuda()
+    a, b = ((0.1 * torch.randn(batch, length, hv, generator=gen)).to(torch.bfloat16).cuda() for _ in range(2))
+    a_log, dt_bias = torch.zeros(hv), torch.zeros(hv)
+    for h, reach in slow.items():                        # softplus(0) = 0.693 nats a token, scaled
+        a_log[h] = math.log(40.0 / (64 * (reach - 0.5)) / 0.693)
+    a_log, dt_bias = a_log.cuda(), dt_bias.cuda()
+    initial = (0.05 * torch.randn(batch, hv, 128, 128, generator=gen)).cuda()
+    rows = batch * length
+    prepared = [x.view(batch, length, *x.shape[1:]) for x in
+                gdn_prepare_inputs(mixed.view(rows, -1), a.view(rows, hv), b.view(rows, hv), a_log, dt_bias, hk, hv)]
+    want_out, want_state = Sm100Forward(native_library)(*prepared, initial, True, configuration="umma")
+    counts = (ctypes.c_int * 2)()
+    assert native_library.lib.actlize_la_sm100_walk_plan_counts(counts, 1) == 0
+    out, state = gdn_forward_projections(mixed, a, b, a_log, dt_bias, hk, hv, initial, True)
+    torch.cuda.synchronize()
+    assert _healthy(native_library)
+    assert native_library.lib.actlize_la_sm100_walk_plan_counts(counts, 1) == 0
+    if split is not None:
+        assert list(counts) == [split, batch * hv - split]
+    for h in range(hv):
+        if split is None or slow.get(h) == 1000:
+            assert torch.equal(out[:, :, h], want_out[:, :, h]) and torch.equal(state[:, h], want_state[:, h])
+        else:                                            # as in test_cuts_follow_the_gates
+            assert oracle.rel_frobenius(out[:, :, h].float().cpu(), want_out[:, :, h].float().cpu()) < 5e-4
+            assert oracle.rel_frobenius(state[:, h].cpu(), want_state[:, h].cpu()) < 8e-6
