@@ -496,6 +496,30 @@ extern "C" int actlize_la_sm100_forward_projections(
 namespace {
 long long align256_ll(long long x) { return (x + 255) & ~255LL; }
 long long varlen_table_bytes(int n_seqs) { return align256_ll((n_seqs + 1LL) * (long long)sizeof(int)); }
+// Few (sequence, value head) items of some chunks each: the two kernels.  The walk of the longest item then counts, at 2.1 us a chunk
+// against 3.8 in the single launch, and the prepare kernel (31 ns a block) and the second launch cost less than that saves;
+// with items for more than half the SMs the single launch deals them out.  The longest sequence is not known here, so the line
+// is drawn by the mean: it meets the measured break-even at 33 to 60 items of 2 to 3 chunks, 80 of 5 and 90 of 19 (two
+// sequences of 1200 tokens, 6 heads: 131 us in the single launch, 89; 10 x 600, 6 heads: 84 and 73; 6 x 1200, 16 heads, 96
+// items: 127 and 134).
+constexpr int kPackedItems = 90, kPackedTokens = 90 * kChunk;
+static_assert(kPackedItems <= kMostPacked, "every sequence has at least one item");
+bool varlen_in_two_kernels(long long total_tokens, int n_seqs, int hv) {
+  const long long items = (long long)n_seqs * hv;
+  return items < kPackedItems && (kPackedItems - items) * total_tokens >= (long long)kPackedTokens * n_seqs;
+}
+long long varlen_factor_bytes(long long total_tokens, int n_seqs, int hv) {
+  return ((total_tokens + kChunk - 1) / kChunk + n_seqs) * hv * kBlockBytes;
+}
+// `offsets` on the device, `factors` behind the table in the workspace
+int run_varlen(const Inputs& in, long long total_tokens, int n_seqs, int hk, int hv, const int* offsets, void* workspace, cudaStream_t stream) {
+  Geometry geo{n_seqs, int(total_tokens), hk, hv};
+  geo.varlen = offsets;                // read by the kernels, clamped there into the tensors: no host read
+  if (!varlen_in_two_kernels(total_tokens, n_seqs, hv)) return launch_forward_fused(in, geo, nullptr, Workspace{}, stream);
+  const Workspace ws = carve_workspace(static_cast<char*>(workspace) + varlen_table_bytes(n_seqs), geo);
+  if (int rc = launch_prepare_umma(in, geo, ws, stream)) return rc;
+  return launch_walk_umma(in, geo, ws, true, stream);
+}
 }  // namespace
 
 extern "C" long long actlize_la_sm100_varlen_workspace_bytes(long long total_tokens, int n_seqs, int hk, int hv) {
@@ -503,7 +527,7 @@ extern "C" long long actlize_la_sm100_varlen_workspace_bytes(long long total_tok
   // every sequence starts a new chunk, so each may add one partly filled chunk to ceil(total / 64)
   const long long max_chunks = (total_tokens + kChunk - 1) / kChunk + n_seqs;
   if (max_chunks * hv > INT_MAX / kDim || (long long)n_seqs * hv > INT_MAX / 8) return -1;
-  return varlen_table_bytes(n_seqs);
+  return varlen_table_bytes(n_seqs) + (varlen_in_two_kernels(total_tokens, n_seqs, hv) ? varlen_factor_bytes(total_tokens, n_seqs, hv) : 0);
 }
 
 extern "C" int actlize_la_sm100_forward_varlen(
@@ -526,12 +550,10 @@ extern "C" int actlize_la_sm100_forward_varlen(
   // pageable source: the runtime has staged the bytes when the call returns
   cudaError_t e = cudaMemcpyAsync(workspace, cu_seqlens_host, (n_seqs + 1) * sizeof(int), cudaMemcpyHostToDevice, stream);
   if (e != cudaSuccess) return int(e);
-  Geometry geo{n_seqs, total, hk, hv};
-  geo.varlen = static_cast<const int*>(workspace);
   const Inputs in{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                   static_cast<const __nv_bfloat16*>(v), g, static_cast<const __nv_bfloat16*>(beta),
                   initial_states, static_cast<__nv_bfloat16*>(output), final_states, gate_fp32 ? 1 : 0};
-  return launch_forward_fused(in, geo, nullptr, Workspace{}, stream);
+  return run_varlen(in, total, n_seqs, hk, hv, static_cast<const int*>(workspace), workspace, stream);
 }
 
 extern "C" int actlize_la_sm100_forward_varlen_device(
@@ -548,12 +570,10 @@ extern "C" int actlize_la_sm100_forward_varlen_device(
       (reinterpret_cast<uintptr_t>(output) & 15))
     return int(cudaErrorInvalidValue);
   cudaStream_t stream = static_cast<cudaStream_t>(opaque_stream);
-  Geometry geo{n_seqs, int(total_tokens), hk, hv};
-  geo.varlen = cu_seqlens_device;      // read by the kernel, clamped there into the tensors: no host read, one launch
   const Inputs in{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
                   static_cast<const __nv_bfloat16*>(v), g, static_cast<const __nv_bfloat16*>(beta),
                   initial_states, static_cast<__nv_bfloat16*>(output), final_states, gate_fp32 ? 1 : 0};
-  return launch_forward_fused(in, geo, nullptr, Workspace{}, stream);
+  return run_varlen(in, total_tokens, n_seqs, hk, hv, cu_seqlens_device, workspace, stream);
 }
 
 namespace {

@@ -22,15 +22,17 @@ struct Geometry {
   // tensor-core kernels only: the launch's chunk range is cut into `parallel` sub-segments per (batch, value head), walked by
   // as many CTAs at the same time (0 or 1 = one CTA walks the whole range); see walk_umma_kernel.
   int parallel = 0;
-  // Packed variable-length mode (single-launch kernel only): the tensors are [1, sequence = total tokens, H, ...],
+  // Packed variable-length mode (tensor-core kernels): the tensors are [1, sequence = total tokens, H, ...],
   // `batch` is the number of sequences and `varlen` points at the token offsets cu_seqlens[0..batch] on the device.
+  // Workspace blocks of the two-kernel form are then indexed hv * slots() + varlen_slot(sequence) + chunk.
   const int* varlen = nullptr;
   __host__ __device__ int chunks() const { return (sequence + kChunk - 1) / kChunk; }
   __host__ __device__ int segment_chunks() const { return chunk_count ? chunk_count : chunks(); }
   __host__ __device__ bool first_segment() const { return chunk_begin == 0; }
   __host__ __device__ bool last_segment() const { return chunk_begin + segment_chunks() == chunks(); }
   __host__ __device__ int group() const { return value_heads / key_heads; }
-  __host__ __device__ long long blocks() const { return (long long)batch * value_heads * chunks(); }
+  __host__ __device__ int slots() const { return chunks() + batch; }
+  __host__ __device__ long long blocks() const { return (long long)value_heads * (varlen ? slots() : (long long)batch * chunks()); }
 };
 
 // Parallel sub-segments of a walk over `chunks` chunks: sub-segment r covers [sub_segment_begin(r), sub_segment_begin(r + 1)).
@@ -44,6 +46,12 @@ __host__ __device__ inline int sub_segment_begin(int chunks, int r, int parallel
   const int body = chunks - kNominalReach;
   return int((long long)(body >= parallel * kNominalReach ? body : chunks) * r / parallel);
 }
+
+// Packed mode, slot of a sequence's first chunk: sequences of any lengths in order get ranges of slots that do not meet (a
+// sequence of n tokens from offset t on has at most floor((t + n) / 64) - floor(t / 64) + 1 chunks), without a table
+// of the chunk counts in front of it.
+__host__ __device__ inline int varlen_slot(int offset, int sequence) { return offset / kChunk + sequence; }
+constexpr int kMostPacked = 96;      // sequences of a packed call in the two-kernel form
 
 // Workspace: structure-of-arrays planes, one entry per (batch, value head, chunk) block,
 // block index = (b * Hv + hv) * chunks + c.  W is stored TRANSPOSED (key-dimension-major), the orientation the

@@ -112,7 +112,7 @@ static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit
 
 #ifdef GDN_SM100_PHASE_TIMING
 #define GDN_PSTAMP(slot) \
-  if (tid == 0) ws.gates[block * kGateWords + 80 + (slot)] = float((clock64() - t_begin) & 0xffffff)
+  if (tid == 0) ws.gates[block * kGateWords + 80 + (slot)] = float((clock64() - clock_begin) & 0xffffff)
 #else
 #define GDN_PSTAMP(slot)
 #endif
@@ -122,7 +122,27 @@ static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit
 // activated on load.
 // kRepair: behind a single-launch forward that left some heads (Repair::flags); a grid that just fills the device takes
 // the chunks of those heads in turn, and leaves at once when there are none.
-template <bool kRaw, bool kRepair>
+// kPacked: the grid holds a CTA per (value head, slot).
+enum PrepareMode { kPlain, kRawInputs, kRepairing, kPackedSequences };
+// Token offset of sequence boundary i, forced into 0 <= ... <= total and non-decreasing (no index can leave the tensors), for one
+// warp: lane l returns boundaries l, l + 32, ... in at[].
+__device__ __forceinline__ void clamped_offsets(const Geometry& geo, int lane, int (&at)[kMostPacked / 32 + 1]) {
+  int most = 0;
+#pragma unroll
+  for (int u = 0; u <= kMostPacked / 32; ++u) {
+    const int i = u * 32 + lane;
+    int x = i && i <= geo.batch ? geo.varlen[i] : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x = max(x, y);
+    }
+    x = max(x, most);
+    most = __shfl_sync(0xffffffffu, x, 31);
+    at[u] = min(x, geo.sequence);
+  }
+}
+template <PrepareMode kMode>
 __global__ void __launch_bounds__(kPrepThreads, 3)
 prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_wh,
@@ -144,6 +164,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* carry = reinterpret_cast<float*>(tmem_slot + 2);
   const AbortFlag abort{abort_word};
+  constexpr bool kRaw = kMode == kRawInputs, kRepair = kMode == kRepairing, kPacked = kMode == kPackedSequences;
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int chunks = geo.chunks(), seg_chunks = geo.segment_chunks();
@@ -170,8 +191,27 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
 #pragma unroll 1
   for (int round = 0;; ++round) {
-  int bh, chunk;
-  if constexpr (kRepair) {
+  int bh, chunk, t_begin = 0, t_end = geo.sequence;
+  if constexpr (kPacked) {
+    // sequence whose slots hold this one: every warp finds it for itself
+    int at[kMostPacked / 32 + 1];
+    clamped_offsets(geo, tid & 31, at);
+    const int slot = int(blockIdx.x) % geo.slots();
+    int seq = -1;
+#pragma unroll
+    for (int u = 0; u <= kMostPacked / 32; ++u) {
+      const int i = u * 32 + (tid & 31);
+      seq += __popc(__ballot_sync(0xffffffffu, i < geo.batch && varlen_slot(at[u], i) <= slot));
+    }
+#pragma unroll
+    for (int u = 0; u <= kMostPacked / 32; ++u) {
+      if (seq >> 5 == u) t_begin = __shfl_sync(0xffffffffu, at[u], seq & 31);
+      if ((seq + 1) >> 5 == u) t_end = __shfl_sync(0xffffffffu, at[u], (seq + 1) & 31);
+    }
+    bh = int(blockIdx.x) / geo.slots();                   // (batch 0)
+    chunk = slot - varlen_slot(t_begin, seq);
+    if (t_begin + chunk * kChunk >= t_end) return;
+  } else if constexpr (kRepair) {
     const int at = int(blockIdx.x) + round * int(gridDim.x);
     if (at >= s_count * chunks) break;
     bh = s_left[at % s_count];
@@ -194,11 +234,11 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   const int b = bh / geo.value_heads, hv = bh % geo.value_heads;
   const int hk = hv / geo.group();
-  const int t0 = chunk * kChunk, t_end = geo.sequence;
-  const long long block = (long long)bh * chunks + chunk;
+  const int t0 = t_begin + chunk * kChunk;
+  const long long block = kPacked ? blockIdx.x : (long long)bh * chunks + chunk;
   const int valid = min(kChunk, t_end - t0);
 #ifdef GDN_SM100_PHASE_TIMING
-  const long long t_begin = clock64();
+  const long long clock_begin = clock64();
 #endif
 
   if (tid == 0) {
@@ -771,12 +811,26 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     if (!__syncthreads_or(mark)) return;
     counted_cut = !__syncthreads_or(mark == 2);
   }
-  const int b = bh / geo.value_heads;
+  int b = bh / geo.value_heads;
   const int hv = bh % geo.value_heads;
   const int hk = hv / geo.group();
   int chunks = geo.segment_chunks();                 // this launch walks `chunks` chunks from token t_first on
-  int t_first = geo.chunk_begin * kChunk;
+  int t_first = geo.chunk_begin * kChunk, tail_valid = kChunk;
   long long block0 = (long long)bh * geo.chunks() + geo.chunk_begin;
+  if (geo.varlen) {
+    // packed sequences: one CTA per (sequence, value head); states are indexed by bh = sequence * Hv + hv
+    int at[kMostPacked / 32 + 1], t_last = 0;
+    clamped_offsets(geo, lane, at);
+#pragma unroll
+    for (int u = 0; u <= kMostPacked / 32; ++u) {
+      if (b >> 5 == u) t_first = __shfl_sync(0xffffffffu, at[u], b & 31);
+      if ((b + 1) >> 5 == u) t_last = __shfl_sync(0xffffffffu, at[u], (b + 1) & 31);
+    }
+    chunks = (t_last - t_first + kChunk - 1) / kChunk;
+    tail_valid = t_last - t_first - (chunks - 1) * kChunk;                  // rows of the sequence's last chunk
+    block0 = (long long)hv * geo.slots() + varlen_slot(t_first, b);
+    b = 0;
+  }
   const float* state_in = geo.first_segment() ? in.initial : ws.carry;
   float* state_out = geo.last_segment() ? in.final_state : ws.carry;
   if (sub > 0) state_in = nullptr;
@@ -1044,6 +1098,16 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       GDN_OSTAMP(1);
       if (c < unstored) continue;
       const int cs = c - unstored;           // count of stored tiles: staging buffers and their barriers follow it
+      if (geo.varlen && c == chunks - 1 && tail_valid < kChunk) {
+        // packed mode, ragged end of a sequence: the rows behind it belong to the next sequence, so the tile
+        // cannot leave through a clipping TMA store; this is the sequence's last chunk, nothing follows it
+        __nv_bfloat16* out = in.output + ((long long)(t_first + c * kChunk) * geo.value_heads + hv) * kDim + v;
+        const long long row = (long long)geo.value_heads * kDim;
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (i < tail_valid) out[i * row] = __float2bfloat16_rn(__uint_as_float(o[i]));
+        break;
+      }
       // stage the tile as two 128-byte-swizzled boxes [token][64 values] and hand it to a TMA store,
       // which also clips the rows of a tail chunk at the sequence end
       uint8_t* stage = sm + L::kOut + (cs & 1) * 2 * kBox + (v >> 6) * kBox + ((v & 7) << 1);
@@ -1222,7 +1286,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 // ======================================================================================= launchers
 int configure_umma() {
   if (int rc = tensor_map_encoder().init()) return rc;
-  for (const auto prepare : {prepare_umma_kernel<false, false>, prepare_umma_kernel<false, true>, prepare_umma_kernel<true, false>})
+  for (const auto prepare : {prepare_umma_kernel<kPlain>, prepare_umma_kernel<kRawInputs>, prepare_umma_kernel<kRepairing>,
+                             prepare_umma_kernel<kPackedSequences>})
     if (cudaError_t e = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem)) return int(e);
   return int(cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem));
 }
@@ -1230,17 +1295,20 @@ int configure_umma() {
 int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, cudaStream_t stream, const Repair& left) {
   TensorMapEncoder& enc = tensor_map_encoder();
   if (int rc = enc.init()) return rc;
+  if (geo.varlen && (geo.batch > kMostPacked || geo.chunk_begin || geo.chunk_count || geo.parallel > 1 || left.flags))
+    return int(cudaErrorInvalidValue);
+  const uint64_t batch = geo.varlen ? 1 : geo.batch;
   CUtensorMap tm_q, tm_k, tm_v;
   if (in.mixed) {
     // one 2-D map over the packed projection rows; the 4-D maps of the normalised planes are store targets
-    if (!in.q || !in.k || left.flags) return int(cudaErrorInvalidValue);
+    if (!in.q || !in.k || geo.varlen || left.flags) return int(cudaErrorInvalidValue);
     if (int rc = enc.bf16_2d(&tm_q, in.mixed, uint64_t(in.mixed_stride), uint64_t(geo.batch) * geo.sequence, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_v, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
   } else {
-    if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-    if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-    if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, geo.batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
+    if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, batch, kChunk)) return rc;
   }
   // W^T planes: [blocks * 128 key rows][64 tokens], one 128-row box per block (the walk loads the same boxes)
   CUtensorMap tm_wh, tm_wl;
@@ -1250,12 +1318,13 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
   const long long grid = (long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel);
   if (!left.flags) {
-    const auto prepare = in.mixed ? prepare_umma_kernel<true, false> : prepare_umma_kernel<false, false>;
-    prepare<<<(unsigned)grid, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
+    const auto prepare = geo.varlen ? prepare_umma_kernel<kPackedSequences>
+                         : in.mixed ? prepare_umma_kernel<kRawInputs> : prepare_umma_kernel<kPlain>;
+    prepare<<<(unsigned)(geo.varlen ? geo.blocks() : grid), kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
     return int(cudaGetLastError());
   }
   const long long resident = 3LL * left.sms;
-  return launch_early(prepare_umma_kernel<false, true>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
+  return launch_early(prepare_umma_kernel<kRepairing>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
                       tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
 }
 
@@ -1264,14 +1333,16 @@ int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws,
   if (int rc = enc.init()) return rc;
   const uint64_t rows = uint64_t(geo.blocks()) * kChunk;
   CUtensorMap tm_wh, tm_wl, tm_q, tm_k, tm_p, tm_out;
-  if (int rc = enc.bf16_4d(&tm_out, in.output, kDim, geo.value_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  const uint64_t batch = geo.varlen ? 1 : geo.batch;
+  if (int rc = enc.bf16_4d(&tm_out, in.output, kDim, geo.value_heads, geo.sequence, batch, kChunk)) return rc;
   // W^T planes: [blocks * 128 key rows][64 tokens], one 128-row box per block
   if (int rc = enc.bf16_2d(&tm_wh, ws.w_hi, kChunk, 2 * rows, kDim)) return rc;
   if (int rc = enc.bf16_2d(&tm_wl, ws.w_lo, kChunk, 2 * rows, kDim)) return rc;
-  if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
-  if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_q, in.q, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
+  if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
   if (int rc = enc.bf16_2d(&tm_p, ws.p, kChunk, rows, kChunk)) return rc;
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
+  if (geo.varlen && (geo.batch > kMostPacked || in.walk_flags || parallel > 1 || left.flags)) return int(cudaErrorInvalidValue);
   if (parallel > 1 && (in.walk_flags || parallel > geo.segment_chunks())) return int(cudaErrorInvalidValue);
   if ((in.walk_flags & kWalkSelftestStall) && in.walk_flags != kWalkSelftestStall) return int(cudaErrorInvalidValue);
   if ((in.walk_flags & (kWalkTail | kWalkPair)) &&

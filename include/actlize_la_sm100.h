@@ -257,11 +257,11 @@ int actlize_la_sm100_forward_projections(
  * marks the boundaries; initial_states / final_states are FP32 [n_seqs,Hv,128,128] (nullable).  Every sequence
  * is chunked from its own start, an empty sequence passes its state through.  The reference has no such entry:
  * its serving prefill pads the requests into a fixed [R,W] batch first (csrc/serving/prefill.cu:196-255,
- * csrc/serving/abi.h:48-56); this entry removes the padding.  One launch on `stream`
- * plus one small host-to-device copy of the offsets (from pageable memory: not for stream capture).
+ * csrc/serving/abi.h:48-56); this entry removes the padding.  One or two launches on
+ * `stream` plus one small host-to-device copy of the offsets (from pageable memory: not for stream capture).
  * Rows behind a sequence's end inside its last chunk are the next sequence's tokens; they are multiplied by
  * exact zeros, so all inputs must be finite.  `workspace` needs actlize_la_sm100_varlen_workspace_bytes(...)
- * bytes (the offsets), 256-byte aligned.  Returns 0 or a cudaError_t value. */
+ * bytes (the offsets and, for few sequences, the factors), 256-byte aligned.  Returns 0 or a cudaError_t value. */
 long long actlize_la_sm100_varlen_workspace_bytes(long long total_tokens, int n_seqs, int hk, int hv);
 int actlize_la_sm100_forward_varlen(
     const void* q, const void* k, const void* v, const void* g, const void* beta,
@@ -270,8 +270,8 @@ int actlize_la_sm100_forward_varlen(
     const int* cu_seqlens_host, int n_seqs, int hk, int hv, int gate_fp32, void* stream);
 
 /* The packed forward with the offsets on the DEVICE: cu_seqlens_device[0..n_seqs] are int32 in device memory, as a
- * serving scheduler produces them; nothing is read on the host, nothing is allocated, and the call is one kernel
- * launch, so it can be captured in a CUDA graph.  `total_tokens` is the token dimension of the tensors.  Offsets are forced into
+ * serving scheduler produces them; nothing is read on the host, nothing is allocated, and the call is kernel
+ * launches only, so it can be captured in a CUDA graph.  `total_tokens` is the token dimension of the tensors.  Offsets are forced into
  * 0 <= ... <= total_tokens and made non-decreasing on the device; tokens behind the last offset are not written. */
 int actlize_la_sm100_forward_varlen_device(
     const void* q, const void* k, const void* v, const void* g, const void* beta,

@@ -122,6 +122,38 @@ def test_packed_sequences_dealt_longest_first(sequences, hv, native_library):
         assert torch.equal(out[:, a:b], want_out) and torch.equal(state[first:last], want_state)
 
 
+@pytest.mark.parametrize("lengths,hv", [([1], 1), ([0, 0, 577, 0, 63, 64, 65, 0], 6), ([300, 1, 129, 700] * 11, 1), ([640] * 44, 2),
+                                        ([255] * 25, 2), ([230] * 25, 2), ([2000, 3], 44)])
+def test_packed_sequences_in_two_kernels(lengths, hv, native_library):
+    """Few packed sequences, both sides of the rule, empty and ragged ones: the bits of the fixed-shape forward.  Device offsets
+    that run back or past the tensors mean what their clamped values mean."""
+    from actlizela_b200 import gdn_forward_varlen
+    bounds = [0]
+    for n in lengths:
+        bounds.append(bounds[-1] + n)
+    w = WORKLOADS["cfg1"].sliced(batch=1, length=bounds[-1], key_heads=1, value_heads=hv, seed=8000 + bounds[-1])
+    q, k, v, g, beta, _ = (x.cuda() if x is not None else None for x in make_inputs(w))
+    init = 0.05 * torch.randn(len(lengths), hv, 128, 128, generator=torch.Generator().manual_seed(len(lengths))).cuda()
+    want_out, want_state = gdn_forward_varlen(q, k, v, g, beta, bounds, init, True, per_sequence=True, algorithm="wy_sm100",
+                                              backend="cuda_sm100", configuration="umma")
+    for initial in (init, None):
+        out, state = gdn_forward_varlen(q, k, v, g, beta, torch.tensor(bounds, dtype=torch.int32, device="cuda"), initial, True)
+        torch.cuda.synchronize()
+        assert _healthy(native_library)
+        if initial is not None:
+            assert torch.equal(out, want_out) and torch.equal(state, want_state)
+    host_out, host_state = gdn_forward_varlen(q, k, v, g, beta, bounds, init, True)
+    assert torch.equal(host_out, want_out) and torch.equal(host_state, want_state)
+    odd = [1 << 30 if i == len(lengths) else at - 5 * (i % 3) for i, at in enumerate(bounds)]
+    clean, most = [0], 0
+    for at in odd[1:]:
+        most = max(most, at)
+        clean.append(min(most, bounds[-1]))
+    odd_out, odd_state = gdn_forward_varlen(q, k, v, g, beta, torch.tensor(odd, dtype=torch.int32, device="cuda"), init, True)
+    want_out, want_state = gdn_forward_varlen(q, k, v, g, beta, clean, init, True)
+    assert torch.equal(odd_out, want_out) and torch.equal(odd_state, want_state)
+
+
 @pytest.mark.parametrize("chunks,reach,split", [
     (300, (4, 20, 60), 2),                   # one for the single launch's 37 pieces, one for eight, one for neither
     (300, (30, 20, 12, 36, 1000), 4),
