@@ -5,7 +5,7 @@ CPU-generated tensors with the shapes and value distributions of the named
 configurations: q,k ~ N(0,1) L2-normalised per head vector (BF16); v ~ N(0,1) BF16;
 g a natural-log decay (FP32 or BF16); beta in (0,1) BF16; optional FP32 initial state.
 Generation is on the CPU with an explicit ``torch.Generator`` so that the device path
-and the CPU checker always see identical bits.
+and the CPU oracle always see identical bits.
 """
 from __future__ import annotations
 

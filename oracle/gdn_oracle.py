@@ -1,6 +1,6 @@
 """CPU oracle for the chunked gated-delta-rule (GDN) forward.  TEST INFRASTRUCTURE ONLY.
 
-Nothing in the product package imports this module; it is the checker used by the
+Nothing in the product package imports this module; it is used by the
 tests, the smoke entry and the CPU-baseline leg of the benchmark.
 
 It restates, in plain torch CPU code, the algorithm of the reference project
