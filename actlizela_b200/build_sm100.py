@@ -51,9 +51,8 @@ def render_policy_table(policy_path, out_path):
     out_path.write_text(
         "// generated from sm100_policy.json (%s); do not edit\n"
         "struct PolicyRow { int b, t, hk, hv, config, segments, parallel; };\n"
-        "constexpr int kPolicyDefault = %d;\n"
         "constexpr PolicyRow kPolicyRows[] = {\n%s\n};\n"
-        % (data["id"], ids[data["default"]], rows))
+        % (data["id"], rows))
 
 
 def host_command(out):

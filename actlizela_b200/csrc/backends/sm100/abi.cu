@@ -281,7 +281,7 @@ extern "C" int actlize_la_sm100_select(int b, int t, int hk, int hv, int gate_fp
   // and whose walk is the faster one per chunk; at most three chunks are over before its second launch, and with many
   // blocks its factors' way through memory costs more than the slower chunk period of the single launch.
   const long long heads = (long long)b * hv, chunks = (t + kChunk - 1) / kChunk;
-  long long parallel = 148 / heads;
+  long long parallel = kSms / heads;
   if (parallel > chunks / 8) parallel = chunks / 8;
   if (parallel > kMaxParallel) parallel = kMaxParallel;
   if (parallel < 1) parallel = 1;
@@ -447,7 +447,7 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
 // T16000: 435 and 378).  One chunk is over before a second launch (B1 T50: 23.6 and 20.4), and with more heads than half
 // the SMs nothing is cut and preparing them all first is never cheap (128 heads, T1000: 128 and 106).
 int projections_config(const Geometry& geo, int config) {
-  return 2LL * geo.batch * geo.value_heads <= 148 && geo.chunks() > 1 ? (config & ~0xf) | 1 : kFused;
+  return 2LL * geo.batch * geo.value_heads <= kSms && geo.chunks() > 1 ? (config & ~0xf) | 1 : kFused;
 }
 extern "C" long long actlize_la_sm100_projections_workspace_bytes(int b, int t, int hk, int hv, int config) {
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config) || ((config & 0xf) != 1 && !is_fused(config)) ||

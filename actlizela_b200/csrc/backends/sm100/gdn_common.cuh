@@ -13,6 +13,7 @@ namespace gdn_sm100 {
 
 constexpr int kChunk = 64;    // tokens per chunk
 constexpr int kDim = 128;     // key and value head dimension
+constexpr int kSms = 148;     // SMs of a B200: rules that read shapes only (no device) count on them
 constexpr float kScale = 0.08838834764831845f;  // 1/sqrt(128), applied exactly once
 
 struct Geometry {

@@ -17,12 +17,6 @@ namespace {
 // a contraction [1]; added to the two-kernel path's counts by read_walk_plan_counts.
 __device__ int g_fused_plan_counts[2];
 
-#ifdef GDN_SM100_PHASE_TIMING
-__device__ long long g_stamps[4][64][16], g_blocks[1024][2];
-#define STAMP(role, n, slot) do { if (blockIdx.x == 0 && (n) < 64) g_stamps[role][n][slot] = clock64(); } while (0)
-#else
-#define STAMP(role, n, slot)
-#endif
 
 // Warps (32, 64 registers a thread):
 //    0      issuer of the chain's tensor-core products
@@ -311,9 +305,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + s * L::kGateStage;
   const float *s_pl2 = gates + L::kPl2, *s_beta = gates + L::kBeta, *s_coefw = gates + L::kCoefW, *s_ecol = gates + L::kECol;
 
-  if (t == 224) STAMP(0, n, 0);
   bool ok = warp_wait(&bar->kq_full[s], (n / kRing) & 1) && !AbortFlag{&bar->abort}.raised();
-  if (t == 224) STAMP(0, n, 1);
   if (kRaw) {
     if (ok) {
 #pragma unroll 1
@@ -343,7 +335,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
 
   // ---- masks and decays on [Q;K] K^T
   ok = warp_wait(&bar->d[group], (n >> 1) & 1);
-  if (t == 224) STAMP(0, n, 2);
   tc_fence_after();
   if (lane == 0) mbar_arrive(&bar->qs_go[s]);
   const int quarter = warp & 3, half = warp >> 2, i = (quarter & 1) * 32 + lane;
@@ -359,7 +350,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   const float pi = s_pl2[i], bi = s_beta[i];
   // A takes the place of the T_u pair of this group's previous chunk, which U was formed from as that chunk began
   if (quarter >= 2 && n >= 2) ok = warp_wait(&bar->u[group], ((n >> 1) - 1) & 1) && ok;
-  if (t == 224) STAMP(0, n, 3);
   float* arow = sAT + i * L::kLd;
   if (ok && (diagonal || below)) {
     uint8_t* prow = tile_p + i * 128;
@@ -437,7 +427,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
     if (quarter >= 2 && diagonal) bad = !(bi >= 0.f && arow[i] <= 2.f);
   }
   not_contraction |= __any_sync(0xffffffffu, bad);
-  if (t == 224) STAMP(0, n, 4);
 
   // ---- T = (I+A)^-1 in place, blocked 16 -> 32 -> 64
   // diagonal 16x16 solves, a column per thread (left-looking, in registers); the 16 threads of a block sit in one warp and
@@ -473,7 +462,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
     for (int r = 0; r < 16; ++r) a0[r * L::kLd + col] = x[r];
   }
   group_sync(id);
-  if (t == 224) STAMP(0, n, 5);
   // block products T21 = -T22 (A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
   // above the diagonal, which holds nothing
   {
@@ -512,11 +500,9 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       if (step == 0) group_sync(id);
     }
   }
-  if (t == 224) STAMP(0, n, 6);
   // T_w has one place: free once the previous chunk's W^T has been formed from it
   if (n >= 1) ok = warp_wait(&bar->w, (n - 1) & 1) && ok;
   group_sync(id);
-  if (t == 224) STAMP(0, n, 7);
   // ---- T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row, 16 columns
   {
     const int row = t & 63, c0 = (t >> 6) * 16;
@@ -537,7 +523,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   }
   __syncwarp();
   if (lane == 0) mbar_arrive(&bar->t_ready[group]);       // P, the gate vector, T_u and T_w of this chunk
-  if (t == 224) STAMP(0, n, 8);
 
   return true;      // the same answer for the whole group; a wait that gave up shows at the next chunk's group_all
 }
@@ -552,9 +537,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const AbortFlag abort{&bar->abort};
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-#ifdef GDN_SM100_PHASE_TIMING
-  if (tid == 0) g_blocks[blockIdx.x][0] = clock64();
-#endif
   dependents_may_start();
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) {
@@ -760,7 +742,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // U^T = V^T (T diag(beta))^T, while the chain warps split the state
         ok = mbar_wait(&bar->t_ready[par], (n >> 1) & 1);
         ok &= mbar_wait(&bar->v_full, par);
-        STAMP(3, n, 0);
         tc_fence_after();
         const uint64_t dU = smem_desc(base + L::kAT + par * L::kATBytes, 16, 1024);
         if (elect_one()) {
@@ -778,7 +759,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
           ok &= mbar_wait(&bar->ops[half], par);
-          STAMP(3, n, 1 + half);
           tc_fence_after();
           const uint64_t dw = dW + uint64_t(half * 256);
           const uint32_t op = half * 16;
@@ -793,10 +773,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (half) mma_commit(&bar->ws);
           }
         }
-        STAMP(3, n, 3);
         ok &= mbar_wait(&bar->qs_done[s], (n / kRing) & 1);
         if (n > 0) ok &= mbar_wait(&bar->ofree, (n - 1) & 1);
-        STAMP(3, n, 4);
         tc_fence_after();
         const uint64_t qd = smem_desc(kq + L::kQ0, 16, 1024);
         if (elect_one()) {
@@ -812,7 +790,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
           ok &= mbar_wait(&bar->opn[half], par);
-          STAMP(3, n, 5 + half);
           tc_fence_after();
           const uint64_t dk = kd + uint64_t(half * 128);
           const uint32_t op = kAccX + half * 16;
@@ -832,7 +809,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
           }
         }
-        STAMP(3, n, 7);
       }
       ok = __all_sync(0xffffffffu, ok);
     }
@@ -951,9 +927,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int par = n & 1;
         const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + (n % kRing) * L::kGateStage;
         ok = mbar_wait(&bar->w_ready, par);            // (the gate vector comes with it)
-        if (tid == 128) STAMP(1, n, 0);
         if (n > 0) ok = ok && mbar_wait(&bar->s, (n - 1) & 1);
-        if (tid == 128) STAMP(1, n, 1);
         if (!ok) break;
         tc_fence_after();
         const float gamma = gates[kChunk];
@@ -984,9 +958,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (lane == 0) mbar_arrive(&bar->ops[part >> 1]);
           }
         }
-        if (tid == 128) STAMP(1, n, 2);
         ok = ok && mbar_wait(&bar->ws, par);
-        if (tid == 128) STAMP(1, n, 3);
         ok = ok && mbar_wait(&bar->u[par], (n >> 1) & 1);
         if (!ok) break;
         tc_fence_after();
@@ -1014,7 +986,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive(&bar->opn[part]);
         }
-        if (tid == 128) STAMP(1, n, 4);
       }
       if (ok && n > 0) ok = mbar_wait(&bar->s, (n - 1) & 1);
       if (ok && (flags & kHasFinal)) {
@@ -1175,12 +1146,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-#ifdef GDN_SM100_PHASE_TIMING
-  if (tid == 0) g_blocks[blockIdx.x][1] = clock64();
-#endif
   if (warp == kIssueWarp) tmem_dealloc(bar->tmem, 512);
 }
-#undef STAMP
 
 template <bool kRaw>
 int launch(const Inputs& in, const Geometry& geo, const Plan& plan, int grid, cudaStream_t stream) {
@@ -1266,7 +1233,3 @@ int read_fused_plan_counts(int* host_out2, int reset) {
 }
 
 }  // namespace gdn_sm100
-#ifdef GDN_SM100_PHASE_TIMING
-extern "C" int gdn_read_stamps(void* host) { return int(cudaMemcpyFromSymbol(host, gdn_sm100::g_stamps, sizeof(gdn_sm100::g_stamps))); }
-extern "C" int gdn_read_blocks(void* host) { return int(cudaMemcpyFromSymbol(host, gdn_sm100::g_blocks, sizeof(gdn_sm100::g_blocks))); }
-#endif

@@ -110,12 +110,6 @@ constexpr int kPrepSmem = PrepLayout::kTotal + 1024;
 constexpr int kPrepTmemCols = 128;   // D1 [0,64), later W^T;  U^T [64,128)
 static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit in one SM's shared memory");
 
-#ifdef GDN_SM100_PHASE_TIMING
-#define GDN_PSTAMP(slot) \
-  if (tid == 0) ws.gates[block * kGateWords + 80 + (slot)] = float((clock64() - clock_begin) & 0xffffff)
-#else
-#define GDN_PSTAMP(slot)
-#endif
 
 // kRaw: the tiles come from the packed projection rows (tm_q is a 2-D map over them, tm_k and tm_v the 4-D maps of the planes
 // of normalised keys and queries, which the walk reads); Q and K rows are L2-normalised in shared memory, gate and beta
@@ -237,9 +231,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const int t0 = t_begin + chunk * kChunk;
   const long long block = kPacked ? blockIdx.x : (long long)bh * chunks + chunk;
   const int valid = min(kChunk, t_end - t0);
-#ifdef GDN_SM100_PHASE_TIMING
-  const long long clock_begin = clock64();
-#endif
 
   if (tid == 0) {
     if (!kRepair || round == 0) {
@@ -284,7 +275,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  GDN_PSTAMP(0);
 
   const float prefix = chunk_prefix64(gate, tid, carry);   // contains a __syncthreads
   if (tid < kChunk) {
@@ -300,7 +290,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   // ---- phase 2: D1 = [Q;K] K^T
   bool ok = mbar_wait(bar_tma, kRepair ? round & 1 : 0, abort, 1, chunk);
-  GDN_PSTAMP(1);
   if (kRaw) {
     static_assert(L::kQ0 == 0 && L::kK0 == kBox && L::kQ1 == 2 * kBox && L::kK1 == 3 * kBox, "tiles as normalise_rows takes them");
     if (ok) {
@@ -331,7 +320,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   ok = ok && mbar_wait(bar_mma, 0, abort, 2, chunk);
   tc_fence_after();
-  GDN_PSTAMP(2);
 
   // ---- phase 3: masks and decays on D1
   // warp -> TMEM lane quarter (warp & 3) and column half (warp >> 2) of the 64 columns
@@ -413,7 +401,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (kRaw && tid == 0) tma_store_wait_read();     // the inverse's scratch and the T tiles reuse the Q boxes from here on
   const int chunk_not_contraction = __syncthreads_or(not_contraction);
   ok = __syncthreads_and(ok);                  // uniform from here on: the warp-level barrier below needs that
-  GDN_PSTAMP(3);
 
   // ---- phase 4: T = (I+A)^-1 in place, blocked 16 -> 32 -> 64, all in FP32 on the CUDA cores
   // level 1: the four 16x16 diagonal blocks, one column per thread (left-looking, in registers); the 16 threads
@@ -447,7 +434,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int i = 0; i < 16; ++i) a0[i * L::kLd + c] = x[i];
   }
   __syncthreads();
-  GDN_PSTAMP(7);
   // level 2: inside each 32x32 diagonal block, T21 = -T22 (A21 T11) with 16x16 blocks, written where A21 was.
   // Levels 2 and 3 are small dense products: they run on the tensor cores as m16n8k8 TF32 tiles with the 3xTF32
   // split (FP32-grade accuracy), one tile per warp, operands read from shared memory one word per lane; as FP32 FMAs
@@ -470,7 +456,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   }
   __syncthreads();
-  GDN_PSTAMP(8);
   // level 3: T21 = -T22 (A21 T11) with 32x32 blocks: eight tiles, one per warp
   {
     const int lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -490,7 +475,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   }
   __syncthreads();
-  GDN_PSTAMP(9);
   // T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row i, sixteen columns (conflict-free:
   // the row pitch of 68 words spreads eight consecutive rows over all banks, the tile rows are swizzled).
   // The W pair goes to the Q boxes at once; the U pair overwrites T, so it waits until every thread has read its part.
@@ -540,7 +524,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
   }
   __syncthreads();
-  GDN_PSTAMP(4);
 
   // ---- phase 5: W^T (into D1's columns, which every thread has read) and U^T
   if (warp == 0 && ok && elect_one()) {
@@ -575,7 +558,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
   ok = ok && mbar_wait(bar_mma, 1, abort, 3, chunk);
   tc_fence_after();
-  GDN_PSTAMP(5);
 
   // ---- phase 6: W (hi/lo) and U leave for the workspace; lrow is the key (W) / value (U) index.
   // W^T: the thread's 32 tokens are contiguous in its row; they are staged as 16-byte pieces in two
@@ -621,7 +603,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tma_store_commit();
     tma_store_wait_read();
   }
-  GDN_PSTAMP(6);
   if (!ok) {
     for (int i = 0; i < 20; ++i) __nanosleep(100000);   // let copies in flight land before the CTA leaves
   }
@@ -633,7 +614,6 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   // (a repair CTA without a block of its own has allocated nothing)
   if (warp == 1 && (!kRepair || int(blockIdx.x) < s_count * chunks)) tmem_dealloc(*tmem_slot, kPrepTmemCols);
 }
-#undef GDN_PSTAMP
 
 // ==================================================================================== walk kernel
 // One CTA per (batch, value head), or per (batch, value head, parallel sub-segment): see the comment above the
@@ -676,17 +656,6 @@ constexpr int kWalkSmem = WalkLayout::kTotal + 1024;
 constexpr uint32_t kAccS = 0, kOpSH = 128, kOpSL = 192, kAccX = 256, kAccO = 384;   // ACC_O: two buffers of 64
 constexpr uint32_t kIdescN64BT = idesc_bf16(128, 64, false, true);     // B MN-major, N = 64
 
-#ifdef GDN_SM100_PHASE_TIMING
-#define GDN_STAMP(slot)                                                                        \
-  if (tid == kChainWarp0 * 32) ws.gates[(block0 + c) * kGateWords + 96 + (slot)] = float((clock64() - t_begin) & 0xffffff)
-#define GDN_MSTAMP(slot) ws.gates[(block0 + c) * kGateWords + 104 + (slot)] = float((clock64() - t_begin) & 0xffffff)
-#define GDN_OSTAMP(slot)                                                                       \
-  if (tid == kOutWarp0 * 32) ws.gates[(block0 + c) * kGateWords + 112 + (slot)] = float((clock64() - t_begin) & 0xffffff)
-#else
-#define GDN_STAMP(slot)
-#define GDN_MSTAMP(slot)
-#define GDN_OSTAMP(slot)
-#endif
 
 // First chunk boundary of a sub-segment at which the decay accumulated since the sub-segment's start is below
 // exp(-40): returns the number of leading chunks an incoming state still reaches (1..count), or -1 when the decay
@@ -841,9 +810,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     identity_in = (flags & kWalkHomogeneous) != 0;
     state_out = in.final_state + ((flags & kWalkTail) ? (long long)heads * kDim * kDim : 0);
   }
-#ifdef GDN_SM100_PHASE_TIMING
-  const long long t_begin = clock64();
-#endif
 
   if (tid == 0) {
     for (int s = 0; s < L::kStages; ++s) {
@@ -984,7 +950,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       ok = ok && mbar_wait(full + s, (c / L::kStages) & 1, abort, 11, c);
       if (!ok) break;
       tc_fence_after();
-      GDN_STAMP(0);
       const float gamma = gates[kChunk];
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
@@ -1016,7 +981,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         if (lane == 0) mbar_arrive(bar_ops + part);
       }
       if (!ok) break;
-      GDN_STAMP(1);
 
       float u[32];
 #pragma unroll
@@ -1025,7 +989,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       ok = mbar_wait(bar_ws, c & 1, abort, 12, c);
       if (!ok) break;
       tc_fence_after();
-      GDN_STAMP(2);
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         const int ks = half * 2 + part;                     // 16-token group
@@ -1052,7 +1015,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_opn + part);
       }
-      GDN_STAMP(3);
     }
     if (ok && chunks > 0) ok = mbar_wait(bar_s, (chunks - 1) & 1, abort, 13, chunks);
     if (ok && state_out) {
@@ -1078,7 +1040,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       ok = mbar_wait(bar_o, c & 1, abort, 20, c);
       if (!ok) break;
       tc_fence_after();
-      GDN_OSTAMP(0);
       const uint32_t taddr = tbase + (c & 1) * 64;
       uint32_t o[64];
       {
@@ -1095,7 +1056,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_ofree + (c & 1));
-      GDN_OSTAMP(1);
       if (c < unstored) continue;
       const int cs = c - unstored;           // count of stored tiles: staging buffers and their barriers follow it
       if (geo.varlen && c == chunks - 1 && tail_valid < kChunk) {
@@ -1132,7 +1092,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         tma_store_wait_read_keep1();
         mbar_arrive(bar_stfree);
       }
-      GDN_OSTAMP(2);
     }
     if (tid == kOutWarp0 * 32) tma_store_wait_all();
   } else if (warp >= kScaleWarp0 && warp < kScaleWarp0 + kScaleWarps) {
@@ -1277,9 +1236,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   __syncthreads();
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
-#undef GDN_STAMP
-#undef GDN_MSTAMP
-#undef GDN_OSTAMP
 
 }  // namespace
 

@@ -320,7 +320,7 @@ int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, 
   // that keeps the CTAs within the slots and at least two K steps in each.
   const long long tiles = ((n + kTileM - 1LL) / kTileM) * ((m + 127LL) / 128), k_tiles = (k + kTileK - 1LL) / kTileK;
   int split = 1;
-  while (split < 8 && tiles * split * 2 <= 2 * 148 && k_tiles >= 4 * split) split *= 2;
+  while (split < 8 && tiles * split * 2 <= 2 * kSms && k_tiles >= 4 * split) split *= 2;
   if (split > 1) {
     if (m <= 16) return launch_skinny<16>(enc, a, w, c, m, n, k, split, stream);
     if (m <= 32) return launch_skinny<32>(enc, a, w, c, m, n, k, split, stream);
@@ -329,7 +329,7 @@ int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, 
   }
   // a K step of all tiles of an SM's turn takes 512 cycles of operand traffic for a 128 x 128 tile, 768 for a 128 x 256 one
   const long long wide = ((n + 255LL) / 256) * ((m + 127LL) / 128);
-  return (wide + 147) / 148 * 768 < (tiles + 147) / 148 * 512 ? launch_tiles<256>(enc, a, w, c, m, n, k, stream)
+  return (wide + kSms - 1) / kSms * 768 < (tiles + kSms - 1) / kSms * 512 ? launch_tiles<256>(enc, a, w, c, m, n, k, stream)
                                                               : launch_tiles<128>(enc, a, w, c, m, n, k, stream);
 }
 

@@ -13,3 +13,11 @@ def test_family_rule(shape, family, native_library):
     choice = sm100_policy.select((*shape, 128, 128), B200)
     assert choice.configuration == family and choice.segments == 1
     assert native_library.lib.actlize_la_sm100_select(*shape, 1) == choice.configuration_id
+
+
+def test_rows_say_what_the_rule_says():
+    """The measured rows and the rule for all other shapes cannot drift apart."""
+    for row in sm100_policy.policy()["rows"]:
+        b, t, _, hv = row["shape"]
+        assert row["configuration"] == sm100_policy.default_configuration(b, t, hv)
+        assert row["parallel"] == sm100_policy.default_parallel(b, t, hv) and row["segments"] == 1
