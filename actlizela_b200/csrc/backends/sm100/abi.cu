@@ -298,7 +298,7 @@ extern "C" long long actlize_la_sm100_workspace_bytes(int b, int t, int hk, int 
 extern "C" int actlize_la_sm100_launches_per_forward(int config) {
   if (!config_ok(config)) return -1;
   if (config & kStageMask) return 1;
-  if (is_fused(config)) return ((config >> kParallelShift) & 0xf) > 1 ? 3 : 1;
+  if (is_fused(config)) return ((config >> kParallelShift) & 0xf) > 1 ? 4 : 1;
   const int segments = (config >> kSegmentShift) & 0xff;
   return ((config & 0xf) == 1 && segments > 1) ? 2 * segments : 2;
 }
@@ -440,14 +440,20 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
 
 // --------------------------------------------------------------- forward on raw projection outputs
 // The raw projections are normalised and activated inside the prepare kernel, which stores the normalised queries and keys for
-// the walk, or inside the single-launch kernel.  The two kernels take every shape whose heads can be cut: a layer's heads
-// decay at very different speeds, and where the single launch has to leave some to the two kernels, one follows the other
-// (B1 T4000, 32 heads, slow gates: 226 us in the two kernels, 374 in the single launch; 8 heads, T1000, ordinary gates: 44
-// and 85).  Only where the sequence is long and every head decays within a piece the single launch would be ahead (32 heads,
-// T16000: 435 and 378).  One chunk is over before a second launch (B1 T50: 23.6 and 20.4), and with more heads than half
-// the SMs nothing is cut and preparing them all first is never cheap (128 heads, T1000: 128 and 106).
+// the walk, or inside the single-launch kernel.  Which form is the faster one is estimated, in ns, from what was measured (B1
+// to B4, T100 to T16000, 6 to 74 heads that decay in about five chunks): the single launch takes 4.9 us a chunk step
+// (every head normalises its rows again), the walk 2.08 us a step of its at most eight pieces and the prepare kernel 35 ns a
+// chunk (B1 T1000, 48 heads: 70 us in the two kernels, 90 in the single launch; B1 T16000, 32 heads: 431 and 376).  One
+// chunk is over before a second launch (B1 T50: 23.6 and 20.4); with more heads than half the SMs nothing is cut and
+// preparing them all first is never cheap (128 heads, T1000: 128 and 106).
 int projections_config(const Geometry& geo, int config) {
-  return 2LL * geo.batch * geo.value_heads <= kSms && geo.chunks() > 1 ? (config & ~0xf) | 1 : kFused;
+  const long long heads = (long long)geo.batch * geo.value_heads, chunks = geo.chunks();
+  if (2 * heads > kSms || chunks == 1) return kFused;
+  long long pieces = kSms / heads < chunks / 8 ? kSms / heads : chunks / 8;
+  if (pieces < 1) pieces = 1;
+  const long long longer = pieces < kMaxParallel ? pieces : kMaxParallel;
+  const bool single = 4900 * (chunks + 5 * pieces) / pieces + 24000 < 2080 * (chunks + 5 * longer) / longer + 35 * heads * chunks + 20000;
+  return (config & ~0xf) | (single && pieces > 1 ? kFused : 1);
 }
 extern "C" long long actlize_la_sm100_projections_workspace_bytes(int b, int t, int hk, int hv, int config) {
   if (!geometry_ok(b, t, hk, hv) || !config_ok(config) || ((config & 0xf) != 1 && !is_fused(config)) ||
@@ -484,12 +490,14 @@ extern "C" int actlize_la_sm100_forward_projections(
   const Geometry geo{b, t, hk, hv};
   config = projections_config(geo, config);
   const cudaStream_t stream = static_cast<cudaStream_t>(opaque_stream);
-  if (is_fused(config)) return run_fused(in, geo, config, workspace, stream);
+  if (is_fused(config) && parallel_of(config, geo.chunks()) == 1) return run_fused(in, geo, config, workspace, stream);
   const int segments = segments_of(config, geo);
-  const char* planes = static_cast<const char*>(workspace) + factor_bytes(geo, segments);
+  char* factors = static_cast<char*>(workspace) + (is_fused(config) ? fused_workspace_bytes() : 0);
+  const char* planes = factors + factor_bytes(geo, segments);
   in.q = reinterpret_cast<const __nv_bfloat16*>(planes);
   in.k = reinterpret_cast<const __nv_bfloat16*>(planes + norm_plane_bytes(geo));
-  return run_forward(in, geo, carve_workspace(workspace, geo), config, segments, stream);
+  if (is_fused(config)) return run_fused(in, geo, config, workspace, stream);
+  return run_forward(in, geo, carve_workspace(factors, geo), config, segments, stream);
 }
 
 // ---------------------------------------------------------------------------------- packed sequences

@@ -209,8 +209,8 @@ int launch_prepare_simt(const Inputs&, const Geometry&, const Workspace&, cudaSt
 int launch_walk_simt(const Inputs&, const Geometry&, const Workspace&, cudaStream_t);
 int configure_simt();
 // Heads that a single-launch forward with cut heads left for the two kernels: flags[head * pieces + piece] != 0 for some
-// piece > 0.  flags == nullptr: every head, the ordinary launch.
-constexpr int kMaxSms = 256;       // CTAs of a single-launch forward at most: its flag words
+// piece > 0 (1: a token is no contraction, 2: some head of the call decays too slowly).  flags == nullptr: every head, the ordinary launch.
+constexpr int kMaxSms = 256;       // CTAs of a single-launch forward at most: its flag and reach words
 struct Repair {
   const int* flags = nullptr;
   int pieces = 0, sms = 0;
@@ -219,8 +219,8 @@ int launch_prepare_umma(const Inputs&, const Geometry&, const Workspace&, cudaSt
 // `early`: the kernel in front of it on the stream is this call's prepare kernel, which lets it set itself up beside it
 int launch_walk_umma(const Inputs&, const Geometry&, const Workspace&, bool early, cudaStream_t, const Repair& = {});
 int configure_umma();
-// single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces (not on raw projections); `flags`
-// is scratch of fused_workspace_bytes, the workspace takes the factors of heads it cannot cut
+// single-launch forward (gdn_fused.cu): Geometry::parallel > 1 lets it cut heads into pieces; `flags` is scratch of
+// fused_workspace_bytes, the workspace takes the factors of heads it does not walk
 int configure_fused();
 long long fused_workspace_bytes();
 int launch_forward_fused(const Inputs&, const Geometry&, int* flags, const Workspace&, cudaStream_t);

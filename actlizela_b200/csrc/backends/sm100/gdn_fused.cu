@@ -6,8 +6,9 @@
 // The arithmetic is that of prepare_umma_kernel and walk_umma_kernel (gdn_umma.cu), operation for operation and in
 // the same order, so both paths give the same bits; orientation and precision are explained there.
 //
-// Bound: the chunk period, 7.1k cycles (B1 T8192, 32 value heads on 128 CTAs: 172 us, 228 as prepare + walk; B8 T4096: 566
-// us, 855).  Of it the state chain takes 5k; the rest is the latency of the preparation, of which two are in flight.
+// Bound: the chunk period, 3.8 us (7.5k cycles) with few CTAs at work, 4.1 to 4.3 us with 128 and more (B1 T8192, 32 value heads
+// on 128 CTAs, 35 steps: 163 us, 228 as prepare + walk; B8 T4096, 128 steps: 554 us, 819).  Of it the state chain takes
+// 5k cycles; the rest is the latency of the preparation, of which two are in flight.
 #include "umma_math.cuh"
 
 namespace gdn_sm100 {
@@ -69,7 +70,7 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory of one SM");
 constexpr uint32_t kAccS = 0, kOpSH = 128, kOpSL = 192, kAccX = 256, kAccU = 320, kAccO = 384, kAccD = 448;
 constexpr uint32_t kIdescN64BT = idesc_bf16(128, 64, false, true);     // B MN-major, N = 64
 
-enum ItemWord { kChunks, kBatch, kHv, kFirst, kEnd, kUnstored, kState, kFlags, kFlagSlot, kOwn };
+enum ItemWord { kChunks, kBatch, kHv, kFirst, kEnd, kUnstored, kState, kFlags, kOwn };
 constexpr int kHasInitial = 1, kHasFinal = 2;
 
 struct Barriers {
@@ -80,9 +81,6 @@ struct Barriers {
   uint32_t tmem;
   int abort;
   int lock, released;
-  // split heads: decay reach of this CTA's sub-segment and of the next one; does some sub-segment of the head not decay
-  // (one word per scanning warp)
-  int reach[2], slow[32];
   uint8_t order[kMostOrdered];      // packed sequences, longest first
 };
 static_assert(sizeof(Barriers) <= 896, "barrier block");
@@ -131,8 +129,9 @@ __device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity)
 // wait with one answer for the whole warp
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
-// ACC_D's lock: taken by the thread that issues into it, given back by the last of the `readers` warps that read it.
-__device__ __noinline__ void acc_lock(Barriers* bar) {
+// ACC_D's lock: taken by the thread that issues into it, given back by the last of the `readers` warps that read it.  Inlined: as a
+// called routine it costs 3 to 9 % (B1 T8192, 32 heads: 181 us, 165 so; B8 T4096: 551, 534).
+__device__ __forceinline__ void acc_lock(Barriers* bar) {
   const AbortFlag abort{&bar->abort};
 #pragma unroll 1
   for (uint32_t spin = 0; spin < kPolls; ++spin) {
@@ -155,59 +154,6 @@ __device__ __forceinline__ void acc_release(Barriers* bar, int lane, int readers
       atomicExch(&bar->lock, 0);
     }
   }
-}
-
-// Gate sums of eight chunks, first_chunk + u * stride (zero behind `count` of them), the same in every lane.  All sixteen
-// loads of a lane are asked for before the first value is used: as loads under a branch each they took a memory latency
-// one after the other (64 heads of 128 chunks that do not decay: 86 us in that launch, now 29).  Rows behind the
-// sequence end are read at its last row and left out.
-__device__ __forceinline__ void eight_gate_sums(const Inputs& in, const Geometry& geo, int b, int hv, int first_chunk, int stride,
-                                                int count, int lane, float (&x)[8]) {
-  uint32_t bits[16];
-  const long long row0 = (long long)b * geo.sequence;
-  const auto token = [&](int i) { return (first_chunk + (i >> 1) * stride) * kChunk + (i & 1) * 32 + lane; };
-  const auto at = [&](int i) { return (row0 + min(token(i), geo.sequence - 1)) * geo.value_heads + hv; };
-  if (in.gate_fp32) {
-    const uint32_t* g = static_cast<const uint32_t*>(in.g);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) bits[i] = g[at(i)];
-  } else {
-    const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(in.g);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) bits[i] = bf16_bits(g + at(i));
-  }
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    x[u] = 0.f;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int i = u * 2 + half;
-      if (u < count && token(i) < geo.sequence) x[u] += in.gate_fp32 ? __uint_as_float(bits[i]) : bf16_lo(bits[i]);
-    }
-  }
-#pragma unroll
-  for (int d = 16; d; d >>= 1) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] += __shfl_xor_sync(0xffffffffu, x[u], d);
-  }
-}
-// First chunk boundary of a range at which the decay accumulated since its start is below exp(-40): number of leading
-// chunks an incoming state still reaches (1..count), or -1 when the decay never gets that far.  Sums the gates
-// themselves, eight chunks at a time; it stops at the boundary, so a typical gate costs one step.  Warp-collective; every
-// caller with the same range gets the same answer.
-__device__ __noinline__ int gate_reach(const Inputs& in, const Geometry& geo, int b, int hv, int first_chunk, int count, int lane) {
-  float total = 0.f;
-#pragma unroll 1
-  for (int c0 = 0; c0 < count; c0 += 8) {
-    float x[8];
-    eight_gate_sums(in, geo, b, hv, first_chunk + c0, 1, count - c0, lane, x);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      total += x[u] * kLog2e;
-      if (c0 + u < count && total < kDecayedLog2) return c0 + u + 1;
-    }
-  }
-  return -1;
 }
 
 // 16 columns of row `row`, scaled per column by `coef`, as BF16 hi/lo pieces of a K-major swizzled tile pair (the lo tile
@@ -249,18 +195,57 @@ struct ItemCursor {
 };
 
 // What a launch walks: the units of the grid, a (batch or sequence, value head) each, or with `pieces` > 1 one of its
-// sub-segments (see walk_umma_kernel), at most one per CTA.  The decay part of the sub-segments' conditions is read off
-// the gates up front, while the contraction part (beta |k|^2 in [0, 2]) shows only when a chunk is prepared: every CTA
-// records what it saw in `flags`, and the two kernels of gdn_umma.cu, launched behind, repair the heads with a violation.
-// Heads that could not be cut are left to them as well (`leave`; a flag word of 2) or, when there are many heads, walked whole
-// by their first CTA.
+// sub-segments (see walk_umma_kernel), at most one per CTA.  The decay part of the sub-segments' conditions is read off the
+// gates by scan_pieces_kernel, launched in front, while the contraction part (beta |k|^2 in [0, 2]) shows only when a chunk is
+// prepared: every CTA records what it saw in `flags`, and the two kernels of gdn_umma.cu, launched behind, repair the heads with
+// a violation.  When some piece does not decay, all heads are left to them (flag words of 2): they follow this launch, and
+// take about as long for one head as for all (B1 T8192, 32 heads of which some decay too slowly for a quarter of the
+// length: 673 us with the others cut here, 407 in the two kernels alone, now 415).
 struct Plan {
-  int units, pieces, leave;
+  int units, pieces;
   int* flags;      // [batch * value_heads][pieces], written when pieces > 1
+  int* reach;      // [batch * value_heads][pieces]: chunks of the piece that an incoming state still reaches, -1: all and more
 };
 constexpr int kLeastPiece = 8;       // chunks: a piece has to outlast the decay, which takes about four at typical gates
-constexpr int kMostLeft = 56;        // heads: more are never left
 constexpr int kWalkPieces = 8;       // pieces at most in the two-kernel form: longer than those here when there are few heads
+
+// First chunk boundary of every piece behind a head's first at which the decay accumulated since the piece's start is below
+// exp(-40).  A CTA per piece, a warp per chunk, eight chunks a step: one memory latency, where a warp per piece in the
+// walking kernel's prologue took one for every chunk and the piece's code as well (first touched there by every SM).
+constexpr int kScanThreads = 256;
+template <bool kRaw>
+__global__ void __launch_bounds__(kScanThreads)
+scan_pieces_kernel(const Inputs in, const Geometry geo, const __grid_constant__ Plan plan) {
+  __shared__ float sums[2][kScanThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = geo.chunks();
+  const int head = blockIdx.x / (plan.pieces - 1), r = 1 + blockIdx.x % (plan.pieces - 1), hv = head % geo.value_heads;
+  const int begin = sub_segment_begin(n, r, plan.pieces), count = sub_segment_begin(n, r + 1, plan.pieces) - begin;
+  const long long row = (long long)(head / geo.value_heads) * geo.sequence;
+  float total = 0.f;
+  int reach = -1;
+#pragma unroll 1
+  for (int c0 = 0, turn = 0; c0 < count && reach < 0; c0 += kScanThreads / 32, turn ^= 1) {
+    float x = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int t = (begin + c0 + warp) * kChunk + half * 32 + lane;
+      if (c0 + warp < count && t < geo.sequence) {
+        const long long at = (row + t) * geo.value_heads + hv;
+        x += kRaw ? raw_gate(in, bf16_bits(in.act_a + at), hv) : load_gate(in.g, at, in.gate_fp32);
+      }
+    }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+    if (lane == 0) sums[turn][warp] = x;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kScanThreads / 32; ++u) {
+      total += sums[turn][u] * kLog2e;
+      if (reach < 0 && c0 + u < count && total < kDecayedLog2) reach = c0 + u + 1;
+    }
+  }
+  if (threadIdx.x == 0) plan.reach[head * plan.pieces + r] = reach;
+}
 
 // Packed sequences are dealt to the CTAs longest first, in turns of alternating direction, so that every CTA gets about the
 // same number of chunks (24 sequences of 1 to 10 chunks, 32 heads: 158 us dealt as they come, now 143).  More than
@@ -268,7 +253,9 @@ constexpr int kWalkPieces = 8;       // pieces at most in the two-kernel form: l
 __device__ __forceinline__ bool is_ordered(const Geometry& geo, const Plan& plan) {
   return geo.varlen && geo.batch <= kMostOrdered && plan.units > int(gridDim.x);
 }
-__device__ __noinline__ void order_sequences(const int* varlen, int n, int total, uint8_t* sm, Barriers* bar) {
+__device__ __forceinline__ void order_sequences(const Geometry& geo, uint8_t* sm, Barriers* bar) {
+  const int* varlen = geo.varlen;
+  const int n = geo.batch, total = geo.sequence;
   int* offset = reinterpret_cast<int*>(sm);                // the stages are still unused
   int* length = offset + kMostOrdered + 4;
   const int tid = threadIdx.x;
@@ -537,6 +524,14 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const AbortFlag abort{&bar->abort};
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  if (plan.pieces > 1) {
+    const bool slow = __syncthreads_or(tid < plan.units && tid % plan.pieces && plan.reach[tid] < 0);
+    if (tid == 0) {
+      if (blockIdx.x % plan.pieces == 0) atomicAdd(&g_fused_plan_counts[slow ? 1 : 0], 1);
+      plan.flags[blockIdx.x] = slow ? 2 : 0;
+    }
+    if (slow) return;
+  }
   dependents_may_start();
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) {
@@ -571,19 +566,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tmem_alloc(&bar->tmem, 512);
     tmem_relinquish();
   }
-  if (!kRaw && plan.pieces > 1 && warp >= kChainWarp) {
-    const int n = geo.chunks(), head = blockIdx.x / plan.pieces, sub = blockIdx.x % plan.pieces;
-    int slow = 0;
-#pragma unroll 1
-    for (int r = 1 + warp - kChainWarp; r < plan.pieces; r += kThreads / 32 - kChainWarp) {
-      const int c0 = sub_segment_begin(n, r, plan.pieces), c1 = sub_segment_begin(n, r + 1, plan.pieces);
-      const int reach = gate_reach(in, geo, head / geo.value_heads, head % geo.value_heads, c0, c1 - c0, lane);
-      if (reach < 0) slow = 1;
-      if (lane == 0 && (r == sub || r == sub + 1)) bar->reach[r - sub] = reach;
-    }
-    if (lane == 0) bar->slow[warp] = slow;
-  }
-  if (is_ordered(geo, plan)) order_sequences(geo.varlen, geo.batch, geo.sequence, sm, bar);
+  if (is_ordered(geo, plan)) order_sequences(geo, sm, bar);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -615,7 +598,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       return true;
     };
-    const bool split = !kRaw && plan.pieces > 1, ordered = is_ordered(geo, plan);
+    const bool split = plan.pieces > 1, ordered = is_ordered(geo, plan);
 #pragma unroll 1
     for (int turn = 0; ok; ++turn) {
       const int across = ordered && (turn & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x);
@@ -623,7 +606,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const bool end = unit >= plan.units;
       const int head = split    ? unit / plan.pieces :
                        ordered && !end ? bar->order[unit / geo.value_heads] * geo.value_heads + unit % geo.value_heads : unit;
-      int b = 0, hv = 0, chunks = -1, t_first = 0, t_end = 0, unstored = 0, flags = 0, own = 0, slot = -1;
+      int b = 0, hv = 0, chunks = -1, t_first = 0, t_end = 0, unstored = 0, flags = 0, own = 0;
       if (!end) {
         b = head / geo.value_heads;
         hv = head % geo.value_heads;
@@ -645,27 +628,17 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
         if (split) {
           const int sub = unit % plan.pieces;
-          const bool serial = __ballot_sync(0xffffffffu, lane >= kChainWarp && bar->slow[lane]);
-          if (lane == 0) {
-            if (sub == 0) atomicAdd(&g_fused_plan_counts[serial ? 1 : 0], 1);
-            plan.flags[unit] = serial && plan.leave ? 2 : 0;
+          const int c0 = sub_segment_begin(chunks, sub, plan.pieces), c1 = sub_segment_begin(chunks, sub + 1, plan.pieces);
+          chunks = c1 - c0;
+          t_first += c0 * kChunk;
+          if (sub) {
+            unstored = plan.reach[unit];
+            flags &= ~kHasInitial;
+            own = c1 - c0;             // chunks that have to be contractions
           }
-          if (serial) {
-            if (sub || plan.leave) continue;
-          } else {
-            const int c0 = sub_segment_begin(chunks, sub, plan.pieces), c1 = sub_segment_begin(chunks, sub + 1, plan.pieces);
-            own = c1 - c0;
-            chunks = own;
-            t_first += c0 * kChunk;
-            if (sub) {
-              unstored = bar->reach[0];
-              flags &= ~kHasInitial;
-              slot = unit;
-            }
-            if (sub + 1 < plan.pieces) {
-              chunks += bar->reach[1];
-              flags &= ~kHasFinal;
-            }
+          if (sub + 1 < plan.pieces) {
+            chunks += plan.reach[unit + 1];
+            flags &= ~kHasFinal;
           }
         }
       }
@@ -683,7 +656,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         item[kUnstored] = unstored;
         item[kState] = head;
         item[kFlags] = flags;
-        item[kFlagSlot] = slot;
         item[kOwn] = own;
         mbar_arrive(&bar->item_full[at]);
         if (end && v_n >= 0) load_v();
@@ -1126,18 +1098,16 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int* item = cursor.open(sm, bar, ok);
       ok = group_all(1 + group, ok);
       if (!ok) break;
-      const int chunks = item[kChunks], slot = item[kFlagSlot], own = item[kOwn];
+      const int chunks = item[kChunks], own = item[kOwn];
       cursor.close(bar, lane);
       if (chunks < 0) break;
-      bool violation = false;
 #pragma unroll 1
       for (int c = 0; c < chunks && ok; ++c, ++n) {
         if ((n & 1) != group) continue;
         bool not_contraction = false;
         ok = prepare_chunk<kRaw>(sm, bar, group, n, not_contraction);
-        violation |= not_contraction && c < own;
+        if (not_contraction && c < own && lane == 0) plan.flags[blockIdx.x] = 1;
       }
-      if (slot >= 0 && violation && lane == 0) plan.flags[slot] = 1;
       ok = group_all(1 + group, ok);
     }
   }
@@ -1164,6 +1134,12 @@ int launch(const Inputs& in, const Geometry& geo, const Plan& plan, int grid, cu
     if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, batch, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_v, in.v, kDim, geo.value_heads, geo.sequence, batch, kChunk)) return rc;
   }
+  if (plan.pieces > 1) {
+    scan_pieces_kernel<kRaw><<<geo.batch * geo.value_heads * (plan.pieces - 1), kScanThreads, 0, stream>>>(in, geo, plan);
+    if (int rc = int(cudaGetLastError())) return rc;
+  }
+  // (Not launched early behind the scan: its CTAs would be dealt to the SMs as the scan leaves them, and a long launch whose
+  // CTAs are not spread evenly is slower, B1 T65536 with 32 heads 1092 us against 1070.)
   forward_umma_kernel<kRaw><<<grid, kThreads, kSmemBytes, stream>>>(tm_q, tm_k, tm_v, in, geo, plan);
   return int(cudaGetLastError());
 }
@@ -1182,15 +1158,16 @@ int configure_fused() {
   return int(e);
 }
 
-long long fused_workspace_bytes() { return kMaxSms * (long long)sizeof(int); }
+long long fused_workspace_bytes() { return 2 * kMaxSms * (long long)sizeof(int); }
 
 // `flags`: fused_workspace_bytes() bytes of scratch (may be null for an unsplit walk)
 int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, const Workspace& ws, cudaStream_t stream) {
   Plan plan{};
   const int heads = geo.batch * geo.value_heads, sms = sm_count(), chunks = geo.segment_chunks();
   const bool split = geo.parallel > 1 && heads > 0;
-  if (split && (in.mixed || geo.varlen || !flags || geo.chunk_begin || geo.chunk_count)) return int(cudaErrorInvalidValue);
+  if (split && (geo.varlen || !flags || geo.chunk_begin || geo.chunk_count)) return int(cudaErrorInvalidValue);
   plan.flags = flags;
+  plan.reach = flags + kMaxSms;
   plan.units = heads;
   plan.pieces = 1;
   if (split) {
@@ -1202,19 +1179,15 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cons
     if (plan.pieces < 1) plan.pieces = 1;
     plan.units = heads * plan.pieces;
   }
-  // A head that is walked whole takes 3.8 us a chunk here; the two kernels take 2.1 us a chunk of the longest head and 31 ns for
-  // every chunk they prepare, which is less up to 56 heads (B1, all heads undecayed, T1024 / T8192: 64 heads 103 / 558 us
-  // left, 95 / 550 walked here; 48 heads at T8192 499 left, 515 walked here).
-  plan.leave = plan.pieces > 1 && heads <= kMostLeft;
   const auto go = in.mixed ? launch<true> : launch<false>;
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
   if (plan.pieces == 1) return 0;
-  // Heads that may not be cut: their chunks prepared by all SMs, then walked at 4.1k cycles a chunk instead of 7.5k by one
-  // CTA each here (B1 T8192, 32 heads that do not decay: 546 us, now 440).  Two launches that leave at once otherwise.
-  // Where this launch's pieces are shorter than an eighth of a head, the walk tries again with eight: gates too slow for the
-  // one are often fast enough for the other (B1, 8 heads, T32768, mean gate -0.02: 1279 us walked uncut, now 372).
+  // Heads left: their chunks prepared by all SMs (31 ns a chunk), then walked at 2.1 us a chunk instead of 3.8 here, in as many
+  // pieces as here or in eight, which are longer when there are more here: gates too slow for the one are often fast enough
+  // for the other (B1, 8 heads, T32768, mean gate -0.02: 1279 us walked uncut, now 347).  Two launches that leave at
+  // once otherwise.
   Geometry again = geo;
-  again.parallel = plan.pieces > kWalkPieces ? kWalkPieces : 0;
+  again.parallel = plan.pieces < kWalkPieces ? plan.pieces : kWalkPieces;
   const Repair left{flags, plan.pieces, sms};
   if (int rc = launch_prepare_umma(in, again, ws, stream, left)) return rc;
   return launch_walk_umma(in, again, ws, true, stream, left);

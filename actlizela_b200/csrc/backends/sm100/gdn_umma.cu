@@ -117,7 +117,7 @@ static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit
 // kRepair: behind a single-launch forward that left some heads (Repair::flags); a grid that just fills the device takes
 // the chunks of those heads in turn, and leaves at once when there are none.
 // kPacked: the grid holds a CTA per (value head, slot).
-enum PrepareMode { kPlain, kRawInputs, kRepairing, kPackedSequences };
+enum PrepareMode { kPlain, kRawInputs, kRepairing, kRawRepairing, kPackedSequences };
 // Token offset of sequence boundary i, forced into 0 <= ... <= total and non-decreasing (no index can leave the tensors), for one
 // warp: lane l returns boundaries l, l + 32, ... in at[].
 __device__ __forceinline__ void clamped_offsets(const Geometry& geo, int lane, int (&at)[kMostPacked / 32 + 1]) {
@@ -158,7 +158,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* carry = reinterpret_cast<float*>(tmem_slot + 2);
   const AbortFlag abort{abort_word};
-  constexpr bool kRaw = kMode == kRawInputs, kRepair = kMode == kRepairing, kPacked = kMode == kPackedSequences;
+  constexpr bool kRaw = kMode == kRawInputs || kMode == kRawRepairing, kRepair = kMode == kRepairing || kMode == kRawRepairing,
+                 kPacked = kMode == kPackedSequences;
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int chunks = geo.chunks(), seg_chunks = geo.segment_chunks();
@@ -186,6 +187,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll 1
   for (int round = 0;; ++round) {
   int bh, chunk, t_begin = 0, t_end = geo.sequence;
+  bool first_of_group = true;                             // kRaw: this CTA stores the tiles of its key head
   if constexpr (kPacked) {
     // sequence whose slots hold this one: every warp finds it for itself
     int at[kMostPacked / 32 + 1];
@@ -208,7 +210,9 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   } else if constexpr (kRepair) {
     const int at = int(blockIdx.x) + round * int(gridDim.x);
     if (at >= s_count * chunks) break;
-    bh = s_left[at % s_count];
+    const int i = at % s_count;
+    bh = s_left[i];
+    first_of_group = i == 0 || s_left[i - 1] / geo.group() != bh / geo.group();
     chunk = chunks - 1 - at / s_count;
   } else {
     // Block order = reverse of the order in which the walk consumes the blocks: the walk's CTAs (one per
@@ -224,6 +228,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int sub_begin = int((long long)seg_chunks * sub / parallel), sub_end = int((long long)seg_chunks * (sub + 1) / parallel);
     if (sub_begin + offset >= sub_end) return;
     bh = unit / parallel;
+    first_of_group = bh % geo.group() == 0;
     chunk = geo.chunk_begin + sub_begin + offset;
   }
   const int b = bh / geo.value_heads, hv = bh % geo.value_heads;
@@ -299,7 +304,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     __syncthreads();
     // the walk reads the normalised queries and keys: one CTA per key head stores the tiles (rows behind T are clipped)
-    if (tid == 0 && ok && hv % geo.group() == 0) {
+    if (tid == 0 && ok && first_of_group) {
       tma_store_4d(&tm_k, sm + L::kK0, 0, hk, t0, b);
       tma_store_4d(&tm_k, sm + L::kK1, 64, hk, t0, b);
       tma_store_4d(&tm_v, sm + L::kQ0, 0, hk, t0, b);
@@ -772,7 +777,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   dependents_may_start();
   bool counted_cut = false;                  // how the single-launch forward counted a head it left
   if (left.flags) {
-    // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: it does not decay)
+    // behind a single-launch forward: only the heads it left (1: a piece met a token that is no contraction, 2: some head decays too slowly)
     // (the wait comes first: the flags live in scratch that is given back behind this call, and a CTA that left without it
     // would let this launch end, and the next one begin, while a late CTA of the repairing prepare kernel still reads them)
     wait_for_previous_kernel();
@@ -1243,7 +1248,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 int configure_umma() {
   if (int rc = tensor_map_encoder().init()) return rc;
   for (const auto prepare : {prepare_umma_kernel<kPlain>, prepare_umma_kernel<kRawInputs>, prepare_umma_kernel<kRepairing>,
-                             prepare_umma_kernel<kPackedSequences>})
+                             prepare_umma_kernel<kRawRepairing>, prepare_umma_kernel<kPackedSequences>})
     if (cudaError_t e = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem)) return int(e);
   return int(cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem));
 }
@@ -1257,7 +1262,7 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   CUtensorMap tm_q, tm_k, tm_v;
   if (in.mixed) {
     // one 2-D map over the packed projection rows; the 4-D maps of the normalised planes are store targets
-    if (!in.q || !in.k || geo.varlen || left.flags) return int(cudaErrorInvalidValue);
+    if (!in.q || !in.k || geo.varlen) return int(cudaErrorInvalidValue);
     if (int rc = enc.bf16_2d(&tm_q, in.mixed, uint64_t(in.mixed_stride), uint64_t(geo.batch) * geo.sequence, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_k, in.k, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
     if (int rc = enc.bf16_4d(&tm_v, in.q, kDim, geo.key_heads, geo.sequence, geo.batch, kChunk)) return rc;
@@ -1280,7 +1285,7 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
     return int(cudaGetLastError());
   }
   const long long resident = 3LL * left.sms;
-  return launch_early(prepare_umma_kernel<kRepairing>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
+  return launch_early(in.mixed ? prepare_umma_kernel<kRawRepairing> : prepare_umma_kernel<kRepairing>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
                       tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
 }
 

@@ -85,7 +85,8 @@ int actlize_la_sm100_configure(void);
 int actlize_la_sm100_select(int batch, int sequence, int key_heads, int value_heads, int gate_fp32);
 
 /* Bytes of caller-owned scratch that forward_prepared needs for this geometry and
- * configuration (the WY factors of every chunk; for the single-launch form flag words only); negative for an unsupported geometry.
+ * configuration (the WY factors of every chunk; the single-launch form needs them only when heads may be cut, and a few
+ * words); negative for an unsupported geometry.
  * Replaces the Python-side workspace table gdn_core_workspace_specs
  * (actlize_la/serving/gdn_core.py:14-22). */
 long long actlize_la_sm100_workspace_bytes(int batch, int sequence, int key_heads, int value_heads,
@@ -93,8 +94,9 @@ long long actlize_la_sm100_workspace_bytes(int batch, int sequence, int key_head
 
 /* Complete forward on caller-owned buffers.  Configuration 4: one kernel, in which every CTA prepares the chunks of a head
  * and walks them (one segment, no stage bits; the sub-segment field says only whether heads may be cut into pieces, 0 or
- * 1 = no, and the launcher chooses how many; heads that do not decay, or hold a token that is no contraction, are left to the
- * two kernels of configuration 1, launched behind it, which leave at once when there are none).  The others: prepare kernel (per-chunk gate prefix, decay-masked
+ * 1 = no, and the launcher chooses how many; a small kernel in front scans the gates: when some piece of some head does
+ * not decay, all heads are left to the two kernels of configuration 1, launched behind it, which also repair heads
+ * that hold a token that is no contraction, and leave at once when there is nothing for them).  The others: prepare kernel (per-chunk gate prefix, decay-masked
  * K.K^T, unit-lower-triangular inverse, WY factors) followed by the sequential chunk walk.
  * `config` is the value returned by actlize_la_sm100_select: kernel family in bits 0..3, number of
  * sequence segments in bits 8..15, number of parallel sub-segments of the walk in bits 16..19 (tcgen05 family only;

@@ -155,13 +155,13 @@ def test_packed_sequences_in_two_kernels(lengths, hv, native_library):
 
 
 @pytest.mark.parametrize("chunks,reach,split", [
-    (300, (4, 20, 60), 2),                   # one for the single launch's 37 pieces, one for eight, one for neither
+    (300, (4, 20, 60), 2),                   # too slow for 37 pieces in the single launch, two of them not for eight
     (300, (30, 20, 12, 36, 1000), 4),
     (131, (9, 17, 25), 1),                   # pieces of 8, and of 16 chunks: the first just too slow for the former
     (130, (2, 3, 64, 65), 2)])
 def test_cuts_follow_the_gates(chunks, reach, split, native_library):
-    """Heads whose state outlives the shortest pieces, each by another factor: cut into as many pieces as the single launch
-    has CTAs for, into eight in the two kernels, or walked whole with the unsplit walk's bits.  Under slow gates a piece's own rounding (16-bit operand pairs: the
+    """Heads whose state outlives the shortest pieces, each by another factor: where the single launch's pieces are too short for
+    one, all are cut into eight in the two kernels, or walked whole with the unsplit walk's bits.  Under slow gates a piece's own rounding (16-bit operand pairs: the
     state is good to 4e-6) is not forgotten within the piece: both walks' errors in the state, and single BF16 flips in the
     output, which has 2^-9 per flipped value (a sixteenth of them is 5e-4)."""
     from actlizela_b200.sm100 import Sm100Forward
@@ -196,13 +196,16 @@ def test_cuts_follow_the_gates(chunks, reach, split, native_library):
     (1, 65, 1, 2, {}, None),
     (1, 700, 2, 8, {}, None),                            # few heads: two kernels, walked whole
     (3, 64 * 9 + 1, 1, 2, {}, None),                     # rows behind a batch element's end are the next one's
-    (1, 64 * 180 + 9, 2, 8, {}, 8),                      # cut into eight
-    (1, 64 * 180 + 9, 2, 8, {3: 18, 5: 1000}, 7),        # one head that just allows that, one that does not
+    (1, 64 * 60 + 9, 2, 8, {}, 8),                       # cut into seven
+    (1, 64 * 60 + 9, 2, 8, {3: 7, 5: 1000}, 7),          # one head that just allows that, one that does not
+    (1, 64 * 180 + 9, 2, 8, {}, 8),                      # single launch, cut into 18
+    (1, 64 * 180 + 9, 2, 8, {3: 18, 5: 1000}, 7),        # left to the two kernels: cut into eight, one head walked whole
+    (2, 64 * 250, 3, 6, {4: 60}, 10),
     (2, 64 * 16 + 3, 37, 37, {3: 1000}, 72),             # the most heads that can be cut, into two
     (5, 64 * 2 + 3, 5, 15, {}, None)])                   # one head more: single launch
 def test_projections_in_every_form(batch, length, hk, hv, slow, split, native_library):
-    """Raw projections in the two kernels (one CTA per key head stores its normalised queries and keys), walked whole and cut, and
-    in the single launch: the outputs of prepare_inputs + forward, bit for bit where that walks them alike.  ``slow``:
+    """Raw projections in the two kernels (one CTA per key head stores its normalised queries and keys), walked whole and cut, in
+    the single launch, and left by it: the outputs of prepare_inputs + forward, bit for bit where that walks them alike.  ``slow``:
     chunks that a head's state outlives."""
     from actlizela_b200 import gdn_forward_projections, gdn_prepare_inputs
     from actlizela_b200.sm100 import Sm100Forward
