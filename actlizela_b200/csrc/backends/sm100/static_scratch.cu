@@ -33,7 +33,7 @@ namespace gdn_sm100 {
 namespace {
 
 constexpr long long kStaticBlocks = ACTLIZE_LA_SM100_STATIC_SCRATCH_MAX_BLOCKS;
-constexpr long long kStaticBytes = kStaticBlocks * kBlockBytes;
+constexpr long long kStaticBytes = kStaticBlocks * kBlockBytes + 2 * kMaxSms * (long long)sizeof(int);   // (a single launch's words)
 
 // In host code this name is only a handle for the runtime; the address a kernel may use is the
 // one cudaGetSymbolAddress returns for the current device.

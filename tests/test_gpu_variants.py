@@ -235,3 +235,16 @@ def test_projections_in_every_form(batch, length, hk, hv, slow, split, native_li
         else:                                            # as in test_cuts_follow_the_gates
             assert oracle.rel_frobenius(out[:, :, h].float().cpu(), want_out[:, :, h].float().cpu()) < 5e-4
             assert oracle.rel_frobenius(state[:, h].cpu(), want_state[:, h].cpu()) < 8e-6
+
+
+def test_static_scratch_takes_cut_heads_at_its_limit(native_library):
+    """64 blocks, the most the built-in array is for, in the form that needs words in front of the factors."""
+    from tests.test_zz_no_alloc import _call
+    w = WORKLOADS["cfg1"].sliced(batch=1, length=64 * 64, key_heads=1, value_heads=1, seed=64)
+    dev = [x.cuda() for x in make_inputs(w)]
+    from actlizela_b200.sm100 import Sm100Forward
+    want_out, want_state = Sm100Forward(native_library)(*dev, True, configuration="fused-split")
+    rc, out, state = _call(native_library.lib, dev, config=4 | (8 << 16))
+    torch.cuda.synchronize()
+    assert rc == 0 and _healthy(native_library)
+    assert torch.equal(out, want_out) and torch.equal(state, want_state)
