@@ -136,7 +136,7 @@ def config_dict(workload, n_gpus):
                          f"Hv{workload.value_heads} D128 chunk64 gate={workload.gate_dtype}"
                          f"{' +initial' if workload.initial is not None else ''} per GPU",
                 sharding=f"batch x{n_gpus}, no collective",
-                l2="working set (inputs, outputs, WY workspace) exceeds the 126 MB L2; no flush between steps")
+                l2="working set (inputs, outputs) exceeds the 126 MB L2; no flush between steps")
 
 
 def reference_arm(args, workload):
@@ -259,7 +259,7 @@ def aux_bench(args):
     print(json.dumps(dict(metric=f"{args.op} {unit}", value=units / (ms * 1e-3), unit=unit, n_gpus=1, steps=args.steps,
                           warmup=max(3, args.warmup), ms_per_step=ms, higher_is_better=True, data="synthetic",
                           config=dict(workload=name, l2="working set exceeds the 126 MB L2"),
-                          gpu_launches=args.steps * (2 if args.op == "varlen" else 8 if args.op == "projections" else 1),
+                          gpu_launches=args.steps * (4 if args.op == "projections" else 1),
                           roofline=dict(bound="hbm", achieved=achieved, peak=peak, unit="GB/s", frac=achieved / peak,
                                         traffic=None, peak_source=source, algorithmic_bytes=nbytes))), flush=True)
 
@@ -727,11 +727,11 @@ def main():
     # against that kernel's own time
     top, ms_top = ("forward", ms_step) if single else max(((k2, kernels_ms[k2]) for k2 in ("prepare", "walk")), key=lambda x: x[1])
     achieved = alg_bytes / (ms_top * 1e-3) / 1e9
-    # DRAM traffic of the two-kernel family per launch from the committed ncu captures of a smaller case (profiles/;
-    # caches flushed before the captured launch, so an upper bound), per (chunk, value head) block and scaled by the
-    # blocks of one launch; the single-launch form moves each tensor once
+    # DRAM traffic per launch from the committed ncu captures (profiles/; caches flushed before the captured launch), of the
+    # headline shape for the single-launch form and of a smaller case for the two-kernel family, per (chunk, value head)
+    # block and scaled by the blocks of one launch
     blocks = shard.batch * shard.value_heads * ((shard.length + 63) // 64)
-    traffic = {"walk": 108.3e3, "prepare": 52.3e3}[top] * blocks if config_name == "umma" else (alg_bytes if single else None)
+    traffic = 46.3e3 * blocks if single else {"walk": 108.3e3, "prepare": 52.3e3}[top] * blocks if config_name == "umma" else None
     whole_ms = max(alg_bytes / (hbm_peak * 1e9), alg_flops / (tensor_peak * 1e12)) * 1e3
     line = dict(
         metric=METRIC, value=workload.tokens * world / (ms_step * 1e-3), unit=UNIT, n_gpus=world,
@@ -744,10 +744,9 @@ def main():
         step_spread=spread,
         roofline=dict(bound="hbm", kernel=top, achieved=achieved, peak=hbm_peak, unit="GB/s",
                       frac=achieved / hbm_peak, traffic=traffic,
-                      traffic_note=("every tensor once: no workspace" if single else
-                                    "dram bytes read + written of one launch in the ncu capture of cfg0 (caches flushed "
-                                    "before the launch; workspace lines still dirty in L2 at its end are not in it), "
-                                    "per block, scaled by the blocks of this launch" if traffic else None),
+                      traffic_note=("dram bytes read + written of one launch in an ncu capture (caches flushed before the "
+                                    "launch; lines still dirty in L2 at its end are not in it), per block, scaled by the "
+                                    "blocks of this launch" if traffic else None),
                       peak_source=peak_source, algorithmic_bytes=alg_bytes, algorithmic_flops=alg_flops,
                       whole_forward_frac=whole_ms / ms_step,
                       tensor_frac=alg_flops / (ms_step * 1e-3) / (tensor_peak * 1e12)),
