@@ -45,7 +45,7 @@ def gdn_forward(q, k, v, g, beta, initial_state=None, output_final_state=True,
     """Complete chunked gated-delta-rule forward.
 
     q,k [B,T,Hk,128] BF16; v [B,T,Hv,128] BF16 (Hv % Hk == 0); g [B,T,Hv] natural-log decay
-    (BF16 or FP32); beta [B,T,Hv] BF16; optional FP32 initial_state [B,Hv,128,128] (K by V).
+    (BF16 or FP32, <= 0: prefix sums within a chunk of 64 must not rise by 88); beta [B,T,Hv] BF16; optional FP32 initial_state [B,Hv,128,128] (K by V).
     Returns (output BF16 [B,T,Hv,128], final FP32 state or None).  Chunk size 64 and the
     1/sqrt(128) query scale are built in; no hidden Q/K normalisation, gate activation,
     rescaling or state conversion takes place.

@@ -177,7 +177,7 @@ class Sm100Forward:
         return held
 
     def varlen(self, q, k, v, g, beta, cu_seqlens, initial_states=None, output_final_state=True):
-        """Packed sequences in one prepare and one walk launch (actlize_la_sm100_forward_varlen)."""
+        """Packed sequences in one or two launches (actlize_la_sm100_forward_varlen)."""
         import ctypes
         import torch
         b, total, hk, hv = _validate(q, k, v, g, beta, None)

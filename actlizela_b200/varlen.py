@@ -4,8 +4,8 @@ The reference's serving prefill pads every request into a fixed ``[R, W]`` batch
 (csrc/serving/prefill.cu:196-255).  Here the sequences stay packed: ``q,k,v,g,beta`` are
 ``[1, total_tokens, H, ...]`` and ``cu_seqlens`` (host integers, or an int32 device tensor, length N+1) marks
 the boundaries.
-The default path is the native entry ``actlize_la_sm100_forward_varlen``: one prepare and one walk launch
-for all sequences, every sequence chunked from its own start.  ``per_sequence=True`` instead hands each
+The default path is the native entry ``actlize_la_sm100_forward_varlen``: one launch for all sequences (few of
+them: a prepare and a walk launch), every sequence chunked from its own start.  ``per_sequence=True`` instead hands each
 sequence (a contiguous slice) to the fixed-shape forward, two launches per sequence; both produce the same
 bits and the second exists as a cross-check.
 """

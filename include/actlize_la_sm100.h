@@ -16,7 +16,9 @@
  *
  * Tensor contract (unchanged from the reference's gdn_forward, README.md:33-46):
  *   q, k      [B, T, Hk, 128] BF16          v, output [B, T, Hv, 128] BF16
- *   g         [B, T, Hv] natural-log decay, FP32 if gate_fp32 else BF16
+ *   g         [B, T, Hv] natural-log decay, FP32 if gate_fp32 else BF16; a decay is <= 0.  Positive values are taken as they
+ *             come: exponentials of differences of the chunk's prefix sums have to stay finite (88), and where the sum rises
+ *             and falls by that much within a chunk, a product of two of them may lose what their difference would have kept
  *   beta      [B, T, Hv] BF16               Hv % Hk == 0, chunk 64, query scale 1/sqrt(128) built in
  *   initial   [B, Hv, 128, 128] FP32, K-by-V order, may be NULL (zero state)
  *   final     [B, Hv, 128, 128] FP32, may be NULL (no export)
