@@ -248,3 +248,57 @@ def test_static_scratch_takes_cut_heads_at_its_limit(native_library):
     torch.cuda.synchronize()
     assert rc == 0 and _healthy(native_library)
     assert torch.equal(out, want_out) and torch.equal(state, want_state)
+
+
+@pytest.mark.parametrize("call", ["cut", "left", "raw-two-kernels", "raw-cut", "raw-left", "packed-two-kernels"])
+def test_forms_under_capture_and_on_a_side_stream(call, native_library):
+    """Every chain of launches captured into a graph and replayed on other inputs in the same buffers, the flags and the scan's
+    words of the capture among them: the eager call's bits."""
+    from actlizela_b200 import gdn_forward, gdn_forward_projections, gdn_forward_varlen
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    draw = lambda *shape: torch.randn(*shape, generator=gen, device="cuda")
+    norm = lambda x: torch.nn.functional.normalize(x, dim=-1).to(torch.bfloat16)
+
+    def inputs(slow):
+        if call.startswith("raw"):
+            t, hk, hv = (700, 2, 4) if call == "raw-two-kernels" else (64 * 250, 2, 6)
+            bias = torch.zeros(hv, device="cuda")
+            if slow:
+                bias[1] = -12.0
+            return [draw(1, t, (2 * hk + hv) * 128).to(torch.bfloat16), draw(1, t, hv).to(torch.bfloat16), draw(1, t, hv).to(torch.bfloat16),
+                    torch.zeros(hv, device="cuda"), bias]
+        t, hk, hv = (1500, 1, 2) if call.startswith("packed") else (64 * 180, 2, 8)
+        g = -torch.rand(1, t, hv, generator=gen, device="cuda")
+        if slow:
+            g[:, :, 1] *= 1e-4
+        return [norm(draw(1, t, hk, 128)), norm(draw(1, t, hk, 128)), draw(1, t, hv, 128).to(torch.bfloat16), g,
+                torch.sigmoid(draw(1, t, hv)).to(torch.bfloat16)]
+
+    slow = call.endswith("left")
+    x, other = inputs(slow), inputs(slow)
+    if call.startswith("packed"):
+        x.append(torch.tensor([0, 100, 100, 900, 1500], dtype=torch.int32, device="cuda"))
+        other.append(torch.tensor([0, 64, 640, 641, 1500], dtype=torch.int32, device="cuda"))
+        run = lambda a: gdn_forward_varlen(*a[:5], a[5], None, True)
+    elif call.startswith("raw"):
+        run = lambda a: gdn_forward_projections(*a, 2, a[3].numel(), None, True)
+    else:
+        run = lambda a: gdn_forward(*a, None, True)
+    want, want_other = run(x), run(other)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        beside = run(x)
+    torch.cuda.current_stream().wait_stream(stream)
+    assert torch.equal(beside[0], want[0]) and torch.equal(beside[1], want[1])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run(x)
+    for values, wanted in ((x, want), (other, want_other), ([y.clone() for y in inputs(not slow)] + x[5:], None)):
+        wanted = wanted or run(values)
+        for slot, value in zip(x, [y.clone() for y in values]):
+            slot.copy_(value)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert _healthy(native_library)
+        assert torch.equal(got[0], wanted[0]) and torch.equal(got[1], wanted[1])
