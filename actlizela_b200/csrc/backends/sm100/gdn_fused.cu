@@ -64,9 +64,10 @@ constexpr int kSmemBytes = Smem::kTotal + 1024;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of one SM");
 
 // Tensor memory (512 columns): the state accumulator, its hi / lo operands, W S (then the N operands of the update: of the
-// 16-token group ks hi at 16 ks, lo at 16 ks + 8), U, the output accumulator, and one accumulator that serves the prepare
-// groups in turn ([Q;K] K^T, then W^T), guarded by a lock word.  N for P N takes the columns of the lo operand, which the
-// product W S has read by then.
+// 16-token group ks hi at 16 ks, lo at 16 ks + 8), W^T and, once that has been converted, U, the output accumulator, and one
+// accumulator that serves the prepare groups in turn ([Q;K] K^T), guarded by a lock word.  (With W^T in that one as well the lock was
+// taken for 6.4k of a chunk's 7.3k cycles: B1 T8192, 32 heads 173 us, 169 so; 48 heads, T65536 1414 and 1392.)  N for P N
+// takes the columns of the lo operand, which the product W S has read by then.
 constexpr uint32_t kAccS = 0, kOpSH = 128, kOpSL = 192, kAccX = 256, kAccU = 320, kAccO = 384, kAccD = 448;
 constexpr uint32_t kIdescN64BT = idesc_bf16(128, 64, false, true);     // B MN-major, N = 64
 
@@ -129,7 +130,7 @@ __device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity)
 // wait with one answer for the whole warp
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
-// ACC_D's lock: taken by the thread that issues into it, given back by the last of the `readers` warps that read it.  Inlined: as a
+// ACC_D's lock: taken by the thread that issues into it, given back by the last of the six warps that read it.  Inlined: as a
 // called routine it costs 3 to 9 % (B1 T8192, 32 heads: 181 us, 165 so; B8 T4096: 551, 534).
 __device__ __forceinline__ void acc_lock(Barriers* bar) {
   const AbortFlag abort{&bar->abort};
@@ -143,12 +144,12 @@ __device__ __forceinline__ void acc_lock(Barriers* bar) {
   }
   abort.raise(1, 100 + (threadIdx.x >> 5), 0);
 }
-__device__ __forceinline__ void acc_release(Barriers* bar, int lane, int readers) {
+__device__ __forceinline__ void acc_release(Barriers* bar, int lane) {
   tc_fence_before();
   __syncwarp();
   if (lane == 0) {
     __threadfence_block();
-    if (atomicAdd(&bar->released, 1) == readers - 1) {
+    if (atomicAdd(&bar->released, 1) == 5) {
       bar->released = 0;
       __threadfence_block();
       atomicExch(&bar->lock, 0);
@@ -346,7 +347,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       uint32_t d[16];
       tmem_ld16(taddr + h * 16, d);
       tmem_wait_ld();
-      if (h & 1) acc_release(bar, lane, 6);      // (the two warps above the diagonal read nothing)
+      if (h & 1) acc_release(bar, lane);      // (the two warps above the diagonal read nothing)
       const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 16 : s_ecol + h * 16);
       const float last = quarter < 2 ? kScale : 1.f, first = quarter < 2 ? 1.f : bi;
       if (diagonal) {
@@ -711,9 +712,10 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int c = 0; c < chunks && ok; ++c, ++n) {
         const int s = n % kRing, par = n & 1;
         const uint32_t kq = base + L::kKQ + s * L::kKQStage;
-        // U^T = V^T (T diag(beta))^T, while the chain warps split the state
+        // U^T = V^T (T diag(beta))^T where W^T was, while the chain warps split the state
         ok = mbar_wait(&bar->t_ready[par], (n >> 1) & 1);
         ok &= mbar_wait(&bar->v_full, par);
+        ok &= mbar_wait(&bar->w_ready, par);
         tc_fence_after();
         const uint64_t dU = smem_desc(base + L::kAT + par * L::kATBytes, 16, 1024);
         if (elect_one()) {
@@ -725,7 +727,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
           mma_commit(&bar->u[par]);
         }
-        ok &= mbar_wait(&bar->w_ready, par);
         // (W S)^T with St ~ SH + SL and W ~ W_hi + W_lo (not lo lo); K steps {0,1,4,5} of the split become available
         // first, {2,3,6,7} second
 #pragma unroll 1
@@ -1009,14 +1010,14 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           // W^T = K^T (T diag(beta exp p))^T; issued here so that the prepare group does not wait for the accumulator
           const uint64_t a = smem_desc(smem_u32(sm) + L::kKQ + (n % kRing) * L::kKQStage + L::kK0, L::kK1 - L::kK0, 1024);
           const uint64_t x = smem_desc(smem_u32(sm) + L::kTw, 16, 1024);
+          if (n > 0) ok = warp_wait(&bar->opn[1], (n - 1) & 1) && ok;      // U of the previous chunk has been read
           if (elect_one()) {
-            acc_lock(bar);
             tc_fence_after();
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks)
-                mma_ss(kAccD, a + uint64_t(ks * 128), x + uint64_t(h * (kBox / 16) + ks * 2), kIdescN64AT, (h | ks) != 0);
+                mma_ss(kAccU, a + uint64_t(ks * 128), x + uint64_t(h * (kBox / 16) + ks * 2), kIdescN64AT, (h | ks) != 0);
             }
             mma_commit(&bar->w);
           }
@@ -1031,9 +1032,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll 1
         for (int h = 0; h < 4; ++h) {
           uint32_t dw[16];
-          tmem_ld16(lanes + kAccD + h * 16, dw);
+          tmem_ld16(lanes + kAccU + h * 16, dw);
           tmem_wait_ld();
-          if (h == 3) acc_release(bar, lane, 4);
 #pragma unroll
           for (int c8 = 0; c8 < 2; ++c8) {
             uint32_t hi[4], lo[4];
@@ -1045,6 +1045,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             *reinterpret_cast<uint4*>(wt + L::kWTile + slot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
         }
+        tc_fence_before();
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar->w_ready);
