@@ -65,8 +65,8 @@ constexpr int kMostPacked = 96;      // sequences of a packed call in the two-ke
 //   gates       FP32 [192]      [0,64): exp(prefix_last - prefix_i), 0 for padding rows;
 //                               [64]: exp(prefix_last); [65] (tcgen05 prepare only): non-zero when some token of the
 //                               chunk is not a contraction of the state (beta < 0 or beta |k|^2 > 2);
-//                               [128,192): exp(prefix_i) / sqrt(128), the scale the walk applies to the rows of its
-//                               Q tile (the scaled queries are not stored: the walk reads q itself); rest unused
+//                               [128,192): exp(prefix_i) / sqrt(128), the scale the walk applies to the columns of its
+//                               product S Q^T (the walk reads q itself); rest unused
 // plus, when the sequence is walked in segments, one FP32 [128][128] state per (batch, value head)
 // that carries the state from one segment's walk to the next (K-by-V order, like the public state).
 struct Workspace {

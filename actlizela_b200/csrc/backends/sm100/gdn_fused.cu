@@ -22,7 +22,7 @@ __device__ int g_fused_plan_counts[2];
 // Warps (32, 64 registers a thread):
 //    0      issuer of the chain's tensor-core products
 //    1      planner (work items of this CTA) and TMA producer
-//    2      query scaling
+//    2      idle
 //    3      gates: prefix sums and exponentials of the coming chunks
 //    4-11   state chain
 //    12-15  W operand (W^T accumulator -> hi/lo tiles) and output
@@ -32,7 +32,7 @@ __device__ int g_fused_plan_counts[2];
 // twice as long, bound by instruction fetches from the cache that the SMs of a GPC share.  Loops are therefore rolled
 // unless a loop's registers need otherwise, and waits call one polling routine.
 constexpr int kThreads = 1024, kPrepThreads = 256;
-constexpr int kIssueWarp = 0, kPlanWarp = 1, kScaleWarp = 2, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
+constexpr int kIssueWarp = 0, kPlanWarp = 1, kGateWarp = 3, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
 constexpr int kRing = 3;      // Q/K tiles, P tiles, gate vectors: one chunk in the chain, two in preparation
 constexpr int kItems = 4;     // work items announced ahead
 constexpr int kMostOrdered = 256;
@@ -75,8 +75,8 @@ enum ItemWord { kChunks, kBatch, kHv, kFirst, kEnd, kUnstored, kState, kFlags, k
 constexpr int kHasInitial = 1, kHasFinal = 2;
 
 struct Barriers {
-  uint64_t kq_full[kRing], kq_free[kRing], g_ready[kRing], qs_go[kRing], qs_done[kRing];
-  uint64_t v_full, w, w_ready, ws, s, o, ofree;
+  uint64_t kq_full[kRing], kq_free[kRing], g_ready[kRing];
+  uint64_t v_full, w, w_ready, ws, qs, scaled, s, o, ofree;
   uint64_t t_ready[2], u[2], d[2], ops[2], opn[2];
   uint64_t item_full[kItems], item_free[kItems];
   uint32_t tmem;
@@ -85,7 +85,7 @@ struct Barriers {
   uint8_t order[kMostOrdered];      // packed sequences, longest first
 };
 static_assert(sizeof(Barriers) <= 896, "barrier block");
-constexpr int kItemReaders = kThreads / 32 - 1;      // every warp but the planner reads the items
+constexpr int kItemReaders = kThreads / 32 - 2;      // every warp but the planner and the idle one reads the items
 
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kPrepThreads) : "memory"); }
 // Barrier of a prepare group that also tells every thread whether all of them are healthy: whoever leaves a loop that
@@ -324,7 +324,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   // ---- masks and decays on [Q;K] K^T
   ok = warp_wait(&bar->d[group], (n >> 1) & 1);
   tc_fence_after();
-  if (lane == 0) mbar_arrive(&bar->qs_go[s]);
   const int quarter = warp & 3, half = warp >> 2, i = (quarter & 1) * 32 + lane;
   const uint32_t taddr = (uint32_t(quarter * 32) << 16) + kAccD;
   bool bad = false;
@@ -538,14 +537,14 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int i = 0; i < kRing; ++i) {
       mbar_init(&bar->kq_full[i], 1);
       mbar_init(&bar->kq_free[i], 1);
-      mbar_init(&bar->qs_go[i], 8);
-      mbar_init(&bar->qs_done[i], 1);
       mbar_init(&bar->g_ready[i], 1);
     }
     mbar_init(&bar->v_full, 1);
     mbar_init(&bar->w, 1);
     mbar_init(&bar->w_ready, 4);
     mbar_init(&bar->ws, 1);
+    mbar_init(&bar->qs, 1);
+    mbar_init(&bar->scaled, 8);
     mbar_init(&bar->s, 1);
     mbar_init(&bar->o, 1);
     mbar_init(&bar->ofree, 4);
@@ -746,7 +745,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (half) mma_commit(&bar->ws);
           }
         }
-        ok &= mbar_wait(&bar->qs_done[s], (n / kRing) & 1);
         if (n > 0) ok &= mbar_wait(&bar->ofree, (n - 1) & 1);
         tc_fence_after();
         const uint64_t qd = smem_desc(kq + L::kQ0, 16, 1024);
@@ -757,6 +755,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             for (int ks = 0; ks < 4; ++ks)
               mma_ts(kAccO, kOpSH + h * 32 + ks * 8, qd + uint64_t(h * (L::kQ1 - L::kQ0) / 16 + ks * 2), kIdescN64, (h | ks) != 0);
           }
+          mma_commit(&bar->qs);
         }
         // St += (N*rel)^T K (the accumulator already holds gamma * St); token groups {0,2} first, {1,3} second
         const uint64_t kd = smem_desc(kq + L::kK0, L::kK1 - L::kK0, 1024), pd = smem_desc(base + L::kP + s * kBox, 16, 1024);
@@ -772,21 +771,23 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
               mma_ts(kAccS, op + h * 32, dk + uint64_t(h * 256), kIdescN128BT, 1);
               mma_ts(kAccS, op + h * 32 + 8, dk + uint64_t(h * 256), kIdescN128BT, 1);
             }
-            if (half) {
-              mma_commit(&bar->s);
-              // O^T += N^T P^T behind the state update: the next chunk's split waits for that, not for the output
-#pragma unroll
-              for (int ks = 0; ks < 4; ++ks) mma_ts(kAccO, kOpSL + ks * 8, pd + uint64_t(ks * 2), kIdescN64, 1);
-              mma_commit(&bar->o);
-              mma_commit(&bar->kq_free[s]);
-            }
+            if (half) mma_commit(&bar->s);
           }
+        }
+        // O^T += N^T P^T behind the state update: the next chunk's split waits for that, not for the output
+        ok &= mbar_wait(&bar->scaled, par);
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) mma_ts(kAccO, kOpSL + ks * 8, pd + uint64_t(ks * 2), kIdescN64, 1);
+          mma_commit(&bar->o);
+          mma_commit(&bar->kq_free[s]);
         }
       }
       ok = __all_sync(0xffffffffu, ok);
     }
-  } else if (warp < kChainWarp) {
-    // ------------------------------------------------------------------ query scaling; gates
+  } else if (warp == kGateWarp) {
+    // ------------------------------------------------------------------ gates
     ItemCursor cursor;
     int n = 0;
 #pragma unroll 1
@@ -800,76 +801,53 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       for (int c = 0; c < chunks && ok; ++c, ++n) {
         const int s = n % kRing;
         float* gates = reinterpret_cast<float*>(sm + L::kGates) + s * L::kGateStage;
-        if (warp == kScaleWarp) {
-          ok = warp_wait(&bar->qs_go[s], (n / kRing) & 1);
-          if (!ok) break;
-          uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
-          const float* scale = gates + kGateQueryScale;
-#pragma unroll 2
-          for (int it = 0; it < 32; ++it) {
-            const int piece = it * 32 + lane, row = piece >> 4, col16 = piece & 15;
-            uint4* at = reinterpret_cast<uint4*>(kq + (col16 < 8 ? L::kQ0 : L::kQ1) + row * 128 + (((col16 & 7) ^ (row & 7)) << 4));
-            const float f = scale[row];
-            const uint4 x = *at;
-            uint4 o;
-            o.x = pack_bf16(bf16_lo(x.x) * f, bf16_hi(x.x) * f);
-            o.y = pack_bf16(bf16_lo(x.y) * f, bf16_hi(x.y) * f);
-            o.z = pack_bf16(bf16_lo(x.z) * f, bf16_hi(x.z) * f);
-            o.w = pack_bf16(bf16_lo(x.w) * f, bf16_hi(x.w) * f);
-            *at = o;
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar->qs_done[s]);
-        } else {
-          // tokens lane and lane + 32: two scans, the second half then adds the first half's total
-          const int t0 = t_first + c * kChunk, valid = min(kChunk, t_end - t0);
-          const long long at = ((long long)b * geo.sequence + t0 + lane) * geo.value_heads + hv;
-          float g[2], beta[2], p[2];
+        // tokens lane and lane + 32: two scans, the second half then adds the first half's total
+        const int t0 = t_first + c * kChunk, valid = min(kChunk, t_end - t0);
+        const long long at = ((long long)b * geo.sequence + t0 + lane) * geo.value_heads + hv;
+        float g[2], beta[2], p[2];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            g[h] = beta[h] = 0.f;
-            if (h * 32 + lane < valid) {
-              const long long gi = at + h * 32LL * geo.value_heads;
-              g[h] = kRaw ? raw_gate(in, bf16_bits(in.act_a + gi), hv) : load_gate(in.g, gi, in.gate_fp32);
-              beta[h] = kRaw ? raw_beta(in, gi) : __bfloat162float(in.beta[gi]);
-            }
+        for (int h = 0; h < 2; ++h) {
+          g[h] = beta[h] = 0.f;
+          if (h * 32 + lane < valid) {
+            const long long gi = at + h * 32LL * geo.value_heads;
+            g[h] = kRaw ? raw_gate(in, bf16_bits(in.act_a + gi), hv) : load_gate(in.g, gi, in.gate_fp32);
+            beta[h] = kRaw ? raw_beta(in, gi) : __bfloat162float(in.beta[gi]);
           }
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const float y = __shfl_up_sync(0xffffffffu, g[0], d), z = __shfl_up_sync(0xffffffffu, g[1], d);
-            if (lane >= d) {
-              g[0] += y;
-              g[1] += z;
-            }
-          }
-          g[1] += __shfl_sync(0xffffffffu, g[0], 31);
-          p[0] = g[0] * kLog2e;
-          p[1] = g[1] * kLog2e;
-          const float last = __shfl_sync(0xffffffffu, valid > 32 ? p[1] : p[0], (valid - 1) & 31);
-          const float p31 = __shfl_sync(0xffffffffu, p[0], 31);
-          // the stage is free once the chain has left the chunk that used it
-          if (n >= kRing) ok = warp_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1);
-          if (!ok) break;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int t = h * 32 + lane;
-            const float e = exp2f(p[h]);
-            gates[t] = t < valid ? fast_exp2(last - p[h]) : 0.f;
-            gates[kGateQueryScale + t] = e * kScale;
-            gates[L::kPl2 + t] = p[h];
-            gates[L::kBeta + t] = beta[h];
-            gates[L::kCoefW + t] = beta[h] * e;
-          }
-          gates[L::kECol + lane] = fast_exp2(p31 - p[0]);
-          if (lane == 0) gates[kChunk] = fast_exp2(last);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar->g_ready[s]);
         }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const float y = __shfl_up_sync(0xffffffffu, g[0], d), z = __shfl_up_sync(0xffffffffu, g[1], d);
+          if (lane >= d) {
+            g[0] += y;
+            g[1] += z;
+          }
+        }
+        g[1] += __shfl_sync(0xffffffffu, g[0], 31);
+        p[0] = g[0] * kLog2e;
+        p[1] = g[1] * kLog2e;
+        const float last = __shfl_sync(0xffffffffu, valid > 32 ? p[1] : p[0], (valid - 1) & 31);
+        const float p31 = __shfl_sync(0xffffffffu, p[0], 31);
+        // the stage is free once the chain has left the chunk that used it
+        if (n >= kRing) ok = warp_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1);
+        if (!ok) break;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int t = h * 32 + lane;
+          const float e = exp2f(p[h]);
+          gates[t] = t < valid ? fast_exp2(last - p[h]) : 0.f;
+          gates[kGateQueryScale + t] = e * kScale;
+          gates[L::kPl2 + t] = p[h];
+          gates[L::kBeta + t] = beta[h];
+          gates[L::kCoefW + t] = beta[h] * e;
+        }
+        gates[L::kECol + lane] = fast_exp2(p31 - p[0]);
+        if (lane == 0) gates[kChunk] = fast_exp2(last);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar->g_ready[s]);
       }
       ok = __all_sync(0xffffffffu, ok);
     }
-  } else if (warp < kOutWarp) {
+  } else if (warp >= kChainWarp && warp < kOutWarp) {
     // ------------------------------------------------------------------ state chain
     const int quarter = warp & 3, half = (warp - kChainWarp) >> 2;
     const int v = quarter * 32 + lane;                     // value row = TMEM lane
@@ -959,6 +937,24 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive(&bar->opn[part]);
         }
+        // S Q^T, which was issued behind W S, becomes the state part of the output while the update runs: token i times
+        // exp(p_i) / sqrt(128).  (Scaling the Q tile instead, by a warp of its own, took 1440 of 17.6k instructions a chunk and rounded
+        // the scaled query: B1 T8192, 32 heads 171 us, 165 so; B8 T4096 540 and 519; output error against FP64 at slow gates 3.06e-3 and 2.72e-3.)
+        ok = mbar_wait(&bar->qs, par);
+        tc_fence_after();
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {
+          uint32_t o[16];
+          const int i0 = half * 32 + part * 16;
+          tmem_ld16(taddr + kAccO + i0, o);
+          tmem_wait_ld();
+          scale_columns(o, gates + kGateQueryScale + i0);
+          tmem_st16(taddr + kAccO + i0, o);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar->scaled);
       }
       if (ok && n > 0) ok = mbar_wait(&bar->s, (n - 1) & 1);
       if (ok && (flags & kHasFinal)) {
@@ -976,7 +972,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       ok = __all_sync(0xffffffffu, ok);
     }
-  } else if (warp < kPrepWarp) {
+  } else if (warp >= kOutWarp && warp < kPrepWarp) {
     // ------------------------------------------------------------------ W operand and output
     // Every chunk's W^T accumulator becomes the hi/lo operand of the chain here, one chunk ahead of the output tile: these
     // four warps are idle most of a chunk, the prepare groups are what a chunk waits for.
@@ -1089,7 +1085,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       ++c;
       ++n;
     }
-  } else {
+  } else if (warp >= kPrepWarp) {
     // ------------------------------------------------------------------ prepare groups
     const int group = (warp - kPrepWarp) >> 3;
     ItemCursor cursor;

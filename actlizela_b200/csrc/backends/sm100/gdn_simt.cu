@@ -3,7 +3,7 @@
 // It exists as an independent device-side cross-check of the tensor-core kernels: the same
 // workspace layout is produced and consumed, so either stage can be exchanged with its
 // tcgen05 counterpart when a numerical difference has to be located.  All contractions are
-// plain FP32 FMAs; only the quantities the tensor-core path rounds to BF16 (P, scaled Q) or to a
+// plain FP32 FMAs; only the quantities the tensor-core path rounds to BF16 (P) or to a
 // BF16 hi+lo pair (W) are rounded.
 //
 // Math (per 64-token chunk, value head h, key head h / (Hv/Hk)); p = inclusive prefix of g:
@@ -187,8 +187,7 @@ walk_simt_kernel(Inputs in, Geometry geo, Workspace ws) {
       if (i < valid) {
         const long long at = (((long long)b * geo.sequence + t0 + i) * geo.key_heads + hk) * kDim + d;
         kv = __bfloat162float(in.k[at]);
-        // the scaled query as the tensor-core walk forms it: one BF16 rounding of q * exp(p) / sqrt(128)
-        qv = __bfloat162float(__float2bfloat16_rn(__bfloat162float(in.q[at]) * ws.gates[block * kGateWords + kGateQueryScale + i]));
+        qv = __bfloat162float(in.q[at]);
       }
       sQ[i * kPad + d] = qv;
       sK[i * kPad + d] = kv;
@@ -210,11 +209,12 @@ walk_simt_kernel(Inputs in, Geometry geo, Workspace ws) {
       sNr[i * kVt + lane_v] = n * sG[i];
     }
     __syncthreads();
-    // O = Qs S + P N   (old state)
+    // O = exp(p) / sqrt(128) Q S + P N   (old state)
     for (int r = 0; r < kChunk / 8; ++r) {
       const int i = row0 + 8 * r;
       float acc = 0.f;
       for (int d = 0; d < kDim; ++d) acc = fmaf(sQ[i * kPad + d], sS[d * kVt + lane_v], acc);
+      acc *= ws.gates[block * kGateWords + kGateQueryScale + i];
       for (int j = 0; j <= i; ++j) acc = fmaf(sP[i * (kChunk + 1) + j], sN[j * kVt + lane_v], acc);
       if (i < valid)
         in.output[(((long long)b * geo.sequence + t0 + i) * geo.value_heads + hv) * kDim + v0 + lane_v] =

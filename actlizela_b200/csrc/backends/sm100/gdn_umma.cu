@@ -12,7 +12,7 @@
 // path to the final state are carried as BF16 pairs x ~= hi + lo (16 significant bits):
 // the triangular inverse T (scaled by beta, exp(prefix)), W, the state operand of W S and N*rel.
 // K, V, Q are exact BF16 inputs.  U is never rounded (FP32 from accumulator to register).
-// Output-side operands (P, scaled Q, N for P N, the state operand of Q S) are single BF16.
+// Output-side operands (P, N for P N, the state operand of Q S) are single BF16; Q S is scaled in FP32.
 //
 // Math reference: the WY chunk form of the reference project (tests/wy_cpu.py:44-88;
 // prepare/state/output kernels csrc/gdn_chunk/gdn_wy_ppu.cu:7-292), re-derived in transposed form.
@@ -628,24 +628,22 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 //   ACC_X [256,320)  (W S)^T = S_hi^T W_hi^T + S_lo^T W_hi^T + S_hi^T W_lo^T;
 //         after N = U - W S has been formed, the columns are reused for the N operands of the
 //         16-token group ks:  (N*rel) hi at 256+16ks, lo at 256+16ks+8,  N (BF16) at 320+16ks
-//   ACC_O [384,448) and [448,512)  O^T = S_hi^T Qs^T + N^T P^T, alternating by chunk: the epilogue drains one
+//   ACC_O [384,448) and [448,512)  O^T = (S_hi^T Q^T) diag(exp p / sqrt(128)) + N^T P^T, alternating by chunk: the epilogue drains one
 //         while the next chunk's products fill the other
-// Per chunk: 24 instructions for W S (N = 64), on which the chain waits; 8 for S Qs and 4 for P N, issued
+// Per chunk: 24 instructions for W S (N = 64), on which the chain waits; 8 for S Q and 4 for P N, issued
 // behind the commits the chain waits for; 8 for the state update (N = 128).
 // Roles: warp 0 MMA issuer and warp 1 TMA producer (the lowest warp ids: their short instruction streams
 //        sit on the critical path and must not queue behind the arithmetic of the chain warps);
 //        warps 4-11 state chain: a warp owns the 32 TMEM lanes of quarter (warp & 3) and, of every tile it
 //        touches, one column half.  Both chain steps are signalled in two halves so that the MMA issuer
 //        starts on the first half of the K range while the second half is still being written.
-//        warps 2-3 query scaling: the Q tile of a ring stage becomes Qs = Q exp(p) / sqrt(128) in place (one BF16
-//        rounding, a row's scale from the gate vector) before the issuer reads it for the state part of the output;
-//        warps 12-15 output epilogue.
+//        While the update runs the chain warps also scale S Q^T, token i by exp(p_i) / sqrt(128) from the gate vector, before
+//        P N is added to it; warps 12-15 output epilogue; warps 2-3 idle.
 struct WalkLayout {
   // one ring stage: W^T hi and lo tiles [128 key lines][64 tokens] (MN-major B operand of the wide product, the
-  // lo tile one 16 KB tile behind the hi tile), Q as two K-major boxes (scaled in place to Qs by the scaling
-  // warps), K as two boxes, P, the gate vector (768 bytes)
+  // lo tile one 16 KB tile behind the hi tile), Q as two K-major boxes, K as two boxes, P, the gate vector (768 bytes)
   static constexpr int kWH = 0, kWL = 2 * kBox;
-  static constexpr int kQS0 = 4 * kBox, kQS1 = 5 * kBox;
+  static constexpr int kQ0 = 4 * kBox, kQ1 = 5 * kBox;
   static constexpr int kK = 6 * kBox, kP = 8 * kBox;
   static constexpr int kGates = 9 * kBox;
   static constexpr int kStage = 9 * kBox + 1024;
@@ -655,7 +653,7 @@ struct WalkLayout {
   static constexpr int kBars = kOut + 4 * kBox;
   static constexpr int kTotal = kBars + 256;
 };
-constexpr int kMmaWarp = 0, kTmaWarp = 1, kScaleWarp0 = 2, kScaleWarps = 2, kChainWarp0 = 4, kChainWarps = 8, kOutWarp0 = 12;
+constexpr int kMmaWarp = 0, kTmaWarp = 1, kChainWarp0 = 4, kChainWarps = 8, kOutWarp0 = 12;
 constexpr int kWalkThreads = 512;
 constexpr int kWalkSmem = WalkLayout::kTotal + 1024;
 constexpr uint32_t kAccS = 0, kOpSH = 128, kOpSL = 192, kAccX = 256, kAccO = 384;   // ACC_O: two buffers of 64
@@ -759,7 +757,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
   uint64_t* bar_ofree = bar_ops + 10;          // [2] output accumulator (c & 1) drained (one arrival per output warp)
   uint64_t* bar_staged = bar_ops + 8;          // output tile staged in shared memory (one arrival per output warp)
   uint64_t* bar_stfree = bar_ops + 9;          // an older output store has finished reading its staging tile
-  uint64_t* bar_qs = bar_ops + 12;             // [2] the ring stage's Q tile has been scaled (one arrival per scaling warp)
+  uint64_t* bar_qs = bar_ops + 12;             // S Q^T complete
+  uint64_t* bar_scaled = bar_ops + 13;         // ... and scaled
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_ops + 14);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* limit_slot = reinterpret_cast<int*>(tmem_slot + 2);      // [4]: [0] chunks of a cut-short walk, [1] transition is zero, [2] suffix of the offset pass
@@ -832,8 +831,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
     mbar_init(bar_ofree + 1, 4);
     mbar_init(bar_staged, 4);
     mbar_init(bar_stfree, 1);
-    mbar_init(bar_qs, kScaleWarps);
-    mbar_init(bar_qs + 1, kScaleWarps);
+    mbar_init(bar_qs, 1);
+    mbar_init(bar_scaled, kChainWarps);
     *abort_word = 0;
     fence_barrier_init();
   }
@@ -1020,6 +1019,23 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_opn + part);
       }
+      // S Q^T was issued behind W S: it becomes the state part of the output while the update runs
+      ok = mbar_wait(bar_qs, c & 1, abort, 15, c);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint32_t o[16];
+        const int i0 = half * 32 + part * 16;
+        tmem_ld16(taddr + kAccO + (c & 1) * 64 + i0, o);
+        tmem_wait_ld();
+        scale_columns(o, gates + kGateQueryScale + i0);
+        tmem_st16(taddr + kAccO + (c & 1) * 64 + i0, o);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_scaled);
     }
     if (ok && chunks > 0) ok = mbar_wait(bar_s, (chunks - 1) & 1, abort, 13, chunks);
     if (ok && state_out) {
@@ -1099,35 +1115,6 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       }
     }
     if (tid == kOutWarp0 * 32) tma_store_wait_all();
-  } else if (warp >= kScaleWarp0 && warp < kScaleWarp0 + kScaleWarps) {
-    // ------------------------------------------------------------------ query scaling
-    // 64 threads turn the 64 x 128 Q tile of a ring stage into Qs in place: 16 pieces of 16 bytes per thread; a
-    // row's 16 pieces lie in two swizzled boxes (columns 0..63 and 64..127)
-    const int t64 = tid - kScaleWarp0 * 32;
-    bool ok = true;
-    for (int c = 0; c < chunks && ok; ++c) {
-      const int s = c % L::kStages;
-      ok = mbar_wait(full + s, (c / L::kStages) & 1, abort, 50, c);
-      if (!ok) break;
-      uint8_t* st = sm + s * L::kStage;
-      const float* scale = reinterpret_cast<const float*>(st + L::kGates) + kGateQueryScale;
-#pragma unroll 4
-      for (int it = 0; it < 16; ++it) {
-        const int piece = it * 64 + t64, row = piece >> 4, col16 = piece & 15;
-        uint4* at = reinterpret_cast<uint4*>(st + (col16 < 8 ? L::kQS0 : L::kQS1) + row * 128 + (((col16 & 7) ^ (row & 7)) << 4));
-        const float f = scale[row];
-        const uint4 v = *at;
-        uint4 o;
-        o.x = pack_bf16(bf16_lo(v.x) * f, bf16_hi(v.x) * f);
-        o.y = pack_bf16(bf16_lo(v.y) * f, bf16_hi(v.y) * f);
-        o.z = pack_bf16(bf16_lo(v.z) * f, bf16_hi(v.z) * f);
-        o.w = pack_bf16(bf16_lo(v.w) * f, bf16_hi(v.w) * f);
-        *at = o;
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_qs + s);
-    }
   } else if (warp == kTmaWarp) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -1146,8 +1133,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         bulk_load(st + L::kGates, ws.gates + (block0 + c) * kGateWords, kGateWords * 4, full + s);
         tma_load_2d(st + L::kWH, &tm_wh, full + s, 0, 2 * row);       // transposed planes: 128 rows per block
         tma_load_2d(st + L::kWL, &tm_wl, full + s, 0, 2 * row);
-        tma_load_4d(st + L::kQS0, &tm_q, full + s, 0, hk, t_first + c * kChunk, b);
-        tma_load_4d(st + L::kQS1, &tm_q, full + s, 64, hk, t_first + c * kChunk, b);
+        tma_load_4d(st + L::kQ0, &tm_q, full + s, 0, hk, t_first + c * kChunk, b);
+        tma_load_4d(st + L::kQ1, &tm_q, full + s, 64, hk, t_first + c * kChunk, b);
         tma_load_4d(st + L::kK, &tm_k, full + s, 0, hk, t_first + c * kChunk, b);
         tma_load_4d(st + L::kK + kBox, &tm_k, full + s, 64, hk, t_first + c * kChunk, b);
         tma_load_2d(st + L::kP, &tm_p, full + s, 0, row);
@@ -1167,7 +1154,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
       // Descriptors of ring stage 0; stage 1 is a constant further on (the start-address field counts 16-byte units).
       static_assert(L::kStages == 2 && L::kStage % 16 == 0, "descriptor arithmetic below assumes a two-stage ring");
       const uint64_t dW = smem_desc(st0 + L::kWH, 16, 1024);      // MN-major, one 64-token group; the lo tile is one tile behind
-      const uint64_t dQ0 = smem_desc(st0 + L::kQS0, 16, 1024), dQ1 = smem_desc(st0 + L::kQS1, 16, 1024);
+      const uint64_t dQ0 = smem_desc(st0 + L::kQ0, 16, 1024), dQ1 = smem_desc(st0 + L::kQ1, 16, 1024);
       const uint64_t dK = smem_desc(st0 + L::kK, kBox, 1024), dP = smem_desc(st0 + L::kP, 16, 1024);
       for (int c = 0; c < chunks && ok; ++c) {
         const uint64_t stage = uint64_t((c & 1) * (L::kStage >> 4));
@@ -1176,7 +1163,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         // (W S)^T with St ~ SH + SL and W ~ W_hi + W_lo (not lo lo), one accumulator.  The B
         // operand is the transposed W tile: key index on the 128-byte lines (K), tokens contiguous (N); one K
         // step of 16 keys is 2048 bytes.  K steps {0,1,4,5} of the split become available first, {2,3,6,7}
-        // second.  The chain waits for this product only; the state part of the output, St Qs^T, reads the same
+        // second.  The chain waits for this product only; the state part of the output, St Q^T, reads the same
         // operands and is issued behind the commit, so that it runs while the chain warps form N.
         ok = mbar_wait(bar_ops, c & 1, abort, 41, c);
         tc_fence_after();
@@ -1199,11 +1186,10 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
           mma_ts(tm + kAccX, tm + kOpSH + ks * 8, bdesc + uint64_t((L::kWL - L::kWH) >> 4), kIdescN64BT, 1);
         }
         mma_commit(bar_ws);
-        ok &= mbar_wait(bar_qs + (c & 1), (c >> 1) & 1, abort, 44, c);     // scaled long ago: the tile landed a chunk ahead
-        tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
           mma_ts(acc_o, tm + kOpSH + ks * 8, ((ks >> 2) ? q1 : q0) + uint64_t((ks & 3) * 2), kIdescN64, ks != 0);
+        mma_commit(bar_qs);
         // St += (N*rel)^T K (accumulator already holds gamma * St); token groups {0,2} first, {1,3} second
         ok &= mbar_wait(bar_opn, c & 1, abort, 43, c);
         tc_fence_after();
@@ -1225,6 +1211,8 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         }
         mma_commit(bar_s);
         // O^T += N^T P^T behind the state update: the next chunk's split waits for that, not for the output
+        ok &= mbar_wait(bar_scaled, c & 1, abort, 44, c);
+        tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           mma_ts(acc_o, tm + kAccX + 64 + ks * 16, pd + uint64_t(ks * 2), kIdescN64, 1);

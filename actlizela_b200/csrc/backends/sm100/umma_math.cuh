@@ -123,5 +123,20 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uin
   lo = pack_bf16(l0, l1);
 }
 
+// 16 columns of an accumulator times a factor per column (shared memory, 16-byte aligned)
+__device__ __forceinline__ void scale_columns(uint32_t (&x)[16], const float* factor) {
+#pragma unroll
+  for (int q4 = 0; q4 < 4; ++q4) {
+    const float4 f = *reinterpret_cast<const float4*>(factor + q4 * 4);
+    float a, b;
+    mul2(a, b, __uint_as_float(x[q4 * 4]), __uint_as_float(x[q4 * 4 + 1]), f.x, f.y);
+    x[q4 * 4] = __float_as_uint(a);
+    x[q4 * 4 + 1] = __float_as_uint(b);
+    mul2(a, b, __uint_as_float(x[q4 * 4 + 2]), __uint_as_float(x[q4 * 4 + 3]), f.z, f.w);
+    x[q4 * 4 + 2] = __float_as_uint(a);
+    x[q4 * 4 + 3] = __float_as_uint(b);
+  }
+}
+
 }  // namespace
 }  // namespace gdn_sm100
