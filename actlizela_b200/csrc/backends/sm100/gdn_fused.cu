@@ -340,7 +340,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   float* arow = sAT + i * L::kLd;
   if (ok && (diagonal || below)) {
     uint8_t* prow = tile_p + i * 128;
-    const float f = below ? fast_exp2(pi - s_pl2[31]) * (quarter < 2 ? kScale : bi) : 0.f;
+    const float f = below ? fast_exp2(pi - s_pl2[31]) * (quarter < 2 ? kScale : -bi) : 0.f;
 #pragma unroll 1
     for (int h = half * 2; h < half * 2 + 2; ++h) {
       uint32_t d[16];
@@ -348,7 +348,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       tmem_wait_ld();
       if (h & 1) acc_release(bar, lane);      // (the two warps above the diagonal read nothing)
       const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 16 : s_ecol + h * 16);
-      const float last = quarter < 2 ? kScale : 1.f, first = quarter < 2 ? 1.f : bi;
+      const float last = quarter < 2 ? kScale : 1.f, first = quarter < 2 ? 1.f : -bi;
       if (diagonal) {
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
@@ -387,11 +387,6 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
           *reinterpret_cast<uint4*>(prow + (((h * 2 + c8) ^ (i & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
       } else {
-        // the upper right 16x16 block of a 32x32 diagonal block is read as zeros
-        if (diagonal && (h & 1) && !(i & 16)) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) d[e] = 0u;
-        }
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4)
           *reinterpret_cast<uint4*>(arow + h * 16 + q4 * 4) = make_uint4(d[q4 * 4], d[q4 * 4 + 1], d[q4 * 4 + 2], d[q4 * 4 + 3]);
@@ -410,8 +405,8 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       for (int c8 = (i >> 3) + 1; c8 < 8; ++c8) *reinterpret_cast<uint4*>(prow + ((c8 ^ (i & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
     }
     // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
-    // (the diagonal of A as stored is beta_i |k_i|^2 exp(0))
-    if (quarter >= 2 && diagonal) bad = !(bi >= 0.f && arow[i] <= 2.f);
+    // (the diagonal of -A as stored is -beta_i |k_i|^2 exp(0))
+    if (quarter >= 2 && diagonal) bad = !(bi >= 0.f && arow[i] >= -2.f);
   }
   not_contraction |= __any_sync(0xffffffffu, bad);
 
@@ -435,10 +430,10 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
 #pragma unroll
       for (int j4 = 0; j4 < r; j4 += 4) {
         const float4 a = cur[j4 >> 2];
-        if (j4 + 0 < r) acc0 = fmaf(-a.x, x[j4 + 0], acc0);
-        if (j4 + 1 < r) acc1 = fmaf(-a.y, x[j4 + 1], acc1);
-        if (j4 + 2 < r) acc0 = fmaf(-a.z, x[j4 + 2], acc0);
-        if (j4 + 3 < r) acc1 = fmaf(-a.w, x[j4 + 3], acc1);
+        if (j4 + 0 < r) acc0 = fmaf(a.x, x[j4 + 0], acc0);
+        if (j4 + 1 < r) acc1 = fmaf(a.y, x[j4 + 1], acc1);
+        if (j4 + 2 < r) acc0 = fmaf(a.z, x[j4 + 2], acc0);
+        if (j4 + 3 < r) acc1 = fmaf(a.w, x[j4 + 3], acc1);
       }
       x[r] = acc0 + acc1;
 #pragma unroll
@@ -449,8 +444,8 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
     for (int r = 0; r < 16; ++r) a0[r * L::kLd + col] = x[r];
   }
   group_sync(id);
-  // block products T21 = -T22 (A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
-  // above the diagonal, which holds nothing
+  // block products T21 = T22 (-A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
+  // above the diagonal, which holds nothing; at 32 the 16x16 blocks above the diagonals of T11 and T22 are left out
   {
     const int g = lane >> 2, tq = lane & 3;
     const int big = (warp >> 1) & 1, o = big * 32, col16 = (warp & 1) * 8;
@@ -461,12 +456,11 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       const uint32_t left = frag + ((o + 16) * L::kLd + o + step * 16) * 4;
       const float* right = (step ? x16 : sAT + o * L::kLd + o + col16) + tq * L::kLd + g;
       float* out = (step ? sAT + (o + 16) * L::kLd + o + col16 : x16) + g * L::kLd + 2 * tq;
-      const float sign = step ? -1.f : 1.f;
       float c[4];
       if (ok && warp < 4) {
-        tile_row_tf32x3(c, left, right, L::kLd, 16);
-        *reinterpret_cast<float2*>(out) = make_float2(sign * c[0], sign * c[1]);
-        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(sign * c[2], sign * c[3]);
+        tile_row_tf32x3<1>(c, left, right, L::kLd, 1);
+        *reinterpret_cast<float2*>(out) = make_float2(c[0], c[1]);
+        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(c[2], c[3]);
       }
       group_sync(id);
     }
@@ -477,12 +471,11 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       const uint32_t left = frag + ((32 + row16) * L::kLd + step * 32) * 4;
       const float* right = sAT + step * 32 + col32 + tq * L::kLd + g;
       float* out = (step ? sAT + (32 + row16) * L::kLd + col32 : sAT + row16 * L::kLd + 32 + col32) + g * L::kLd + 2 * tq;
-      const float sign = step ? -1.f : 1.f;
       float c[4];
       if (ok) {
-        tile_row_tf32x3(c, left, right, L::kLd, 32);
-        *reinterpret_cast<float2*>(out) = make_float2(sign * c[0], sign * c[1]);
-        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(sign * c[2], sign * c[3]);
+        tile_row_tf32x3<2>(c, left, right, L::kLd, step ? (row16 ? 3 : 1) : (col32 < 16 ? 3 : 2));
+        *reinterpret_cast<float2*>(out) = make_float2(c[0], c[1]);
+        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(c[2], c[3]);
       }
       if (step == 0) group_sync(id);
     }
@@ -909,8 +902,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (lane == 0) mbar_arrive(&bar->ops[part >> 1]);
           }
         }
-        ok = ok && mbar_wait(&bar->ws, par);
-        ok = ok && mbar_wait(&bar->u[par], (n >> 1) & 1);
+        ok = ok && mbar_wait(&bar->ws, par);            // (U was issued in front of W S)
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
@@ -921,13 +913,17 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           tmem_ld16(taddr + kAccU + ks * 16, u);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const int i = ks * 16 + j;
-            float n0, n1, r0, r1;
-            sub2(n0, n1, __uint_as_float(u[j]), __uint_as_float(u[j + 1]), __uint_as_float(x[j]), __uint_as_float(x[j + 1]));
-            mul2(r0, r1, n0, n1, gates[i], gates[i + 1]);
-            split_pair(r0, r1, nh[j >> 1], nl[j >> 1]);
-            n16[j >> 1] = pack_bf16(n0, n1);
+          for (int q4 = 0; q4 < 4; ++q4) {
+            const float4 rel = *reinterpret_cast<const float4*>(gates + ks * 16 + q4 * 4);
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const int j = q4 * 4 + e;
+              float n0, n1, r0, r1;
+              sub2(n0, n1, __uint_as_float(u[j]), __uint_as_float(u[j + 1]), __uint_as_float(x[j]), __uint_as_float(x[j + 1]));
+              mul2(r0, r1, n0, n1, e ? rel.z : rel.x, e ? rel.w : rel.y);
+              split_pair(r0, r1, nh[j >> 1], nl[j >> 1]);
+              n16[j >> 1] = pack_bf16(n0, n1);
+            }
           }
           tmem_st8(taddr + kAccX + ks * 16, nh);
           tmem_st8(taddr + kAccX + ks * 16 + 8, nl);

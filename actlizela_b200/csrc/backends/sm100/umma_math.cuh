@@ -40,9 +40,13 @@ GDN_F32X2(mul2, "mul")
 template <int kN>
 __device__ __forceinline__ void split_tf32(const float (&x)[kN], uint32_t (&hi)[kN], uint32_t (&lo)[kN]) {
 #pragma unroll
-  for (int i = 0; i < kN; ++i) {
+  for (int i = 0; i < kN; i += 2) {
     hi[i] = __float_as_uint(x[i]) & 0xffffe000u;
-    lo[i] = __float_as_uint(x[i] - __uint_as_float(hi[i]));
+    hi[i + 1] = __float_as_uint(x[i + 1]) & 0xffffe000u;
+    float l0, l1;
+    sub2(l0, l1, x[i], x[i + 1], __uint_as_float(hi[i]), __uint_as_float(hi[i + 1]));
+    lo[i] = __float_as_uint(l0);
+    lo[i + 1] = __float_as_uint(l1);
   }
 }
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -58,22 +62,27 @@ __device__ __forceinline__ void load_fragment_a(float (&a)[4], uint32_t addr) {
 }
 // row piece of a lane: rows 0..15, columns 0 or 4 (floats, pitch lda)
 __device__ __forceinline__ int fragment_row(int lane, int lda) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * lda + (lane >> 4) * 4; }
-// One m16n8 tile D = A B over k in [0, kdim): A at this lane's `a_addr`, B row-major with pitch ldb, b = this lane's
-// B[t][g].  The three TF32 products of the split run as three chains that are added at the end (one chain of dependent
-// products would be three times as long, some 25 cycles each).
-__device__ __forceinline__ void tile_row_tf32x3(float (&d)[4], uint32_t a_addr, const float* b, int ldb, int kdim) {
+// One m16n8 tile D = A B over k in [0, 16 kSteps): A at this lane's `a_addr`, B row-major with pitch ldb, b = this lane's
+// B[t][g]; of the 16-wide steps those in the mask `steps` are taken.  The three TF32 products of the split run as three chains
+// that are added at the end (one chain of dependent products would be three times as long, some 25 cycles each).
+template <int kSteps>
+__device__ __forceinline__ void tile_row_tf32x3(float (&d)[4], uint32_t a_addr, const float* b, int ldb, int steps) {
   float lh[4] = {}, hl[4] = {}, hh[4] = {};
 #pragma unroll
-  for (int k0 = 0; k0 < kdim; k0 += 8) {
-    float av[4];
-    uint32_t ah[4], al[4], bh[2], bl[2];
-    load_fragment_a(av, a_addr + k0 * 4);
-    const float bv[2] = {b[k0 * ldb], b[(k0 + 4) * ldb]};
-    split_tf32(av, ah, al);
-    split_tf32(bv, bh, bl);
-    mma_tf32(lh, al, bh);
-    mma_tf32(hl, ah, bl);
-    mma_tf32(hh, ah, bh);
+  for (int step = 0; step < kSteps; ++step) {
+    if (kSteps > 1 && !(steps >> step & 1)) continue;
+#pragma unroll
+    for (int k0 = step * 16; k0 < step * 16 + 16; k0 += 8) {
+      float av[4];
+      uint32_t ah[4], al[4], bh[2], bl[2];
+      load_fragment_a(av, a_addr + k0 * 4);
+      const float bv[2] = {b[k0 * ldb], b[(k0 + 4) * ldb]};
+      split_tf32(av, ah, al);
+      split_tf32(bv, bh, bl);
+      mma_tf32(lh, al, bh);
+      mma_tf32(hl, ah, bl);
+      mma_tf32(hh, ah, bh);
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) d[i] = (lh[i] + hl[i]) + hh[i];
