@@ -348,7 +348,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       tmem_wait_ld();
       if (h & 1) acc_release(bar, lane);      // (the two warps above the diagonal read nothing)
       const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 16 : s_ecol + h * 16);
-      const float last = quarter < 2 ? kScale : 1.f, first = quarter < 2 ? 1.f : -bi;
+const float row = quarter < 2 ? kScale : -bi;
       if (diagonal) {
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
@@ -357,9 +357,8 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
           for (int e = 0; e < 4; e += 2) {
             float x0 = __uint_as_float(d[q4 * 4 + e]), x1 = __uint_as_float(d[q4 * 4 + e + 1]), e0, e1;
             sub2(e0, e1, pi, pi, e ? p4.z : p4.x, e ? p4.w : p4.y);
-            mul2(x0, x1, x0, x1, first, first);
+            mul2(x0, x1, x0, x1, row, row);
             mul2(x0, x1, x0, x1, fast_exp2(e0), fast_exp2(e1));
-            mul2(x0, x1, x0, x1, last, last);
             d[q4 * 4 + e] = __float_as_uint(x0);
             d[q4 * 4 + e + 1] = __float_as_uint(x1);
           }
@@ -401,8 +400,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       x.z &= keep > 5 ? ~0u : (keep == 5 ? 0xffffu : 0u);
       x.w &= keep > 7 ? ~0u : (keep == 7 ? 0xffffu : 0u);
       *at = x;
-#pragma unroll 1
-      for (int c8 = (i >> 3) + 1; c8 < 8; ++c8) *reinterpret_cast<uint4*>(prow + ((c8 ^ (i & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+      if (!(i & 8)) *reinterpret_cast<uint4*>(prow + ((((i >> 3) + 1) ^ (i & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
     }
     // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
     // (the diagonal of -A as stored is -beta_i |k_i|^2 exp(0))
@@ -486,18 +484,17 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   // ---- T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row, 16 columns
   {
     const int row = t & 63, c0 = (t >> 6) * 16;
-    const bool empty = c0 >= 32 && row < 32;          // above the diagonal
+    const bool empty = c0 >= 32 && row < 32;          // above the diagonal: not read
     const float* trow = sAT + row * L::kLd + c0;
-    float4 x[4];
+    float4 x[4] = {};
+    if (!empty) {
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
-      x[q4] = *reinterpret_cast<const float4*>(trow + q4 * 4);
-      if (empty) x[q4] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int q4 = 0; q4 < 4; ++q4) x[q4] = *reinterpret_cast<const float4*>(trow + q4 * 4);
     }
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
       if (pass) group_sync(id);          // every thread holds its part of T: the U pair may take its place
-      scaled_row(x, (pass ? s_beta : s_coefw) + c0, sm + (pass ? L::kAT + group * L::kATBytes : L::kTw) + row * 128, c0 >> 3, row);
+      if (!empty) scaled_row(x, (pass ? s_beta : s_coefw) + c0, sm + (pass ? L::kAT + group * L::kATBytes : L::kTw) + row * 128, c0 >> 3, row);
     }
     fence_proxy_async_smem();
   }
@@ -715,7 +712,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           for (int h = 0; h < 2; ++h) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              mma_ss(kAccU, dV + uint64_t(ks * 128), dU + uint64_t(h * (kBox >> 4) + ks * 2), kIdescN64AT, (h | ks) != 0);
+              mma_ss(kAccU + 16 * ks, dV + uint64_t(ks * 128), dU + uint64_t(h * (kBox >> 4) + ks * 2 + rows_from(ks)), idesc_rows_from(ks, true), (h | ks) != 0);
           }
           mma_commit(&bar->u[par]);
         }
@@ -772,7 +769,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) mma_ts(kAccO, kOpSL + ks * 8, pd + uint64_t(ks * 2), kIdescN64, 1);
+          for (int ks = 0; ks < 4; ++ks) mma_ts(kAccO + 16 * ks, kOpSL + ks * 8, pd + uint64_t(ks * 2 + rows_from(ks)), idesc_rows_from(ks, false), 1);
           mma_commit(&bar->o);
           mma_commit(&bar->kq_free[s]);
         }
@@ -1009,7 +1006,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             for (int h = 0; h < 2; ++h) {
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks)
-                mma_ss(kAccU, a + uint64_t(ks * 128), x + uint64_t(h * (kBox / 16) + ks * 2), kIdescN64AT, (h | ks) != 0);
+                mma_ss(kAccU + 16 * ks, a + uint64_t(ks * 128), x + uint64_t(h * (kBox / 16) + ks * 2 + rows_from(ks)), idesc_rows_from(ks, true), (h | ks) != 0);
             }
             mma_commit(&bar->w);
           }

@@ -374,8 +374,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             a0 = a0 * pj[jj] * row_factor;
             a1 = a1 * pj[jj + 1] * row_factor;
           } else {
-            a0 = a0 * fast_exp2(pi - pj[jj]) * kScale;
-            a1 = a1 * fast_exp2(pi - pj[jj + 1]) * kScale;
+            a0 = a0 * kScale * fast_exp2(pi - pj[jj]);
+            a1 = a1 * kScale * fast_exp2(pi - pj[jj + 1]);
           }
           packed[jj >> 1] = pack_bf16(j <= i ? a0 : 0.f, j + 1 <= i ? a1 : 0.f);
         }
