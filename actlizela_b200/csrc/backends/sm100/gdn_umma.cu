@@ -17,7 +17,7 @@
 // Math reference: the WY chunk form of the reference project (tests/wy_cpu.py:44-88;
 // prepare/state/output kernels csrc/gdn_chunk/gdn_wy_ppu.cu:7-292), re-derived in transposed form.
 #include "gdn_common.cuh"
-#include "umma_math.cuh"
+#include "chunk_factors.cuh"
 
 namespace gdn_sm100 {
 using namespace ptx;
@@ -76,7 +76,7 @@ __device__ int g_walk_plan_counts[2];
 // accumulator it reads, the column half (warp >> 2).
 //   phase 1  TMA: Q, K chunk tiles (key head of the group) and V tile; gate prefix by two warps
 //   phase 2  D1[128x64] = [Q;K] K^T                                  (one tcgen05 product, 8 instructions)
-//   phase 3  rows 0..63  -> P = tril(QK^T * decay)/sqrt(128) -> BF16 -> workspace
+//   phase 3  rows 0..63  -> P = tril(QK^T * decay)/sqrt(128) -> BF16 -> swizzled tile -> TMA store
 //            rows 64..127-> A = tril(beta_i KK^T * decay, -1) -> shared (FP32);
 //            the diagonal k_i.k_i decides whether token i is a contraction (word 65 of the gate vector)
 //   phase 4  T = (I+A)^-1 IN PLACE, blocked: four 16x16 diagonal solves in FP32 registers, then
@@ -92,18 +92,15 @@ __device__ int g_walk_plan_counts[2];
 struct PrepLayout {
   static constexpr int kQ0 = 0, kK0 = kBox, kQ1 = 2 * kBox, kK1 = 3 * kBox;   // [Q;K] stacked, two K atoms
   static constexpr int kV0 = 4 * kBox, kV1 = 5 * kBox;
-  static constexpr int kLd = 68;                           // row pitch (floats) of the FP32 64x64 matrix
-  static constexpr int kAT = 6 * kBox;                     // float [64][68]: A, then T in place
-  static constexpr int kTwH = kQ0, kTwL = kQ1;             // written after phase 4, when Q and the scratch are dead
+  static constexpr int kAT = 6 * kBox;                     // FP32 matrix: A, then T in place
+  static constexpr int kP = 8 * kBox;
+  static constexpr int kTwH = kQ0, kTwL = kQ1;             // written after phase 4, when Q is dead
   static constexpr int kTuH = kAT, kTuL = kAT + kBox;      // written once T sits in registers
-  static constexpr int kX = kQ0;                           // block products of the inverse, on the dead Q box
   static constexpr int kStageWH = 0, kStageWL = 2 * kBox;  // phase 6: W^T hi / lo tiles [128][64] over the Q/K boxes
-  static constexpr int kLdX = 20, kLdX3 = 36;
-  static constexpr int kVec = kAT + 64 * kLd * 4;          // float [4][64]: pl2, beta, beta*exp(p), exp(p)/sqrt(128)
+  static constexpr int kVec = 9 * kBox;                    // float [4][64]: pl2, beta, beta*exp(p), exp(p)/sqrt(128)
   static constexpr int kBars = kVec + (4 * 64 + 32) * 4;   // (and 32 column factors) 2 mbarriers, tmem slot, abort flag, carry
   static constexpr int kTotal = kBars + 64;
-  static_assert(2 * kBox <= 64 * kLd * 4 && kAT % 1024 == 0, "the U pair of T tiles must fit on T, box aligned");
-  static_assert(32 * kLdX3 * 4 <= kBox && 32 * kLdX * 4 <= kBox, "block-product scratch must fit in one Q box");
+  static_assert(2 * kBox == kMatrixBytes, "the U pair of T tiles takes the place of T");
 };
 constexpr int kPrepThreads = 256;
 constexpr int kPrepSmem = PrepLayout::kTotal + 1024;
@@ -140,13 +137,13 @@ template <PrepareMode kMode>
 __global__ void __launch_bounds__(kPrepThreads, 3)
 prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_wh,
-                    const __grid_constant__ CUtensorMap tm_wl, Inputs in, Geometry geo, Workspace ws, Repair left) {
+                    const __grid_constant__ CUtensorMap tm_wl, const __grid_constant__ CUtensorMap tm_p, Inputs in, Geometry geo,
+                    Workspace ws, Repair left) {
   // Indexing the declared array (no integer round trip) keeps these accesses in the shared state space.
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
   using L = PrepLayout;
-  float* sAT = reinterpret_cast<float*>(sm + L::kAT);
-  float* sX = reinterpret_cast<float*>(sm + L::kX);
+  const uint32_t matrix = smem_u32(sm + L::kAT);
   float* s_pl2 = reinterpret_cast<float*>(sm + L::kVec);
   float* s_beta = s_pl2 + 64;
   float* s_coefw = s_beta + 64;
@@ -327,206 +324,44 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   tc_fence_after();
 
   // ---- phase 3: masks and decays on D1
-  // warp -> TMEM lane quarter (warp & 3) and column half (warp >> 2) of the 64 columns
-  const int quarter = warp & 3, chalf = warp >> 2;
-  const int lrow = quarter * 32 + (tid & 31);          // accumulator row owned by this thread
+  const int lane = tid & 31, quarter = warp & 3, chalf = warp >> 2;
+  const int lrow = quarter * 32 + lane;                // accumulator row owned by this thread
   const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16);
   bool not_contraction = false;
   if (ok) {
-    const int i = lrow & 63;
-    const float pi = s_pl2[i], bi = s_beta[i];
-    uint32_t d[2][16];
-    tmem_ld16(taddr + chalf * 32, d[0]);
-    tmem_ld16(taddr + chalf * 32 + 16, d[1]);
-    tmem_wait_ld();
-    float kk = 0.f;                                      // k_i . k_i when the diagonal lies in this column half
+    not_contraction = mask_chunk(tmem, s_pl2, s_beta, s_ecol, smem_u32(sm + L::kP), matrix, warp, lane);
+    // P above its 16x16 diagonal blocks: by the warps of the diagonal blocks in them, by warp 4 rows ..31, columns 32..
+    if (warp == 4 || (lrow < 64 && (lrow >> 5) == chalf && !(lrow & 16))) {
+      const int row = lrow & 63;
 #pragma unroll
-    for (int piece = 0; piece < 2; ++piece) {
-      const int j0 = chalf * 32 + piece * 16;
-      if (j0 > (i | 31)) {
-        // the whole piece lies above the diagonal for every row of this warp (rows (i & ~31) .. (i | 31)): zeros
-        if (lrow < 64) {
-          uint4* dst = reinterpret_cast<uint4*>(ws.p + (block * kChunk + i) * kChunk + j0);
-          dst[0] = dst[1] = make_uint4(0u, 0u, 0u, 0u);
-        } else {
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4)
-            *reinterpret_cast<float4*>(sAT + i * L::kLd + j0 + q4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        continue;
-      }
-      // in the 32x32 block off the diagonal exp(p_i - p_j) = exp(p_i - p_31) exp(p_31 - p_j): a factor per row, one per column
-      const bool off = quarter & 1 && chalf == 0;
-      const float row_factor = off ? fast_exp2(pi - s_pl2[31]) * (lrow < 64 ? kScale : bi) : 0.f;
-      float pj[16];
-#pragma unroll
-      for (int q4 = 0; q4 < 4; ++q4) {
-        const float4 t = *reinterpret_cast<const float4*>((off ? s_ecol : s_pl2) + j0 + q4 * 4);
-        pj[q4 * 4] = t.x; pj[q4 * 4 + 1] = t.y; pj[q4 * 4 + 2] = t.z; pj[q4 * 4 + 3] = t.w;
-      }
-      if (lrow < 64) {
-        uint32_t packed[8];
-#pragma unroll
-        for (int jj = 0; jj < 16; jj += 2) {
-          const int j = j0 + jj;
-          float a0 = __uint_as_float(d[piece][jj]), a1 = __uint_as_float(d[piece][jj + 1]);
-          if (off) {
-            a0 = a0 * pj[jj] * row_factor;
-            a1 = a1 * pj[jj + 1] * row_factor;
-          } else {
-            a0 = a0 * kScale * fast_exp2(pi - pj[jj]);
-            a1 = a1 * kScale * fast_exp2(pi - pj[jj + 1]);
-          }
-          packed[jj >> 1] = pack_bf16(j <= i ? a0 : 0.f, j + 1 <= i ? a1 : 0.f);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(ws.p + (block * kChunk + i) * kChunk + j0);
-        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      } else {
-        float* arow = sAT + i * L::kLd + j0;
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          float a[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int jj = q4 * 4 + e;
-            const float x = __uint_as_float(d[piece][jj]);
-            const float y = off ? x * pj[jj] * row_factor : bi * x * fast_exp2(pi - pj[jj]);
-            a[e] = j0 + jj < i ? y : 0.f;
-            kk = j0 + jj == i ? x : kk;
-          }
-          *reinterpret_cast<float4*>(arow + q4 * 4) = make_float4(a[0], a[1], a[2], a[3]);
-        }
-      }
+      for (int c8 = 0; c8 < 4; ++c8)
+        if (warp == 4 || c8 >= 2) *reinterpret_cast<uint4*>(sm + L::kP + row * 128 + (((chalf * 4 + c8) ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
     }
     tc_fence_before();      // D1's columns are overwritten by the W^T product once every thread has passed the barriers
-    // token i multiplies the state by exp(g_i) (I - beta_i k_i k_i^T): a contraction iff 0 <= beta_i |k_i|^2 <= 2
-    if (lrow >= 64) not_contraction = !(bi >= 0.f && bi * kk <= 2.f);
+    fence_proxy_async_smem();
   }
-  if (kRaw && tid == 0) tma_store_wait_read();     // the inverse's scratch and the T tiles reuse the Q boxes from here on
+  if (kRaw && tid == 0) tma_store_wait_read();     // the T tiles reuse the Q boxes from here on
   const int chunk_not_contraction = __syncthreads_or(not_contraction);
-  ok = __syncthreads_and(ok);                  // uniform from here on: the warp-level barrier below needs that
+  ok = __syncthreads_and(ok);                  // uniform from here on: the warp-level barriers below need that
+  if (tid == 0 && ok) {
+    tma_store_2d(&tm_p, sm + L::kP, 0, int(block * kChunk));
+    tma_store_commit();
+  }
 
-  // ---- phase 4: T = (I+A)^-1 in place, blocked 16 -> 32 -> 64, all in FP32 on the CUDA cores
-  // level 1: the four 16x16 diagonal blocks, one column per thread (left-looking, in registers); the 16 threads
-  // of a block sit in one warp and overwrite the block only after all of them have read it
-  if (ok && tid < 64) {
-    const int blk = tid >> 4, c = tid & 15;
-    float* a0 = sAT + (blk * 16) * L::kLd + blk * 16;
-    float x[16];
-    float4 cur[4], nxt[4] = {};
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      // fetch the next row's lower-triangle part before the dependent FMA chain of this row
-#pragma unroll
-      for (int j4 = 0; j4 < i + 1 && i + 1 < 16; j4 += 4)
-        nxt[j4 >> 2] = *reinterpret_cast<const float4*>(a0 + (i + 1) * L::kLd + j4);
-      float acc0 = (i == c) ? 1.f : 0.f, acc1 = 0.f;
-#pragma unroll
-      for (int j4 = 0; j4 < i; j4 += 4) {
-        const float4 a = cur[j4 >> 2];
-        if (j4 + 0 < i) acc0 = fmaf(-a.x, x[j4 + 0], acc0);
-        if (j4 + 1 < i) acc1 = fmaf(-a.y, x[j4 + 1], acc1);
-        if (j4 + 2 < i) acc0 = fmaf(-a.z, x[j4 + 2], acc0);
-        if (j4 + 3 < i) acc1 = fmaf(-a.w, x[j4 + 3], acc1);
-      }
-      x[i] = acc0 + acc1;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) cur[q] = nxt[q];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 16; ++i) a0[i * L::kLd + c] = x[i];
-  }
+  // ---- phase 4: T = (I+A)^-1 in place, blocked 16 -> 32 -> 64
+  if (ok && warp < 2) solve_diagonal(matrix, warp, lane);
   __syncthreads();
-  // level 2: inside each 32x32 diagonal block, T21 = -T22 (A21 T11) with 16x16 blocks, written where A21 was.
-  // Levels 2 and 3 are small dense products: they run on the tensor cores as m16n8k8 TF32 tiles with the 3xTF32
-  // split (FP32-grade accuracy), one tile per warp, operands read from shared memory one word per lane; as FP32 FMAs
-  // with vector loads they made up more than half of the kernel's shared-memory traffic, which is what bounds it.
-  {
-    const int lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int big = warp >> 1, nt = warp & 1, o = big * 32;        // warps 0..3: (diagonal block, 8-column tile)
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    if (ok && warp < 4) {
-      tile_product_tf32x3(c, sAT + (o + 16) * L::kLd + o, L::kLd, sAT + o * L::kLd + o + nt * 8, L::kLd, 16, g, t);
-      *reinterpret_cast<float2*>(sX + (big * 16 + g) * L::kLdX + nt * 8 + 2 * t) = make_float2(c[0], c[1]);
-      *reinterpret_cast<float2*>(sX + (big * 16 + g + 8) * L::kLdX + nt * 8 + 2 * t) = make_float2(c[2], c[3]);
-    }
-    __syncthreads();
-    if (ok && warp < 4) {
-      c[0] = c[1] = c[2] = c[3] = 0.f;
-      tile_product_tf32x3(c, sAT + (o + 16) * L::kLd + o + 16, L::kLd, sX + big * 16 * L::kLdX + nt * 8, L::kLdX, 16, g, t);
-      *reinterpret_cast<float2*>(sAT + (o + 16 + g) * L::kLd + o + nt * 8 + 2 * t) = make_float2(-c[0], -c[1]);
-      *reinterpret_cast<float2*>(sAT + (o + 16 + g + 8) * L::kLd + o + nt * 8 + 2 * t) = make_float2(-c[2], -c[3]);
-    }
-  }
+  merge_blocks(matrix, ok, warp, lane, [] { __syncthreads(); });
   __syncthreads();
-  // level 3: T21 = -T22 (A21 T11) with 32x32 blocks: eight tiles, one per warp
+  // T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles.  The W pair goes to the Q boxes at once; the U pair
+  // overwrites T, so it waits until every thread has read its part.
   {
-    const int lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int mt = warp >> 2, nt = warp & 3;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    if (ok) {
-      tile_product_tf32x3(c, sAT + (32 + mt * 16) * L::kLd, L::kLd, sAT + nt * 8, L::kLd, 32, g, t);
-      *reinterpret_cast<float2*>(sX + (mt * 16 + g) * L::kLdX3 + nt * 8 + 2 * t) = make_float2(c[0], c[1]);
-      *reinterpret_cast<float2*>(sX + (mt * 16 + g + 8) * L::kLdX3 + nt * 8 + 2 * t) = make_float2(c[2], c[3]);
-    }
+    float4 x[4];
+    const bool mine = ok && inverse_part(matrix, tid, x);
+    if (mine) scaled_part<L::kTwL - L::kTwH>(x, s_coefw, smem_u32(sm + L::kTwH), tid);
     __syncthreads();
-    if (ok) {
-      c[0] = c[1] = c[2] = c[3] = 0.f;
-      tile_product_tf32x3(c, sAT + (32 + mt * 16) * L::kLd + 32, L::kLd, sX + nt * 8, L::kLdX3, 32, g, t);
-      *reinterpret_cast<float2*>(sAT + (32 + mt * 16 + g) * L::kLd + nt * 8 + 2 * t) = make_float2(-c[0], -c[1]);
-      *reinterpret_cast<float2*>(sAT + (32 + mt * 16 + g + 8) * L::kLd + nt * 8 + 2 * t) = make_float2(-c[2], -c[3]);
-    }
-  }
-  __syncthreads();
-  // T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row i, sixteen columns (conflict-free:
-  // the row pitch of 68 words spreads eight consecutive rows over all banks, the tile rows are swizzled).
-  // The W pair goes to the Q boxes at once; the U pair overwrites T, so it waits until every thread has read its part.
-  {
-    const int i = tid & 63, c0 = (tid >> 6) * 16;      // a warp's lanes: consecutive rows, the same columns
-    uint32_t uh[8], ul[8];
-    if (ok) {
-#pragma unroll
-      for (int g8 = 0; g8 < 2; ++g8) {
-        const int c = c0 + g8 * 8;
-        float t[8], cw[8], cu[8];
-#pragma unroll
-        for (int q4 = 0; q4 < 2; ++q4) {
-          const float4 tv = *reinterpret_cast<const float4*>(sAT + i * L::kLd + c + q4 * 4);
-          const float4 wv = *reinterpret_cast<const float4*>(s_coefw + c + q4 * 4);
-          const float4 uv = *reinterpret_cast<const float4*>(s_beta + c + q4 * 4);
-          t[q4 * 4] = tv.x; t[q4 * 4 + 1] = tv.y; t[q4 * 4 + 2] = tv.z; t[q4 * 4 + 3] = tv.w;
-          cw[q4 * 4] = wv.x; cw[q4 * 4 + 1] = wv.y; cw[q4 * 4 + 2] = wv.z; cw[q4 * 4 + 3] = wv.w;
-          cu[q4 * 4] = uv.x; cu[q4 * 4 + 1] = uv.y; cu[q4 * 4 + 2] = uv.z; cu[q4 * 4 + 3] = uv.w;
-        }
-        uint32_t wh[4], wl[4];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const float w0 = t[e] * cw[e], w1 = t[e + 1] * cw[e + 1];
-          const float u0 = t[e] * cu[e], u1 = t[e + 1] * cu[e + 1];
-          const uint32_t hw = pack_bf16(w0, w1), hu = pack_bf16(u0, u1);
-          wh[e >> 1] = hw;
-          wl[e >> 1] = pack_bf16(w0 - bf16_lo(hw), w1 - bf16_hi(hw));
-          uh[g8 * 4 + (e >> 1)] = hu;
-          ul[g8 * 4 + (e >> 1)] = pack_bf16(u0 - bf16_lo(hu), u1 - bf16_hi(hu));
-        }
-        const int off = i * 128 + (((c >> 3) ^ (i & 7)) << 4);
-        *reinterpret_cast<uint4*>(sm + L::kTwH + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-        *reinterpret_cast<uint4*>(sm + L::kTwL + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-      }
-    }
-    __syncthreads();
-    if (ok) {
-#pragma unroll
-      for (int g8 = 0; g8 < 2; ++g8) {
-        const int c = c0 + g8 * 8;
-        const int off = i * 128 + (((c >> 3) ^ (i & 7)) << 4);
-        *reinterpret_cast<uint4*>(sm + L::kTuH + off) = make_uint4(uh[g8 * 4], uh[g8 * 4 + 1], uh[g8 * 4 + 2], uh[g8 * 4 + 3]);
-        *reinterpret_cast<uint4*>(sm + L::kTuL + off) = make_uint4(ul[g8 * 4], ul[g8 * 4 + 1], ul[g8 * 4 + 2], ul[g8 * 4 + 3]);
-      }
-      fence_proxy_async_smem();
-    }
+    if (mine) scaled_part<L::kTuL - L::kTuH>(x, s_beta, smem_u32(sm + L::kTuH), tid);
+    fence_proxy_async_smem();
   }
   __syncthreads();
 
@@ -538,8 +373,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         const uint64_t a = smem_desc(base + L::kK0 + ks * 2048, L::kK1 - L::kK0, 1024);
-        const uint64_t bb = smem_desc(base + (part ? L::kTwL : L::kTwH) + ks * 32, 16, 1024);
-        mma_ss(tmem + 0, a, bb, kIdescN64AT, (part | ks) != 0);
+        const uint64_t bb = smem_desc(base + (part ? L::kTwL : L::kTwH) + ks * 32, 16, 1024) + rows_from(ks);
+        mma_ss(tmem + 0 + 16 * ks, a, bb, idesc_rows_from(ks, true), (part | ks) != 0);
       }
     }
 #pragma unroll
@@ -547,8 +382,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         const uint64_t a = smem_desc(base + L::kV0 + ks * 2048, L::kV1 - L::kV0, 1024);
-        const uint64_t bb = smem_desc(base + (part ? L::kTuL : L::kTuH) + ks * 32, 16, 1024);
-        mma_ss(tmem + 64, a, bb, kIdescN64AT, (part | ks) != 0);
+        const uint64_t bb = smem_desc(base + (part ? L::kTuL : L::kTuH) + ks * 32, 16, 1024) + rows_from(ks);
+        mma_ss(tmem + 64 + 16 * ks, a, bb, idesc_rows_from(ks, true), (part | ks) != 0);
       }
     }
     mma_commit(bar_mma);
@@ -1215,7 +1050,7 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          mma_ts(acc_o, tm + kAccX + 64 + ks * 16, pd + uint64_t(ks * 2), kIdescN64, 1);
+          mma_ts(acc_o + 16 * ks, tm + kAccX + 64 + ks * 16, pd + uint64_t(ks * 2) + rows_from(ks), idesc_rows_from(ks, false), 1);
         mma_commit(bar_o);
         mma_commit(empty + (c & 1));
       }
@@ -1264,17 +1099,19 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   const uint64_t plane_rows = uint64_t(geo.blocks()) * kDim;
   if (int rc = enc.bf16_2d(&tm_wh, ws.w_hi, kChunk, plane_rows, kDim)) return rc;
   if (int rc = enc.bf16_2d(&tm_wl, ws.w_lo, kChunk, plane_rows, kDim)) return rc;
+  CUtensorMap tm_p;
+  if (int rc = enc.bf16_2d(&tm_p, ws.p, kChunk, uint64_t(geo.blocks()) * kChunk, kChunk)) return rc;
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
   const long long grid = (long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel);
   if (!left.flags) {
     const auto prepare = geo.varlen ? prepare_umma_kernel<kPackedSequences>
                          : in.mixed ? prepare_umma_kernel<kRawInputs> : prepare_umma_kernel<kPlain>;
-    prepare<<<(unsigned)(geo.varlen ? geo.blocks() : grid), kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
+    prepare<<<(unsigned)(geo.varlen ? geo.blocks() : grid), kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, tm_p, in, geo, ws, left);
     return int(cudaGetLastError());
   }
   const long long resident = 3LL * left.sms;
   return launch_early(in.mixed ? prepare_umma_kernel<kRawRepairing> : prepare_umma_kernel<kRepairing>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
-                      tm_q, tm_k, tm_v, tm_wh, tm_wl, in, geo, ws, left);
+                      tm_q, tm_k, tm_v, tm_wh, tm_wl, tm_p, in, geo, ws, left);
 }
 
 int launch_walk_umma(const Inputs& in, const Geometry& geo, const Workspace& ws, bool early, cudaStream_t stream, const Repair& left) {

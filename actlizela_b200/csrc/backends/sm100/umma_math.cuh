@@ -91,24 +91,6 @@ __device__ __forceinline__ void tile_row_tf32x3(float (&d)[4], uint32_t a_addr, 
 #pragma unroll
   for (int i = 0; i < 4; ++i) d[i] = (lh[i] + hl[i]) + hh[i];
 }
-// The same with both operands read word by word: A row-major with pitch lda (rows {g, g+8}).
-__device__ __forceinline__ void tile_product_tf32x3(float (&d)[4], const float* a, int lda, const float* b, int ldb,
-                                                    int kdim, int g, int t) {
-  float lh[4] = {}, hl[4] = {}, hh[4] = {};
-#pragma unroll
-  for (int k0 = 0; k0 < kdim; k0 += 8) {
-    const float av[4] = {a[g * lda + k0 + t], a[(g + 8) * lda + k0 + t], a[g * lda + k0 + t + 4], a[(g + 8) * lda + k0 + t + 4]};
-    const float bv[2] = {b[(k0 + t) * ldb + g], b[(k0 + t + 4) * ldb + g]};
-    uint32_t ah[4], al[4], bh[2], bl[2];
-    split_tf32(av, ah, al);
-    split_tf32(bv, bh, bl);
-    mma_tf32(lh, al, bh);
-    mma_tf32(hl, ah, bl);
-    mma_tf32(hh, ah, bh);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] = (lh[i] + hl[i]) + hh[i];
-}
 __device__ __forceinline__ float bf16_lo(uint32_t packed) { return __uint_as_float(packed << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t packed) { return __uint_as_float(packed & 0xffff0000u); }
 // L2-normalises 16 of the 128 rows of a [Q0 K0 Q1 K1] tile group in place, the pass-th sixteen of the 64 Q rows and then the 64 K
