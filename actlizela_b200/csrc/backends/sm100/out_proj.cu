@@ -1,12 +1,12 @@
 // out_proj of the layer's output gate: C[M,N] = A[M,K] W[N,K]^T, BF16 operands, FP32 accumulation, BF16 result
 // (the reference's out_proj_gemm / out_proj_gemm_cutlass, csrc/output_gate/output_gate.cu and
 // csrc/output_gate/output_gate_cutlass.cu, docs/OUTPUT_GATE.md:17-24: an mma.sync kernel and a CUTLASS SM80 GEMM).
-// Here: one tcgen05 kernel.  A CTA owns a 128 x 128 tile of C; both operands are K-major as they lie in memory
-// (A row-major, W in the Linear layout [N][K]), so their 128 x 64 tiles come straight from TMA into
-// 128-byte-swizzled shared memory, three stages deep; the accumulator lives in 128 columns of tensor memory.
-// Roles: warp 0 TMA producer, warp 1 MMA issuer (owns the tensor-memory allocation), warps 2-5 epilogue
-// (TMEM -> registers -> BF16 -> 256 contiguous bytes per row and thread).  Two CTAs per SM, so the epilogue of one
-// tile overlaps the main loop of another.  Rows and columns beyond M, N and the K tail read as zeros (TMA fill).
+// Here: one tcgen05 kernel.  A CTA owns a tile of C of 128 or 256 rows; both operands are K-major as they lie in memory
+// (A row-major, W in the Linear layout [N][K]), so their 64-wide K steps come straight from TMA into 128-byte-swizzled
+// shared memory, three or four stages deep; the accumulators live in tensor memory.
+// Roles: warp 0 TMA producer, warp 1 MMA issuer (owns the tensor-memory allocation), then four epilogue warps per 128 rows
+// (TMEM -> registers -> BF16 -> swizzled tile -> TMA store).  Rows and columns beyond M, N and the K tail
+// read as zeros (TMA fill).
 #include "actlize_la_sm100.h"
 #include "gdn_common.cuh"
 #include "umma.cuh"
@@ -15,25 +15,28 @@ namespace gdn_sm100 {
 using namespace ptx;
 namespace {
 
-constexpr int kTileM = 128, kTileK = 64, kGemmThreads = 192;
+constexpr int kTileM = 128, kTileK = 64;
 constexpr int kOperandBytes = kTileM * kTileK * 2;                 // 16 KB per 128-row operand tile
-// Tiles of 128 x kN.  Bound by the operands' way into shared memory (about 64 bytes a cycle and SM): a 128 x 128 step takes in
-// 32 KB, a 128 x 256 step 48 KB for twice the products.  Two CTAs of the narrow tile share an SM, the wide one has it alone.
-// (M 8192, K 4096, N 2560: 165 us with 128 columns, 145 with 256, 1.18 PFLOP/s; M 3000: 68 and 62.)
-template <int kN> struct GemmLayout {
-  static constexpr int kStage = kOperandBytes * (1 + kN / 128);
-  static constexpr int kStages = kN == 256 ? 4 : 3, kPerSm = kN == 256 ? 1 : 2;
+// Tiles of 128 kRows x kN.  Bound by shared memory, 128 bytes a cycle: a K step of 64 of a 128 x 128 tile is written (32 KB) and
+// read by the tensor core (32 KB) in 512 cycles, of a 128 x 256 tile in 768 (512 of products), of a 256 x 256 tile in 1280
+// (1024 of products; its two accumulators fill tensor memory).  Two CTAs of the smallest share an SM, the others have it alone.
+// M 3000, K 4096, N 2560: 68, 61 and 53 us; M 6000: 121 as 128 x 256, 102; M 8192: 165, 148, 147 (1.16 PFLOP/s).
+template <int kN, int kRows> struct GemmLayout {
+  static constexpr int kStage = kOperandBytes * kRows + kN * kTileK * 2;
+  static constexpr int kStages = kRows == 1 && kN == 256 ? 4 : 3, kPerSm = kN == 128 ? 2 : 1;
+  static constexpr int kThreads = 64 + 128 * kRows;
   static constexpr int kBars = kStages * kStage;
   static constexpr int kBytes = kBars + 128 + 1024;
   static constexpr uint32_t kIdesc = idesc_bf16(kTileM, kN, false, false);
-  static_assert(kPerSm * (kBytes + 1024) <= 227 * 1024, "shared memory of one SM");
+  static_assert(kN % 64 == 0 && kRows * (kN / 64) * kOperandBytes <= kBars, "the output tile must fit on the stages");
+  static_assert(kPerSm * (kBytes + 1024) <= 227 * 1024 && kPerSm * kRows * kN <= 512, "shared and tensor memory of one SM");
 };
 
-template <int kN>
-__global__ void __launch_bounds__(kGemmThreads, GemmLayout<kN>::kPerSm)
+template <int kN, int kRows>
+__global__ void __launch_bounds__(GemmLayout<kN, kRows>::kThreads, GemmLayout<kN, kRows>::kPerSm)
 out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                     __nv_bfloat16* __restrict__ c, int m, int n, int k) {
-  using L = GemmLayout<kN>;
+                     const __grid_constant__ CUtensorMap tm_c, int m, int n, int k) {
+  using L = GemmLayout<kN, kRows>;
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + L::kBars);       // [stages] tiles landed
@@ -44,7 +47,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   const AbortFlag abort{abort_word};
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * kN, m0 = blockIdx.y * kTileM;
+  const int n0 = blockIdx.x * kN, m0 = blockIdx.y * kTileM * kRows;
   const int k_tiles = (k + kTileK - 1) / kTileK;
 
   if (tid == 0) {
@@ -57,7 +60,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, kN);
+    tmem_alloc(tmem_slot, kN * kRows);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -77,7 +80,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         uint8_t* stage = sm + s * L::kStage;
         mbar_arrive_expect_tx(full + s, L::kStage);
         tma_load_2d(stage, &tm_a, full + s, kt * kTileK, m0);
-        tma_load_2d(stage + kOperandBytes, &tm_w, full + s, kt * kTileK, n0);
+        tma_load_2d(stage + kOperandBytes * kRows, &tm_w, full + s, kt * kTileK, n0);
       }
     }
     __syncwarp();
@@ -90,51 +93,63 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         ok = mbar_wait(full + s, (kt / L::kStages) & 1, abort, 61, kt);
         tc_fence_after();
         const uint64_t da = smem_desc(base + s * L::kStage, 16, 1024);
-        const uint64_t db = smem_desc(base + s * L::kStage + kOperandBytes, 16, 1024);
+        const uint64_t db = smem_desc(base + s * L::kStage + kOperandBytes * kRows, 16, 1024);
 #pragma unroll
         for (int ks = 0; ks < kTileK / 16; ++ks)          // 16 BF16 (32 bytes) along K per instruction
-          mma_ss(tmem, da + uint64_t(ks * 2), db + uint64_t(ks * 2), L::kIdesc, (kt | ks) != 0);
+#pragma unroll
+          for (int r = 0; r < kRows; ++r)
+            mma_ss(tmem + r * kN, da + uint64_t(r * (kOperandBytes >> 4) + ks * 2), db + uint64_t(ks * 2), L::kIdesc, (kt | ks) != 0);
         mma_commit(empty + s);
       }
       mma_commit(done);
     }
     __syncwarp();
   } else {
-    // epilogue: a warp may only touch the TMEM lane quarter (warp % 4); warps 2..5 cover quarters 2, 3, 0, 1
-    const int quarter = warp & 3;
-    const int row = m0 + quarter * 32 + lane;
+    // epilogue: a warp may only touch the TMEM lane quarter (warp % 4); warps 2..5 cover quarters 2, 3, 0, 1, warps 6..9 those
+    // of the second 128 rows
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
+    // The tile leaves through boxes of 128 rows x 64 columns on the dead stages and TMA stores, which clip it at M and N.
+    // (Straight from registers a warp's 16-byte stores go to 32 rows, two to a sector: about 4 us a turn of the wide tiles.)
+    const int row = quarter * 32 + lane;
     const bool ok = mbar_wait(done, 0, abort, 62, 0);
     tc_fence_after();
-    if (ok) {
-      const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16);
+    const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + part * kN;
+    const bool leader = ((warp - 2) & 3) == 0 && lane == 0;
+#pragma unroll 1
+    for (int box = 0; box < (kN + 63) / 64; ++box) {
+      uint8_t* tile = sm + (part * ((kN + 63) / 64) + box) * kOperandBytes;
 #pragma unroll
-      for (int piece = 0; piece < kN / 32; ++piece) {
-        uint32_t d[32];
-        tmem_ld32(taddr + piece * 32, d);        // warp-collective: every lane takes part, also rows beyond M
-        tmem_wait_ld();
-        if (row < m) {
-          __nv_bfloat16* dst = c + (long long)row * n + n0 + piece * 32;
+      for (int half = 0; half < 2; ++half) {
+        if (box * 64 + half * 32 < kN && ok) {
+          uint32_t d[32];
+          tmem_ld32(taddr + box * 64 + half * 32, d);
+          tmem_wait_ld();
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            if (n0 + piece * 32 + q * 8 < n) {     // N is a multiple of 8: a 16-byte piece is inside or outside
-              uint4 o;
-              o.x = pack_bf16(__uint_as_float(d[q * 8 + 0]), __uint_as_float(d[q * 8 + 1]));
-              o.y = pack_bf16(__uint_as_float(d[q * 8 + 2]), __uint_as_float(d[q * 8 + 3]));
-              o.z = pack_bf16(__uint_as_float(d[q * 8 + 4]), __uint_as_float(d[q * 8 + 5]));
-              o.w = pack_bf16(__uint_as_float(d[q * 8 + 6]), __uint_as_float(d[q * 8 + 7]));
-              *reinterpret_cast<uint4*>(dst + q * 8) = o;
-            }
+            uint4 o;
+            o.x = pack_bf16(__uint_as_float(d[q * 8 + 0]), __uint_as_float(d[q * 8 + 1]));
+            o.y = pack_bf16(__uint_as_float(d[q * 8 + 2]), __uint_as_float(d[q * 8 + 3]));
+            o.z = pack_bf16(__uint_as_float(d[q * 8 + 4]), __uint_as_float(d[q * 8 + 5]));
+            o.w = pack_bf16(__uint_as_float(d[q * 8 + 6]), __uint_as_float(d[q * 8 + 7]));
+            *reinterpret_cast<uint4*>(tile + row * 128 + (((half * 4 + q) ^ (row & 7)) << 4)) = o;
           }
         }
       }
+      fence_proxy_async_smem();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
+      if (leader && ok && m0 + part * kTileM < m && n0 + box * 64 < n) {
+        tma_store_2d(&tm_c, tile, n0 + box * 64, m0 + part * kTileM);
+        tma_store_commit();
+      }
     }
+    if (leader) tma_store_wait_all();
   }
   if (abort.raised()) {
     for (int i = 0; i < 20; ++i) __nanosleep(100000);   // let copies in flight land before the CTA leaves
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, kN);
+  if (warp == 1) tmem_dealloc(tmem, kN * kRows);
 }
 
 // ------------------------------------------------------------------------------------------- few rows: split over K
@@ -289,13 +304,15 @@ int launch_skinny(TensorMapEncoder& enc, const void* a, const void* w, void* c, 
 }
 
 
-template <int kN>
+template <int kN, int kRows>
 int launch_tiles(TensorMapEncoder& enc, const void* a, const void* w, void* c, int m, int n, int k, cudaStream_t stream) {
-  CUtensorMap tm_a, tm_w;
-  if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM)) return rc;
+  using L = GemmLayout<kN, kRows>;
+  CUtensorMap tm_a, tm_w, tm_c;
+  if (int rc = enc.bf16_2d(&tm_c, c, uint64_t(n), uint64_t(m), kTileM)) return rc;
+  if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM * kRows)) return rc;
   if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kN)) return rc;
-  return launch_early(out_proj_umma_kernel<kN>, dim3((n + kN - 1) / kN, (m + kTileM - 1) / kTileM), kGemmThreads,
-                      GemmLayout<kN>::kBytes, true, stream, tm_a, tm_w, static_cast<__nv_bfloat16*>(c), m, n, k);
+  return launch_early(out_proj_umma_kernel<kN, kRows>, dim3((n + kN - 1) / kN, (m + kTileM * kRows - 1) / (kTileM * kRows)), L::kThreads,
+                      L::kBytes, true, stream, tm_a, tm_w, tm_c, m, n, k);
 }
 }  // namespace
 
@@ -304,8 +321,9 @@ GDN_SM100_DEFINE_STATUS_HOOKS(gemm)
 int configure_out_proj() {
   if (int rc = tensor_map_encoder().init()) return rc;
   const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(out_proj_umma_kernel<128>, smem, GemmLayout<128>::kBytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<256>, smem, GemmLayout<256>::kBytes);
+  cudaError_t e = cudaFuncSetAttribute(out_proj_umma_kernel<128, 1>, smem, GemmLayout<128, 1>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<256, 1>, smem, GemmLayout<256, 1>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<256, 2>, smem, GemmLayout<256, 2>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<16>, smem, SkinnyLayout<16>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<32>, smem, SkinnyLayout<32>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<64>, smem, SkinnyLayout<64>::kBytes);
@@ -327,10 +345,13 @@ int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, 
     if (m <= 64) return launch_skinny<64>(enc, a, w, c, m, n, k, split, stream);
     return launch_skinny<128>(enc, a, w, c, m, n, k, split, stream);
   }
-  // a K step of all tiles of an SM's turn takes 512 cycles of operand traffic for a 128 x 128 tile, 768 for a 128 x 256 one
-  const long long wide = ((n + 255LL) / 256) * ((m + 127LL) / 128);
-  return (wide + kSms - 1) / kSms * 768 < (tiles + kSms - 1) / kSms * 512 ? launch_tiles<256>(enc, a, w, c, m, n, k, stream)
-                                                              : launch_tiles<128>(enc, a, w, c, m, n, k, stream);
+  // A K step takes an SM 512 cycles for a 128 x 128 tile, 768 for a 128 x 256 and 1280 for a 256 x 256 one (shared memory, see
+  // GemmLayout; measured 0.43 us and 0.69 for the last two): the form whose turns are the shortest in all.
+  const auto turns = [](long long all) { return (all + kSms - 1) / kSms; };
+  const long long columns = (n + 255LL) / 256, small = turns(tiles) * 512;
+  const long long wide = turns(columns * ((m + 127LL) / 128)) * 768, square = turns(columns * ((m + 255LL) / 256)) * 1280;
+  if (square < wide && square < small) return launch_tiles<256, 2>(enc, a, w, c, m, n, k, stream);
+  return wide < small ? launch_tiles<256, 1>(enc, a, w, c, m, n, k, stream) : launch_tiles<128, 1>(enc, a, w, c, m, n, k, stream);
 }
 
 }  // namespace gdn_sm100

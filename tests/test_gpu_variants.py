@@ -29,6 +29,20 @@ def test_out_proj_with_few_rows(m, k, n):
     assert torch.equal(got, out_proj_gemm(a, w))                  # the sum over the cluster has one order
 
 
+@pytest.mark.parametrize("m,k,n", [(2900, 72, 2504), (3001, 136, 2504), (5000, 64, 1288), (6000, 1024, 2560)])
+def test_out_proj_square_tiles(m, k, n):
+    """Tiles of 256 x 256: rows that end in either 128-row half, ragged columns, one K step, a K tail, several turns.  An element is one
+    BF16 rounding (2^-8 relative, two neighbours) from the FP32 sum; sums of K products differ by K 2^-24 of their terms."""
+    from actlizela_b200 import out_proj_gemm
+    gen = torch.Generator().manual_seed(m + k)
+    a = torch.randn(m, k, generator=gen).to(torch.bfloat16).cuda()
+    w = (torch.randn(n, k, generator=gen) * k ** -0.5).to(torch.bfloat16).cuda()
+    want = a.double() @ w.double().t()
+    got = out_proj_gemm(a, w)
+    assert got.shape == (m, n)
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all())
+
+
 @pytest.mark.parametrize("m,k,n", [(1100, 264, 2560), (1930, 136, 2312), (2049, 72, 5128), (3000, 4096, 2560), (1999, 64, 5000)])
 def test_out_proj_tile_widths(m, k, n):
     """Tiles of 128 and 256 columns, both sides of the rule: ragged rows, columns that end in either half of a wide tile,
