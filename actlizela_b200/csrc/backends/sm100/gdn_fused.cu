@@ -297,7 +297,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   if (kRaw) {
     if (ok) {
 #pragma unroll 1
-      for (int pass = 0; pass < 8; ++pass) normalise_rows(kq, pass, t);
+      for (int pass = 0; pass < 4; ++pass) normalise_rows(kq, pass, t);
       fence_proxy_async_smem();
     }
     group_sync(id);

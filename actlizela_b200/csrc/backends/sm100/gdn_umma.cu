@@ -296,7 +296,7 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     static_assert(L::kQ0 == 0 && L::kK0 == kBox && L::kQ1 == 2 * kBox && L::kK1 == 3 * kBox, "tiles as normalise_rows takes them");
     if (ok) {
 #pragma unroll
-      for (int pass = 0; pass < 8; ++pass) normalise_rows(sm, pass, tid);
+      for (int pass = 0; pass < 4; ++pass) normalise_rows(sm, pass, tid);
       fence_proxy_async_smem();
     }
     __syncthreads();
