@@ -204,8 +204,8 @@ __device__ __forceinline__ void merge_blocks(uint32_t matrix, bool ok, int warp,
   }
 }
 
-// A thread's part of T (row t & 63, 16 columns from (t >> 6) * 16 on), and the same scaled per column by `coef` as BF16 hi/lo
-// pieces of a K-major swizzled tile pair, the lo tile `kLo` bytes behind.  The block above the diagonal is left out.
+// A thread's part of T (row t & 63, 16 columns from (t >> 6) * 16 on), the same scaled per column by `coef` as BF16 hi/lo pieces, and
+// their place in a K-major swizzled tile pair, the lo tile `kLo` bytes behind.  The block above the diagonal is left out.
 __device__ __forceinline__ bool inverse_part(uint32_t matrix, int t, float4 (&x)[4]) {
   const int row = t & 63, c4 = (t >> 6) * 4;
   if (c4 >= 8 && row < 32) return false;
@@ -214,24 +214,34 @@ __device__ __forceinline__ bool inverse_part(uint32_t matrix, int t, float4 (&x)
   for (int q4 = 0; q4 < 4; ++q4) x[q4] = *shared_at<const float4>(at ^ uint32_t(q4 << 4));
   return true;
 }
-template <int kLo>
-__device__ __forceinline__ void scaled_part(const float4 (&x)[4], const float* coef, uint32_t tile, int t) {
-  const int row = t & 63, c0 = (t >> 6) * 16;
-  const uint32_t at = (tile + row * 128 + (row & 7) * 16) ^ uint32_t(c0 << 1);
+struct ScaledPart { uint4 hi[2], lo[2]; };
+__device__ __forceinline__ ScaledPart scaled_part(const float4 (&x)[4], const float* coef, int t) {
+  ScaledPart out;
 #pragma unroll
   for (int g8 = 0; g8 < 2; ++g8) {
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int q4 = 0; q4 < 2; ++q4) {
-      const float4 y = x[g8 * 2 + q4], c = *reinterpret_cast<const float4*>(coef + c0 + (g8 * 2 + q4) * 4);
+      const float4 y = x[g8 * 2 + q4], c = *reinterpret_cast<const float4*>(coef + (t >> 6) * 16 + (g8 * 2 + q4) * 4);
       float a0, a1, b0, b1;
       mul2(a0, a1, y.x, y.y, c.x, c.y);
       mul2(b0, b1, y.z, y.w, c.z, c.w);
       split_pair(a0, a1, hi[q4 * 2], lo[q4 * 2]);
       split_pair(b0, b1, hi[q4 * 2 + 1], lo[q4 * 2 + 1]);
     }
-    *shared_at<uint4>(at ^ uint32_t(g8 << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *shared_at<uint4>((at ^ uint32_t(g8 << 4)) + kLo) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    out.hi[g8] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    out.lo[g8] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+  return out;
+}
+template <int kLo>
+__device__ __forceinline__ void store_part(const ScaledPart& p, uint32_t tile, int t) {
+  const int row = t & 63, c0 = (t >> 6) * 16;
+  const uint32_t at = (tile + row * 128 + (row & 7) * 16) ^ uint32_t(c0 << 1);
+#pragma unroll
+  for (int g8 = 0; g8 < 2; ++g8) {
+    *shared_at<uint4>(at ^ uint32_t(g8 << 4)) = p.hi[g8];
+    *shared_at<uint4>((at ^ uint32_t(g8 << 4)) + kLo) = p.lo[g8];
   }
 }
 

@@ -70,11 +70,13 @@ namespace {
 __device__ int g_walk_plan_counts[2];
 
 // ================================================================================= prepare kernel
-// One CTA per (batch, value head, chunk) block, 256 threads, THREE CTAs per SM (at most 80 registers, 67 KB of
-// shared memory, 128 tensor-memory columns): the phases of a block are serial and latency bound, so the
-// throughput comes from the blocks in flight.  A warp owns the TMEM lane quarter (warp & 3) and, of every
-// accumulator it reads, the column half (warp >> 2).
-//   phase 1  TMA: Q, K chunk tiles (key head of the group) and V tile; gate prefix by two warps
+// One CTA per (batch, value head, chunk) block, 256 threads, three or four CTAs per SM (50 KB of shared memory, 128
+// tensor-memory columns; see launch_prepare_umma): the phases of a block are serial and latency bound, so the
+// throughput comes from the blocks in flight.  The V tile comes over the dead Q tile, and one scaled pair of tiles of T after the
+// other takes the place of T (with places of their own a CTA took 75 KB, three to an SM: T2048, 32 heads 67.6 us in all, 64.9 so;
+// T8192 201.7 and 193.5).  A warp owns the TMEM lane quarter (warp & 3) and, of every accumulator it reads, the column half
+// (warp >> 2).
+//   phase 1  TMA: Q, K chunk tiles (key head of the group); gate prefix by two warps
 //   phase 2  D1[128x64] = [Q;K] K^T                                  (one tcgen05 product, 8 instructions)
 //   phase 3  rows 0..63  -> P = tril(QK^T * decay)/sqrt(128) -> BF16 -> swizzled tile -> TMA store
 //            rows 64..127-> A = tril(beta_i KK^T * decay, -1) -> shared (FP32);
@@ -82,30 +84,26 @@ __device__ int g_walk_plan_counts[2];
 //   phase 4  T = (I+A)^-1 IN PLACE, blocked: four 16x16 diagonal solves in FP32 registers, then
 //            T21 = -T22 (A21 T11) at block size 16 and 32 as 3xTF32 mma.sync tiles (the blocked scheme and the
 //            TF32x3 merges of the reference's tests/wy_cpu.py:10-41)
-//            T diag(beta exp(p)) and T diag(beta) -> BF16 hi/lo K-major tiles: the first pair over the dead Q
-//            boxes, the second over T itself (every thread holds its part of T in registers by then)
-//   phase 5  W^T = K^T (T diag(beta exp p))^T (into the columns D1 occupied),  U^T = V^T (T diag(beta))^T
+//   phase 5  T diag(beta exp(p)) -> BF16 hi/lo K-major tiles over T (every thread holds its part in registers by then),
+//            W^T = K^T (T diag(beta exp p))^T into the columns D1 occupied; then T diag(beta) and U^T = V^T (T diag(beta))^T
 //            (A = transposed K / V tiles)
 //   phase 6  accumulators -> registers -> workspace.  W is stored transposed, [key dim][token]: a thread owns one
 //            row and stages its 32 tokens as 16-byte pieces in swizzled tiles that leave through TMA stores; U is
 //            token-major and leaves straight from registers (a warp writes 128 contiguous bytes per token)
 struct PrepLayout {
   static constexpr int kQ0 = 0, kK0 = kBox, kQ1 = 2 * kBox, kK1 = 3 * kBox;   // [Q;K] stacked, two K atoms
-  static constexpr int kV0 = 4 * kBox, kV1 = 5 * kBox;
-  static constexpr int kAT = 6 * kBox;                     // FP32 matrix: A, then T in place
-  static constexpr int kP = 8 * kBox;
-  static constexpr int kTwH = kQ0, kTwL = kQ1;             // written after phase 4, when Q is dead
-  static constexpr int kTuH = kAT, kTuL = kAT + kBox;      // written once T sits in registers
+  static constexpr int kP = kQ0, kV0 = kQ0, kV1 = kQ1;     // Q is dead behind D1: P passes through its first box, then V is loaded
+  static constexpr int kAT = 4 * kBox;                     // FP32 matrix: A, then T in place, then the scaled pair hi | lo
   static constexpr int kStageWH = 0, kStageWL = 2 * kBox;  // phase 6: W^T hi / lo tiles [128][64] over the Q/K boxes
-  static constexpr int kVec = 9 * kBox;                    // float [4][64]: pl2, beta, beta*exp(p), exp(p)/sqrt(128)
-  static constexpr int kBars = kVec + (4 * 64 + 32) * 4;   // (and 32 column factors) 2 mbarriers, tmem slot, abort flag, carry
+  static constexpr int kVec = 6 * kBox;                    // float [4][64]: pl2, beta, beta*exp(p), exp(p)/sqrt(128)
+  static constexpr int kBars = kVec + (4 * 64 + 32) * 4;   // (and 32 column factors) 3 mbarriers, tmem slot, abort flag, carry
   static constexpr int kTotal = kBars + 64;
-  static_assert(2 * kBox == kMatrixBytes, "the U pair of T tiles takes the place of T");
+  static_assert(2 * kBox == kMatrixBytes, "the scaled pair takes the place of T");
 };
 constexpr int kPrepThreads = 256;
 constexpr int kPrepSmem = PrepLayout::kTotal + 1024;
 constexpr int kPrepTmemCols = 128;   // D1 [0,64), later W^T;  U^T [64,128)
-static_assert(3 * (kPrepSmem + 1024) <= 227 * 1024, "three prepare CTAs must fit in one SM's shared memory");
+static_assert(4 * (kPrepSmem + 1024) <= 227 * 1024, "four prepare CTAs must fit in one SM's shared memory");
 
 
 // kRaw: the tiles come from the packed projection rows (tm_q is a 2-D map over them, tm_k and tm_v the 4-D maps of the planes
@@ -133,8 +131,8 @@ __device__ __forceinline__ void clamped_offsets(const Geometry& geo, int lane, i
     at[u] = min(x, geo.sequence);
   }
 }
-template <PrepareMode kMode>
-__global__ void __launch_bounds__(kPrepThreads, 3)
+template <PrepareMode kMode, int kPerSm>
+__global__ void __launch_bounds__(kPrepThreads, kPerSm)
 prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_wh,
                     const __grid_constant__ CUtensorMap tm_wl, const __grid_constant__ CUtensorMap tm_p, Inputs in, Geometry geo,
@@ -151,7 +149,8 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   float* s_ecol = s_qscale + 64;
   uint64_t* bar_tma = reinterpret_cast<uint64_t*>(sm + L::kBars);
   uint64_t* bar_mma = bar_tma + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tma + 2);
+  uint64_t* bar_v = bar_tma + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tma + 3);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* carry = reinterpret_cast<float*>(tmem_slot + 2);
   const AbortFlag abort{abort_word};
@@ -238,29 +237,26 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     if (!kRepair || round == 0) {
       mbar_init(bar_tma, 1);
       mbar_init(bar_mma, 1);
+      mbar_init(bar_v, 1);
       *abort_word = 0;
       fence_barrier_init();
     }
     // the input tiles do not depend on tensor memory: start them before the allocation
-    mbar_arrive_expect_tx(bar_tma, 6 * kBox);
+    mbar_arrive_expect_tx(bar_tma, 4 * kBox);
     if (kRaw) {
       // packed rows [q heads | k heads | v heads]; rows behind the batch element's end belong to the next one
       // (or read as zero behind the last) and are neutralised by beta = 0 / zero gate weights
       const int row = b * geo.sequence + t0;
-      const int xq = hk * kDim, xk = (geo.key_heads + hk) * kDim, xv = (2 * geo.key_heads + hv) * kDim;
+      const int xq = hk * kDim, xk = (geo.key_heads + hk) * kDim;
       tma_load_2d(sm + L::kQ0, &tm_q, bar_tma, xq, row);
       tma_load_2d(sm + L::kQ1, &tm_q, bar_tma, xq + 64, row);
       tma_load_2d(sm + L::kK0, &tm_q, bar_tma, xk, row);
       tma_load_2d(sm + L::kK1, &tm_q, bar_tma, xk + 64, row);
-      tma_load_2d(sm + L::kV0, &tm_q, bar_tma, xv, row);
-      tma_load_2d(sm + L::kV1, &tm_q, bar_tma, xv + 64, row);
     } else {
       tma_load_4d(sm + L::kQ0, &tm_q, bar_tma, 0, hk, t0, b);
       tma_load_4d(sm + L::kQ1, &tm_q, bar_tma, 64, hk, t0, b);
       tma_load_4d(sm + L::kK0, &tm_k, bar_tma, 0, hk, t0, b);
       tma_load_4d(sm + L::kK1, &tm_k, bar_tma, 64, hk, t0, b);
-      tma_load_4d(sm + L::kV0, &tm_v, bar_tma, 0, hv, t0, b);
-      tma_load_4d(sm + L::kV1, &tm_v, bar_tma, 64, hv, t0, b);
     }
   }
   if (warp == 1 && (!kRepair || round == 0)) {
@@ -320,8 +316,13 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     mma_commit(bar_mma);
   }
-  ok = ok && mbar_wait(bar_mma, 0, abort, 2, chunk);
+  const uint32_t phase = kRepair ? round & 1 : 0;          // three products a round
+  ok = ok && mbar_wait(bar_mma, phase, abort, 2, chunk);
   tc_fence_after();
+  if (kRaw) {
+    if (tid == 0) tma_store_wait_read();         // P and V take the Q boxes
+    __syncthreads();
+  }
 
   // ---- phase 3: masks and decays on D1
   const int lane = tid & 31, quarter = warp & 3, chalf = warp >> 2;
@@ -340,63 +341,70 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tc_fence_before();      // D1's columns are overwritten by the W^T product once every thread has passed the barriers
     fence_proxy_async_smem();
   }
-  if (kRaw && tid == 0) tma_store_wait_read();     // the T tiles reuse the Q boxes from here on
   const int chunk_not_contraction = __syncthreads_or(not_contraction);
   ok = __syncthreads_and(ok);                  // uniform from here on: the warp-level barriers below need that
-  if (tid == 0 && ok) {
+  if (tid == kPrepThreads - 32 && ok) {          // (a warp that has nothing to do in the next two phases)
     tma_store_2d(&tm_p, sm + L::kP, 0, int(block * kChunk));
     tma_store_commit();
+    tma_store_wait_read();
+    mbar_arrive_expect_tx(bar_v, 2 * kBox);
+    if (kRaw) {
+      const int row = b * geo.sequence + t0, xv = (2 * geo.key_heads + hv) * kDim;
+      tma_load_2d(sm + L::kV0, &tm_q, bar_v, xv, row);
+      tma_load_2d(sm + L::kV1, &tm_q, bar_v, xv + 64, row);
+    } else {
+      tma_load_4d(sm + L::kV0, &tm_v, bar_v, 0, hv, t0, b);
+      tma_load_4d(sm + L::kV1, &tm_v, bar_v, 64, hv, t0, b);
+    }
   }
+  __syncwarp();
 
   // ---- phase 4: T = (I+A)^-1 in place, blocked 16 -> 32 -> 64
   if (ok && warp < 2) solve_diagonal(matrix, warp, lane);
   __syncthreads();
   merge_blocks(matrix, ok, warp, lane, [] { __syncthreads(); });
   __syncthreads();
-  // T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles.  The W pair goes to the Q boxes at once; the U pair
-  // overwrites T, so it waits until every thread has read its part.
+  // ---- phase 5: T diag(beta exp p) as a BF16 hi/lo pair of K-major tiles over T (every thread holds its part in registers by
+  // then), W^T into D1's columns, which every thread has read; then T diag(beta) and U^T likewise
   {
     float4 x[4];
     const bool mine = ok && inverse_part(matrix, tid, x);
-    if (mine) scaled_part<L::kTwL - L::kTwH>(x, s_coefw, smem_u32(sm + L::kTwH), tid);
+    ScaledPart pair{};
+    if (mine) pair = scaled_part(x, s_coefw, tid);
     __syncthreads();
-    if (mine) scaled_part<L::kTuL - L::kTuH>(x, s_beta, smem_u32(sm + L::kTuH), tid);
-    fence_proxy_async_smem();
-  }
-  __syncthreads();
-
-  // ---- phase 5: W^T (into D1's columns, which every thread has read) and U^T
-  if (warp == 0 && ok && elect_one()) {
-    tc_fence_after();
+#pragma unroll 1
+    for (int product = 0; product < 2; ++product) {
+      if (mine) store_part<kBox>(pair, matrix, tid);
+      fence_proxy_async_smem();
+      __syncthreads();
+      if (warp == 0 && ok) {
+        if (product) ok = mbar_wait(bar_v, phase, abort, 4, chunk);
+        if (__all_sync(0xffffffffu, ok) && elect_one()) {
+          tc_fence_after();
+          const uint32_t tile = base + (product ? L::kV0 : L::kK0);          // both pairs of boxes lie 16 KB apart
 #pragma unroll
-    for (int part = 0; part < 2; ++part) {
+          for (int part = 0; part < 2; ++part) {
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const uint64_t a = smem_desc(base + L::kK0 + ks * 2048, L::kK1 - L::kK0, 1024);
-        const uint64_t bb = smem_desc(base + (part ? L::kTwL : L::kTwH) + ks * 32, 16, 1024) + rows_from(ks);
-        mma_ss(tmem + 0 + 16 * ks, a, bb, idesc_rows_from(ks, true), (part | ks) != 0);
+            for (int ks = 0; ks < 4; ++ks)
+              mma_ss(tmem + product * 64 + 16 * ks, smem_desc(tile + ks * 2048, L::kK1 - L::kK0, 1024),
+                     smem_desc(base + L::kAT + part * kBox + ks * 32, 16, 1024) + rows_from(ks), idesc_rows_from(ks, true), (part | ks) != 0);
+          }
+          mma_commit(bar_mma);
+        }
+        __syncwarp();
       }
-    }
-#pragma unroll
-    for (int part = 0; part < 2; ++part) {
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const uint64_t a = smem_desc(base + L::kV0 + ks * 2048, L::kV1 - L::kV0, 1024);
-        const uint64_t bb = smem_desc(base + (part ? L::kTuL : L::kTuH) + ks * 32, 16, 1024) + rows_from(ks);
-        mma_ss(tmem + 64 + 16 * ks, a, bb, idesc_rows_from(ks, true), (part | ks) != 0);
+      if (product == 0 && ok) {
+        // the gate vector does not depend on the products: write it while they run
+        const float last = s_pl2[valid - 1];
+        if (tid < kChunk) ws.gates[block * kGateWords + tid] = (tid < valid) ? fast_exp2(last - s_pl2[tid]) : 0.f;
+        if (tid == kChunk) ws.gates[block * kGateWords + kChunk] = fast_exp2(last);
+        if (tid == kChunk + 1) ws.gates[block * kGateWords + kChunk + 1] = chunk_not_contraction ? 1.f : 0.f;
+        if (tid >= 128 && tid < 128 + kChunk) ws.gates[block * kGateWords + kGateQueryScale + tid - 128] = s_qscale[tid - 128];
       }
+      if (product == 0 && mine) pair = scaled_part(x, s_beta, tid);          // while W^T is formed
+      ok = ok && mbar_wait(bar_mma, phase ^ (product ? 0 : 1), abort, 3, chunk);
     }
-    mma_commit(bar_mma);
   }
-  // the gate vector does not depend on the products: write it while they run
-  if (ok) {
-    const float last = s_pl2[valid - 1];
-    if (tid < kChunk) ws.gates[block * kGateWords + tid] = (tid < valid) ? fast_exp2(last - s_pl2[tid]) : 0.f;
-    if (tid == kChunk) ws.gates[block * kGateWords + kChunk] = fast_exp2(last);
-    if (tid == kChunk + 1) ws.gates[block * kGateWords + kChunk + 1] = chunk_not_contraction ? 1.f : 0.f;
-    if (tid >= 128 && tid < 128 + kChunk) ws.gates[block * kGateWords + kGateQueryScale + tid - 128] = s_qscale[tid - 128];
-  }
-  ok = ok && mbar_wait(bar_mma, 1, abort, 3, chunk);
   tc_fence_after();
 
   // ---- phase 6: W (hi/lo) and U leave for the workspace; lrow is the key (W) / value (U) index.
@@ -412,26 +420,23 @@ prepare_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
     for (int piece = 0; piece < 2; ++piece) {
       const int tk0 = chalf * 32 + piece * 16;
-      uint32_t dw[16], du[16];
-      tmem_ld16(taddr + tk0, dw);
-      tmem_ld16(taddr + 64 + tk0, du);
+      uint32_t d[16];
+      tmem_ld16(taddr + tk0, d);
       tmem_wait_ld();
-      uint32_t hi[8], lo[8];
-#pragma unroll
-      for (int jj = 0; jj < 16; jj += 2) {
-        const float w0 = __uint_as_float(dw[jj]), w1 = __uint_as_float(dw[jj + 1]);
-        const uint32_t h = pack_bf16(w0, w1);
-        hi[jj >> 1] = h;
-        lo[jj >> 1] = pack_bf16(w0 - bf16_lo(h), w1 - bf16_hi(h));
-      }
 #pragma unroll
       for (int h8 = 0; h8 < 2; ++h8) {          // eight tokens = one 16-byte slot of the swizzled row
-        const int slot = (((tk0 >> 3) + h8) ^ (lrow & 7)) << 4;
-        *reinterpret_cast<uint4*>(stage_hi + slot) = make_uint4(hi[h8 * 4], hi[h8 * 4 + 1], hi[h8 * 4 + 2], hi[h8 * 4 + 3]);
-        *reinterpret_cast<uint4*>(stage_lo + slot) = make_uint4(lo[h8 * 4], lo[h8 * 4 + 1], lo[h8 * 4 + 2], lo[h8 * 4 + 3]);
-      }
+        uint32_t hi[4], lo[4];
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) dst_u[(tk0 + jj) * kDim] = __uint_as_float(du[jj]);
+        for (int e = 0; e < 4; ++e)
+          split_pair(__uint_as_float(d[h8 * 8 + 2 * e]), __uint_as_float(d[h8 * 8 + 2 * e + 1]), hi[e], lo[e]);
+        const int slot = (((tk0 >> 3) + h8) ^ (lrow & 7)) << 4;
+        *reinterpret_cast<uint4*>(stage_hi + slot) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(stage_lo + slot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      tmem_ld16(taddr + 64 + tk0, d);
+      tmem_wait_ld();
+#pragma unroll
+      for (int jj = 0; jj < 16; ++jj) dst_u[(tk0 + jj) * kDim] = __uint_as_float(d[jj]);
     }
     fence_proxy_async_smem();
   }
@@ -1070,8 +1075,9 @@ walk_umma_kernel(const __grid_constant__ CUtensorMap tm_wh, const __grid_constan
 // ======================================================================================= launchers
 int configure_umma() {
   if (int rc = tensor_map_encoder().init()) return rc;
-  for (const auto prepare : {prepare_umma_kernel<kPlain>, prepare_umma_kernel<kRawInputs>, prepare_umma_kernel<kRepairing>,
-                             prepare_umma_kernel<kRawRepairing>, prepare_umma_kernel<kPackedSequences>})
+  for (const auto prepare : {prepare_umma_kernel<kPlain, 3>, prepare_umma_kernel<kPlain, 4>, prepare_umma_kernel<kRawInputs, 3>,
+                             prepare_umma_kernel<kRawInputs, 4>, prepare_umma_kernel<kPackedSequences, 3>,
+                             prepare_umma_kernel<kPackedSequences, 4>, prepare_umma_kernel<kRepairing, 4>, prepare_umma_kernel<kRawRepairing, 4>})
     if (cudaError_t e = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem)) return int(e);
   return int(cudaFuncSetAttribute(walk_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem));
 }
@@ -1104,13 +1110,19 @@ int launch_prepare_umma(const Inputs& in, const Geometry& geo, const Workspace& 
   const int parallel = geo.parallel > 1 ? geo.parallel : 1;
   const long long grid = (long long)geo.batch * geo.value_heads * parallel * ((geo.segment_chunks() + parallel - 1) / parallel);
   if (!left.flags) {
-    const auto prepare = geo.varlen ? prepare_umma_kernel<kPackedSequences>
-                         : in.mixed ? prepare_umma_kernel<kRawInputs> : prepare_umma_kernel<kPlain>;
-    prepare<<<(unsigned)(geo.varlen ? geo.blocks() : grid), kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, tm_p, in, geo, ws, left);
+    // Three CTAs an SM (80 registers) while all blocks are resident at once, four (64 registers) when they take turns: a block is
+    // faster with more registers, the turns are shorter with more blocks (1024 blocks, whole forward 65.7 and 64.9 us, 4096 blocks
+    // 201.8 and 193.5; 256 blocks, one turn in either form, 39.4 and 40.7).
+    const long long blocks = geo.varlen ? geo.blocks() : grid;
+    const bool turns = blocks > 3LL * kSms;
+    const auto prepare = geo.varlen ? (turns ? prepare_umma_kernel<kPackedSequences, 4> : prepare_umma_kernel<kPackedSequences, 3>)
+                         : in.mixed ? (turns ? prepare_umma_kernel<kRawInputs, 4> : prepare_umma_kernel<kRawInputs, 3>)
+                                    : (turns ? prepare_umma_kernel<kPlain, 4> : prepare_umma_kernel<kPlain, 3>);
+    prepare<<<(unsigned)blocks, kPrepThreads, kPrepSmem, stream>>>(tm_q, tm_k, tm_v, tm_wh, tm_wl, tm_p, in, geo, ws, left);
     return int(cudaGetLastError());
   }
-  const long long resident = 3LL * left.sms;
-  return launch_early(in.mixed ? prepare_umma_kernel<kRawRepairing> : prepare_umma_kernel<kRepairing>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
+  const long long resident = 4LL * left.sms;
+  return launch_early(in.mixed ? prepare_umma_kernel<kRawRepairing, 4> : prepare_umma_kernel<kRepairing, 4>, unsigned(grid < resident ? grid : resident), kPrepThreads, kPrepSmem, true, stream,
                       tm_q, tm_k, tm_v, tm_wh, tm_wl, tm_p, in, geo, ws, left);
 }
 

@@ -75,6 +75,31 @@ def test_single_launch_form_equals_the_two_kernels_bitwise(batch, length, hk, hv
     assert none is None and torch.equal(out_only, want_out)
 
 
+@pytest.mark.parametrize("length,hv", [(64 * 110 + 1, 4), (64 * 89, 5)])
+@pytest.mark.parametrize("raw", [False, True])
+def test_both_occupancies_of_the_prepare_kernel(length, hv, raw, native_library):
+    """444 blocks, one turn of three CTAs an SM, and 445, which four take: the single launch's bits, from prepared tensors and
+    from raw projections (two kernels against the same in three launches)."""
+    from actlizela_b200 import gdn_forward_projections, gdn_prepare_inputs
+    from actlizela_b200.sm100 import Sm100Forward
+    forward = Sm100Forward(native_library)
+    if raw:
+        gen = torch.Generator().manual_seed(length)
+        mixed = torch.randn(1, length, (2 + hv) * 128, generator=gen).to(torch.bfloat16).cuda()
+        a, b = (torch.randn(1, length, hv, generator=gen).to(torch.bfloat16).cuda() for _ in range(2))
+        a_log, dt_bias = torch.zeros(hv, device="cuda"), torch.full((hv,), -8.0, device="cuda")       # slow: two kernels
+        q, k, v, g, beta = (x.unsqueeze(0) for x in gdn_prepare_inputs(mixed[0], a[0], b[0], a_log, dt_bias, 1, hv))
+        out, state = gdn_forward_projections(mixed, a, b, a_log, dt_bias, 1, hv, None)
+    else:
+        w = WORKLOADS["cfg1"].sliced(batch=1, length=length, key_heads=1, value_heads=hv, seed=length)
+        q, k, v, g, beta, _ = [x.cuda() if x is not None else None for x in make_inputs(w)]
+        out, state = forward(q, k, v, g, beta, None, True, configuration="umma")
+    want_out, want_state = forward(q, k, v, g, beta, None, True, configuration="fused")
+    torch.cuda.synchronize()
+    assert _healthy(native_library)
+    assert torch.equal(out, want_out) and torch.equal(state, want_state)
+
+
 def _healthy(native_library):
     status = (ctypes.c_int * 4)()
     return native_library.lib.actlize_la_sm100_device_status(status, 1) == 0 and status[0] == 0
