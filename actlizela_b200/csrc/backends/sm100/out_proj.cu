@@ -19,23 +19,25 @@ constexpr int kTileM = 128, kTileK = 64;
 constexpr int kOperandBytes = kTileM * kTileK * 2;                 // 16 KB per 128-row operand tile
 // Tiles of 128 kRows x kN.  Bound by shared memory, 128 bytes a cycle: a K step of 64 of a 128 x 128 tile is written (32 KB) and
 // read by the tensor core (32 KB) in 512 cycles, of a 128 x 256 tile in 768 (512 of products), of a 256 x 256 tile in 1280
-// (1024 of products; its two accumulators fill tensor memory).  Two CTAs of the smallest share an SM, the others have it alone.
-// M 3000, K 4096, N 2560: 68, 61 and 53 us; M 6000: 121 as 128 x 256, 102; M 8192: 165, 148, 147 (1.16 PFLOP/s).
+// (1024 of products; its two accumulators fill tensor memory), of 256 x 224 in 1184, which fits the turns of some sizes better.  Two
+// CTAs of the smallest share an SM, the others have it alone.  K 4096, N 2560, in this order: M 3000 68, 61, 53 and 49 us; M 6000 as
+// 128 x 256 121, then 102 and 94; M 8192 165, 148, 147 and 137 (1.25 PFLOP/s).
 template <int kN, int kRows> struct GemmLayout {
   static constexpr int kStage = kOperandBytes * kRows + kN * kTileK * 2;
   static constexpr int kStages = kRows == 1 && kN == 256 ? 4 : 3, kPerSm = kN == 128 ? 2 : 1;
+  static constexpr int kAccStride = kN == 224 ? 256 : kN, kColumns = kAccStride * kRows;      // tensor memory
   static constexpr int kThreads = 64 + 128 * kRows;
   static constexpr int kBars = kStages * kStage;
   static constexpr int kBytes = kBars + 128 + 1024;
   static constexpr uint32_t kIdesc = idesc_bf16(kTileM, kN, false, false);
-  static_assert(kN % 64 == 0 && kRows * (kN / 64) * kOperandBytes <= kBars, "the output tile must fit on the stages");
-  static_assert(kPerSm * (kBytes + 1024) <= 227 * 1024 && kPerSm * kRows * kN <= 512, "shared and tensor memory of one SM");
+  static_assert(kN % 32 == 0 && kRows * (kN / 64) * kOperandBytes <= kBars, "the output tile must fit on the stages");
+  static_assert(kPerSm * (kBytes + 1024) <= 227 * 1024 && kPerSm * kColumns <= 512, "shared and tensor memory of one SM");
 };
 
 template <int kN, int kRows>
 __global__ void __launch_bounds__(GemmLayout<kN, kRows>::kThreads, GemmLayout<kN, kRows>::kPerSm)
 out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                     const __grid_constant__ CUtensorMap tm_c, int m, int n, int k) {
+                     const __grid_constant__ CUtensorMap tm_c, __nv_bfloat16* __restrict__ c, int m, int n, int k) {
   using L = GemmLayout<kN, kRows>;
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   uint8_t* sm = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
@@ -60,7 +62,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, kN * kRows);
+    tmem_alloc(tmem_slot, L::kColumns);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -98,7 +100,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         for (int ks = 0; ks < kTileK / 16; ++ks)          // 16 BF16 (32 bytes) along K per instruction
 #pragma unroll
           for (int r = 0; r < kRows; ++r)
-            mma_ss(tmem + r * kN, da + uint64_t(r * (kOperandBytes >> 4) + ks * 2), db + uint64_t(ks * 2), L::kIdesc, (kt | ks) != 0);
+            mma_ss(tmem + r * L::kAccStride, da + uint64_t(r * (kOperandBytes >> 4) + ks * 2), db + uint64_t(ks * 2), L::kIdesc, (kt | ks) != 0);
         mma_commit(empty + s);
       }
       mma_commit(done);
@@ -113,14 +115,14 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const int row = quarter * 32 + lane;
     const bool ok = mbar_wait(done, 0, abort, 62, 0);
     tc_fence_after();
-    const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + part * kN;
+    const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + part * L::kAccStride;
     const bool leader = ((warp - 2) & 3) == 0 && lane == 0;
 #pragma unroll 1
-    for (int box = 0; box < (kN + 63) / 64; ++box) {
-      uint8_t* tile = sm + (part * ((kN + 63) / 64) + box) * kOperandBytes;
+    for (int box = 0; box < kN / 64; ++box) {
+      uint8_t* tile = sm + (part * (kN / 64) + box) * kOperandBytes;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        if (box * 64 + half * 32 < kN && ok) {
+        if (ok) {
           uint32_t d[32];
           tmem_ld32(taddr + box * 64 + half * 32, d);
           tmem_wait_ld();
@@ -142,6 +144,19 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         tma_store_commit();
       }
     }
+    if (kN % 64 && ok) {
+      // 32 columns more: too narrow for a box
+      uint32_t d[32];
+      tmem_ld32(taddr + kN - 32, d);
+      tmem_wait_ld();
+      const int r = m0 + part * kTileM + row, first = n0 + kN - 32;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (r < m && first + q * 8 < n)      // N is a multiple of 8: a 16-byte piece is inside or outside
+          *reinterpret_cast<uint4*>(c + (long long)r * n + first + q * 8) =
+              make_uint4(pack_bf16(__uint_as_float(d[q * 8]), __uint_as_float(d[q * 8 + 1])), pack_bf16(__uint_as_float(d[q * 8 + 2]), __uint_as_float(d[q * 8 + 3])),
+                         pack_bf16(__uint_as_float(d[q * 8 + 4]), __uint_as_float(d[q * 8 + 5])), pack_bf16(__uint_as_float(d[q * 8 + 6]), __uint_as_float(d[q * 8 + 7])));
+    }
     if (leader) tma_store_wait_all();
   }
   if (abort.raised()) {
@@ -149,7 +164,7 @@ out_proj_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, kN * kRows);
+  if (warp == 1) tmem_dealloc(tmem, L::kColumns);
 }
 
 // ------------------------------------------------------------------------------------------- few rows: split over K
@@ -312,7 +327,7 @@ int launch_tiles(TensorMapEncoder& enc, const void* a, const void* w, void* c, i
   if (int rc = enc.bf16_2d(&tm_a, a, uint64_t(k), uint64_t(m), kTileM * kRows)) return rc;
   if (int rc = enc.bf16_2d(&tm_w, w, uint64_t(k), uint64_t(n), kN)) return rc;
   return launch_early(out_proj_umma_kernel<kN, kRows>, dim3((n + kN - 1) / kN, (m + kTileM * kRows - 1) / (kTileM * kRows)), L::kThreads,
-                      L::kBytes, true, stream, tm_a, tm_w, tm_c, m, n, k);
+                      L::kBytes, true, stream, tm_a, tm_w, tm_c, static_cast<__nv_bfloat16*>(c), m, n, k);
 }
 }  // namespace
 
@@ -324,6 +339,7 @@ int configure_out_proj() {
   cudaError_t e = cudaFuncSetAttribute(out_proj_umma_kernel<128, 1>, smem, GemmLayout<128, 1>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<256, 1>, smem, GemmLayout<256, 1>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<256, 2>, smem, GemmLayout<256, 2>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_umma_kernel<224, 2>, smem, GemmLayout<224, 2>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<16>, smem, SkinnyLayout<16>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<32>, smem, SkinnyLayout<32>::kBytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(out_proj_skinny_kernel<64>, smem, SkinnyLayout<64>::kBytes);
@@ -345,12 +361,15 @@ int launch_out_proj(const void* a, const void* w, void* c, int m, int n, int k, 
     if (m <= 64) return launch_skinny<64>(enc, a, w, c, m, n, k, split, stream);
     return launch_skinny<128>(enc, a, w, c, m, n, k, split, stream);
   }
-  // A K step takes an SM 512 cycles for a 128 x 128 tile, 768 for a 128 x 256 and 1280 for a 256 x 256 one (shared memory, see
-  // GemmLayout; measured 0.43 us and 0.69 for the last two): the form whose turns are the shortest in all.
-  const auto turns = [](long long all) { return (all + kSms - 1) / kSms; };
-  const long long columns = (n + 255LL) / 256, small = turns(tiles) * 512;
-  const long long wide = turns(columns * ((m + 127LL) / 128)) * 768, square = turns(columns * ((m + 255LL) / 256)) * 1280;
-  if (square < wide && square < small) return launch_tiles<256, 2>(enc, a, w, c, m, n, k, stream);
+  // A K step takes an SM 512 cycles for a 128 x 128 tile, 768 for a 128 x 256, 1280 for a 256 x 256 and 1184 for a 256 x 224 one
+  // (shared memory, see GemmLayout; measured 0.43 us and 0.69 for the second and third): the form whose turns are the shortest in all.
+  const auto cost = [&](long long width, int rows, int cycles) {
+    const long long all = ((n + width - 1) / width) * ((m + rows - 1LL) / rows);
+    return (all + kSms - 1) / kSms * cycles;
+  };
+  const long long small = cost(128, 128, 512), wide = cost(256, 128, 768), square = cost(256, 256, 1280), narrow = cost(224, 256, 1184);
+  if (square < wide && square < small && square <= narrow) return launch_tiles<256, 2>(enc, a, w, c, m, n, k, stream);
+  if (narrow < wide && narrow < small) return launch_tiles<224, 2>(enc, a, w, c, m, n, k, stream);
   return wide < small ? launch_tiles<256, 1>(enc, a, w, c, m, n, k, stream) : launch_tiles<128, 1>(enc, a, w, c, m, n, k, stream);
 }
 

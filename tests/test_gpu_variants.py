@@ -29,9 +29,10 @@ def test_out_proj_with_few_rows(m, k, n):
     assert torch.equal(got, out_proj_gemm(a, w))                  # the sum over the cluster has one order
 
 
-@pytest.mark.parametrize("m,k,n", [(2900, 72, 2504), (3001, 136, 2504), (5000, 64, 1288), (6000, 1024, 2560)])
+@pytest.mark.parametrize("m,k,n", [(13900, 72, 2504), (14001, 136, 2504), (2900, 72, 2504), (3001, 136, 2448), (5000, 64, 1288), (6000, 1024, 2560)])
 def test_out_proj_square_tiles(m, k, n):
-    """Tiles of 256 x 256: rows that end in either 128-row half, ragged columns, one K step, a K tail, several turns.  An element is one
+    """Tiles of 256 x 256 (the first two) and 256 x 224: rows that end in either 128-row half, columns that end in a
+    box and in the 32 behind the boxes, one K step, a K tail, several turns.  An element is one
     BF16 rounding (2^-8 relative, two neighbours) from the FP32 sum; sums of K products differ by K 2^-24 of their terms."""
     from actlizela_b200 import out_proj_gemm
     gen = torch.Generator().manual_seed(m + k)
