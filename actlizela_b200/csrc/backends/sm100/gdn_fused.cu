@@ -6,9 +6,12 @@
 // The arithmetic is that of prepare_umma_kernel and walk_umma_kernel (gdn_umma.cu), operation for operation and in
 // the same order, so both paths give the same bits; orientation and precision are explained there.
 //
-// Bound: the chunk period, 3.8 us (7.5k cycles) with few CTAs at work, 4.1 to 4.3 us with 128 and more (B1 T8192, 32 value heads
-// on 128 CTAs, 35 steps: 163 us, 228 as prepare + walk; B8 T4096, 128 steps: 554 us, 819).  Of it the state chain takes
-// 5k cycles; the rest is the latency of the preparation, of which two are in flight.
+// Bound: the chunk period, about 3.75 us (7k cycles) with 128 CTAs at work (B1 T8192, 32 value heads, 35 steps: 150 us, 194 as
+// prepare + walk; B8 T4096, 128 steps: 518 us).  A chunk takes 16k warp instructions, 58 % of the issue slots, 5k of the cycles
+// in shared memory (3k wavefronts of the warps, 2k of the tensor core's operands), and three ring stages are in flight for about three
+// periods: load 2k, preparation 9k, W 3k, chain 5k cycles.  The roles compete for the issue slots: instructions taken out of
+// the preparation gain 1.5 times their share, while handing work on earlier (the split in front of W's arrival, W or U in columns of
+// their own, the output through shared memory) only slows the preparation and gained nothing.
 #include "umma_math.cuh"
 
 namespace gdn_sm100 {
@@ -348,7 +351,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       tmem_wait_ld();
       if (h & 1) acc_release(bar, lane);      // (the two warps above the diagonal read nothing)
       const float4* pj = reinterpret_cast<const float4*>(diagonal ? s_pl2 + h * 16 : s_ecol + h * 16);
-const float row = quarter < 2 ? kScale : -bi;
+      const float row = quarter < 2 ? kScale : -bi;
       if (diagonal) {
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
@@ -443,7 +446,9 @@ const float row = quarter < 2 ? kScale : -bi;
   }
   group_sync(id);
   // block products T21 = T22 (-A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
-  // above the diagonal, which holds nothing; at 32 the 16x16 blocks above the diagonals of T11 and T22 are left out
+  // above the diagonal, which holds nothing; at 32 the 16x16 blocks above the diagonals of T11 and T22 are left out (the
+  // products are 2.6k of a chunk's 17k instructions: B1 T8192, 32 heads 165 us with all blocks, signs and unpacked
+  // subtractions in the split, 163 so)
   {
     const int g = lane >> 2, tq = lane & 3;
     const int big = (warp >> 1) & 1, o = big * 32, col16 = (warp & 1) * 8;

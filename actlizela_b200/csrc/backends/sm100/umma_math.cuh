@@ -11,7 +11,6 @@ namespace {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kBox = 8192;            // one TMA box: 64 rows x 128 bytes
 constexpr uint32_t kIdescN64 = idesc_bf16(128, 64, false, false);      // A K-major (smem or TMEM), B K-major
-constexpr uint32_t kIdescN64AT = idesc_bf16(128, 64, true, false);     // A MN-major (transposed smem tile)
 constexpr uint32_t kIdescN128BT = idesc_bf16(128, 128, false, true);   // B MN-major
 // K step ks (16 tokens j) of a product whose B operand is a lower-triangular K-major [i][j] tile: only rows i from 16 ks on; what lies
 // above need not even be written

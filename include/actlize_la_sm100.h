@@ -194,8 +194,8 @@ int actlize_la_sm100_rmsnorm_gated(const void* y, const void* z, const void* wei
 
 /* Step after, second half: the output projection C[M,N] = A[M,K] W[N,K]^T with BF16 operands, FP32 accumulation and
  * a BF16 result; A row-major, W in the Linear layout [N][K], C row-major; K and N multiples of 8, all pointers
- * 16-byte aligned.  One tcgen05 kernel (128 x 128 tiles, TMA-fed, accumulator in tensor memory); call
- * actlize_la_sm100_configure once per device first.
+ * 16-byte aligned.  One tcgen05 kernel (tiles of 128 x 128 to 256 x 256, TMA-fed, accumulators in tensor memory;
+ * few rows: K split over a cluster); call actlize_la_sm100_configure once per device first.
  * Replaces out_proj_gemm / out_proj_gemm_cutlass (csrc/output_gate/output_gate.cu, output_gate_cutlass.cu;
  * docs/OUTPUT_GATE.md:17-24). */
 int actlize_la_sm100_out_proj(const void* a, const void* w, void* c, int m, int n, int k, void* stream);
