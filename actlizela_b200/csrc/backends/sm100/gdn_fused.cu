@@ -79,7 +79,7 @@ constexpr int kHasInitial = 1, kHasFinal = 2;
 
 struct Barriers {
   uint64_t kq_full[kRing], kq_free[kRing], g_ready[kRing];
-  uint64_t v_full, w, w_ready, ws, qs, scaled, s, o, ofree;
+  uint64_t v_full, w, w_ready, ws, qs, scaled, o, ofree;
   uint64_t t_ready[2], u[2], d[2], ops[2], opn[2];
   uint64_t item_full[kItems], item_free[kItems];
   uint32_t tmem;
@@ -534,7 +534,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     mbar_init(&bar->ws, 1);
     mbar_init(&bar->qs, 1);
     mbar_init(&bar->scaled, 8);
-    mbar_init(&bar->s, 1);
     mbar_init(&bar->o, 1);
     mbar_init(&bar->ofree, 4);
     for (int i = 0; i < 2; ++i) {
@@ -760,10 +759,9 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
               mma_ts(kAccS, op + h * 32, dk + uint64_t(h * 256), kIdescN128BT, 1);
               mma_ts(kAccS, op + h * 32 + 8, dk + uint64_t(h * 256), kIdescN128BT, 1);
             }
-            if (half) mma_commit(&bar->s);
           }
         }
-        // O^T += N^T P^T behind the state update: the next chunk's split waits for that, not for the output
+        // O^T += N^T P^T behind the state update
         ok &= mbar_wait(&bar->scaled, par);
         tc_fence_after();
         if (elect_one()) {
@@ -867,13 +865,12 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int par = n & 1;
         const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + (n % kRing) * L::kGateStage;
         ok = mbar_wait(&bar->w_ready, par);            // (the gate vector comes with it)
-        if (n > 0) ok = ok && mbar_wait(&bar->s, (n - 1) & 1);
+        // The previous chunk's products, of which P N was issued last: the update has left the new state, and P N has read its N
+        // from the columns of the lo operand.  One wait for both, ahead of the fence that orders the accesses below behind it.
+        if (n > 0) ok = ok && mbar_wait(&bar->o, (n - 1) & 1);
         if (!ok) break;
         tc_fence_after();
         const float gamma = gates[kChunk];
-        // P N of the previous chunk reads its N from the columns of the lo operand.  (Waited for here, not in the loop in front of the
-        // first store to them, where the wait had to be inlined and unrolled: 2.3 of 79 KB of code; B8 T4096 502 us, 490 so, T8192 161 and 159.)
-        if (n > 0) ok = mbar_wait(&bar->o, (n - 1) & 1);
 #pragma unroll 1
         for (int part = 0; part < 4; ++part) {
           uint32_t d[16], hi[8], lo[8];
@@ -949,9 +946,9 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar->scaled);
       }
-      if (ok && n > 0) ok = mbar_wait(&bar->s, (n - 1) & 1);
+      if (ok && n > 0) ok = mbar_wait(&bar->o, (n - 1) & 1);
+      tc_fence_after();                              // also for the next item's first state
       if (ok && (flags & kHasFinal)) {
-        tc_fence_after();
         float* fin = in.final_state + (long long)bh * kDim * kDim + v;
 #pragma unroll 1
         for (int part = 0; part < 4; ++part) {
