@@ -277,9 +277,10 @@ extern "C" int actlize_la_sm100_select(int b, int t, int hk, int hv, int gate_fp
       return row.config | (row.segments << kSegmentShift) | (row.parallel << kParallelShift);
   // no measured row: integer rules (sm100_policy.py::default_configuration / default_parallel are the same).  Parallel
   // sub-segments: as many as fill the 148 SMs with one walk CTA each, at least 8 chunks per sub-segment, at most 8.
-  // Family: the two-kernel form for few (head, chunk) blocks, which its prepare kernel has done in two to three waves
+  // Family: the two-kernel form for few (head, chunk) blocks, which its prepare kernel has done in one to three turns
   // and whose walk is the faster one per chunk; at most three chunks are over before its second launch, and with many
-  // blocks its factors' way through memory costs more than the slower chunk period of the single launch.
+  // blocks its factors' way through memory costs more than the slower chunk period of the single launch (both sides measured:
+  // sm100_policy.py::default_configuration).
   const long long heads = (long long)b * hv, chunks = (t + kChunk - 1) / kChunk;
   long long parallel = kSms / heads;
   if (parallel > chunks / 8) parallel = chunks / 8;
@@ -440,12 +441,14 @@ int run_forward(const Inputs& in, Geometry geo, const Workspace& ws, int config,
 
 // --------------------------------------------------------------- forward on raw projection outputs
 // The raw projections are normalised and activated inside the prepare kernel, which stores the normalised queries and keys for
-// the walk, or inside the single-launch kernel.  Which form is the faster one is estimated, in ns, from what was measured (B1
-// to B4, T100 to T16000, 6 to 74 heads that decay in about five chunks): the single launch takes 4.9 us a chunk step
-// (every head normalises its rows again), the walk 2.08 us a step of its at most eight pieces and the prepare kernel 35 ns a
-// chunk (B1 T1000, 48 heads: 70 us in the two kernels, 90 in the single launch; B1 T16000, 32 heads: 431 and 376).  One
-// chunk is over before a second launch (B1 T50: 23.6 and 20.4); with more heads than half the SMs nothing is cut and
-// preparing them all first is never cheap (128 heads, T1000: 128 and 106).
+// the walk, or inside the single-launch kernel.  Which form is the faster one is estimated, in ns, from a step of the single
+// launch (every head normalises its rows again), a step of the walk's at most eight pieces and the prepare kernel's time a
+// chunk.  One chunk is over before a second launch (B1 T50, 32 heads: 16.4 us in two kernels, 18.5 in one, when they run alone); with more heads
+// than half the SMs nothing is cut and preparing them all first is never cheap (128 heads, T1000: 128 and 106).
+// The constants were fitted when a step and a chunk took 4.9 us and 35 ns.  They take 4.4 us and 25 ns now, but the line these
+// would draw is no better: over 278 calls (B1 to B4, T50 to T16000, 6 to 74 heads, half of them with gates too slow to be cut)
+// the line below costs 2.1 % of the better form's time on average and 14 % at most (B2 T1500, 32 heads, slow gates: 118
+// us in two kernels, 134 in one), the other 2.0 % and 17 % (B2 T4000, 16 heads, gates that decay: 130 and 112).
 int projections_config(const Geometry& geo, int config) {
   const long long heads = (long long)geo.batch * geo.value_heads, chunks = geo.chunks();
   if (2 * heads > kSms || chunks == 1) return kFused;
@@ -504,12 +507,13 @@ extern "C" int actlize_la_sm100_forward_projections(
 namespace {
 long long align256_ll(long long x) { return (x + 255) & ~255LL; }
 long long varlen_table_bytes(int n_seqs) { return align256_ll((n_seqs + 1LL) * (long long)sizeof(int)); }
-// Few (sequence, value head) items of some chunks each: the two kernels.  The walk of the longest item then counts, at 2.1 us a chunk
-// against 3.8 in the single launch, and the prepare kernel (31 ns a block) and the second launch cost less than that saves;
+// Few (sequence, value head) items of some chunks each: the two kernels.  The walk of the longest item then counts, at 2.1 to 2.6 us a chunk
+// against 3.6 in the single launch, and the prepare kernel (25 to 30 ns a block) and the second launch cost less than that saves;
 // with items for more than half the SMs the single launch deals them out.  The longest sequence is not known here, so the line
-// is drawn by the mean: it meets the measured break-even at 33 to 60 items of 2 to 3 chunks, 80 of 5 and 90 of 19 (two
-// sequences of 1200 tokens, 6 heads: 131 us in the single launch, 89; 10 x 600, 6 heads: 84 and 73; 6 x 1200, 16 heads, 96
-// items: 127 and 134).
+// is drawn by the mean: it met the measured break-even at 33 to 60 items of 2 to 3 chunks, 80 of 5 and 90 of 19.  Both forms have
+// become faster by about as much since: over 203 batches (2 to 20 sequences of 60 to 2500 tokens on average, 6 to 48 heads) the
+// line costs 0.3 % of the better form's time on average and 10 % at most, two timer steps (2 sequences of 1200 tokens, 6 heads: 119 us
+// in the single launch, 83 in the two kernels; 14 x 600, 6 heads, on the other side: 90 and 85).
 constexpr int kPackedItems = 90, kPackedTokens = 90 * kChunk;
 static_assert(kPackedItems <= kMostPacked, "every sequence has at least one item");
 bool varlen_in_two_kernels(long long total_tokens, int n_seqs, int hv) {

@@ -135,7 +135,9 @@ __device__ __forceinline__ void prefetch_state(const float* state) {
 // state held in registers and NOT written back; besides the outputs it records delta_t = beta_t (v_t - k_t^T S),
 // from which commit_step_kernel later applies the accepted prefix.  Thread layout as in decode_step_kernel; the
 // arithmetic per token is the decode step's, operation for operation.  Bound: the latency of a token's two reductions and
-// the state's way from HBM.  A token's operands come one token ahead (behind the barriers their latency was most of a
+// the state's way from HBM, times the CTAs an SM has to take one behind the other: 118 registers a thread let two be resident, 296
+// in all, each of which lives about 9 us, so that from 4 to 32 requests of 32 heads and 4 tokens the step grows by 0.95 us a
+// request (12.3, 16.4 at 8, 22.6 at 16, 38.9 at 32).  A token's operands come one token ahead (behind the barriers their latency was most of a
 // token's time), k and q are read 16 bytes at a time, the state is on its way to L2 before the launch's turn: 16 requests
 // x 4 tokens with the commit 32.2 -> 26.1 us, 90 x 8 249 -> 188.  (One barrier a token instead of four, with three k/q buffers,
 // was slower from 16 requests on: 26.3 and 193.)

@@ -6,12 +6,14 @@
 // The arithmetic is that of prepare_umma_kernel and walk_umma_kernel (gdn_umma.cu), operation for operation and in
 // the same order, so both paths give the same bits; orientation and precision are explained there.
 //
-// Bound: the chunk period, about 3.75 us (7k cycles) with 128 CTAs at work (B1 T8192, 32 value heads, 35 steps: 150 us, 194 as
-// prepare + walk; B8 T4096, 128 steps: 518 us).  A chunk takes 16k warp instructions, 58 % of the issue slots, 5k of the cycles
-// in shared memory (3k wavefronts of the warps, 2k of the tensor core's operands), and three ring stages are in flight for about three
-// periods: load 2k, preparation 9k, W 3k, chain 5k cycles.  The roles compete for the issue slots: instructions taken out of
+// What a pass takes is chunk periods, 3.6 us (7k cycles) each with 128 CTAs at work (B1 T8192, 32 value heads, 35 steps, timed in
+// turn: 194 us as prepare + walk, 159 so).  No unit is full: a chunk takes 16k warp instructions, 58 % of the issue slots, and 5k of the
+// cycles in shared memory (3k wavefronts of the warps, 2k of the tensor core's operands).  Three ring stages are in flight for about three
+// periods: load 2k, preparation 9k, W 3k, chain 5k cycles, and the roles slow each other down: instructions taken out of
 // the preparation gain 1.5 times their share, while handing work on earlier (the split in front of W's arrival, W or U in columns of
 // their own, the output through shared memory) only slows the preparation and gained nothing.
+// (Times in pairs, here and below, were taken in turn when the choice was made, by events around a cold call: the two of a pair compare
+// with each other, not with those of another comment.)
 #include "umma_math.cuh"
 
 namespace gdn_sm100 {
@@ -69,7 +71,7 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory of one SM");
 // Tensor memory (512 columns): the state accumulator, its hi / lo operands, W S (then the N operands of the update: of the
 // 16-token group ks hi at 16 ks, lo at 16 ks + 8), W^T and, once that has been converted, U, the output accumulator, and one
 // accumulator that serves the prepare groups in turn ([Q;K] K^T), guarded by a lock word.  (With W^T in that one as well the lock was
-// taken for 6.4k of a chunk's 7.3k cycles: B1 T8192, 32 heads 173 us, 169 so; 48 heads, T65536 1414 and 1392.)  N for P N
+// taken for 6.4k of a chunk's 7.3k cycles: B1 T8192, 32 heads 175 us, 171 so; 48 heads, T65536 1420 and 1403.)  N for P N
 // takes the columns of the lo operand, which the product W S has read by then.
 constexpr uint32_t kAccS = 0, kOpSH = 128, kOpSL = 192, kAccX = 256, kAccU = 320, kAccO = 384, kAccD = 448;
 constexpr uint32_t kIdescN64BT = idesc_bf16(128, 64, false, true);     // B MN-major, N = 64
@@ -198,7 +200,7 @@ struct ItemCursor {
 // prepared: every CTA records what it saw in `flags`, and the two kernels of gdn_umma.cu, launched behind, repair the heads with
 // a violation.  When some piece does not decay, all heads are left to them (flag words of 2): they follow this launch, and
 // take about as long for one head as for all (B1 T8192, 32 heads of which some decay too slowly for a quarter of the
-// length: 673 us with the others cut here, 407 in the two kernels alone, now 415).
+// length: 673 us with the others cut here, 407 in the two kernels alone, 415 so).
 struct Plan {
   int units, pieces;
   int* flags;      // [batch * value_heads][pieces], written when pieces > 1
@@ -246,7 +248,7 @@ scan_pieces_kernel(const Inputs in, const Geometry geo, const __grid_constant__ 
 }
 
 // Packed sequences are dealt to the CTAs longest first, in turns of alternating direction, so that every CTA gets about the
-// same number of chunks (24 sequences of 1 to 10 chunks, 32 heads: 158 us dealt as they come, now 143).  More than
+// same number of chunks (24 sequences of 1 to 10 chunks, 32 heads: 158 us dealt as they come, 143 so).  More than
 // kMostOrdered are many items a CTA, which even out by themselves, and would make the ranking long.
 __device__ __forceinline__ bool is_ordered(const Geometry& geo, const Plan& plan) {
   return geo.varlen && geo.batch <= kMostOrdered && plan.units > int(gridDim.x);
@@ -1169,9 +1171,9 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cons
   const auto go = in.mixed ? launch<true> : launch<false>;
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
   if (plan.pieces == 1) return 0;
-  // Heads left: their chunks prepared by all SMs (31 ns a chunk), then walked at 2.1 us a chunk instead of 3.8 here, in as many
+  // Heads left: their chunks prepared by all SMs (25 ns a chunk), then walked at 2.1 us a chunk instead of 3.6 here, in as many
   // pieces as here or in eight, which are longer when there are more here: gates too slow for the one are often fast enough
-  // for the other (B1, 8 heads, T32768, mean gate -0.02: 1279 us walked uncut, now 347).  Two launches that leave at
+  // for the other (B1, 8 heads, T32768, mean gate -0.02: 1279 us walked uncut, 347 so).  Two launches that leave at
   // once otherwise.
   Geometry again = geo;
   again.parallel = plan.pieces < kWalkPieces ? plan.pieces : kWalkPieces;

@@ -76,10 +76,17 @@ def default_segments(batch, length, value_heads):
 
 def default_configuration(batch, length, value_heads):
     """Kernel family for a shape without a measured row.  Few (head, chunk) blocks: the two-kernel form, whose prepare
-    kernel takes them all at once (444 fit on the device) and whose walk then needs 4.4k cycles a chunk; the single-launch
-    form has a period of 7.1k but no second launch, no factors through memory and no prepare time that grows with the blocks.
-    The two meet near 1280 blocks (16, 32, 48 heads: at 4700, 2800, 1750 tokens), up to three chunks the
-    second launch is all that counts, and from 64 heads on prepare is never short.  The native selector computes the same."""
+    kernel takes them in one to three turns (592 blocks at a time) and whose walk has the shorter step (2.1 to 2.6 us a chunk
+    against 3.6); the single-launch form has no second launch, no factors through memory and no prepare time that grows with
+    the blocks.  Up to three chunks the second launch is all that counts, and from 64 heads on prepare is never short.
+
+    The line at 1280 blocks was drawn when the single launch took 4.2 us a chunk (the two met at 4700, 2800 and 1750 tokens
+    with 16, 32 and 48 heads).  Both are faster now; with gates that decay they meet at 3800, 2200 and 1700 (16 heads, T4000:
+    75 us in two kernels, 73 in one; 32 heads, T2048: 69 and 71, T2560: 83 and 77), and with fewer heads at about 120 chunks
+    (6 heads, T6000: 63 and 71, T8192: 79 and 71).  In between the rule takes the slower form: of 153 shapes with such gates
+    16 are more than 5 % above the better form, the worst 6 heads, T12000 (101 and 75 us).  With gates that decay too slowly to
+    cut a head the single launch leaves all of them to the two kernels, 8 to 20 us later than these alone (32 heads, T2560: 142
+    and 134 us).  The native selector computes the same."""
     heads, chunks = batch * value_heads, (length + 63) // 64
     return "umma" if heads < 64 and chunks > 3 and heads * chunks < 1280 else "fused"
 
