@@ -731,7 +731,7 @@ def main():
     # headline shape for the single-launch form and of a smaller case for the two-kernel family, per (chunk, value head)
     # block and scaled by the blocks of one launch
     blocks = shard.batch * shard.value_heads * ((shard.length + 63) // 64)
-    traffic = 45.8e3 * blocks if single else {"walk": 109.1e3, "prepare": 50.6e3}[top] * blocks if config_name == "umma" else None
+    traffic = 45.5e3 * blocks if single else {"walk": 107.5e3, "prepare": 51.0e3}[top] * blocks if config_name == "umma" else None
     whole_ms = max(alg_bytes / (hbm_peak * 1e9), alg_flops / (tensor_peak * 1e12)) * 1e3
     line = dict(
         metric=METRIC, value=workload.tokens * world / (ms_step * 1e-3), unit=UNIT, n_gpus=world,
