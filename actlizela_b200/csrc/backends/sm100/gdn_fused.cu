@@ -33,9 +33,10 @@ __device__ int g_fused_plan_counts[2];
 //    12-15  W operand (W^T accumulator -> hi/lo tiles) and output
 //    16-23, 24-31  two prepare groups: even and odd chunks of the CTA's stream.  The phases of a chunk's preparation
 //           are serial and latency bound (about two chunk periods long), so two chunks are in preparation at a time.
-// All roles share one instruction cache of some tens of KB: with every loop unrolled (134 KB of code) a chunk took
-// twice as long, bound by instruction fetches from the cache that the SMs of a GPC share.  Loops are therefore rolled
-// unless a loop's registers need otherwise, and waits call one polling routine.
+// All roles share one instruction cache of 32 KB (straight-line code of 30 KB runs at one cycle an instruction, of 36 KB at 2.4): with every
+// loop unrolled (134 KB of code) a chunk took twice as long, and now that some 40 KB pass through it in a chunk, the SMs that happen to miss
+// most, 250 lines a chunk instead of 120, take 15 % longer than the others and end the launch.  Loops are therefore rolled
+// unless a loop's registers or its latency in the chain need otherwise, and waits call one polling routine.
 constexpr int kThreads = 1024, kPrepThreads = 256;
 constexpr int kIssueWarp = 0, kPlanWarp = 1, kGateWarp = 3, kChainWarp = 4, kOutWarp = 12, kPrepWarp = 16;
 constexpr int kRing = 3;      // Q/K tiles, P tiles, gate vectors: one chunk in the chain, two in preparation
@@ -106,28 +107,26 @@ __device__ __forceinline__ uint8_t* shared_base() {
   extern __shared__ __align__(1024) uint8_t raw_smem[];
   return raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);      // (no integer round trip: stays in the shared space)
 }
-// Bounded waits as in umma.cuh, with a polling routine that takes two arguments and loads nothing: a wait is in nearly
-// fifty places of this kernel.  The record names the warp (100 + warp).
+// Bounded waits as in umma.cuh, with a polling routine that takes two arguments and loads nothing, and without an answer: a wait is in
+// more than forty places of this kernel, whose roles together pass some 40 KB of code a chunk through an instruction cache of 32 KB.
+// Waits that each role tested and joined across its warp were 2 KB of that and 2.5 of 70 million instructions (B1 T8192, 32 heads; with
+// waits that others already vouch for left out: 148.5 us with them, 142.2 so; B4 T3000 178 and 171).  The record names the warp (100 + warp).
 constexpr uint32_t kPolls = 1u << 20;
-__device__ __noinline__ bool fused_wait_poll(uint32_t bar_addr, uint32_t parity) {
+__device__ __noinline__ void fused_wait_poll(uint32_t bar_addr, uint32_t parity) {
   const AbortFlag abort{&reinterpret_cast<Barriers*>(shared_base() + Smem::kBars)->abort};
 #pragma unroll 1
   for (uint32_t spin = 0; spin < kPolls; ++spin) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(bar_addr), "r"(parity) : "memory");
-    if (done) return true;
-    if ((spin & 255u) == 255u && abort.raised()) return false;
+    if (done) return;
+    if ((spin & 255u) == 255u && abort.raised()) return;
   }
   abort.raise(1, 100 + (threadIdx.x >> 5), int(bar_addr));
-  return false;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  return fused_wait_poll(smem_u32(bar), parity);
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
+  if (!mbar_try_wait(bar, parity)) fused_wait_poll(smem_u32(bar), parity);
 }
-// wait with one answer for the whole warp
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 
 // ACC_D's lock: taken by the thread that issues into it, given back by the last of the six warps that read it.  Inlined: as a
 // called routine it costs 3 to 9 % (B1 T8192, 32 heads: 181 us, 165 so; B8 T4096: 551, 534).
@@ -180,11 +179,16 @@ __device__ __forceinline__ void scaled_row(const float4 (&x)[4], const float* co
   }
 }
 
+// Whether no role has given up, one answer for the warp.  Asked once an item and once a chunk: a wait that gave up, or that returned
+// because another had, leaves its role to run on through the chunk on what is there.
+__device__ __forceinline__ bool healthy(Barriers* bar) { return __all_sync(0xffffffffu, !AbortFlag{&bar->abort}.raised()); }
+
 // One read of a work item by a warp; `ring` counts items.
 struct ItemCursor {
   int ring = 0;
   __device__ __forceinline__ const int* open(uint8_t* sm, Barriers* bar, bool& ok) {
-    ok = warp_wait(&bar->item_full[ring % kItems], (ring / kItems) & 1);
+    mbar_wait(&bar->item_full[ring % kItems], (ring / kItems) & 1);
+    ok = healthy(bar);
     return reinterpret_cast<const int*>(sm + Smem::kItem) + (ring % kItems) * 16;
   }
   __device__ __forceinline__ void close(Barriers* bar, int lane) {
@@ -292,16 +296,14 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + s * L::kGateStage;
   const float *s_pl2 = gates + L::kPl2, *s_beta = gates + L::kBeta, *s_coefw = gates + L::kCoefW, *s_ecol = gates + L::kECol;
 
-  bool ok = warp_wait(&bar->kq_full[s], (n / kRing) & 1) && !AbortFlag{&bar->abort}.raised();
+  if (kRaw || warp == 7) mbar_wait(&bar->kq_full[s], (n / kRing) & 1);
   if (kRaw) {
-    if (ok) {
 #pragma unroll 1
-      for (int pass = 0; pass < 4; ++pass) normalise_rows(kq, pass, t);
-      fence_proxy_async_smem();
-    }
+    for (int pass = 0; pass < 4; ++pass) normalise_rows(kq, pass, t);
+    fence_proxy_async_smem();
     group_sync(id);
   }
-  if (warp == 7 && ok) {
+  if (warp == 7) {
     const uint64_t a = smem_desc(smem_u32(kq) + L::kQ0, 16, 1024), x = smem_desc(smem_u32(kq) + L::kK0, 16, 1024);
     if (elect_one()) {
       acc_lock(bar);
@@ -316,12 +318,15 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
     }
   }
   __syncwarp();
-  ok = warp_wait(&bar->g_ready[s], (n / kRing) & 1) && ok;
-  ok = group_all(id, ok);
-  if (!ok) return false;
+  if (warp == 0) {
+    mbar_wait(&bar->g_ready[s], (n / kRing) & 1);
+    // A takes the place of the T_u pair of this group's previous chunk, which U was formed from as that chunk began
+    if (n >= 2) mbar_wait(&bar->u[group], ((n >> 1) - 1) & 1);
+  }
+  if (!group_all(id, !AbortFlag{&bar->abort}.raised())) return false;
 
   // ---- masks and decays on [Q;K] K^T
-  ok = warp_wait(&bar->d[group], (n >> 1) & 1);
+  mbar_wait(&bar->d[group], (n >> 1) & 1);
   tc_fence_after();
   const int quarter = warp & 3, half = warp >> 2, i = (quarter & 1) * 32 + lane;
   const uint32_t taddr = (uint32_t(quarter * 32) << 16) + kAccD;
@@ -334,10 +339,8 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   // special-function unit eight cycles per warp).
   const bool diagonal = half == (quarter & 1), below = half < (quarter & 1);      // else above: nothing there
   const float pi = s_pl2[i], bi = s_beta[i];
-  // A takes the place of the T_u pair of this group's previous chunk, which U was formed from as that chunk began
-  if (quarter >= 2 && n >= 2) ok = warp_wait(&bar->u[group], ((n >> 1) - 1) & 1) && ok;
   float* arow = sAT + i * L::kLd;
-  if (ok && (diagonal || below)) {
+  if (diagonal || below) {
     uint8_t* prow = tile_p + i * 128;
     const float f = below ? fast_exp2(pi - s_pl2[31]) * (quarter < 2 ? kScale : -bi) : 0.f;
 #pragma unroll 1
@@ -412,7 +415,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   // overwrite the block only after all of them have read it
   // (the two warps that wrote the diagonal 32x32 blocks of A solve the two 16x16 blocks in theirs)
   __syncwarp();
-  if (ok && quarter >= 2 && diagonal) {
+  if (quarter >= 2 && diagonal) {
     const int col = lane & 15;
     const int o = (quarter & 1) * 32 + (lane & 16);
     float* a0 = sAT + o * L::kLd + o;
@@ -456,7 +459,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       const float* right = (step ? x16 : sAT + o * L::kLd + o + col16) + tq * L::kLd + g;
       float* out = (step ? sAT + (o + 16) * L::kLd + o + col16 : x16) + g * L::kLd + 2 * tq;
       float c[4];
-      if (ok && warp < 4) {
+      if (warp < 4) {
         tile_row_tf32x3<1>(c, left, right, L::kLd, 1);
         *reinterpret_cast<float2*>(out) = make_float2(c[0], c[1]);
         *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(c[2], c[3]);
@@ -471,16 +474,14 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
       const float* right = sAT + step * 32 + col32 + tq * L::kLd + g;
       float* out = (step ? sAT + (32 + row16) * L::kLd + col32 : sAT + row16 * L::kLd + 32 + col32) + g * L::kLd + 2 * tq;
       float c[4];
-      if (ok) {
-        tile_row_tf32x3<2>(c, left, right, L::kLd, step ? (row16 ? 3 : 1) : (col32 < 16 ? 3 : 2));
-        *reinterpret_cast<float2*>(out) = make_float2(c[0], c[1]);
-        *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(c[2], c[3]);
-      }
+      tile_row_tf32x3<2>(c, left, right, L::kLd, step ? (row16 ? 3 : 1) : (col32 < 16 ? 3 : 2));
+      *reinterpret_cast<float2*>(out) = make_float2(c[0], c[1]);
+      *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(c[2], c[3]);
       if (step == 0) group_sync(id);
     }
   }
   // T_w has one place: free once the previous chunk's W^T has been formed from it
-  if (n >= 1) ok = warp_wait(&bar->w, (n - 1) & 1) && ok;
+  if (n >= 1 && warp == 0) mbar_wait(&bar->w, (n - 1) & 1);
   group_sync(id);
   // ---- T diag(beta exp p) and T diag(beta) as BF16 hi/lo K-major tiles; thread -> row, 16 columns
   {
@@ -575,8 +576,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // The V tile of a chunk is asked for one step behind its Q and K tiles: its single buffer is given back at the start
     // of the previous chunk's chain step, ring stages at the end of one.
     int v_n = -1, v_row = 0, v_t0 = 0, v_b = 0, v_hv = 0;
-    auto load_v = [&]() -> bool {
-      if (v_n >= 1 && !mbar_wait(&bar->u[(v_n - 1) & 1], ((v_n - 1) >> 1) & 1)) return false;
+    auto load_v = [&]() {
+      if (v_n >= 1) mbar_wait(&bar->u[(v_n - 1) & 1], ((v_n - 1) >> 1) & 1);
       uint8_t* sv = sm + L::kV;
       mbar_arrive_expect_tx(&bar->v_full, 2 * kBox);
       if (kRaw) {
@@ -586,7 +587,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tma_load_4d(sv, &tm_v, &bar->v_full, 0, v_hv, v_t0, v_b);
         tma_load_4d(sv + kBox, &tm_v, &bar->v_full, 64, v_hv, v_t0, v_b);
       }
-      return true;
     };
     const bool split = plan.pieces > 1, ordered = is_ordered(geo, plan);
 #pragma unroll 1
@@ -633,8 +633,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
       }
       const int at = ring % kItems;
-      if (ring >= kItems) ok = warp_wait(&bar->item_free[at], ((ring / kItems) - 1) & 1);
-      if (!ok) break;
+      if (ring >= kItems) mbar_wait(&bar->item_free[at], ((ring / kItems) - 1) & 1);
+      if (!healthy(bar)) break;
       const int hk = hv / geo.group();
       if (lane == 0) {
         int* item = reinterpret_cast<int*>(sm + L::kItem) + at * 16;
@@ -650,9 +650,9 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         mbar_arrive(&bar->item_full[at]);
         if (end && v_n >= 0) load_v();
 #pragma unroll 1
-        for (int c = 0; c < chunks; ++c, ++n) {
+        for (int c = 0; c < chunks && !abort.raised(); ++c, ++n) {
           const int s = n % kRing, t0 = t_first + c * kChunk;
-          if (n >= kRing && !mbar_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1)) break;
+          if (n >= kRing) mbar_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1);
           uint8_t* kq = sm + L::kKQ + s * L::kKQStage;
           mbar_arrive_expect_tx(&bar->kq_full[s], 4 * kBox);
           if (kRaw) {
@@ -669,7 +669,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             tma_load_4d(kq + L::kK0, &tm_k, &bar->kq_full[s], 0, hk, t0, b);
             tma_load_4d(kq + L::kK1, &tm_k, &bar->kq_full[s], 64, hk, t0, b);
           }
-          if (n >= 1 && !load_v()) break;
+          if (n >= 1) load_v();
           v_row = b * geo.sequence + t0;
           v_t0 = t0;
           v_b = b;
@@ -679,7 +679,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       __syncwarp();
       n = __shfl_sync(0xffffffffu, n, 0);
-      ok = __all_sync(0xffffffffu, !abort.raised());
+      ok = healthy(bar);
       ++ring;
       if (end) break;
     }
@@ -698,13 +698,12 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       cursor.close(bar, lane);
       if (chunks < 0) break;
 #pragma unroll 1
-      for (int c = 0; c < chunks && ok; ++c, ++n) {
+      for (int c = 0; c < chunks && healthy(bar); ++c, ++n) {
         const int s = n % kRing, par = n & 1;
         const uint32_t kq = base + L::kKQ + s * L::kKQStage;
         // U^T = V^T (T diag(beta))^T where W^T was, while the chain warps split the state
-        ok = mbar_wait(&bar->t_ready[par], (n >> 1) & 1);
-        ok &= mbar_wait(&bar->v_full, par);
-        ok &= mbar_wait(&bar->w_ready, par);
+        mbar_wait(&bar->v_full, par);
+        mbar_wait(&bar->w_ready, par);
         tc_fence_after();
         const uint64_t dU = smem_desc(base + L::kAT + par * L::kATBytes, 16, 1024);
         if (elect_one()) {
@@ -720,7 +719,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // first, {2,3,6,7} second
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
-          ok &= mbar_wait(&bar->ops[half], par);
+          mbar_wait(&bar->ops[half], par);
           tc_fence_after();
           const uint64_t dw = dW + uint64_t(half * 256);
           const uint32_t op = half * 16;
@@ -735,7 +734,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (half) mma_commit(&bar->ws);
           }
         }
-        if (n > 0) ok &= mbar_wait(&bar->ofree, (n - 1) & 1);
+        if (n > 0) mbar_wait(&bar->ofree, (n - 1) & 1);
         tc_fence_after();
         const uint64_t qd = smem_desc(kq + L::kQ0, 16, 1024);
         if (elect_one()) {
@@ -751,7 +750,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint64_t kd = smem_desc(kq + L::kK0, L::kK1 - L::kK0, 1024), pd = smem_desc(base + L::kP + s * kBox, 16, 1024);
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
-          ok &= mbar_wait(&bar->opn[half], par);
+          mbar_wait(&bar->opn[half], par);
           tc_fence_after();
           const uint64_t dk = kd + uint64_t(half * 128);
           const uint32_t op = kAccX + half * 16;
@@ -764,7 +763,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
         }
         // O^T += N^T P^T behind the state update
-        ok &= mbar_wait(&bar->scaled, par);
+        mbar_wait(&bar->scaled, par);
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -773,7 +772,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           mma_commit(&bar->kq_free[s]);
         }
       }
-      ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp == kGateWarp) {
     // ------------------------------------------------------------------ gates
@@ -787,7 +785,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       cursor.close(bar, lane);
       if (chunks < 0) break;
 #pragma unroll 1
-      for (int c = 0; c < chunks && ok; ++c, ++n) {
+      for (int c = 0; c < chunks && healthy(bar); ++c, ++n) {
         const int s = n % kRing;
         float* gates = reinterpret_cast<float*>(sm + L::kGates) + s * L::kGateStage;
         // tokens lane and lane + 32: two scans, the second half then adds the first half's total
@@ -817,8 +815,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const float last = __shfl_sync(0xffffffffu, valid > 32 ? p[1] : p[0], (valid - 1) & 31);
         const float p31 = __shfl_sync(0xffffffffu, p[0], 31);
         // the stage is free once the chain has left the chunk that used it
-        if (n >= kRing) ok = warp_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1);
-        if (!ok) break;
+        if (n >= kRing) mbar_wait(&bar->kq_free[s], ((n / kRing) - 1) & 1);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int t = h * 32 + lane;
@@ -834,7 +831,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar->g_ready[s]);
       }
-      ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp >= kChainWarp && warp < kOutWarp) {
     // ------------------------------------------------------------------ state chain
@@ -863,14 +859,13 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tmem_wait_st();
       }
 #pragma unroll 1
-      for (int c = 0; c < chunks && ok; ++c, ++n) {
+      for (int c = 0; c < chunks && healthy(bar); ++c, ++n) {
         const int par = n & 1;
         const float* gates = reinterpret_cast<const float*>(sm + L::kGates) + (n % kRing) * L::kGateStage;
-        ok = mbar_wait(&bar->w_ready, par);            // (the gate vector comes with it)
+        mbar_wait(&bar->w_ready, par);                 // (the gate vector comes with it)
         // The previous chunk's products, of which P N was issued last: the update has left the new state, and P N has read its N
         // from the columns of the lo operand.  One wait for both, ahead of the fence that orders the accesses below behind it.
-        if (n > 0) ok = ok && mbar_wait(&bar->o, (n - 1) & 1);
-        if (!ok) break;
+        if (n > 0) mbar_wait(&bar->o, (n - 1) & 1);
         tc_fence_after();
         const float gamma = gates[kChunk];
 #pragma unroll 1
@@ -898,8 +893,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (lane == 0) mbar_arrive(&bar->ops[part >> 1]);
           }
         }
-        ok = ok && mbar_wait(&bar->ws, par);            // (U was issued in front of W S)
-        if (!ok) break;
+        mbar_wait(&bar->ws, par);                       // (U was issued in front of W S)
         tc_fence_after();
 #pragma unroll 1
         for (int part = 0; part < 2; ++part) {
@@ -932,7 +926,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // S Q^T, which was issued behind W S, becomes the state part of the output while the update runs: token i times
         // exp(p_i) / sqrt(128).  (Scaling the Q tile instead, by a warp of its own, took 1440 of 17.6k instructions a chunk and rounded
         // the scaled query: B1 T8192, 32 heads 171 us, 165 so; B8 T4096 540 and 519; output error against FP64 at slow gates 3.06e-3 and 2.72e-3.)
-        ok = mbar_wait(&bar->qs, par);
+        mbar_wait(&bar->qs, par);
         tc_fence_after();
 #pragma unroll 1
         for (int part = 0; part < 2; ++part) {
@@ -948,9 +942,9 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar->scaled);
       }
-      if (ok && n > 0) ok = mbar_wait(&bar->o, (n - 1) & 1);
+      if (n > 0) mbar_wait(&bar->o, (n - 1) & 1);
       tc_fence_after();                              // also for the next item's first state
-      if (ok && (flags & kHasFinal)) {
+      if (flags & kHasFinal) {
         float* fin = in.final_state + (long long)bh * kDim * kDim + v;
 #pragma unroll 1
         for (int part = 0; part < 4; ++part) {
@@ -962,7 +956,6 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           for (int j = 0; j < 16; ++j) fin[(k0 + j) * kDim] = __uint_as_float(d[j]);
         }
       }
-      ok = __all_sync(0xffffffffu, ok);
     }
   } else if (warp >= kOutWarp && warp < kPrepWarp) {
     // ------------------------------------------------------------------ W operand and output
@@ -977,8 +970,9 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     int o_rows = 0;                             // rows of it to be stored
     int chunks = 0, c = 0, b = 0, hv = 0, t_first = 0, t_end = 0, unstored = 0;
 #pragma unroll 1
-    for (bool ok = true; ok;) {
+    while (healthy(bar)) {
       if (c == chunks) {
+        bool ok;
         const int* item = cursor.open(sm, bar, ok);
         if (!ok) break;
         c = 0;
@@ -993,12 +987,12 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       const bool end = chunks < 0;
       if (!end) {
-        ok = warp_wait(&bar->t_ready[n & 1], (n >> 1) & 1);                // (what it announces is passed on with W)
         if (warp == kOutWarp) {
+          mbar_wait(&bar->t_ready[n & 1], (n >> 1) & 1);                     // (what it announces is passed on with W)
           // W^T = K^T (T diag(beta exp p))^T; issued here so that the prepare group does not wait for the accumulator
           const uint64_t a = smem_desc(smem_u32(sm) + L::kKQ + (n % kRing) * L::kKQStage + L::kK0, L::kK1 - L::kK0, 1024);
           const uint64_t x = smem_desc(smem_u32(sm) + L::kTw, 16, 1024);
-          if (n > 0) ok = warp_wait(&bar->opn[1], (n - 1) & 1) && ok;      // U of the previous chunk has been read
+          if (n > 0) mbar_wait(&bar->opn[1], (n - 1) & 1);                 // U of the previous chunk has been read
           if (elect_one()) {
             tc_fence_after();
 #pragma unroll 1
@@ -1011,10 +1005,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
           __syncwarp();
         }
-        ok = warp_wait(&bar->w, n & 1) && ok;
-        if (n > 0) ok = warp_wait(&bar->ws, (n - 1) & 1) && ok;            // W of the previous chunk has been read
+        mbar_wait(&bar->w, n & 1);
         tc_fence_after();
-        if (!ok) break;
         const int key = quarter * 32 + lane;
         uint8_t* wt = sm + L::kW + key * 128;
 #pragma unroll 1
@@ -1042,8 +1034,7 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // The output tile leaves straight from registers: neighbouring lanes (value columns) swap halves of a token pair,
         // so that an even lane holds two columns of the first token and an odd lane of the second, and a warp writes
         // two 64-byte pieces.  (No staging tile: its 16 KB are what lets T_w have a place of its own.)
-        ok = warp_wait(&bar->o, (n - 1) & 1);
-        if (!ok) break;
+        mbar_wait(&bar->o, (n - 1) & 1);
         tc_fence_after();
         __nv_bfloat16* at = o_at;
         int rows = o_rows - (lane & 1);
