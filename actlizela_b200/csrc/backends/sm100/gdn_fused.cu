@@ -453,19 +453,22 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
     const int big = (warp >> 1) & 1, o = big * 32, col16 = (warp & 1) * 8;
     float* x16 = sAT + (big * 16) * L::kLd + 32 + col16;
     const uint32_t frag = smem_u32(sAT) + fragment_row(lane, L::kLd) * 4;
+    // 16 wide: a warp's second tile reads its own first, so there is no barrier of the group in between (B1 T8192, 32 heads: 140.8 us
+    // with one, 137.6 so)
+    if (warp < 4) {
 #pragma unroll 1
-    for (int step = 0; step < 2; ++step) {
-      const uint32_t left = frag + ((o + 16) * L::kLd + o + step * 16) * 4;
-      const float* right = (step ? x16 : sAT + o * L::kLd + o + col16) + tq * L::kLd + g;
-      float* out = (step ? sAT + (o + 16) * L::kLd + o + col16 : x16) + g * L::kLd + 2 * tq;
-      float c[4];
-      if (warp < 4) {
+      for (int step = 0; step < 2; ++step) {
+        const uint32_t left = frag + ((o + 16) * L::kLd + o + step * 16) * 4;
+        const float* right = (step ? x16 : sAT + o * L::kLd + o + col16) + tq * L::kLd + g;
+        float* out = (step ? sAT + (o + 16) * L::kLd + o + col16 : x16) + g * L::kLd + 2 * tq;
+        float c[4];
         tile_row_tf32x3<1>(c, left, right, L::kLd, 1);
         *reinterpret_cast<float2*>(out) = make_float2(c[0], c[1]);
         *reinterpret_cast<float2*>(out + 8 * L::kLd) = make_float2(c[2], c[3]);
+        __syncwarp();
       }
-      group_sync(id);
     }
+    group_sync(id);
     // 32 wide: eight tiles, one per warp
     const int row16 = (warp & 1) * 16, col32 = (warp >> 1) * 8;
 #pragma unroll 1
@@ -928,14 +931,12 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // the scaled query: B1 T8192, 32 heads 171 us, 165 so; B8 T4096 540 and 519; output error against FP64 at slow gates 3.06e-3 and 2.72e-3.)
         mbar_wait(&bar->qs, par);
         tc_fence_after();
-#pragma unroll 1
-        for (int part = 0; part < 2; ++part) {
-          uint32_t o[16];
-          const int i0 = half * 32 + part * 16;
-          tmem_ld16(taddr + kAccO + i0, o);
+        {
+          uint32_t o[32];
+          tmem_ld32(taddr + kAccO + half * 32, o);
           tmem_wait_ld();
-          scale_columns(o, gates + kGateQueryScale + i0);
-          tmem_st16(taddr + kAccO + i0, o);
+          scale_columns(o, gates + kGateQueryScale + half * 32);
+          tmem_st32(taddr + kAccO + half * 32, o);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -1033,7 +1034,8 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       if (n > 0) {
         // The output tile leaves straight from registers: neighbouring lanes (value columns) swap halves of a token pair,
         // so that an even lane holds two columns of the first token and an odd lane of the second, and a warp writes
-        // two 64-byte pieces.  (No staging tile: its 16 KB are what lets T_w have a place of its own.)
+        // two 64-byte pieces.  (No staging tile: its 16 KB are what lets T_w have a place of its own.)  Rows that are not stored are left out
+        // by the predicate alone: with a branch around the shuffles, whose lanes the compiler then has to gather, the kernel's code was 2 KB longer.
         mbar_wait(&bar->o, (n - 1) & 1);
         tc_fence_after();
         __nv_bfloat16* at = o_at;
@@ -1048,15 +1050,13 @@ forward_umma_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar->ofree);
           }
-          if (o_rows > 0) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const uint32_t x = pack_bf16(__uint_as_float(d[2 * j]), __uint_as_float(d[2 * j + 1]));
-              const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1);
-              const uint32_t pair = __byte_perm(x, y, (lane & 1) ? 0x3276 : 0x5410);
-              if (2 * j < rows) *reinterpret_cast<uint32_t*>(at) = pair;
-              at += 2 * row_stride;
-            }
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t x = pack_bf16(__uint_as_float(d[2 * j]), __uint_as_float(d[2 * j + 1]));
+            const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1);
+            const uint32_t pair = __byte_perm(x, y, (lane & 1) ? 0x3276 : 0x5410);
+            if (2 * j < rows) *reinterpret_cast<uint32_t*>(at) = pair;
+            at += 2 * row_stride;
           }
           rows -= 16;
         }

@@ -136,10 +136,11 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uin
   lo = pack_bf16(l0, l1);
 }
 
-// 16 columns of an accumulator times a factor per column (shared memory, 16-byte aligned)
-__device__ __forceinline__ void scale_columns(uint32_t (&x)[16], const float* factor) {
+// kN columns of an accumulator times a factor per column (shared memory, 16-byte aligned)
+template <int kN>
+__device__ __forceinline__ void scale_columns(uint32_t (&x)[kN], const float* factor) {
 #pragma unroll
-  for (int q4 = 0; q4 < 4; ++q4) {
+  for (int q4 = 0; q4 < kN / 4; ++q4) {
     const float4 f = *reinterpret_cast<const float4*>(factor + q4 * 4);
     float a, b;
     mul2(a, b, __uint_as_float(x[q4 * 4]), __uint_as_float(x[q4 * 4 + 1]), f.x, f.y);
