@@ -508,7 +508,7 @@ namespace {
 long long align256_ll(long long x) { return (x + 255) & ~255LL; }
 long long varlen_table_bytes(int n_seqs) { return align256_ll((n_seqs + 1LL) * (long long)sizeof(int)); }
 // Few (sequence, value head) items of some chunks each: the two kernels.  The walk of the longest item then counts, at 2.1 to 2.6 us a chunk
-// against 3.6 in the single launch, and the prepare kernel (25 to 30 ns a block) and the second launch cost less than that saves;
+// against 3.2 in the single launch, and the prepare kernel (25 to 30 ns a block) and the second launch cost less than that saves;
 // with items for more than half the SMs the single launch deals them out.  The longest sequence is not known here, so the line
 // is drawn by the mean: it met the measured break-even at 33 to 60 items of 2 to 3 chunks, 80 of 5 and 90 of 19.  Both forms have
 // become faster by about as much since: over 203 batches (2 to 20 sequences of 60 to 2500 tokens on average, 6 to 48 heads) the

@@ -6,12 +6,16 @@
 // The arithmetic is that of prepare_umma_kernel and walk_umma_kernel (gdn_umma.cu), operation for operation and in
 // the same order, so both paths give the same bits; orientation and precision are explained there.
 //
-// What a pass takes is chunk periods, 3.6 us (7k cycles) each with 128 CTAs at work (B1 T8192, 32 value heads, 35 steps, timed in
-// turn: 194 us as prepare + walk, 159 so).  No unit is full: a chunk takes 16k warp instructions, 58 % of the issue slots, and 5k of the
-// cycles in shared memory (3k wavefronts of the warps, 2k of the tensor core's operands).  Three ring stages are in flight for about three
-// periods: load 2k, preparation 9k, W 3k, chain 5k cycles, and the roles slow each other down: instructions taken out of
-// the preparation gain 1.5 times their share, while handing work on earlier (the split in front of W's arrival, W or U in columns of
-// their own, the output through shared memory) only slows the preparation and gained nothing.
+// What a pass takes is chunk periods, 3.2 us (6.3k cycles) each with 128 CTAs at work (B1 T8192, 32 value heads, 35 steps; it was 3.6 us,
+// 7k cycles).  No unit is full: a chunk takes 14.7k warp instructions, 58 % of the issue slots, and 5k of the
+// cycles in shared memory (3k wavefronts of the warps, 2k of the tensor core's operands).  Two loops of waits take the same time, by time stamps:
+// from one N to the next (W's product 0.7k, its conversion 1.1k, split 1.6k, W S 0.8k, N 1.0k cycles and the waits in between), and three periods of a
+// ring stage (load 2k, preparation 9.3k, W 1.3k, conversion 1.1k, chain 4.4k).  Cutting one of them alone gained nothing and mostly cost something,
+// because the roles then meet elsewhere: the split in front of W's arrival 1.02 to 1.03, W in the accumulator of [Q;K] K^T 1.02 to 1.04, four
+// stages with K and Q loaded a second time for the chain 1.06, K and Q prefetched to L2 1.06 to 1.08, conversions in 32 columns or with the next
+// piece in flight 1.01, W's conversion shared with the chain warps 1.03, products issued from loops 1.04, all unrolled 1.00 to 1.02, the preparation's work
+// spread evenly over the schedulers 1.00.  What gained were instructions and code taken out of all roles alike.  Long launches run at the board's power
+// limit (990 W at 1.79 to 1.93 GHz).
 // (Times in pairs, here and below, were taken in turn when the choice was made, by events around a cold call: the two of a pair compare
 // with each other, not with those of another comment.)
 #include "umma_math.cuh"
@@ -446,7 +450,7 @@ __device__ __forceinline__ bool prepare_chunk(uint8_t* sm, Barriers* bar, int gr
   group_sync(id);
   // block products T21 = T22 (-A21 T11) at block size 16, then 32, two steps each; the scratch is the 32x32 block
   // above the diagonal, which holds nothing; at 32 the 16x16 blocks above the diagonals of T11 and T22 are left out (the
-  // products are 2.6k of a chunk's 17k instructions: B1 T8192, 32 heads 165 us with all blocks, signs and unpacked
+  // products are 2.6k of a chunk's instructions, which were 17k then: B1 T8192, 32 heads 165 us with all blocks, signs and unpacked
   // subtractions in the split, 163 so)
   {
     const int g = lane >> 2, tq = lane & 3;
@@ -1162,7 +1166,7 @@ int launch_forward_fused(const Inputs& in, const Geometry& geo, int* flags, cons
   const auto go = in.mixed ? launch<true> : launch<false>;
   if (int rc = go(in, geo, plan, plan.units < sms ? plan.units : sms, stream)) return rc;
   if (plan.pieces == 1) return 0;
-  // Heads left: their chunks prepared by all SMs (25 ns a chunk), then walked at 2.1 us a chunk instead of 3.6 here, in as many
+  // Heads left: their chunks prepared by all SMs (25 ns a chunk), then walked at 2.1 us a chunk instead of 3.2 here, in as many
   // pieces as here or in eight, which are longer when there are more here: gates too slow for the one are often fast enough
   // for the other (B1, 8 heads, T32768, mean gate -0.02: 1279 us walked uncut, 347 so).  Two launches that leave at
   // once otherwise.

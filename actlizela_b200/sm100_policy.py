@@ -77,7 +77,7 @@ def default_segments(batch, length, value_heads):
 def default_configuration(batch, length, value_heads):
     """Kernel family for a shape without a measured row.  Few (head, chunk) blocks: the two-kernel form, whose prepare
     kernel takes them in one to three turns (592 blocks at a time) and whose walk has the shorter step (2.1 to 2.6 us a chunk
-    against 3.6); the single-launch form has no second launch, no factors through memory and no prepare time that grows with
+    against 3.2); the single-launch form has no second launch, no factors through memory and no prepare time that grows with
     the blocks.  Up to three chunks the second launch is all that counts, and from 64 heads on prepare is never short.
 
     The line at 1280 blocks was drawn when the single launch took 4.2 us a chunk (the two met at 4700, 2800 and 1750 tokens
